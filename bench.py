@@ -688,11 +688,11 @@ def main():
         "batched_vs_plain": round(value / plain["device_pairs_per_s"], 2) if plain else None,
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": traffic, "peak_source": peak_src,
-                     "kernel": "xted_dp_kernel", "bytes_per_cell": BYTES_PER_CELL},
+                     "kernel": "xted_flow_kernel", "bytes_per_cell": BYTES_PER_CELL},
         "cpu_baseline": cpu,
         "cpu_baseline_pair_parallel": cpu_pp,  # the same reference code, 1 thread per pair x all cores
         "serve": serve,
-        "gpu_launches": 3 * args.steps,  # ready-queue init, DP, gather per step
+        "gpu_launches": 2 * args.steps,  # DP, gather per step
         "clocks": clk.summary(),
         "tasks": st["tasks"], "units": st["units"], "grid": st["grid"], "host_plan_ms": round(plan_ms, 2),
         "cuda_graph": bool(st["graph"]),  # the timed steps replayed the step's captured CUDA graph

@@ -297,7 +297,7 @@ int xted_serve_options(xted_ctx *ctx, int32_t prune, int32_t first_round);
  * to the device, then disarms itself.
  *   XTED_FAULT_HOLD_PAIR: level 0 of one computed pair (the batch's pair 0,
  *     or the query's first computed corpus tree) is never published into the
- *     ready queue, so its tables never become ready. A batch then ends when
+ *     launch's data, so its tables never become ready. A batch then ends when
  *     the persistent launch's bounded idle wait (wait_timeout_s) runs out and
  *     returns XTED_ETIMEOUT; a serving launch goes idle and ends, and the
  *     query fails with XTED_ETIMEOUT. The context stays usable. */

@@ -1,0 +1,80 @@
+"""The DP launch at the sizes where its item kinds change (needs a B200):
+chunks of up to 256 and up to 512 columns a warp, column stripes of 512 beyond
+that (a stripe boundary may fall on any node), row runs around the 32 rows that
+a warp looks ahead, stacks deeper than the shared-memory window, and the form
+for chunks with more than 64 columns on a right path or across a stripe
+boundary. Exact against the oracle: distances are whole numbers."""
+import numpy as np
+import pytest
+
+import oracle
+import xted
+from xted import gen, trees
+
+pytestmark = pytest.mark.gpu
+
+
+def _comb(n, seed, leaf_first):
+    """A spine on which every node carries one leaf, before or after the next
+    spine node: right-path keyroots nested to depth n / 2, or one long path."""
+    adj = []
+    for v in range(n):
+        if v % 2 or v + 1 >= n:
+            adj.append([])
+        elif leaf_first:
+            adj.append([c for c in (v + 1, v + 2) if c < n])
+        else:
+            adj.append([])
+    if not leaf_first:  # spine 0 .. d-1, then the leaves from the innermost out
+        d = n // 2 + 1
+        adj = [[] for _ in range(n)]
+        for v in range(d - 1):
+            adj[v].append(v + 1)
+        for k in range(n - d):
+            adj[d - 2 - k].append(d + k)
+    labels = np.random.default_rng(seed).integers(0, 4, n)
+    return trees.from_adjacency([int(x) for x in labels], adj)
+
+
+@pytest.mark.timeout(300)
+@pytest.mark.parametrize("n", [253, 256, 257, 260, 508, 511, 512, 513, 516, 1023, 1025, 1537])
+def test_chunk_widths(n):
+    """Column trees around every width limit, both decompositions."""
+    pairs = []
+    for k, shape in enumerate(("random", "wide", "deep", "caterpillar")):
+        pairs.append((gen.tree(shape, 31 + 2 * k, n + k, "uniform", 5), gen.tree("random", n, 7 * n + k, "uniform", 5)))
+        pairs.append((gen.tree("random", 64 + k, n + k, "uniform", 5), gen.tree(shape, n, 3 * n + k, "uniform", 5)))
+    want = oracle.distance_batch(pairs, nthreads=8)
+    for orient in (xted.ORIENT_RIGHT, xted.ORIENT_LEFT):
+        with xted.Context(orientation=orient) as ctx:
+            assert np.array_equal(ctx.distance_batch(pairs), want)
+
+
+@pytest.mark.timeout(300)
+@pytest.mark.parametrize("m,n", [(1, 700), (2, 513), (32, 600), (33, 257), (35, 1030), (97, 129)])
+def test_long_lists_and_deep_stacks(m, n):
+    """Combs: every second column of the root chunk on its right path, or one
+    export per nested keyroot (lists longer than 64), and row stacks as deep as
+    half the tree; also under general costs."""
+    pairs = [(_comb(m, 1, a), _comb(n, 2, b)) for a in (True, False) for b in (True, False)]
+    pairs += [(_comb(n, 3, a), _comb(m, 4, True)) for a in (True, False)]
+    for orient in (xted.ORIENT_AUTO, xted.ORIENT_RIGHT, xted.ORIENT_LEFT):
+        with xted.Context(orientation=orient) as ctx:
+            assert np.array_equal(ctx.distance_batch(pairs), oracle.distance_batch(pairs, nthreads=8))
+    with xted.Context(costs=(2, 3, 7)) as ctx:  # a rename dearer than delete + insert
+        assert ctx.distance_batch(pairs).tolist() == [oracle.distance(a, b, costs=(2, 3, 7)) for a, b in pairs]
+
+
+@pytest.mark.timeout(300)
+@pytest.mark.parametrize("narrow,run_rows", [(256, 1), (64, 7), (0, 33), (256, 200)])
+def test_many_segments(narrow, run_rows):
+    """Chunks of many small segments (caterpillars, wide trees) and runs of many
+    small tables, at several granularities."""
+    rng = np.random.default_rng(narrow + run_rows)
+    pairs = []
+    for k in range(24):
+        m, n = int(rng.integers(1, 400)), int(rng.integers(1, 400))
+        pairs.append((gen.tree(("caterpillar", "wide", "random")[k % 3], m, k, "uniform", 3),
+                      gen.tree(("wide", "caterpillar", "deep")[k // 3 % 3], n, 50 + k, "uniform", 3)))
+    with xted.Context(narrow_width=narrow, run_rows=run_rows) as ctx:
+        assert np.array_equal(ctx.distance_batch(pairs), oracle.distance_batch(pairs, nthreads=8))

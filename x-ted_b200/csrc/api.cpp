@@ -2,9 +2,9 @@
 //
 // xted_distance / xted_distance_batch replace the reference's
 // standard_ted (X-TED_CPU/TED.cpp:177-190; X-TED_GPU/TED.cu:116-128): the
-// planner (plan.cpp) lays out every keyroot table of every pair as device
-// tasks, one cooperative launch of the persistent DP kernel (kernels.cu)
-// drains them, and a gather kernel reads Dtree[0][0] of each pair
+// planner (prep.cu) lays out every keyroot table of every pair as a list of
+// items, one cooperative launch of the persistent DP kernel (flow.cu) runs
+// them, and a gather kernel reads Dtree[0][0] of each pair
 // (X-TED_CPU/TED.cpp:188). Errors are returned, never printed or exited on
 // (the reference prints CUDA errors and continues, X-TED_GPU/utils/cuda_utils.h:35-41,
 // or exits, X-TED_GPU/help.h:6-14).
@@ -28,9 +28,8 @@
 namespace xted {
 int dp_occupancy(int *blocks_per_sm);
 cudaError_t launch_dp(const XKernelParams &P, int grid, cudaStream_t s);
-cudaError_t launch_rq_init(const XKernelParams &P, cudaStream_t s);
 cudaError_t launch_gather(const XPair *pairs, const int32_t *trivial, const int32_t *dt, int npairs,
-                          int32_t *out, int c_del, int c_ins, cudaStream_t s);
+                          int32_t *out, int c_del, int c_ins, int32_t *error, cudaStream_t s);
 }  // namespace xted
 
 using namespace xted;
@@ -106,15 +105,13 @@ int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npa
     K.c_del = c->opts.cost_del;
     K.c_ins = c->opts.cost_ins;
     K.c_ren = c->opts.cost_ren;
-    rc = ctx_dev_reserve(c, c->dt, (size_t)std::max<int64_t>(c->plan_dt_elems, 1) * sizeof(int32_t));
+    // (a stripe of slack: a row's copies name, without reading, words up to a stripe past its end)
+    rc = ctx_dev_reserve(c, c->dt, (size_t)(c->plan_dt_elems + XTED_SW) * sizeof(int32_t));
     if (rc) return rc;
-    const int64_t stack_rows = c->plan_stack_rows, max_wide = c->plan_max_wide;
-    // per-block scratch: far-row stacks (+ rows of the generic wide path)
-    int64_t per = stack_rows * (XTED_WARPS * XTED_NARROW_MAX);
-    if (max_wide > 0 && max_wide <= XTED_WIDE_REG_MAX) per = std::max<int64_t>(per, stack_rows * max_wide);
-    if (max_wide > XTED_WIDE_REG_MAX) per = std::max<int64_t>(per, xted_wide_big_scratch(max_wide, stack_rows));
-    per = (int64_t)align_up((size_t)per, 64);
-    rc = ctx_dev_reserve(c, c->scratch, (size_t)per * (size_t)c->grid * sizeof(int32_t));
+    // per-warp scratch: the far-row stack's rows outside the shared window
+    const int64_t stack_rows = c->plan_stack_rows;
+    const int64_t per = stack_rows * XTED_SW;
+    rc = ctx_dev_reserve(c, c->scratch, (size_t)per * (size_t)c->grid * XTED_FLOW_WARPS * sizeof(int32_t));
     if (rc) return rc;
     // counters: [1] error, [2..5] error info, then out[npairs]
     rc = ctx_dev_reserve(c, c->counters, (8 + 2 * (size_t)npairs) * sizeof(int32_t));
@@ -124,17 +121,17 @@ int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npa
     int32_t *cnt = (int32_t *)c->counters.p;
     K.dt = (int32_t *)c->dt.p;
     K.scratch = (int32_t *)c->scratch.p;
-    K.scratch_per_cta = per;
+    K.scratch_per_warp = per;
     K.stack_rows = (int32_t)stack_rows;
     K.error = cnt + 1;
     K.error_info = cnt + 2;
     K.timeout_ns = (uint64_t)(c->opts.wait_timeout_s * 1e9);
-    // Optional per-task trace (XTED_TRACE=<file>): timestamps of every task,
+    // Optional per-item trace (XTED_TRACE=<file>): timestamps of every item,
     // written as raw uint64 quadruples after each run.
     const char *tr = std::getenv("XTED_TRACE");
     K.trace = nullptr;
-    if (tr && *tr && K.ntasks > 0) {
-        rc = ctx_dev_reserve(c, c->trace, (size_t)K.ntasks * 4 * sizeof(unsigned long long));
+    if (tr && *tr && K.nitems > 0) {
+        rc = ctx_dev_reserve(c, c->trace, (size_t)K.nitems * 4 * sizeof(unsigned long long));
         if (rc) return rc;
         K.trace = (unsigned long long *)c->trace.p;
     }
@@ -146,8 +143,7 @@ int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npa
 // Runs the prepared plan: counter reset, the persistent DP launch, the
 // gather, and the copy of results + error word to pinned memory. Synchronous.
 // One step of the prepared plan, enqueued on the context's stream: counter
-// reset, the ready queue's level 0, the persistent DP launch, the gather, and
-// the copy of results + error word to pinned memory.
+// resets, the persistent DP launch, the gather, and the copy of results + error word to pinned memory.
 static int enqueue_step(xted_ctx *c, bool events) {
     const XKernelParams &K = c->kp;
     const int npairs = c->npairs;
@@ -156,22 +152,18 @@ static int enqueue_step(xted_ctx *c, bool events) {
     int32_t *hres = (int32_t *)c->result.p;
     const size_t res_bytes = (size_t)npairs * sizeof(int32_t);
     if (events && cudaEventRecord(c->ev0, c->stream) != cudaSuccess) return XTED_ECUDA;
-    // per-run reset of the error words and the ready queue, then level 0 of every pair
-    const size_t ne = (size_t)K.nentries;
+    // per-run reset: the error words and the claim counter; every table and hand-off word to -1 (not written)
     if (cudaMemsetAsync(cnt, 0, 8 * sizeof(int32_t), c->stream) != cudaSuccess ||
-        (K.ntasks > 0 &&
-         (cudaMemsetAsync(K.entry_state, 0, XTED_ESTATE * ne * sizeof(int32_t), c->stream) != cudaSuccess ||
-          cudaMemsetAsync(K.rq, 0xff, ((size_t)XTED_RINGS << K.rq_log2) * sizeof(unsigned long long),
-                          c->stream) != cudaSuccess ||
-          cudaMemsetAsync(K.rq_ctl, 0, (2 * XTED_RINGS + 8) * sizeof(int32_t), c->stream) != cudaSuccess ||
-          (K.nstriped > 0 &&
-           cudaMemsetAsync(K.sbuf, 0, (size_t)K.sbuf_words * sizeof(unsigned long long), c->stream) != cudaSuccess) ||
-          launch_rq_init(K, c->stream) != cudaSuccess)))
+        (K.nitems > 0 &&
+         (cudaMemsetAsync(K.next, 0, 2 * sizeof(int32_t), c->stream) != cudaSuccess ||
+          cudaMemsetAsync(K.dt, 0xff, (size_t)c->plan_dt_elems * sizeof(int32_t), c->stream) != cudaSuccess ||
+          (c->plan_words > 0 &&
+           cudaMemsetAsync(K.buf, 0xff, (size_t)c->plan_words * sizeof(int32_t), c->stream) != cudaSuccess))))
         return XTED_ECUDA;
     if (events && cudaEventRecord(c->evk0, c->stream) != cudaSuccess) return XTED_ECUDA;
-    if (K.ntasks > 0 && launch_dp(K, c->grid, c->stream) != cudaSuccess) return XTED_ECUDA;
+    if (K.nitems > 0 && launch_dp(K, c->grid, c->stream) != cudaSuccess) return XTED_ECUDA;
     if (events && cudaEventRecord(c->evk1, c->stream) != cudaSuccess) return XTED_ECUDA;
-    if (launch_gather(K.pairs, c->d_trivial, K.dt, npairs, d_out, K.c_del, K.c_ins, c->stream) != cudaSuccess)
+    if (launch_gather(K.pairs, c->d_trivial, K.dt, npairs, d_out, K.c_del, K.c_ins, K.error, c->stream) != cudaSuccess)
         return XTED_ECUDA;
     if ((events && cudaEventRecord(c->ev1, c->stream) != cudaSuccess) ||
         cudaMemcpyAsync(hres, cnt, 8 * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
@@ -223,7 +215,7 @@ int ctx_run(xted_ctx *c, int32_t *out, bool allow_graph) {
     c->runs_prepared++;
     if (replay) {
         // timed from outside: the DP time of a replay includes the step's
-        // small kernels (ready-queue init and gather, a few microseconds)
+        // clearing of the tables and its gather
         if (cudaEventRecord(c->ev0, c->stream) != cudaSuccess || cudaEventRecord(c->evk0, c->stream) != cudaSuccess ||
             cudaGraphLaunch(c->step_graph, c->stream) != cudaSuccess ||
             cudaEventRecord(c->evk1, c->stream) != cudaSuccess || cudaEventRecord(c->ev1, c->stream) != cudaSuccess) {
@@ -253,28 +245,21 @@ int ctx_run(xted_ctx *c, int32_t *out, bool allow_graph) {
     c->stats.grid = c->grid;
     std::memcpy(c->err_info, hres + 2, sizeof(c->err_info));
     if (K.trace) {
-        std::vector<unsigned long long> tr((size_t)K.ntasks * 4);
+        std::vector<unsigned long long> tr((size_t)K.nitems * 4);
         if (cudaMemcpy(tr.data(), K.trace, tr.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost) ==
             cudaSuccess) {
             if (FILE *f = std::fopen(std::getenv("XTED_TRACE"), "wb")) {
                 std::fwrite(tr.data(), sizeof(unsigned long long), tr.size(), f);
                 std::fclose(f);
             }
-            // the plan beside it: tasks (pair, entry, kind, first unit) and entries
-            std::vector<XTask> tk((size_t)K.ntasks);
-            std::vector<XEntry> en((size_t)K.nentries);
+            // the plan beside it: the items in list order
+            std::vector<XItem> it((size_t)K.nitems);
             const std::string base = std::getenv("XTED_TRACE");
-            if (cudaMemcpy(tk.data(), K.tasks, tk.size() * sizeof(XTask), cudaMemcpyDeviceToHost) == cudaSuccess &&
-                cudaMemcpy(en.data(), K.entries, en.size() * sizeof(XEntry), cudaMemcpyDeviceToHost) == cudaSuccess) {
-                if (FILE *f = std::fopen((base + ".tasks").c_str(), "wb")) {
-                    std::fwrite(tk.data(), sizeof(XTask), tk.size(), f);
+            if (cudaMemcpy(it.data(), K.items, it.size() * sizeof(XItem), cudaMemcpyDeviceToHost) == cudaSuccess)
+                if (FILE *f = std::fopen((base + ".items").c_str(), "wb")) {
+                    std::fwrite(it.data(), sizeof(XItem), it.size(), f);
                     std::fclose(f);
                 }
-                if (FILE *f = std::fopen((base + ".entries").c_str(), "wb")) {
-                    std::fwrite(en.data(), sizeof(XEntry), en.size(), f);
-                    std::fclose(f);
-                }
-            }
         }
     }
     if (hres[1] != 0) return hres[1];
@@ -295,8 +280,8 @@ void fill_stats(xted_ctx *c, double plan_ms) {
     c->stats.pairs = c->npairs;
     c->stats.cells = c->plan_cells;
     c->stats.cells_right = c->plan_cells_right;
-    c->stats.tasks = c->kp.ntasks;
-    c->stats.units = c->plan_units;
+    c->stats.tasks = c->kp.nitems;
+    c->stats.units = c->kp.nitems;
     c->stats.levels_max = c->plan_levels_max;
     c->stats.host_plan_ms = plan_ms;
 }

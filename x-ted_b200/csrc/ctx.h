@@ -52,8 +52,8 @@ struct xted_ctx {
     std::vector<xted::TreeView> uniq;
     std::vector<int32_t> pair_trees;
     std::vector<xted::DTree> htrees;
-    int64_t plan_dt_elems = 0, plan_cells = 0, plan_cells_right = 0, plan_units = 0;
-    int32_t plan_stack_rows = 1, plan_max_wide = 0, plan_levels_max = 0;
+    int64_t plan_dt_elems = 0, plan_cells = 0, plan_cells_right = 0, plan_words = 0;
+    int32_t plan_stack_rows = 1, plan_levels_max = 0;
     // the prepared plan (xted_prepare_batch / every batch call)
     XKernelParams kp{};
     int32_t npairs = 0;

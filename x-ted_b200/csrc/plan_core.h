@@ -41,6 +41,9 @@ struct DDepth {
     int32_t chunk_lo, nnarrow, nwide;  // chunks: narrow, then half-block, then whole-block ones
     int32_t maxrows, maxw_n, maxw_w;   // largest run and chunk widths (cost estimates)
     int32_t nhalf, maxw_h;
+    int32_t nitems, wsum;  // as columns: items per row run, hand-off words per row (flow_plan.h)
+    int32_t rows;          // as rows: all rows of the depth's tables
+    int32_t pad;
 };
 
 // One tree in one orientation (index 2 * tree + o; o = 1 mirrored).

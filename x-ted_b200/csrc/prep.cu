@@ -11,18 +11,22 @@
 //                  column-list positions, row runs, column chunks (the records
 //                  plan_core.h's orient_tree builds for the host planners)
 //   k_pair_setup   decomposition choice, level count
-//   k_level_*      unit/task counts and estimates per (pair, level), ready-
-//                  queue priority, then the units and tasks themselves
+//   k_map_reserve, k_chunk_maps   export maps of column chunks too wide for a warp
+//   k_depth_totals items and hand-off words per keyroot depth (flow_plan.h)
+//   k_level_*      item counts per (pair, level), the levels in the order of
+//                  the launch's list, then the items themselves
 //
-// Each (pair, level) entry gets a ready-queue priority bucket from the pair's
-// remaining estimated critical path; the DP kernel publishes an entry when the
-// previous level of its pair has finished (see xted_internal.h).
-// Two small device-to-host reads size the buffers (entries; tasks and units).
+// The list holds the levels of all pairs by the time estimated to be left of
+// their pair behind them, longest first (a pair's levels in order), so the
+// pairs with the longest chains of tables start first and the launch ends
+// with short ones. Two small device-to-host reads size the buffers.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 
 #include "ctx.h"
+#include "flow_plan.h"
 #include "plan_core.h"
 
 namespace xted {
@@ -365,23 +369,24 @@ __global__ void k_orient_warp(PlanPools P) {
 }
 
 __global__ void k_pair_setup(const DTree *trees, const DOTree *ot, const int32_t *pair_trees, int orientation,
-                             int npairs, DPair *pairs, int64_t *L, int64_t *cells) {
+                             int npairs, DPair *pairs, int64_t *L, int64_t *cells, int32_t *used) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npairs) return;
     pair_setup(trees, ot, pair_trees, orientation, p, pairs);
-    L[p] = pairs[p].L;
-    cells[p] = pairs[p].trivial >= 0 ? 0 : (int64_t)trees[pairs[p].ta].n * trees[pairs[p].tb].n;
+    const DPair q = pairs[p];
+    L[p] = q.L;
+    cells[p] = q.trivial >= 0 ? 0 : (int64_t)trees[q.ta].n * table_pitch(trees[q.tb].n);
+    if (q.trivial < 0) used[2 * q.tb + q.o] = 1;  // a column tree
 }
 
-// Exclusive scan of n int64 values in one block; out[n] = total. Optional
-// permutation: scans v[perm[i]] in the order i and writes out[i].
-__global__ void k_scan64(const int64_t *v, const int32_t *perm, int n, int64_t *out) {
+// Exclusive scan of n int64 values in one block; out[n] = total.
+__global__ void k_scan64(const int64_t *v, int n, int64_t *out) {
     __shared__ int64_t part[1024];
     const int tid = threadIdx.x, nt = blockDim.x;
     const int per = (n + nt - 1) / nt;
-    const int lo = tid * per, hi = min(lo + per, n);
+    const int lo = min(tid * per, n), hi = min(lo + per, n);
     int64_t s = 0;
-    for (int i = lo; i < hi; i++) s += v[perm ? perm[i] : i];
+    for (int i = lo; i < hi; i++) s += v[i];
     part[tid] = s;
     __syncthreads();
     for (int d = 1; d < nt; d <<= 1) {
@@ -393,17 +398,16 @@ __global__ void k_scan64(const int64_t *v, const int32_t *perm, int n, int64_t *
     int64_t run = part[tid] - s;
     for (int i = lo; i < hi; i++) {
         out[i] = run;
-        run += v[perm ? perm[i] : i];
+        run += v[i];
     }
     if (tid == nt - 1) out[n] = part[nt - 1];
 }
 
 struct Summary {
     int64_t entries, dt_elems;
-    int64_t tasks, units;
-    int64_t nstriped, nstripes;  // striped units and their stripes
-    int64_t stripe_buf;          // 64-bit words of the striped units' buffers
-    int32_t stack_rows, max_wide;
+    int64_t items, words;        // items of the launch, hand-off words of striped units
+    int64_t map_ints;            // export maps of striped chunks
+    int32_t nmaps, stack_rows;
     int64_t cells, cells_right;
     int32_t levels_max, pad;
     int64_t chain_max;
@@ -421,9 +425,8 @@ __global__ void k_pair_offsets(DPair *pairs, const DTree *trees, const DOTree *o
     q.lvl_base = (int32_t)Lscan[p];
     q.dt_off = dtscan[p];
     if (q.trivial < 0) {
-        const DOTree &A = ot[2 * q.ta + q.o], &B = ot[2 * q.tb + q.o];
+        const DOTree &A = ot[2 * q.ta + q.o];
         atomicMax(&sum->stack_rows, A.maxka + 1);
-        atomicMax(&sum->max_wide, B.maxw_wide);
         atomicMax(&sum->levels_max, q.L);
         atomicAdd((unsigned long long *)&sum->cells, (unsigned long long)q.cells);
         atomicAdd((unsigned long long *)&sum->cells_right,
@@ -431,116 +434,59 @@ __global__ void k_pair_offsets(DPair *pairs, const DTree *trees, const DOTree *o
     }
 }
 
-__global__ void k_level_expand(const DPair *pairs, int npairs, DLevel *lv) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npairs) return;
-    const DPair q = pairs[p];
-    for (int d = 0; d < q.L; d++) {
-        DLevel &E = lv[q.lvl_base + d];
-        E.pair = p;
-        E.level = d;
+// A warp per oriented tree: reserves export-map space for the striped chunks
+// of the trees that some pair uses as its column tree, and lists them.
+__global__ void k_map_reserve(PlanPools P, const int32_t *used, XChunkX *chunkx, int32_t *list, Summary *sum) {
+    const int lane = threadIdx.x & 31;
+    const int ot = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (ot >= 2 * P.ntrees || !used[ot]) return;
+    const DOTree O = P.otrees[ot];
+    for (int d = 0; d <= O.D; d++) {
+        const DDepth &dd = P.depths[O.depth_base + d];
+        const int hi = dd.chunk_lo + dd.nnarrow + dd.nhalf + dd.nwide;
+        for (int c = dd.chunk_lo + lane; c < hi; c += 32)
+            if (chunk_stripes(P.chunks[c], P.krd) > 1) {
+                chunkx[c].map = (int64_t)atomicAdd((unsigned long long *)&sum->map_ints,
+                                                   (unsigned long long)P.chunks[c].width);
+                list[atomicAdd(&sum->nmaps, 1)] = c;
+            }
     }
 }
 
-__global__ void k_level_count(LevelCtx C, DLevel *lv, int64_t nent, int64_t *units, int64_t *tasks,
-                              int64_t *striped, int64_t *stripes) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nent) return;
-    DLevel E = lv[e];
-    double est;
-    level_count(C, E, &est);
-    E.key = (int64_t)(est / 64.0) + 1;  // >= 1: strictly decreasing ranks below
-    lv[e] = E;
-    units[e] = (int64_t)E.nwide + E.nnarrow + E.nhalf;
-    tasks[e] = E.ntasks;
-    striped[e] = E.nstriped;
-    stripes[e] = E.nstripes;
-}
-
-// Per pair: est(d) is the estimated time of level d's slowest task; EST(d) =
-// sum of est below d; the pair's chain C = sum of all est. A level's ready-
-// queue bucket grows with the pair's remaining chain C - EST(d) relative to
-// the longest chain of the batch.
-__global__ void k_pair_rank(const DPair *pairs, int npairs, DLevel *lv, int64_t *chain, Summary *sum) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npairs) return;
-    const DPair q = pairs[p];
-    int64_t acc = 0;
-    for (int d = 0; d < q.L; d++) {
-        DLevel &E = lv[q.lvl_base + d];
-        const int64_t est = E.key;
-        E.key = acc;
-        acc += est;
-    }
-    chain[p] = acc;
-    atomicMax((unsigned long long *)&sum->chain_max, (unsigned long long)acc);
-}
-
-__global__ void k_level_offsets(DLevel *lv, int64_t nent, const int64_t *task_scan, const int64_t *unit_scan,
-                                const int64_t *striped_scan, const int64_t *stripes_scan, const int64_t *chain,
-                                const DPair *pairs, XEntry *entries, Summary *sum) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e == 0) {
-        sum->tasks = task_scan[nent];
-        sum->units = unit_scan[nent];
-        sum->nstriped = striped_scan[nent];
-        sum->nstripes = stripes_scan[nent];
-    }
-    if (e >= nent) return;
-    DLevel &E = lv[e];
-    E.task_off = (int32_t)task_scan[e];
-    E.unit_off = (int32_t)unit_scan[e];
-    E.stripe_off = (int32_t)striped_scan[e];
-    E.entry = (int32_t)e;
-    XEntry X;
-    X.task_off = E.task_off;
-    X.ntasks = E.ntasks;
-    X.bucket = level_bucket(chain[E.pair] - E.key, sum->chain_max);
-    X.next = E.level + 1 < pairs[E.pair].L ? (int32_t)e + 1 : -1;
-    X.nnarrow = E.nntasks;
-    X.pad = 0;
-    entries[e] = X;
-}
-
-__global__ void k_level_fill(LevelCtx C, const DLevel *lv, int64_t nent, XUnit *units, XTask *tasks,
-                             XStripe *stripes) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < nent) level_fill(C, lv[e], units, tasks, stripes);
-}
-
-// One block per striped unit: its export map, the far columns that a stripe
-// reads from a stripe to its right (f = orl(j) + 1 in another stripe), numbered
-// in column order (-1 elsewhere), and the words its buffer needs: carries and
-// first columns of every stripe and row, and the exported values of every row.
-__global__ void k_stripe_prep(XStripe *stripes, int32_t *smap, int64_t map_stride, const XUnit *units,
-                              const XChunk *chunks, const XPair *pairs, const int2 *rowinfo, const int32_t *krd,
-                              int64_t *need) {
+// One block per striped chunk: its export map, the far columns that a stripe
+// reads from a stripe to its right, numbered in column order (-1 elsewhere).
+// The tree whose node records it needs is found from the chunk's
+// keyroot pool index, which lies in the tree's range of the node pool.
+__global__ void k_chunk_maps(PlanPools P, const int32_t *list, XChunkX *chunkx, int32_t *smap) {
     __shared__ int ends[XTED_WARPS];
-    const int i = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const XStripe S = stripes[i];
-    const XChunk ch = chunks[units[S.unit].chunk];
-    const XPair pr = pairs[S.pair];
-    const int w = S.w, SW = XTED_CTA_THREADS * S.sww;
-    int32_t *expmap = smap + (int64_t)i * map_stride;
-    for (int c = tid; c < w; c += XTED_CTA_THREADS) expmap[c] = 0;
+    __shared__ int s_base;
+    const int c0 = list[blockIdx.x], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const XChunk ch = P.chunks[c0];
+    if (tid == 0) {  // the oriented tree whose pool range holds the chunk
+        int lo = 0, hi = 2 * P.ntrees - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (P.otrees[mid].node_base <= ch.k_lo) lo = mid;
+            else hi = mid - 1;
+        }
+        s_base = P.otrees[lo].node_base;
+    }
     __syncthreads();
-    const int2 *nodes = rowinfo + pr.col_base;
-    const int j0 = krd[ch.k_lo];
+    const int w = ch.width, j0 = P.krd[ch.k_lo], lead = j0 & (XTED_PITCH - 1);
+    const int2 *nodes = P.node + s_base;
+    int32_t *map = smap + chunkx[c0].map;
+    for (int c = tid; c < w; c += XTED_CTA_THREADS) map[c] = 0;
+    __syncthreads();
     for (int c = tid; c < w; c += XTED_CTA_THREADS) {
-        const int j = j0 + c;
-        const int f = c + ((nodes[j].y & XTED_ROW_ORL_MASK) + 1 - j);
-        if (f < w && f / SW != c / SW) expmap[f] = 1;
+        const int foff = (nodes[j0 + c].y & XTED_ROW_ORL_MASK) + 1 - (j0 + c);
+        if (far_crosses(c, foff, w, lead)) map[c + foff] = 1;
     }
     __syncthreads();
     const int per = (w + XTED_CTA_THREADS - 1) / XTED_CTA_THREADS;
     const int a0 = min(tid * per, w), a1 = min(a0 + per, w);
     int cnt = 0;
-    for (int c = a0; c < a1; c++) cnt += expmap[c];
-    int incl = cnt;
-    for (int d = 1; d < 32; d <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += y;
-    }
+    for (int c = a0; c < a1; c++) cnt += map[c];
+    const int incl = warp_incl_sum(cnt, lane);
     if (lane == 31) ends[warp] = incl;
     __syncthreads();
     int before = incl - cnt, total = 0;
@@ -549,35 +495,199 @@ __global__ void k_stripe_prep(XStripe *stripes, int32_t *smap, int64_t map_strid
         total += ends[q];
     }
     for (int c = a0; c < a1; c++) {
-        const int m = expmap[c];
-        expmap[c] = m ? before : -1;
+        const int m = map[c];
+        map[c] = m ? before : -1;
         before += m;
     }
-    if (tid == 0) {
-        stripes[i].X = total;
-        stripes[i].map_off = (int64_t)i * map_stride;
-        need[i] = (2 * (int64_t)S.K * S.R + (int64_t)S.R * total + 15) & ~(int64_t)15;
+    if (tid == 0) chunkx[c0].X = total;
+}
+
+// A warp per oriented tree: stripes and hand-off words of its chunks summed
+// per depth (flow_depth_totals, flow_plan.h, with the lanes over the chunks).
+__global__ void k_depth_totals(PlanPools P, XChunkX *chunkx) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int ot = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (ot >= 2 * P.ntrees) return;
+    const DOTree O = P.otrees[ot];
+    for (int d = 0; d <= O.D; d++) {
+        DDepth &dd = P.depths[O.depth_base + d];
+        const int lo = dd.chunk_lo, hi = lo + dd.nnarrow + dd.nhalf + dd.nwide;
+        int k = 0, w = 0;
+        for (int cb = lo; cb < hi; cb += 32) {
+            const int c = cb + lane;
+            int K = 0, words = 0;
+            if (c < hi) {
+                K = chunk_stripes(P.chunks[c], P.krd);
+                if (K == 1) chunkx[c].X = 0;
+                words = chunk_words(K, chunkx[c].X);
+            }
+            const int ki = warp_incl_sum(K, lane), wi = warp_incl_sum(words, lane);
+            if (c < hi) {
+                chunkx[c].K = K;
+                chunkx[c].kpre = k + ki - K;
+                chunkx[c].wpre = w + wi - words;
+            }
+            k += __shfl_sync(FULL, ki, 31);
+            w += __shfl_sync(FULL, wi, 31);
+        }
+        if (lane == 0) {
+            dd.nitems = k;
+            dd.wsum = w;
+            const int last = dd.run_hi - 1;
+            dd.rows = P.cumw[P.runs[last].kr_lo] + P.runs[last].rows;  // every depth up to D has a keyroot
+        }
     }
 }
 
-__global__ void k_stripe_bufoff(XStripe *stripes, int64_t n, const int64_t *scan, Summary *sum) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) sum->stripe_buf = scan[n];
-    if (i < n) stripes[i].buf_off = scan[i];
+// One (pair, level) of the batch.
+struct Level {
+    int32_t pair, level;
+    int64_t items, words;
+    int64_t rem;              // estimate, then the time left of the pair from this level on
+    int64_t item_off, buf_off;
+};
+
+// A pair's levels: their counts, and the time left of the pair from each on.
+__global__ void k_level_count(FlowCtx C, const DPair *pairs, int npairs, Level *lv, Summary *sum) {
+    const int lane = threadIdx.x & 31;
+    const int p = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (p >= npairs) return;
+    const DPair q = pairs[p];
+    if (q.L == 0) return;
+    const DOTree A = C.ot[2 * q.ta + q.o], B = C.ot[2 * q.tb + q.o];
+    int64_t rem = 0;
+    for (int hi = q.L; hi > 0; hi -= 32) {  // from the last level down, 32 at a time
+        const int d = hi - 1 - lane;
+        int64_t items = 0, words = 0, est = 0;
+        if (d >= 0) flow_level_count(C, A, B, d, &items, &words, &est);
+        int64_t incl = est;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (d >= 0) {
+            Level &E = lv[q.lvl_base + d];
+            E.pair = p;
+            E.level = d;
+            E.items = items;
+            E.words = words;
+            E.rem = rem + incl;
+        }
+        rem += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) atomicMax((unsigned long long *)&sum->chain_max, (unsigned long long)rem);
+}
+
+// The order of the levels in the launch's list and their offsets, in one
+// block: a stable radix sort (four passes of four bits) of the levels by the
+// time left of their pair, longest first (stable: a pair's levels stay in
+// order), then the scans of items and hand-off words in that order.
+#define ORDER_THREADS 512
+__global__ void __launch_bounds__(ORDER_THREADS) k_level_order(Level *lv, int n, bool sort, int32_t *ord0, int32_t *ord1,
+                                                               Summary *sum) {
+    __shared__ int32_t cnt[16 * ORDER_THREADS];
+    __shared__ int64_t part[2][ORDER_THREADS];
+    const int tid = threadIdx.x;
+    const int per = (n + ORDER_THREADS - 1) / ORDER_THREADS, lo = min(tid * per, n), hi = min(lo + per, n);
+    int32_t *src = ord0, *dst = ord1;
+    for (int i = lo; i < hi; i++) src[i] = i;
+    if (sort) {
+        const double scale = 65535.0 / (double)max(sum->chain_max, (int64_t)1);
+        for (int shift = 0; shift < 16; shift += 4) {
+            auto digit = [&](int e) { return ((65535 - (int)((double)lv[e].rem * scale)) >> shift) & 15; };
+            for (int b = 0; b < 16; b++) cnt[b * ORDER_THREADS + tid] = 0;
+            for (int i = lo; i < hi; i++) cnt[digit(src[i]) * ORDER_THREADS + tid]++;
+            __syncthreads();
+            int s = 0;
+            for (int b = 0; b < 16; b++) s += cnt[16 * tid + b];
+            part[0][tid] = s;
+            __syncthreads();
+            for (int d = 1; d < ORDER_THREADS; d <<= 1) {
+                const int64_t x = tid >= d ? part[0][tid - d] : 0;
+                __syncthreads();
+                part[0][tid] += x;
+                __syncthreads();
+            }
+            int run = (int)part[0][tid] - s;
+            for (int b = 0; b < 16; b++) {
+                const int c = cnt[16 * tid + b];
+                cnt[16 * tid + b] = run;
+                run += c;
+            }
+            __syncthreads();
+            for (int i = lo; i < hi; i++) {
+                const int e = src[i];
+                dst[cnt[digit(e) * ORDER_THREADS + tid]++] = e;
+            }
+            __syncthreads();
+            int32_t *x = src;
+            src = dst;
+            dst = x;
+        }
+    }
+    int64_t a = 0, b = 0;
+    for (int i = lo; i < hi; i++) {
+        a += lv[src[i]].items;
+        b += lv[src[i]].words;
+    }
+    part[0][tid] = a;
+    part[1][tid] = b;
+    __syncthreads();
+    for (int d = 1; d < ORDER_THREADS; d <<= 1) {
+        const int64_t x = tid >= d ? part[0][tid - d] : 0, y = tid >= d ? part[1][tid - d] : 0;
+        __syncthreads();
+        part[0][tid] += x;
+        part[1][tid] += y;
+        __syncthreads();
+    }
+    int64_t ia = part[0][tid] - a, ib = part[1][tid] - b;
+    for (int i = lo; i < hi; i++) {
+        Level &E = lv[src[i]];
+        E.item_off = ia;
+        E.buf_off = ib;
+        ia += E.items;
+        ib += E.words;
+    }
+    if (tid == ORDER_THREADS - 1) {
+        sum->items = part[0][tid];
+        sum->words = part[1][tid];
+    }
+}
+
+// The items of the list, a block per level: by row depth from the deepest
+// down (the longest runs first), then by run, then by chunk.
+__global__ void k_level_fill(FlowCtx C, const DPair *pairs, const Level *lv, int64_t nent, XItem *items) {
+    for (int64_t e = blockIdx.x; e < nent; e += gridDim.x) {
+        const Level E = lv[e];
+        const DPair q = pairs[E.pair];
+        const DOTree A = C.ot[2 * q.ta + q.o], B = C.ot[2 * q.tb + q.o];
+        const int lo = max(E.level - B.D, 0), hi = min(A.D, E.level);
+        int64_t at = E.item_off, buf = E.buf_off;
+        for (int a = hi; a >= lo; a--) {
+            const DDepth ra = C.depths[A.depth_base + a], cb = C.depths[B.depth_base + E.level - a];
+            const int64_t n = (int64_t)(ra.run_hi - ra.run_lo) * cb.nitems;
+            for (int64_t k = threadIdx.x; k < n; k += blockDim.x) items[at + k] = flow_item(C, ra, cb, E.pair, k, buf);
+            at += n;
+            buf += (int64_t)ra.rows * cb.wsum;
+        }
+    }
 }
 
 __global__ void k_pair_finalize(const DPair *pairs, const DTree *trees, const DOTree *ot, int npairs, XPair *xp,
-                                int32_t *trivial, int32_t *first) {
+                                int32_t *trivial) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npairs) return;
     const DPair q = pairs[p];
-    first[p] = q.L > 0 ? q.lvl_base : -1;
     XPair x;
     x.dt_off = q.dt_off;
     x.m = trees[q.ta].n;
     x.n = trees[q.tb].n;
     x.row_base = ot[2 * q.ta + q.o].node_base;
     x.col_base = ot[2 * q.tb + q.o].node_base;
+    x.pitch = table_pitch(x.n);
+    x.pad = 0;
     xp[p] = x;
     trivial[p] = q.trivial;
 }
@@ -607,6 +717,7 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     std::vector<int32_t> &pt = c->pair_trees;
     pt.resize(2 * (size_t)npairs);
     int64_t N = 0, R = 0;
+    int32_t maxn = 0;
     for (int p = 0; p < npairs; p++) {
         for (int side = 0; side < 2; side++) {
             const xted_tree &t = side ? b[p] : a[p];
@@ -620,6 +731,7 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
                 c->uniq.push_back(TreeView{t.n, t.labels, t.child_off, t.child_idx});
                 N += t.n;
                 R += 3 * (int64_t)t.n + 1;
+                maxn = std::max(maxn, t.n);
             } else {
                 id = it->second;
             }
@@ -684,9 +796,10 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     const size_t N2 = 2 * (size_t)std::max<int64_t>(N, 1);
     size_t need = upload + 4096;
     need += 3 * sizeof(int32_t) * (size_t)std::max<int64_t>(N, 1);  // size, depth, parent
-    need += N2 * (sizeof(int2) + 2 * sizeof(int32_t) + sizeof(XRun) + sizeof(XChunk) + 3 * sizeof(int32_t));
-    need += sizeof(DDepth) * (N2 + 2 * (size_t)T) + sizeof(DOTree) * 2 * (size_t)T + sizeof(DTree) * (size_t)T;
-    need += (size_t)npairs * (sizeof(DPair) + sizeof(XPair) + 4 + 5 * 8) + 20 * 256 + sizeof(Summary);
+    need += N2 * (sizeof(int2) + 2 * sizeof(int32_t) + sizeof(XRun) + sizeof(XChunk) + sizeof(XChunkX) + 4 * sizeof(int32_t));
+    need += sizeof(DDepth) * (N2 + 2 * (size_t)T) + sizeof(DOTree) * 2 * (size_t)T + sizeof(DTree) * (size_t)T +
+            2 * sizeof(int32_t) * (size_t)T;
+    need += (size_t)npairs * (sizeof(DPair) + sizeof(XPair) + 4 + 4 * 8) + 24 * 256 + sizeof(Summary);
     rc = ctx_dev_reserve(c, c->meta, need);
     if (rc) return rc;
     Carver cv{(char *)c->meta.p};
@@ -725,23 +838,27 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     XPair *d_xpairs = cv.take<XPair>((size_t)npairs);
     int32_t *d_trivial = cv.take<int32_t>((size_t)npairs);
     int64_t *d_L = cv.take<int64_t>((size_t)npairs + 1);
-    int64_t *d_chain = cv.take<int64_t>((size_t)npairs + 1);
     int64_t *d_cells = cv.take<int64_t>((size_t)npairs + 1);
     int64_t *d_Ls = cv.take<int64_t>((size_t)npairs + 1);
     int64_t *d_dts = cv.take<int64_t>((size_t)npairs + 1);
+    XChunkX *d_chunkx = cv.take<XChunkX>(N2);
+    int32_t *d_list = cv.take<int32_t>(N2);
+    int32_t *d_used = cv.take<int32_t>(2 * (size_t)T);
     Summary *d_sum = cv.take<Summary>(1);
     if (cv.off > c->meta.cap) return XTED_ENOMEM;
+    const bool stripes = maxn + XTED_PITCH > XTED_SW;  // some chunk may be wider than a warp holds
 
     const int BS = 128;
-    cudaMemsetAsync(d_sum, 0, sizeof(Summary), s);
+    cudaMemsetAsync(d_used, 0, (size_t)((char *)(d_sum + 1) - (char *)d_used), s);
     k_tree_basic_warp<<<blocks_for(32 * (int64_t)T, BS), BS, 0, s>>>(P, d_trees);
     k_orient_warp<<<blocks_for(64 * (int64_t)T, BS), BS, 0, s>>>(P);
-    k_pair_setup<<<blocks_for(npairs, BS), BS, 0, s>>>(d_trees, P.otrees, d_pt, c->opts.orientation, npairs,
-                                                       d_pairs, d_L, d_cells);
-    k_scan64<<<1, 1024, 0, s>>>(d_L, nullptr, npairs, d_Ls);
-    k_scan64<<<1, 1024, 0, s>>>(d_cells, nullptr, npairs, d_dts);
+    k_pair_setup<<<blocks_for(std::max(npairs, 1), BS), BS, 0, s>>>(d_trees, P.otrees, d_pt, c->opts.orientation, npairs,
+                                                                    d_pairs, d_L, d_cells, d_used);
+    k_scan64<<<1, 1024, 0, s>>>(d_L, npairs, d_Ls);
+    k_scan64<<<1, 1024, 0, s>>>(d_cells, npairs, d_dts);
     k_pair_offsets<<<blocks_for(std::max(npairs, 1), BS), BS, 0, s>>>(d_pairs, d_trees, P.otrees, npairs, d_Ls,
                                                                       d_dts, d_sum);
+    if (stripes) k_map_reserve<<<blocks_for(64 * (int64_t)T, BS), BS, 0, s>>>(P, d_used, d_chunkx, d_list, d_sum);
     rc = ctx_host_reserve(c->summary, sizeof(Summary));
     if (rc) return rc;
     Summary *hs = (Summary *)c->summary.p;
@@ -751,92 +868,53 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
         return XTED_ECUDA;
     }
     const int64_t nent = hs->entries;
-    if (nent > INT32_MAX / XTED_BUCKETS) return XTED_ENOMEM;
-    // ---- buffer B: level entries and scans ----
+    if (nent > INT32_MAX / 2) return XTED_ENOMEM;
+    if (hs->nmaps > 0) {
+        rc = ctx_dev_reserve(c, c->smap, (size_t)hs->map_ints * sizeof(int32_t));
+        if (rc) return rc;
+        k_chunk_maps<<<(unsigned)hs->nmaps, XTED_CTA_THREADS, 0, s>>>(P, d_list, d_chunkx, (int32_t *)c->smap.p);
+    }
+    // ---- buffer B: the levels ----
     const size_t E1 = (size_t)nent + 1;
-    size_t needB = sizeof(DLevel) * E1 + sizeof(XEntry) * E1 + 8 * 8 * E1 + 16 * 256;
-    rc = ctx_dev_reserve(c, c->levels, needB);
+    rc = ctx_dev_reserve(c, c->levels, sizeof(Level) * E1 + 2 * sizeof(int32_t) * E1 + 4 * 256);
     if (rc) return rc;
     Carver cb{(char *)c->levels.p};
-    DLevel *d_lv = cb.take<DLevel>(E1);
-    XEntry *d_entries = cb.take<XEntry>(E1);
-    int64_t *d_units = cb.take<int64_t>(E1), *d_tasks = cb.take<int64_t>(E1);
-    int64_t *d_uscan = cb.take<int64_t>(E1), *d_tscan = cb.take<int64_t>(E1);
-    int64_t *d_striped = cb.take<int64_t>(E1), *d_stripes = cb.take<int64_t>(E1);
-    int64_t *d_sdscan = cb.take<int64_t>(E1), *d_spscan = cb.take<int64_t>(E1);
-    LevelCtx C;
+    Level *d_lv = cb.take<Level>(E1);
+    int32_t *d_ord0 = cb.take<int32_t>(E1), *d_ord1 = cb.take<int32_t>(E1);
+    FlowCtx C;
     C.ot = P.otrees;
     C.depths = P.depths;
     C.runs = P.runs;
     C.chunks = P.chunks;
-    C.pairs = d_pairs;
-    C.narrow_width = c->opts.narrow_width;
-    C.wide_rows = c->opts.wide_rows > 0 ? c->opts.wide_rows : -1;
-    C.stripe_min_cells = c->opts.stripe_min_cells < 0 ? 0
-                         : (c->opts.stripe_min_cells > 0 ? c->opts.stripe_min_cells : XTED_STRIPE_MIN_CELLS_DEFAULT);
+    C.chunkx = d_chunkx;
+    C.cumw = P.cumw;
+    k_pair_finalize<<<blocks_for(std::max(npairs, 1), BS), BS, 0, s>>>(d_pairs, d_trees, P.otrees, npairs, d_xpairs,
+                                                                       d_trivial);
     if (nent > 0) {
-        k_level_expand<<<blocks_for(npairs, BS), BS, 0, s>>>(d_pairs, npairs, d_lv);
-        k_level_count<<<blocks_for(nent, BS), BS, 0, s>>>(C, d_lv, nent, d_units, d_tasks, d_striped, d_stripes);
-        k_pair_rank<<<blocks_for(npairs, BS), BS, 0, s>>>(d_pairs, npairs, d_lv, d_chain, d_sum);
-        k_scan64<<<1, 1024, 0, s>>>(d_tasks, nullptr, (int)nent, d_tscan);
-        k_scan64<<<1, 1024, 0, s>>>(d_units, nullptr, (int)nent, d_uscan);
-        k_scan64<<<1, 1024, 0, s>>>(d_striped, nullptr, (int)nent, d_sdscan);
-        k_scan64<<<1, 1024, 0, s>>>(d_stripes, nullptr, (int)nent, d_spscan);
-        k_level_offsets<<<blocks_for(nent, BS), BS, 0, s>>>(d_lv, nent, d_tscan, d_uscan, d_sdscan, d_spscan,
-                                                              d_chain, d_pairs, d_entries, d_sum);
+        k_depth_totals<<<blocks_for(64 * (int64_t)T, BS), BS, 0, s>>>(P, d_chunkx);
+        k_level_count<<<blocks_for(32 * (int64_t)npairs, BS), BS, 0, s>>>(C, d_pairs, npairs, d_lv, d_sum);
+        k_level_order<<<1, ORDER_THREADS, 0, s>>>(d_lv, (int)nent, npairs > 1, d_ord0, d_ord1, d_sum);
     }
     cudaMemcpyAsync(hs, d_sum, sizeof(Summary), cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) {
         cudaGetLastError();
         return XTED_ECUDA;
     }
-    const int64_t ntasks = nent > 0 ? hs->tasks : 0, nunits = nent > 0 ? hs->units : 0;
-    const int64_t nstriped = nent > 0 ? hs->nstriped : 0, nstripes = nent > 0 ? hs->nstripes : 0;
-    if (ntasks > INT32_MAX / 2 || nunits > INT32_MAX / 2 || nstripes > INT32_MAX / 2) return XTED_ENOMEM;
-    // ---- buffer C: units, tasks and the ready queue's state ----
-    int rq_log2 = 0;
-    while (((int64_t)1 << rq_log2) < (int64_t)E1) rq_log2++;
-    const size_t rq_slots = (size_t)XTED_RINGS << rq_log2;
-    rc = ctx_dev_reserve(c, c->work, sizeof(XUnit) * (size_t)(nunits + 1) + sizeof(XTask) * (size_t)(ntasks + 1) +
-                                         8 * rq_slots + 4 * (XTED_ESTATE * E1 + (size_t)npairs + 2 * XTED_RINGS + 8) +
-                                         sizeof(XStripe) * (size_t)(nstriped + 1) + 8 * 2 * (size_t)(nstriped + 1) +
-                                         12 * 256);
+    const int64_t nitems = hs->items;
+    if (nitems > INT32_MAX / 2) return XTED_ENOMEM;
+    // ---- buffer C: the items and the launch's counters; the hand-off words ----
+    rc = ctx_dev_reserve(c, c->work, sizeof(XItem) * (size_t)(nitems + 1) + 2 * 256 + 64);
     if (rc) return rc;
     Carver cw{(char *)c->work.p};
-    XUnit *d_units_out = cw.take<XUnit>((size_t)nunits);
-    XTask *d_tasks_out = cw.take<XTask>((size_t)ntasks);
-    int32_t *d_first = cw.take<int32_t>((size_t)npairs);
-    int32_t *d_state = cw.take<int32_t>(XTED_ESTATE * E1);  // narrow claimed, group claimed, done per entry
-    unsigned long long *d_rq = cw.take<unsigned long long>(rq_slots);
-    int32_t *d_ctl = cw.take<int32_t>(2 * XTED_RINGS + 8);  // heads/tails, then the done counter
-    XStripe *d_st = cw.take<XStripe>((size_t)nstriped + 1);
-    int64_t *d_need = cw.take<int64_t>((size_t)nstriped + 1), *d_needscan = cw.take<int64_t>((size_t)nstriped + 1);
-    if (nent > 0)
-        k_level_fill<<<blocks_for(nent, 64), 64, 0, s>>>(C, d_lv, nent, d_units_out, d_tasks_out, d_st);
-    k_pair_finalize<<<blocks_for(std::max(npairs, 1), BS), BS, 0, s>>>(d_pairs, d_trees, P.otrees, npairs, d_xpairs,
-                                                                       d_trivial, d_first);
-    if (cudaGetLastError() != cudaSuccess) return XTED_ECUDA;
-    // striped units: export maps (one stride of the widest segment each), then
-    // the buffers, whose sizes the maps give
-    int64_t stripe_buf = 0;
-    if (nstriped > 0) {
-        const int64_t map_stride = ((int64_t)hs->max_wide + 31) & ~(int64_t)31;
-        rc = ctx_dev_reserve(c, c->smap, (size_t)(nstriped * map_stride) * sizeof(int32_t));
-        if (rc) return rc;
-        k_stripe_prep<<<(unsigned)nstriped, XTED_CTA_THREADS, 0, s>>>(d_st, (int32_t *)c->smap.p, map_stride,
-                                                                      d_units_out, P.chunks, d_xpairs, P.node,
-                                                                      P.krd, d_need);
-        k_scan64<<<1, 1024, 0, s>>>(d_need, nullptr, (int)nstriped, d_needscan);
-        k_stripe_bufoff<<<blocks_for(nstriped, BS), BS, 0, s>>>(d_st, nstriped, d_needscan, d_sum);
-        cudaMemcpyAsync(hs, d_sum, sizeof(Summary), cudaMemcpyDeviceToHost, s);
-        if (cudaStreamSynchronize(s) != cudaSuccess) {
-            cudaGetLastError();
-            return XTED_ECUDA;
-        }
-        stripe_buf = hs->stripe_buf;
-        rc = ctx_dev_reserve(c, c->sbuf, (size_t)std::max<int64_t>(stripe_buf, 1) * sizeof(unsigned long long));
+    XItem *d_items = cw.take<XItem>((size_t)nitems);
+    int32_t *d_ctl = cw.take<int32_t>(2);  // items claimed, items finished
+    if (hs->words > 0) {
+        rc = ctx_dev_reserve(c, c->sbuf, (size_t)hs->words * sizeof(int32_t));
         if (rc) return rc;
     }
+    if (nent > 0)
+        k_level_fill<<<(unsigned)std::min<int64_t>(nent, 1 << 16), 128, 0, s>>>(C, d_pairs, d_lv, nent, d_items);
+    if (cudaGetLastError() != cudaSuccess) return XTED_ECUDA;
 
     std::memset(&K, 0, sizeof(K));
     K.rowinfo = P.node;
@@ -845,32 +923,22 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     K.runs = P.runs;
     K.chunks = P.chunks;
     K.pairs = d_xpairs;
-    K.units = d_units_out;
-    K.tasks = d_tasks_out;
-    K.entries = d_entries;
-    K.first = d_first;
-    K.ntasks = (int32_t)ntasks;
-    K.nentries = (int32_t)nent;
+    K.chunkx = d_chunkx;
+    K.items = d_items;
+    K.nitems = (int32_t)nitems;
     K.npairs = npairs;
-    K.entry_state = d_state;
-    K.rq = d_rq;
-    K.rq_log2 = rq_log2;
-    K.rq_ctl = d_ctl;
-    K.done_total = d_ctl + 2 * XTED_RINGS;
-    K.stripes = d_st;
-    K.nstriped = (int32_t)nstriped;
-    K.smap = nstriped > 0 ? (const int32_t *)c->smap.p : nullptr;
-    K.sbuf = nstriped > 0 ? (unsigned long long *)c->sbuf.p : nullptr;
-    K.sbuf_words = stripe_buf;
+    K.next = d_ctl;
+    K.progress = d_ctl + 1;
+    K.smap = (const int32_t *)c->smap.p;
+    K.buf = (int32_t *)c->sbuf.p;
     K.hold_pair = -1;
     c->d_trivial = d_trivial;
     c->plan_dt_elems = hs->dt_elems;
     c->plan_stack_rows = std::max(hs->stack_rows, 1);
-    c->plan_max_wide = hs->max_wide;
+    c->plan_words = hs->words;
     c->plan_cells = hs->cells;
     c->plan_cells_right = hs->cells_right;
     c->plan_levels_max = hs->levels_max;
-    c->plan_units = nunits;
     return XTED_OK;
 }
 

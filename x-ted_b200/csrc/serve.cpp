@@ -10,20 +10,19 @@
 // the device. A query is one more tree planned into one of XTED_SERVE_SLOTS
 // slots: its node pools, its pairs (query x every corpus tree, the corpus
 // tree as the row tree so the far-row stack depth is a corpus property),
-// their level entries, units and tasks. Distance tables come from a pool of
-// device memory; a query is admitted when a slot is free and its tables,
-// units, tasks and entries fit ("DP scratch bytes"), in arrival order.
+// their items. Tables, hand-off words and export maps come from a pool of
+// device memory; a query is admitted when a slot is free and these and its
+// items fit ("DP scratch bytes"), in arrival order.
 //
 // Continuous batching. An admitted query's plan is copied to the device on a
-// copy stream, followed by a mailbox record and the posted count. The DP
-// kernel, launched once and kept running while there is work, claims the
-// record, publishes level 0 of the query's pairs into its ready queue and
-// runs them beside the queries already in flight. Each query owns one
-// priority bucket (by arrival), and blocks probe the oldest query's bucket
-// first, so earlier queries finish first while later ones fill idle blocks.
-// A finished pair writes its distance into pinned host memory; the last pair
-// of a query raises the slot's flag. Blocks leave the launch after an idle
-// spell; a worker thread relaunches when new work arrives.
+// copy stream, its tables set to "not written", and its slot's list word
+// (first item, end) written last. The warps of the DP kernel, launched once
+// and kept running while there is work, claim items from the lists of all
+// slots, the oldest query's first, so earlier queries finish first while later
+// ones fill idle warps. The item that ends a pair writes its distance into
+// pinned host memory; the last item of a query raises the slot's flag. Warps
+// leave the launch after an idle spell; a worker thread relaunches when new
+// work arrives.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -52,7 +51,6 @@ cudaError_t launch_dp(const XKernelParams &P, int grid, cudaStream_t s);
 }
 
 static_assert(XTED_SERVE_SLOTS == XTED_SERVE_SLOTS_MAX, "slot count of the ABI and the kernels");
-static_assert(XTED_SERVE_SLOTS <= XTED_BUCKETS, "one ready-queue bucket per query in flight");
 
 namespace xted {
 
@@ -63,49 +61,23 @@ double now_ms() {
     return duration<double, std::milli>(steady_clock::now().time_since_epoch()).count();
 }
 
-// Allocator over [0, cap) (elements): first fit, or next fit from a cursor
-// that follows the last allocation (freed ranges are then reused only after
-// the cursor has gone round the whole pool).
+// First-fit allocator over [0, cap) (elements).
 class Extents {
 public:
-    void reset(int64_t cap, bool next_fit = false) {
+    void reset(int64_t cap) {
         free_.clear();
         if (cap > 0) free_[0] = cap;
         cap_ = cap;
-        next_fit_ = next_fit;
-        cursor_ = 0;
     }
     int64_t cap() const { return cap_; }
     bool alloc(int64_t n, int64_t *off) {
         n = std::max<int64_t>(n, 1);
-        auto take = [&](std::map<int64_t, int64_t>::iterator it, int64_t at) {
-            // [at, at + n) lies inside the free range it
-            const int64_t lo = it->first, len = it->second;
-            free_.erase(it);
-            if (at > lo) free_[lo] = at - lo;
-            if (lo + len > at + n) free_[at + n] = lo + len - (at + n);
-            *off = at;
-            cursor_ = at + n;
-        };
-        if (next_fit_) {
-            // a free range holding the cursor, then ranges after it, then from the start
-            auto it = free_.upper_bound(cursor_);
-            if (it != free_.begin()) {
-                auto pv = std::prev(it);
-                if (pv->first + pv->second >= cursor_ + n) {
-                    take(pv, std::max(pv->first, cursor_));
-                    return true;
-                }
-            }
-            for (auto jt = it; jt != free_.end(); ++jt)
-                if (jt->second >= n) {
-                    take(jt, jt->first);
-                    return true;
-                }
-        }
         for (auto it = free_.begin(); it != free_.end(); ++it)
             if (it->second >= n) {
-                take(it, it->first);
+                const int64_t lo = it->first, len = it->second;
+                free_.erase(it);
+                if (len > n) free_[lo + n] = len - n;
+                *off = lo;
                 return true;
             }
         return false;
@@ -130,8 +102,7 @@ public:
 
 private:
     std::map<int64_t, int64_t> free_;
-    int64_t cap_ = 0, cursor_ = 0;
-    bool next_fit_ = false;
+    int64_t cap_ = 0;
 };
 
 struct Query {
@@ -145,15 +116,13 @@ struct Query {
 
 struct Slot {
     bool busy = false;
-    bool planned = false;
     int round = 1;               // 1: the most promising corpus trees; 2: what may still beat them
     bool need_post = false;      // a planned next round waits for device room
     std::vector<uint8_t> inc;    // corpus trees computed in this round
     uint64_t ticket = 0;
     int64_t seq = 0;
     int32_t gen = 0;
-    int32_t rec = -1;            // mailbox record of the posted round
-    int64_t dt_off = 0, dt_n = 0, u_off = 0, u_n = 0, t_off = 0, t_n = 0, e_off = 0, e_n = 0;
+    int64_t dt_off = 0, dt_n = 0, i_off = 0, i_n = 0;  // table pool and item pool ranges
     QPlan plan;
 };
 
@@ -168,24 +137,20 @@ struct ServeState {
     // device
     std::vector<void *> dev_allocs;
     int2 *d_node = nullptr;
-    int32_t *d_krd = nullptr, *d_cumw = nullptr, *d_first = nullptr, *d_state = nullptr, *d_ctl = nullptr,
-            *d_mbox = nullptr, *d_slot = nullptr, *d_err = nullptr, *d_scratch = nullptr, *d_dt = nullptr;
+    int32_t *d_krd = nullptr, *d_cumw = nullptr, *d_ctl = nullptr, *d_slot = nullptr, *d_err = nullptr,
+            *d_scratch = nullptr, *d_dt = nullptr;
     XRun *d_runs = nullptr;
     XChunk *d_chunks = nullptr;
     XPair *d_pairs = nullptr;
-    XEntry *d_entries = nullptr;
-    XUnit *d_units = nullptr;
-    XTask *d_tasks = nullptr;
-    unsigned long long *d_rq = nullptr;
+    XChunkX *d_chunkx = nullptr;
+    XItem *d_items = nullptr;
+    unsigned long long *d_lists = nullptr;
     int32_t *h_results = nullptr, *h_flags = nullptr;  // mapped pinned host memory
-    Extents dt_ext, u_ext, t_ext, e_ext;
-    int rq_log2 = 12;
+    Extents dt_ext, i_ext;
     XKernelParams K{};
     cudaStream_t ks = nullptr, cs = nullptr;
     cudaEvent_t kev = nullptr;
     bool running = false;
-    int32_t posted = 0;
-    int32_t top_written = -1;
     // requests
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
@@ -212,7 +177,7 @@ struct ServeState {
 namespace {
 
 constexpr int kMaxPending = 1 << 16;
-constexpr int64_t kUnitCap = 24 << 20, kTaskCap = 12 << 20, kEntryCap = 2 << 20;
+constexpr int64_t kItemCap = 24 << 20;
 constexpr int64_t kDtCapMax = (int64_t)4 << 30;  // int32 elements (16 GiB)
 
 template <class T>
@@ -245,99 +210,87 @@ void free_all(ServeState *s) {
     s->ks = s->cs = nullptr;
 }
 
+// Table-pool elements of a planned query: tables, hand-off words, export maps
+// (whole 16-byte pieces, so every query's tables start on one).
+int64_t pool_elems(const QPlan &p) {
+    const int64_t n = std::max<int64_t>(p.dt_elems + p.words + (int64_t)p.smap.size(), 1);
+    return (n + XTED_PITCH - 1) / XTED_PITCH * XTED_PITCH;
+}
+
 // Reserves device room for a planned query; false if it does not fit now.
 bool reserve(ServeState *s, Slot &sl) {
     const QPlan &p = sl.plan;
-    sl.dt_n = std::max<int64_t>(p.dt_elems, 1);
-    sl.u_n = std::max<int64_t>((int64_t)p.units.size(), 1);
-    sl.t_n = std::max<int64_t>((int64_t)p.tasks.size(), 1);
-    sl.e_n = std::max<int64_t>((int64_t)p.entries.size(), 1);
+    sl.dt_n = pool_elems(p);
+    sl.i_n = std::max<int64_t>((int64_t)p.items.size(), 1);
     if (!s->dt_ext.alloc(sl.dt_n, &sl.dt_off)) return false;
-    if (!s->u_ext.alloc(sl.u_n, &sl.u_off)) {
+    if (!s->i_ext.alloc(sl.i_n, &sl.i_off)) {
         s->dt_ext.release(sl.dt_off, sl.dt_n);
-        return false;
-    }
-    if (!s->t_ext.alloc(sl.t_n, &sl.t_off)) {
-        s->dt_ext.release(sl.dt_off, sl.dt_n);
-        s->u_ext.release(sl.u_off, sl.u_n);
-        return false;
-    }
-    if (!s->e_ext.alloc(sl.e_n, &sl.e_off)) {
-        s->dt_ext.release(sl.dt_off, sl.dt_n);
-        s->u_ext.release(sl.u_off, sl.u_n);
-        s->t_ext.release(sl.t_off, sl.t_n);
         return false;
     }
     return true;
 }
 
 bool never_fits(ServeState *s, const QPlan &p) {
-    return p.dt_elems > s->dt_ext.cap() || (int64_t)p.units.size() > s->u_ext.cap() ||
-           (int64_t)p.tasks.size() > s->t_ext.cap() || (int64_t)p.entries.size() > s->e_ext.cap();
+    return pool_elems(p) > s->dt_ext.cap() || (int64_t)p.items.size() > s->i_ext.cap();
 }
 
 void release_extents(ServeState *s, Slot &sl) {
     s->dt_ext.release(sl.dt_off, sl.dt_n);
-    s->u_ext.release(sl.u_off, sl.u_n);
-    s->t_ext.release(sl.t_off, sl.t_n);
-    s->e_ext.release(sl.e_off, sl.e_n);
-    sl.dt_n = sl.u_n = sl.t_n = sl.e_n = 0;
+    s->i_ext.release(sl.i_off, sl.i_n);
+    sl.dt_n = sl.i_n = 0;
 }
 
 void release(ServeState *s, Slot &sl) {
-    s->dt_ext.release(sl.dt_off, sl.dt_n);
-    s->u_ext.release(sl.u_off, sl.u_n);
-    s->t_ext.release(sl.t_off, sl.t_n);
-    s->e_ext.release(sl.e_off, sl.e_n);
+    release_extents(s, sl);
     sl = Slot{};
 }
 
-// Fixes the plan up to its device offsets and copies it, its slot words and
-// a mailbox record to the device, in that order, on the copy stream.
+// Fixes the plan up to its device offsets, clears its tables, and copies it,
+// its slot words and last its list word to the device, in that order, on the
+// copy stream.
 int post(ServeState *s, int slot, Slot &sl) {
     QPlan &p = sl.plan;
     const int T = s->T;
     const int64_t pair_base = (int64_t)slot * T;
-    serve_fixup(p, slot, T, sl.dt_off, sl.u_off, sl.t_off, sl.e_off, (int32_t)((-sl.seq) & (XTED_BUCKETS - 1)));
+    serve_fixup_items(s->pools, p, slot, sl.dt_off);
     const ServePools &H = s->pools;
     const DTree &Q = H.trees[(size_t)(T + slot)];
     const size_t nb = 2 * (size_t)Q.nbase, n2 = 2 * (size_t)Q.n;
     cudaStream_t st = s->cs;
-    const std::vector<int32_t> zeros(XTED_ESTATE * p.entries.size(), 0);
-    std::vector<int32_t> first_held;  // test hook: one computed pair's level 0 is never published
-    if (s->c->fault == XTED_FAULT_HOLD_PAIR) {
-        first_held = p.first;
-        for (int32_t &f : first_held)
-            if (f >= 0) {
-                f = -1;
-                break;
-            }
+    const int32_t words[2] = {(int32_t)p.items.size(), sl.gen};
+    if (s->c->fault == XTED_FAULT_HOLD_PAIR) {  // test hook: one computed pair is never computed
+        const int32_t held = p.items[0].pair;
+        p.items.erase(std::remove_if(p.items.begin(), p.items.end(), [&](const XItem &i) { return i.pair == held; }),
+                      p.items.end());
         s->c->fault = 0;
     }
-    const std::vector<int32_t> &first = first_held.empty() ? p.first : first_held;
-    const int32_t words[2] = {p.need, sl.gen};
-    const int32_t rec[4] = {slot, (int32_t)pair_base, T, 0};
-    const int32_t posted = s->posted + 1;
+    const unsigned long long list =
+        ((unsigned long long)(sl.i_off + (int64_t)p.items.size()) << 32) | (unsigned long long)sl.i_off;
+    const int32_t age = (int32_t)sl.seq;
     int rc = XTED_OK;
+    if (cudaMemsetAsync(s->d_dt + sl.dt_off, 0xff, (size_t)(p.dt_elems + p.words) * 4, st) != cudaSuccess)
+        rc = XTED_ECUDA;
+    rc |= upload(s->d_dt + sl.dt_off + p.dt_elems + p.words, p.smap.data(), p.smap.size() * 4, st);
     rc |= upload(s->d_node + nb, H.node.data() + nb, n2 * sizeof(int2), st);
     rc |= upload(s->d_krd + nb, H.krd.data() + nb, n2 * 4, st);
     rc |= upload(s->d_cumw + nb, H.cumw.data() + nb, n2 * 4, st);
     rc |= upload(s->d_runs + nb, H.runs.data() + nb, n2 * sizeof(XRun), st);
     rc |= upload(s->d_chunks + nb, H.chunks.data() + nb, n2 * sizeof(XChunk), st);
+    rc |= upload(s->d_chunkx + nb, H.chunkx.data() + nb, n2 * sizeof(XChunkX), st);
     rc |= upload(s->d_pairs + pair_base, p.pairs.data(), p.pairs.size() * sizeof(XPair), st);
-    rc |= upload(s->d_first + pair_base, first.data(), first.size() * 4, st);
-    rc |= upload(s->d_entries + sl.e_off, p.entries.data(), p.entries.size() * sizeof(XEntry), st);
-    rc |= upload(s->d_state + XTED_ESTATE * sl.e_off, zeros.data(), zeros.size() * 4, st);
-    rc |= upload(s->d_units + sl.u_off, p.units.data(), p.units.size() * sizeof(XUnit), st);
-    rc |= upload(s->d_tasks + sl.t_off, p.tasks.data(), p.tasks.size() * sizeof(XTask), st);
+    rc |= upload(s->d_items + sl.i_off, p.items.data(), p.items.size() * sizeof(XItem), st);
     rc |= upload(s->d_slot + XTED_SERVE_SLOTS + slot, &words[0], 4, st);      // slot_need
     rc |= upload(s->d_slot + 2 * XTED_SERVE_SLOTS + slot, &words[1], 4, st);  // slot_gen
-    rc |= upload(s->d_mbox + XTED_MBOX_REC + 4 * (s->posted & (XTED_SERVE_RECS - 1)), rec, sizeof(rec), st);
-    rc |= upload(s->d_mbox + XTED_MBOX_POSTED, &posted, 4, st);
-    if (rc) return XTED_ECUDA;
-    sl.rec = s->posted;
-    s->posted = posted;
-    return XTED_OK;
+    rc |= upload(s->d_slot + 3 * XTED_SERVE_SLOTS + slot, &age, 4, st);
+    rc |= upload(s->d_lists + slot, &list, sizeof(list), st);
+    return rc ? XTED_ECUDA : XTED_OK;
+}
+
+// Empties a slot's list, so that no launch claims the rest of it.
+void close_list(ServeState *s, int slot) {
+    if (cudaMemset(s->d_lists + slot, 0, sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMemset(s->d_slot + slot, 0, 4) != cudaSuccess)
+        cudaGetLastError();
 }
 
 // Finishes a query from its known distances: every corpus tree not computed
@@ -426,13 +379,6 @@ void first_round(ServeState *s, const Query &q, std::vector<int32_t> &lb, std::v
     prune_round1(lb, dist, std::max<size_t>((size_t)s->first_round, 4 * (size_t)q.k), level > 0, inc);
 }
 
-int64_t oldest_seq(ServeState *s) {
-    int64_t o = INT64_MAX;
-    for (const Slot &sl : s->slots)
-        if (sl.busy && sl.planned) o = std::min(o, sl.seq);  // between rounds too: its bucket stays its own
-    return o;
-}
-
 void fail_inflight(ServeState *s, int code) {
     for (int i = 0; i < s->S; i++) {
         Slot &sl = s->slots[i];
@@ -467,18 +413,16 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
             if (sl.plan.trivial[(size_t)t] < 0 && sl.inc[(size_t)t]) q.dist[(size_t)t] = res[t];
         if (sl.round == 1 && s->prune > 0) {
             std::vector<uint8_t> inc2;
-            if (prune_round2(q.lb, q.dist, q.k, inc2)) {  // plan round 2 in the same slot (its bucket stays reserved)
+            if (prune_round2(q.lb, q.dist, q.k, inc2)) {  // plan round 2 in the same slot
                 release_extents(s, sl);
                 sl.gen = 0;
                 sl.round = 2;
                 sl.inc = std::move(inc2);
                 Query qcopy = q;
-                const int wr = s->c->opts.wide_rows;
                 lk.unlock();
                 const double t1 = now_ms();
-                serve_plan_query(s->pools, i, qcopy.lab.data(), qcopy.off.data(), qcopy.idx.data(), qcopy.n,
-                                 s->c->opts.orientation, s->c->opts.narrow_width, wr > 0 ? wr : -1, sl.plan,
-                                 sl.inc.data());
+                serve_plan_items(s->pools, i, qcopy.lab.data(), qcopy.off.data(), qcopy.idx.data(), qcopy.n,
+                                 s->c->opts.orientation, sl.plan, sl.inc.data());
                 const double t2 = now_ms();
                 lk.lock();
                 s->plan_us += (int64_t)((t2 - t1) * 1e3);
@@ -516,55 +460,45 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
     const cudaError_t kq = s->running ? cudaEventQuery(s->kev) : cudaErrorNotReady;
     if (s->running && kq == cudaSuccess) {
         s->running = false;
-        int32_t err = 0, cons = 0;
-        if (cudaMemcpy(&err, s->d_err, 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
-            cudaMemcpy(&cons, s->d_mbox + XTED_MBOX_CONSUMED, 4, cudaMemcpyDeviceToHost) != cudaSuccess)
-            err = XTED_ECUDA;
-        int32_t consumed = cons & ~XTED_MBOX_CLOSED;
+        int32_t err = 0;
+        if (cudaMemcpy(&err, s->d_err, 4, cudaMemcpyDeviceToHost) != cudaSuccess) err = XTED_ECUDA;
+        cudaStreamSynchronize(s->cs);  // every list posted so far is in place
         if (err != 0) {
             s->error = err;
             fail_inflight(s, err);
             cudaMemset(s->d_err, 0, 8 * sizeof(int32_t));
-            cudaMemset(s->d_slot, 0, XTED_SERVE_SLOTS * sizeof(int32_t));
-            // records of the failed queries are void: the next launch starts after them
-            cudaStreamSynchronize(s->cs);
-            consumed = s->posted;
+            for (int i = 0; i < s->S; i++) close_list(s, i);  // what is left of them is void
             s->cv_done.notify_all();
             progress = true;
         } else {
-            // Every query whose record this launch claimed has finished: a
-            // launch leaves only when all of its blocks are idle. One that
-            // has not (its work was lost) fails instead of waiting forever.
+            // A launch leaves only when every warp is idle, so a query whose
+            // items were all claimed has finished. One that has not (its work
+            // was lost) fails instead of waiting forever; one with items left
+            // goes on in the next launch.
+            unsigned long long lists[XTED_SERVE_SLOTS] = {};
+            if (cudaMemcpy(lists, s->d_lists, sizeof(lists), cudaMemcpyDeviceToHost) != cudaSuccess) cudaGetLastError();
             for (int i = 0; i < s->S; i++) {
                 Slot &sl = s->slots[i];
-                if (!sl.busy || sl.gen == 0 || sl.rec < 0 || sl.rec >= consumed) continue;
+                if (!sl.busy || sl.gen == 0) continue;
                 if (((volatile int32_t *)s->h_flags)[i] == sl.gen) continue;  // done: step 1 takes it
+                if ((uint32_t)lists[i] < (uint32_t)(lists[i] >> 32)) continue;
                 if (std::getenv("XTED_SERVE_DEBUG")) {
                     int32_t done = -1;
                     cudaMemcpy(&done, s->d_slot + i, 4, cudaMemcpyDeviceToHost);
                     std::fprintf(stderr,
-                                 "xted serve: launch %lld ended with slot %d unfinished: round %d gen %d rec %d "
-                                 "consumed %d posted %d need %d done %d flag %d\n",
-                                 (long long)s->launches, i, sl.round, sl.gen, sl.rec, consumed, s->posted,
-                                 sl.plan.need, done, ((volatile int32_t *)s->h_flags)[i]);
+                                 "xted serve: launch %lld ended with slot %d unfinished: round %d gen %d items %zu "
+                                 "done %d flag %d\n",
+                                 (long long)s->launches, i, sl.round, sl.gen, sl.plan.items.size(), done,
+                                 ((volatile int32_t *)s->h_flags)[i]);
                 }
                 auto it = s->queries.find(sl.ticket);
                 if (it != s->queries.end()) it->second.state = XTED_ETIMEOUT;
                 s->error = XTED_ETIMEOUT;
-                const int32_t zero = 0;  // the slot's finished-pair count restarts for its next query
-                if (cudaMemcpy(s->d_slot + i, &zero, 4, cudaMemcpyHostToDevice) != cudaSuccess) cudaGetLastError();
+                close_list(s, i);  // the slot's finished-item count restarts for its next query
                 release(s, sl);
                 s->cv_done.notify_all();
                 progress = true;
             }
-        }
-        // reopen the claim word for the next launch
-        if (cons != consumed &&
-            cudaMemcpy(s->d_mbox + XTED_MBOX_CONSUMED, &consumed, 4, cudaMemcpyHostToDevice) != cudaSuccess) {
-            cudaGetLastError();
-            s->error = XTED_ECUDA;
-            fail_inflight(s, XTED_ECUDA);
-            s->cv_done.notify_all();
         }
     } else if (s->running && kq != cudaErrorNotReady) {
         cudaGetLastError();
@@ -587,8 +521,6 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
             if (s->slots[i].busy && s->slots[i].ticket == ticket) slot = i;
         if (slot < 0) {
             const int64_t seq = s->next_seq;
-            const int64_t old = oldest_seq(s);
-            if (old != INT64_MAX && seq - old >= XTED_BUCKETS) break;  // keep buckets distinct by age
             for (int i = 0; i < s->S && slot < 0; i++)
                 if (!s->slots[i].busy) slot = i;
             if (slot < 0) break;
@@ -604,10 +536,8 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
             std::vector<uint8_t> inc;
             first_round(s, qcopy, lb, dist, inc);
             const double t1 = now_ms();
-            const int wr = s->c->opts.wide_rows;
-            serve_plan_query(s->pools, slot, qcopy.lab.data(), qcopy.off.data(), qcopy.idx.data(), qcopy.n,
-                             s->c->opts.orientation, s->c->opts.narrow_width, wr > 0 ? wr : -1,
-                             sl.plan, inc.data());
+            serve_plan_items(s->pools, slot, qcopy.lab.data(), qcopy.off.data(), qcopy.idx.data(), qcopy.n,
+                             s->c->opts.orientation, sl.plan, inc.data());
             const double t2 = now_ms();
             lk.lock();
             s->bound_us += (int64_t)((t1 - t0) * 1e3);
@@ -617,7 +547,6 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
             q.dist = std::move(dist);
             sl.inc = std::move(inc);
             sl.round = 1;
-            sl.planned = true;
             progress = true;
         }
         Slot &sl = s->slots[slot];
@@ -651,20 +580,11 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
         q.t_admit = now_ms();
         progress = true;
     }
-    // 4. priority: the oldest query in flight goes first
-    const int64_t old = oldest_seq(s);
-    if (old != INT64_MAX) {
-        const int32_t top = (int32_t)((-old) & (XTED_BUCKETS - 1));
-        if (top != s->top_written) {
-            s->top_written = top;
-            cudaMemcpyAsync(s->d_mbox + XTED_MBOX_TOP, &top, 4, cudaMemcpyHostToDevice, s->cs);
-        }
-    }
-    // 5. keep a launch running while queries are in flight
+    // 4. keep a launch running while queries are in flight
     bool inflight = false;
     for (const Slot &sl : s->slots) inflight |= sl.busy && sl.gen != 0;
     if (inflight && !s->running && s->stop) {
-        // shutting down: a query whose record no launch claimed is not started again
+        // shutting down: a query that its launch has not finished is not started again
         for (int i = 0; i < s->S; i++) {
             Slot &sl = s->slots[i];
             if (!sl.busy || sl.gen == 0) continue;
@@ -677,10 +597,8 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
         return true;
     }
     if (inflight && !s->running) {
-        // every earlier launch ended with all of its work done: start from empty rings
         cudaStreamSynchronize(s->cs);
-        bool ok = cudaMemsetAsync(s->d_rq, 0xff, ((size_t)XTED_RINGS << s->rq_log2) * 8, s->ks) == cudaSuccess &&
-                  cudaMemsetAsync(s->d_ctl, 0, (2 * XTED_RINGS + 8) * 4, s->ks) == cudaSuccess &&
+        bool ok = cudaMemsetAsync(s->d_ctl, 0, XTED_CTL_INTS * 4, s->ks) == cudaSuccess &&
                   launch_dp(s->K, s->c->grid, s->ks) == cudaSuccess &&
                   cudaEventRecord(s->kev, s->ks) == cudaSuccess;
         if (!ok) {
@@ -721,7 +639,7 @@ void stop_worker(ServeState *s) {
         for (Slot &sl : s->slots)
             if (sl.busy && sl.gen == 0) sl = Slot{};  // planned but never posted
         const int32_t one = 1;
-        if (s->cs) cudaMemcpyAsync(s->d_mbox + XTED_MBOX_STOP, &one, 4, cudaMemcpyHostToDevice, s->cs);
+        if (s->cs) cudaMemcpyAsync(s->d_ctl + XTED_CTL_STOP, &one, 4, cudaMemcpyHostToDevice, s->cs);
     }
     s->cv_work.notify_all();
     if (s->worker.joinable()) s->worker.join();
@@ -763,9 +681,6 @@ int load(xted_ctx *c, ServeState *s, const xted_tree *tr, int32_t ntrees) {
     const ServePools &H = s->pools;
     const size_t n2 = H.node.size();
     // device memory
-    int rq_log2 = 12;
-    while (((int64_t)1 << rq_log2) < 4 * (int64_t)XTED_SERVE_SLOTS * std::max(T, 1)) rq_log2++;
-    s->rq_log2 = rq_log2;
     int64_t dt_cap = std::min<int64_t>(kDtCapMax, (int64_t)S * Qm * std::max<int64_t>(nonempty, 1));
     if (c->opts.mem_limit > 0) dt_cap = std::min<int64_t>(dt_cap, c->opts.mem_limit / 8);  // half of the limit
     dt_cap = std::max<int64_t>(dt_cap, 1);
@@ -776,24 +691,16 @@ int load(xted_ctx *c, ServeState *s, const xted_tree *tr, int32_t ntrees) {
     rc |= dev_alloc(s, &s->d_runs, n2);
     rc |= dev_alloc(s, &s->d_chunks, n2);
     rc |= dev_alloc(s, &s->d_pairs, (size_t)S * T);
-    rc |= dev_alloc(s, &s->d_first, (size_t)S * T);
-    rc |= dev_alloc(s, &s->d_entries, (size_t)kEntryCap);
-    rc |= dev_alloc(s, &s->d_state, XTED_ESTATE * (size_t)kEntryCap);
-    rc |= dev_alloc(s, &s->d_units, (size_t)kUnitCap);
-    rc |= dev_alloc(s, &s->d_tasks, (size_t)kTaskCap);
-    rc |= dev_alloc(s, &s->d_rq, (size_t)XTED_RINGS << rq_log2);
-    rc |= dev_alloc(s, &s->d_ctl, 2 * XTED_RINGS + 8);
-    rc |= dev_alloc(s, &s->d_mbox, XTED_MBOX_INTS);
-    rc |= dev_alloc(s, &s->d_slot, 3 * XTED_SERVE_SLOTS);
+    rc |= dev_alloc(s, &s->d_chunkx, n2);
+    rc |= dev_alloc(s, &s->d_items, (size_t)kItemCap);
+    rc |= dev_alloc(s, &s->d_lists, XTED_SERVE_SLOTS);
+    rc |= dev_alloc(s, &s->d_ctl, XTED_CTL_INTS);
+    rc |= dev_alloc(s, &s->d_slot, 4 * XTED_SERVE_SLOTS);
     rc |= dev_alloc(s, &s->d_err, 8);
-    rc |= dev_alloc(s, &s->d_dt, (size_t)dt_cap);
-    // per-block scratch: far-row stacks, and rows of the wide paths for queries up to Qmax columns
-    const int64_t sr = H.stack_rows;
-    int64_t per = sr * (XTED_WARPS * XTED_NARROW_MAX);
-    per = std::max<int64_t>(per, sr * std::min(Qm, XTED_WIDE_REG_MAX));
-    if (Qm > XTED_WIDE_REG_MAX) per = std::max<int64_t>(per, xted_wide_big_scratch(Qm, sr));
-    per = (per + 63) / 64 * 64;
-    rc |= dev_alloc(s, &s->d_scratch, (size_t)per * (size_t)c->grid);
+    rc |= dev_alloc(s, &s->d_dt, (size_t)dt_cap + XTED_SW);  // (slack: see ctx_prepare)
+    // per-warp scratch: the far-row stack's rows outside the shared window
+    const int64_t per = (int64_t)H.stack_rows * XTED_SW;
+    rc |= dev_alloc(s, &s->d_scratch, (size_t)per * (size_t)c->grid * XTED_FLOW_WARPS);
     if (rc) return XTED_ENOMEM;
     if (cudaHostAlloc((void **)&s->h_results, sizeof(int32_t) * std::max<size_t>((size_t)S * T, 1),
                       cudaHostAllocMapped) != cudaSuccess ||
@@ -816,16 +723,15 @@ int load(xted_ctx *c, ServeState *s, const xted_tree *tr, int32_t ntrees) {
         upload(s->d_krd, H.krd.data(), ncorp * 4, s->cs) || upload(s->d_cumw, H.cumw.data(), ncorp * 4, s->cs) ||
         upload(s->d_runs, H.runs.data(), ncorp * sizeof(XRun), s->cs) ||
         upload(s->d_chunks, H.chunks.data(), ncorp * sizeof(XChunk), s->cs) ||
-        cudaMemsetAsync(s->d_mbox, 0, XTED_MBOX_INTS * 4, s->cs) != cudaSuccess ||
-        cudaMemsetAsync(s->d_slot, 0, 3 * XTED_SERVE_SLOTS * 4, s->cs) != cudaSuccess ||
+        cudaMemsetAsync(s->d_lists, 0, XTED_SERVE_SLOTS * 8, s->cs) != cudaSuccess ||
+        cudaMemsetAsync(s->d_slot, 0, 4 * XTED_SERVE_SLOTS * 4, s->cs) != cudaSuccess ||
+        cudaMemsetAsync(s->d_ctl, 0, XTED_CTL_INTS * 4, s->cs) != cudaSuccess ||
         cudaMemsetAsync(s->d_err, 0, 8 * 4, s->cs) != cudaSuccess || cudaStreamSynchronize(s->cs) != cudaSuccess) {
         cudaGetLastError();
         return XTED_ECUDA;
     }
     s->dt_ext.reset(dt_cap);
-    s->u_ext.reset(kUnitCap);
-    s->t_ext.reset(kTaskCap);
-    s->e_ext.reset(kEntryCap, true);  // entry ids: reused as late as possible
+    s->i_ext.reset(kItemCap);
     XKernelParams &K = s->K;
     std::memset(&K, 0, sizeof(K));
     K.rowinfo = s->d_node;
@@ -834,22 +740,15 @@ int load(xted_ctx *c, ServeState *s, const xted_tree *tr, int32_t ntrees) {
     K.runs = s->d_runs;
     K.chunks = s->d_chunks;
     K.pairs = s->d_pairs;
-    K.units = s->d_units;
-    K.tasks = s->d_tasks;
-    K.entries = s->d_entries;
-    K.first = s->d_first;
-    K.dt = s->d_dt;
+    K.chunkx = s->d_chunkx;
+    K.items = s->d_items;
+    K.dt = K.buf = s->d_dt;
+    K.smap = s->d_dt;
     K.scratch = s->d_scratch;
-    K.scratch_per_cta = per;
+    K.scratch_per_warp = per;
     K.stack_rows = H.stack_rows;
-    K.ntasks = INT32_MAX;
-    K.nentries = (int32_t)kEntryCap;
     K.npairs = S * T;
-    K.entry_state = s->d_state;
-    K.rq = s->d_rq;
-    K.rq_log2 = rq_log2;
-    K.rq_ctl = s->d_ctl;
-    K.done_total = s->d_ctl + 2 * XTED_RINGS;
+    K.progress = s->d_ctl + XTED_CTL_PROGRESS;
     K.error = s->d_err;
     K.error_info = s->d_err + 1;
     K.timeout_ns = (uint64_t)(c->opts.wait_timeout_s * 1e9);
@@ -857,7 +756,9 @@ int load(xted_ctx *c, ServeState *s, const xted_tree *tr, int32_t ntrees) {
     K.serve = 1;
     K.serve_pairs = T;
     K.idle_exit_ns = 2000000;  // 2 ms
-    K.mbox = s->d_mbox;
+    K.lists = s->d_lists;
+    K.ages = s->d_slot + 3 * XTED_SERVE_SLOTS;
+    K.ctl = s->d_ctl;
     K.slot_done = s->d_slot;
     K.slot_need = s->d_slot + XTED_SERVE_SLOTS;
     K.slot_gen = s->d_slot + 2 * XTED_SERVE_SLOTS;

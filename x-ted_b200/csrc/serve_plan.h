@@ -15,6 +15,8 @@
 #include <vector>
 
 #include "../../include/xted.h"
+#include "flow_plan.h"
+#include "plan.h"
 #include "plan_core.h"
 
 namespace xted {
@@ -30,13 +32,15 @@ struct ServePools {
     std::vector<XChunk> chunks;
     std::vector<DDepth> depths;
     std::vector<DOTree> otrees;
+    std::vector<XChunkX> chunkx;
     PlanPools P{};
     int32_t stack_rows = 1;  // far-row stack rows any pair needs (corpus rows)
 };
 
-// A planned query. Offsets are relative (pairs from 0, entries, units and
-// tasks from 0, tables from 0) until serve_fixup moves them to the slot's
-// device ranges.
+// A planned query. Offsets are relative (pairs, items, tables, hand-off words
+// and export maps from 0) until serve_fixup_items moves them to the slot's
+// device ranges; likewise entries, units and tasks (the per-level view of the
+// same tables that the planner's CPU emulation runs) and serve_fixup.
 struct QPlan {
     std::vector<XPair> pairs;     // [T]
     std::vector<int32_t> first;   // [T] level-0 entry, -1 for an empty-tree pair
@@ -44,6 +48,9 @@ struct QPlan {
     std::vector<XEntry> entries;
     std::vector<XUnit> units;
     std::vector<XTask> tasks;
+    std::vector<XItem> items;     // the launch's items, in list order
+    std::vector<int32_t> smap;    // export maps of the query's striped chunks
+    int64_t words = 0;            // hand-off words of striped units
     int64_t dt_elems = 0, cells = 0;
     int32_t need = 0;             // pairs the device computes
 };
@@ -103,6 +110,7 @@ inline void serve_pools_build(ServePools &s, const xted_tree *tr, int T, int S, 
     s.chunks.assign(n2, XChunk{0, 0, 0, 0});
     s.depths.assign(2 * (n1 + (size_t)(T + S)), DDepth{});
     s.otrees.assign(2 * (size_t)(T + S), DOTree{});
+    s.chunkx.assign(n2, XChunkX{1, 0, 0, 0, 0});
     PlanPools &P = s.P;
     P.raw = s.raw.data();
     P.trees = s.trees.data();
@@ -130,18 +138,23 @@ inline void serve_pools_build(ServePools &s, const xted_tree *tr, int T, int S, 
         tree_basic(P, t, s.trees.data());
         orient_tree(P, 2 * t);
         orient_tree(P, 2 * t + 1);
-        for (int o = 0; o < 2; o++) s.stack_rows = std::max(s.stack_rows, s.otrees[2 * (size_t)t + o].maxka + 1);
+        for (int o = 0; o < 2; o++) {
+            const DOTree &O = s.otrees[2 * (size_t)t + o];
+            s.stack_rows = std::max(s.stack_rows, O.maxka + 1);
+            for (int d = 0; d <= O.D; d++)  // corpus trees are row trees only: their depths' rows
+                flow_depth_totals(s.depths[(size_t)(O.depth_base + d)], P.runs, P.cumw, s.chunkx.data());
+        }
     }
 }
 
-// Plans query (lab, off, idx, n <= Qmax, valid) in slot `slot`: the tree into
-// the slot's region, then every (corpus tree, query) pair as the batch
-// planner does (k_pair_setup ... k_level_fill in prep.cu); with `include`,
+// Query (lab, off, idx, n <= Qmax, valid) in slot `slot`: the tree into the
+// slot's region, then every (corpus tree, query) pair as the batch planner
+// sets it up (k_pair_setup ... in prep.cu) and its levels; with `include`,
 // only the pairs of the corpus trees it marks (pairs with an empty tree are
 // always answered on the host).
-inline void serve_plan_query(ServePools &s, int slot, const int32_t *lab, const int32_t *off, const int32_t *idx,
-                             int n, int orientation, int narrow_width, int wide_rows, QPlan &out,
-                             const uint8_t *include = nullptr) {
+inline void serve_plan_pairs(ServePools &s, int slot, const int32_t *lab, const int32_t *off, const int32_t *idx,
+                             int n, int orientation, QPlan &out, const uint8_t *include, std::vector<DPair> &dp,
+                             std::vector<DLevel> &lv) {
     const int T = s.T, tq = T + slot;
     DTree &Q = s.trees[(size_t)tq];
     Q.n = n;
@@ -158,11 +171,11 @@ inline void serve_plan_query(ServePools &s, int slot, const int32_t *lab, const 
     orient_tree(s.P, 2 * tq + 1);
 
     out = QPlan{};
-    std::vector<DPair> dp((size_t)T);
+    dp.resize((size_t)T);
     out.pairs.resize((size_t)T);
     out.first.assign((size_t)T, -1);
     out.trivial.assign((size_t)T, -1);
-    std::vector<DLevel> lv;
+    lv.clear();
     int64_t dt = 0;
     for (int t = 0; t < T; t++) {
         const int32_t pt[2] = {t, tq};
@@ -180,7 +193,8 @@ inline void serve_plan_query(ServePools &s, int slot, const int32_t *lab, const 
         x.n = n;
         x.row_base = s.otrees[2 * (size_t)t + d.o].node_base;
         x.col_base = s.otrees[2 * (size_t)tq + d.o].node_base;
-        dt += (int64_t)x.m * x.n;
+        x.pitch = table_pitch(n);
+        dt += (int64_t)x.m * x.pitch;
         d.lvl_base = (int32_t)lv.size();
         out.first[(size_t)t] = d.lvl_base;
         for (int l = 0; l < d.L; l++) {
@@ -193,6 +207,109 @@ inline void serve_plan_query(ServePools &s, int slot, const int32_t *lab, const 
         out.need++;
     }
     out.dt_elems = dt;
+}
+
+// Plans a query as the launch's items: the levels of all its pairs by the time
+// estimated to be left of their pair, longest first (a counting sort, so a
+// pair's levels stay in order), as k_level_order in prep.cu.
+inline void serve_plan_items(ServePools &s, int slot, const int32_t *lab, const int32_t *off, const int32_t *idx,
+                             int n, int orientation, QPlan &out, const uint8_t *include = nullptr) {
+    std::vector<DPair> dp;
+    std::vector<DLevel> lv;
+    serve_plan_pairs(s, slot, lab, off, idx, n, orientation, out, include, dp, lv);
+    const int tq = s.T + slot;
+    for (int o = 0; o < 2; o++) {
+        const DOTree &O = s.otrees[2 * (size_t)tq + o];
+        for (int d = 0; d <= O.D; d++) {
+            DDepth &dd = s.depths[(size_t)(O.depth_base + d)];
+            for (int32_t c = dd.chunk_lo; c < dd.chunk_lo + dd.nnarrow + dd.nhalf + dd.nwide; c++) {
+                const XChunk &ch = s.chunks[(size_t)c];
+                XChunkX &x = s.chunkx[(size_t)c];
+                x = XChunkX{chunk_stripes(ch, s.P.krd), 0, 0, 0, 0};
+                if (x.K > 1) {
+                    x.map = (int64_t)out.smap.size();
+                    out.smap.resize(out.smap.size() + (size_t)ch.width);
+                    x.X = chunk_export_map(ch, s.P.krd, s.P.node + O.node_base, &out.smap[(size_t)x.map]);
+                }
+            }
+            flow_depth_totals(dd, s.P.runs, s.P.cumw, s.chunkx.data());
+        }
+    }
+    const FlowCtx C{s.otrees.data(), s.depths.data(), s.P.runs, s.P.chunks, s.chunkx.data(), s.P.cumw};
+    const size_t E = lv.size();
+    std::vector<int64_t> items(E), words(E), rem(E);
+    parallel_for((int64_t)E, 4096, [&](int64_t lo, int64_t hi) {
+        for (int64_t e = lo; e < hi; e++) {
+            const DPair &q = dp[(size_t)lv[(size_t)e].pair];
+            flow_level_count(C, s.otrees[2 * (size_t)lv[(size_t)e].pair + q.o], s.otrees[2 * (size_t)tq + q.o],
+                             lv[(size_t)e].level, &items[(size_t)e], &words[(size_t)e], &rem[(size_t)e]);
+        }
+    });
+    int64_t chain_max = 1;
+    for (size_t e = E; e-- > 0;) {
+        if (e + 1 < E && lv[e + 1].pair == lv[e].pair) rem[e] += rem[e + 1];
+        chain_max = std::max(chain_max, rem[e]);
+    }
+    constexpr int B = 4096;
+    std::vector<int32_t> at(B + 1, 0), order(E);
+    auto bucket = [&](size_t e) { return B - 1 - (int)(rem[e] * (B - 1) / chain_max); };
+    for (size_t e = 0; e < E; e++) at[(size_t)bucket(e) + 1]++;
+    for (int b = 0; b < B; b++) at[(size_t)b + 1] += at[(size_t)b];
+    for (size_t e = 0; e < E; e++) order[(size_t)at[(size_t)bucket(e)]++] = (int32_t)e;
+    std::vector<int64_t> ioff(E), boff(E);
+    int64_t ni = 0, nw = 0;
+    for (int32_t e : order) {
+        ioff[(size_t)e] = ni;
+        boff[(size_t)e] = nw;
+        ni += items[(size_t)e];
+        nw += words[(size_t)e];
+    }
+    out.items.resize((size_t)ni);
+    out.words = nw;
+    parallel_for((int64_t)E, 256, [&](int64_t lo, int64_t hi) {
+        for (int64_t k = lo; k < hi; k++) {
+            const DLevel &L = lv[(size_t)k];
+            const DPair &q = dp[(size_t)L.pair];
+            const DOTree &A = s.otrees[2 * (size_t)L.pair + q.o], &Bt = s.otrees[2 * (size_t)tq + q.o];
+            int64_t i = ioff[(size_t)k], buf = boff[(size_t)k];
+            for (int a = std::min(A.D, L.level); a >= std::max(L.level - Bt.D, 0); a--) {
+                const DDepth &ra = s.depths[(size_t)(A.depth_base + a)];
+                const DDepth &cb = s.depths[(size_t)(Bt.depth_base + L.level - a)];
+                const int64_t cnt = (int64_t)(ra.run_hi - ra.run_lo) * cb.nitems;
+                for (int64_t x = 0; x < cnt; x++) out.items[(size_t)(i++)] = flow_item(C, ra, cb, L.pair, x, buf);
+                buf += (int64_t)ra.rows * cb.wsum;
+            }
+        }
+    });
+}
+
+// Moves a plan's items to their slot: pairs of slot `slot` start at slot * T;
+// the query's device range at `off` holds its tables, hand-off words and
+// export maps in that order.
+inline void serve_fixup_items(ServePools &s, QPlan &p, int slot, int64_t off) {
+    const int32_t pair_base = (int32_t)((int64_t)slot * s.T);
+    for (XPair &x : p.pairs) x.dt_off += off;
+    for (XItem &i : p.items) {
+        i.pair += pair_base;
+        i.buf += off + p.dt_elems;
+    }
+    for (int o = 0; o < 2; o++) {
+        const DOTree &O = s.otrees[2 * (size_t)(s.T + slot) + o];
+        if (O.D < 0) continue;
+        const DDepth &last = s.depths[(size_t)(O.depth_base + O.D)];
+        for (int32_t c = O.node_base; c < last.chunk_lo + last.nnarrow + last.nhalf + last.nwide; c++)
+            s.chunkx[(size_t)c].map += off + p.dt_elems + p.words;
+    }
+}
+
+// Plans a query level by level as entries, units and tasks (plan_core.h), the
+// view that the planner's CPU emulation checks and runs.
+inline void serve_plan_query(ServePools &s, int slot, const int32_t *lab, const int32_t *off, const int32_t *idx,
+                             int n, int orientation, int narrow_width, int wide_rows, QPlan &out,
+                             const uint8_t *include = nullptr) {
+    std::vector<DPair> dp;
+    std::vector<DLevel> lv;
+    serve_plan_pairs(s, slot, lab, off, idx, n, orientation, out, include, dp, lv);
     LevelCtx C;
     C.ot = s.otrees.data();
     C.depths = s.depths.data();

@@ -73,6 +73,8 @@ struct XPair {
     int32_t m, n;     // rows (A) and columns (B)
     int32_t row_base; // index of A's node 0 in the node-record pool
     int32_t col_base; // index of B's node 0 in the node-record pool
+    int32_t pitch;    // row pitch of the table: n rounded up to XTED_PITCH columns
+    int32_t pad;
 };
 
 struct XUnit {
@@ -160,65 +162,78 @@ struct XEntry {
     int32_t pad;
 };
 
+// ---- the DP launch (flow.cu) ----
+//
+// Every warp of the launch claims *items* from one list and runs each to its
+// end. An item is a unit (row run x chunk) or, for a single segment wider
+// than a warp holds, one column stripe of a unit. The list is sorted so that
+// an item only needs values of items before it: a unit of keyroot depths
+// (a, b) reads tables of depths (a', b') with a' <= a, b' <= b, and the
+// stripes of a unit go rightmost first. A warp that needs a value which is not
+// there yet waits for it: every word that one item writes for another starts
+// at -1 and is written once, with a value >= 0.
+#define XTED_PITCH 4          // rows of a table start on 16 bytes
+#define XTED_SW 512           // columns of a stripe: the widest slice one warp holds (16 per lane)
+#define XTED_FLOW_WARPS 4     // warps per block, each with its own shared memory
+
+struct XItem {
+    int32_t run, chunk, pair;
+    int32_t stripe;           // stripe of the unit's chunk (0 for a chunk one warp holds)
+    int64_t buf;              // striped unit: its hand-off words in XKernelParams::buf
+    int32_t pad[2];
+};
+
+// What a column chunk adds to the plan (same index as its XChunk).
+struct XChunkX {
+    int32_t K;     // stripes (1: one warp holds the chunk)
+    int32_t kpre;  // stripes of the chunks before it at its depth
+    int32_t X;     // columns that a stripe further left reads as far columns
+    int32_t wpre;  // hand-off words per row of the chunks before it at its depth
+    int64_t map;   // striped: its export map in XKernelParams::smap (width ints: export index or -1)
+};
+
 struct XKernelParams {
     const int2 *rowinfo;  // node records of every oriented tree
     const int32_t *krd;   // keyroots grouped by depth (node ids within their tree)
     const int32_t *cumw;  // position of each keyroot's segment in its depth's column list
     const XRun *runs;
     const XChunk *chunks;
+    const XChunkX *chunkx;
     const XPair *pairs;
-    const XUnit *units;
-    const XTask *tasks;
-    const XEntry *entries;
-    const int32_t *first;  // [npairs] level-0 entry of every pair, -1 for pairs with an empty tree
-    int32_t *dt;          // all distance tables
-    int32_t *scratch;     // per-block far-row stacks (and wide generic rows)
-    int64_t scratch_per_cta; // int32 elements
+    const XItem *items;
+    int32_t *dt;          // every pair's tree-distance savings, -1 = not computed yet
+    int32_t *buf;         // hand-off words of striped units, -1 = not written yet
+    const int32_t *smap;  // export maps of striped chunks
+    int32_t *scratch;     // per-warp far-row stacks: rows that left the shared window
+    int64_t scratch_per_warp;  // int32 elements
     int32_t stack_rows;   // stack capacity in rows
-    int32_t ntasks;
-    int32_t nentries, npairs;
-    int32_t *entry_state; // [XTED_ESTATE * nentries]: narrow claimed, group claimed, done
-    // Ring g's slots are rq[g << rq_log2 ...]; queue position pos lives in
-    // slot pos & (2^rq_log2 - 1) as (pos << 32 | entry), so a reader knows a
-    // slot holds position pos and not an older or not-yet-written one.
-    unsigned long long *rq;
-    int32_t rq_log2;
-    int32_t *rq_ctl;      // [2 * XTED_RINGS]: head, tail of each ring (unsigned positions), then counters
-    int32_t *done_total;  // finished tasks
+    int32_t nitems, npairs;
+    int32_t *next;        // items claimed (batch launch)
+    int32_t *progress;    // items finished
     int32_t *error;       // 0 = ok; else an XTED error code
     int32_t *error_info;  // [4] diagnostics of the first error
-    uint64_t timeout_ns;  // bound on every idle wait
-    unsigned long long *trace; // optional, 4 words per task: claim ns, start ns, end ns, info
-    // ---- striped units (nstriped = 0: none) ----
-    const XStripe *stripes;
-    const int32_t *smap;        // export maps
-    unsigned long long *sbuf;   // carries, first columns, exports (zeroed per run)
-    int64_t sbuf_words;
-    int32_t nstriped;
+    uint64_t timeout_ns;  // bound on every wait, without progress of any item
+    unsigned long long *trace; // optional, 4 words per item: claim ns, start ns, end ns, info
     // ---- serving session (serve = 1); a batch launch leaves these zero ----
     int32_t serve;
     int32_t serve_pairs;    // pairs per query slot (the corpus size)
-    uint64_t idle_exit_ns;  // a block with no work for this long leaves the launch
-    int32_t *mbox;          // XTED_MBOX_* words and records, device memory
-    int32_t *slot_done;     // [XTED_SERVE_SLOTS] pairs finished in the slot's current query
-    const int32_t *slot_need, *slot_gen;  // pairs to finish, generation to report
+    uint64_t idle_exit_ns;  // the launch ends once every warp has had no work for this long
+    unsigned long long *lists;  // [XTED_SERVE_SLOTS] (end << 32) | next item of the slot's list
+    const int32_t *ages;    // [XTED_SERVE_SLOTS] arrival number of the slot's query
+    int32_t *ctl;           // XTED_CTL_* words
+    int32_t *slot_done;     // [XTED_SERVE_SLOTS] items finished in the slot's current round
+    const int32_t *slot_need, *slot_gen;  // items to finish, generation to report
     int32_t *results;       // [slots * serve_pairs] distances, mapped host memory
-    int32_t *flags;         // [XTED_SERVE_SLOTS] generation of the last finished query, mapped host memory
-    // ---- test hook (xted_test_fault): level 0 of this pair is never published; -1: none ----
+    int32_t *flags;         // [XTED_SERVE_SLOTS] generation of the last finished round, mapped host memory
+    // ---- test hook (xted_test_fault): level 0 of this pair is never computed; -1: none ----
     int32_t hold_pair;
     // ---- edit costs: delete a row-tree node, insert a column-tree node, change a label ----
     int32_t c_del, c_ins, c_ren;
 };
 
-// Serving mailbox in device memory. The host writes records and then the
-// posted count with stream-ordered copies; blocks claim records in order and
-// publish level 0 of the record's pairs into the running launch's ready queue.
 #define XTED_SERVE_SLOTS 16
-#define XTED_SERVE_RECS 64
-#define XTED_MBOX_POSTED 0    // records posted (host)
-#define XTED_MBOX_STOP 1      // nonzero: blocks leave when idle (host)
-#define XTED_MBOX_CONSUMED 2  // records claimed (device), | XTED_MBOX_CLOSED once the launch leaves
-#define XTED_MBOX_CLOSED (1 << 30)  // set by the block that ends the launch: no record is claimed after it
-#define XTED_MBOX_TOP 3       // bucket of the oldest query in flight (host)
-#define XTED_MBOX_REC 4       // records: 4 ints each {slot, pair_lo, npairs, 0}
-#define XTED_MBOX_INTS (XTED_MBOX_REC + 4 * XTED_SERVE_RECS)
+#define XTED_CTL_IDLE 0     // warps currently without work
+#define XTED_CTL_CLOSED 1   // nonzero: the launch is ending, warps claim nothing more
+#define XTED_CTL_STOP 2     // nonzero: warps leave when idle (host)
+#define XTED_CTL_PROGRESS 3 // items finished
+#define XTED_CTL_INTS 8
