@@ -1,8 +1,8 @@
 """The DP launch at the sizes where its item kinds change (needs a B200):
-chunks of up to 256 and up to 512 columns a warp, column stripes of 512 beyond
-that (a stripe boundary may fall on any node), row runs around the 32 rows that
-a warp looks ahead, stacks deeper than the shared-memory window, and the form
-for chunks with more than 64 columns on a right path or across a stripe
+chunks of up to 256 columns on one warp, column stripes of 256 beyond
+that (a boundary may fall on any node), row runs around the 32 rows that
+a warp looks ahead, stacks deeper than the shared-memory window, and long
+lists of path columns, exports and far columns across a stripe
 boundary. Exact against the oracle: distances are whole numbers."""
 import numpy as np
 import pytest
@@ -78,3 +78,14 @@ def test_many_segments(narrow, run_rows):
                       gen.tree(("wide", "caterpillar", "deep")[k // 3 % 3], n, 50 + k, "uniform", 3)))
     with xted.Context(narrow_width=narrow, run_rows=run_rows) as ctx:
         assert np.array_equal(ctx.distance_batch(pairs), oracle.distance_batch(pairs, nthreads=8))
+
+
+@pytest.mark.timeout(300)
+@pytest.mark.parametrize("n", [301, 601])
+def test_more_far_values_than_places(n):
+    """Forced right-path tables of a comb whose nested keyroots cross every
+    stripe boundary with a far column each: more than have a place in shared
+    memory (64)."""
+    a, b = _comb(9, 5, False), _comb(n, 6, False)
+    with xted.Context(orientation=xted.ORIENT_RIGHT) as ctx:
+        assert ctx.distance(a, b) == oracle.distance(a, b)

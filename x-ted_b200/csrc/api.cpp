@@ -105,8 +105,7 @@ int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npa
     K.c_del = c->opts.cost_del;
     K.c_ins = c->opts.cost_ins;
     K.c_ren = c->opts.cost_ren;
-    // (a stripe of slack: a row's copies name, without reading, words up to a stripe past its end)
-    rc = ctx_dev_reserve(c, c->dt, (size_t)(c->plan_dt_elems + XTED_SW) * sizeof(int32_t));
+    rc = ctx_dev_reserve(c, c->dt, (size_t)std::max<int64_t>(c->plan_dt_elems, 1) * sizeof(int32_t));
     if (rc) return rc;
     // per-warp scratch: the far-row stack's rows outside the shared window
     const int64_t stack_rows = c->plan_stack_rows;

@@ -72,15 +72,16 @@ __device__ __forceinline__ void set_error(const XKernelParams &P, int code, int 
     }
 }
 
-// Both copy `bytes` (0 up to their size) and zero the rest of the destination.
 // Copies of table rows go through L2 (.cg) or, four bytes at a time, may
 // allocate in L1 (.ca): a stale L1 line can only hold -1 where the value has
-// since arrived, and a reader that finds -1 looks again through L2.
-__device__ __forceinline__ void cp_async16(unsigned smem, const int32_t *gmem, int bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem), "l"(gmem), "r"(bytes) : "memory");
+// since arrived, and a reader that finds -1 looks again through L2. Whole
+// pieces only: with a size operand (to zero what lies past a segment) a row's
+// copies cost some 50 more instructions.
+__device__ __forceinline__ void cp_async16(unsigned smem, const int32_t *gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async4(unsigned smem, const int32_t *gmem, int bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem), "l"(gmem), "r"(bytes) : "memory");
+__device__ __forceinline__ void cp_async4(unsigned smem, const int32_t *gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -115,27 +116,37 @@ __device__ __forceinline__ int warp_suffix_max(int v) {
     return v;
 }
 
-// A warp's shared memory: a ring of FLOW_PF table rows in flight and the stack
-// window. A stack row holds column c (lane c / W, its k-th column) at 32 k + lane, so reading or writing
-// every lane's k-th column touches 32 banks, then a zero word that stands for
-// the border, then (W = 16) the far values a stripe takes from others. W = 16 leaves a window of 4 rows (the stack leaves it on 2.5% of
-// the mixed batch's rows, against 1.7% for 8 rows), W = 8 keeps 8.
+// A warp's shared memory: a ring of FLOW_PF table rows in flight, the stack
+// window, and lists of the chunk's special columns. A stack row holds column c
+// (lane c / W, its k-th column) at 32 k + lane, so reading or writing every
+// lane's k-th column touches 32 banks, then a zero word that stands for the
+// border, then the far values a stripe takes from other stripes. The stack
+// leaves a window of 4 rows on 2.5% of the mixed batch's rows, one of 8 on 1.7%.
+#define FLOW_W 8                   // columns per lane
 #define FLOW_PF 4
+#define FLOW_IMPORTS 64            // far values of other stripes kept beside a stack row
+#define FLOW_STACK_ROWS 4
+#define FLOW_ZERO (32 * FLOW_W)    // place of the zero word in a stack row
+#define FLOW_PITCH (FLOW_ZERO + 4 + FLOW_IMPORTS)
 #define FLOW_RING (FLOW_PF * XTED_SW)
-#define FLOW_IMPORTS 64  // far values of other stripes kept beside a stack row
-template <int W>
-struct StackWin {
-    static constexpr int ROWS = W == 16 ? 4 : 8;
-    static constexpr int PITCH = 32 * W + 4 + (W == 16 ? FLOW_IMPORTS : 0);
-};
-#define FLOW_STACK 2320  // the larger ROWS * PITCH
-static_assert(StackWin<16>::ROWS * StackWin<16>::PITCH <= FLOW_STACK && StackWin<8>::ROWS * StackWin<8>::PITCH <= FLOW_STACK,
-              "stack window");
-#define FLOW_WARP_INTS (FLOW_RING + FLOW_STACK)
-#define FLOW_ZERO 584  // a stack row of zeros, one per block: what tree rows read as far values
-static_assert(StackWin<16>::PITCH <= FLOW_ZERO && FLOW_ZERO % 4 == 0, "row of zeros");
-#define FLOW_SMEM ((FLOW_ZERO + XTED_FLOW_WARPS * FLOW_WARP_INTS) * 4)
-// A row's flags in a run's row sequence, beside those of its node record.
+#define FLOW_STACK (FLOW_STACK_ROWS * FLOW_PITCH)
+// path columns (column | segment << 8 | node << 16), their labels, exported columns (16 bits each)
+#define FLOW_LISTS (XTED_SW + XTED_SW + XTED_SW / 2)
+#define FLOW_WARP_INTS (FLOW_RING + FLOW_STACK + FLOW_LISTS)
+// a stack row of zeros, one per block: what tree rows read as far values
+#define FLOW_SMEM ((FLOW_PITCH + XTED_FLOW_WARPS * FLOW_WARP_INTS) * 4)
+static_assert(XTED_SW == 32 * FLOW_W && XTED_MAX_NODES < 65536 && FLOW_PITCH % 4 == 0, "list entries and row places");
+// A row's flags in a run's row sequence, beside orl (20 bits) and the flags of
+// its node record (bits 29, 30). The ITEM_ flags are the same for every row of
+// an item: what the row loop asks of the item. They come with the row, through
+// the same shuffle, because the compiler would make a copy of the loop for
+// every answer it can tell to be constant.
+#define ITEM_MULTI (1u << 20)    // a chunk of several segments
+#define ITEM_RIGHT (1u << 21)    // a stripe has a right neighbour
+#define ITEM_LEFT (1u << 22)     // ... a left one
+#define ITEM_IMPORTS (1u << 23)  // it takes far values from other stripes
+#define ITEM_EXPORTS (1u << 24)  // it has columns that other stripes take
+#define ITEM_EDGE (1u << 25)     // its first or last 16-byte piece holds words of other segments
 #define ROW_NEXTTREE (1u << 26)  // the next row of the table is on its right path
 #define ROW_TREE (1u << 27)      // the row is on its table's right path
 #define ROW_FIRST (1u << 28)     // first row of its table (the table's last node)
@@ -148,56 +159,54 @@ static_assert(StackWin<16>::PITCH <= FLOW_ZERO && FLOW_ZERO % 4 == 0, "row of ze
 // later shuffle of the row compiled to a check and a slow path (2.3 KB of
 // code for the five of a row's suffix maximum, times every use).
 __device__ __forceinline__ bool warp_wait(const XKernelParams &P, const int32_t *p, bool need, int &v) {
-    uint64_t t0 = global_ns();
-    int pg = ld_relaxed(P.progress);
-    unsigned ns = 32;
-    for (;;) {
+    uint64_t t0 = 0;
+    int pg = 0;
+#pragma unroll 1
+    for (unsigned n = 1;; n++) {
         if (need) v = ld_relaxed(p);
         if (!__any_sync(FULLMASK, need && v < 0)) return true;
-        bool out = ld_relaxed(P.error) != 0;
-        const uint64_t now = global_ns();
-        if (now - t0 > P.timeout_ns) {
-            const int q = ld_relaxed(P.progress);
-            if (q == pg) {
-                set_error(P, XTED_ETIMEOUT, 1, 0, 0);
-                out = true;
+        __nanosleep(n < 8 ? 40 * n : 320);
+        if ((n & 31) == 0) {  // every few microseconds: has the launch failed, or stopped?
+            bool out = ld_relaxed(P.error) != 0;
+            const uint64_t now = global_ns();
+            if (t0 == 0 || now - t0 > P.timeout_ns) {
+                const int q = ld_relaxed(P.progress);
+                if (t0 != 0 && q == pg) {
+                    set_error(P, XTED_ETIMEOUT, 1, 0, 0);
+                    out = true;
+                }
+                pg = q;
+                t0 = now;
             }
-            pg = q;
-            t0 = now;
+            if (__any_sync(FULLMASK, out)) return false;
         }
-        if (__any_sync(FULLMASK, out)) return false;
-        __nanosleep(ns);
-        if (ns < 512) ns <<= 1;
     }
 }
 
-// One item on one warp. MULTI: the chunk holds several segments (copied word
-// by word; at most 32 W columns), else one segment (16-byte copies). W = 16:
-// stripe s of K of a segment (K = 1: all of it).
+// One item on one warp: a chunk of several segments (multi, copied word by
+// word), a segment one warp holds, or stripe s of K of a wider one (both
+// copied in 16-byte pieces).
 //
-// A few columns of a segment need more than the common step: those on its
-// right path (on tree rows they take the diagonal and their value goes out),
-// those that stripes further left read, and those whose far column lies in
-// another stripe. LISTS: there are at most 64 of each, and lane q takes the
-// q-th and (q + 32)-th through shared memory; otherwise (LISTS = false, and
-// for several segments, where most columns are on a path) every lane tests its
-// own W columns. Testing them all on every row cost 100-200 of a row's 400
-// instructions, and code: the instruction cache is what the first form of this
-// kernel, with six unrolled bodies, ran out of (15.6 of 24.5 cycles per issued
-// instruction waited for instructions on a 256-pair mixed batch).
-// What a row rarely needs (waiting, the stack leaving its window) is marked
-// unlikely. Returns 0, FLOW_FAILED once the launch has failed, or FLOW_LISTS
-// (nothing done) if LISTS is set and a list would be longer than 64.
+// There is one row loop for all of them, of 8 columns a lane. What bounds it
+// is the instruction cache and the latency of a row: with a loop per kind of
+// chunk and width (six, unrolled) 15.6 of 24.5 cycles per issued instruction
+// went on waiting for instructions, with three (8 columns, 8 of several
+// segments, 16 a lane) 3.6 of 9.6. So the few columns that need more than the
+// common step are listed and taken by whole warps, not tested on every lane:
+// those on their segment's right path (on tree rows they take the diagonal
+// and their value goes out), those that stripes further left read, and those
+// whose far column lies in another stripe. What a row rarely needs (waiting,
+// the stack leaving its window) is marked unlikely. OVER: a stripe that takes
+// more far values from other stripes than have a place in shared memory.
+// Returns 0, FLOW_FAILED once the launch has failed, or FLOW_OVER (nothing
+// done) if OVER is needed.
 #define FLOW_FAILED 1
-#define FLOW_LISTS 2
-template <int W, bool MULTI, bool LISTS>
+#define FLOW_OVER 2
+template <bool OVER>
 __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it, const XPair &pr, const XRun &run,
-                                     const XChunk &ch, unsigned zeros, int32_t *ring, int32_t *gstk) {
-    constexpr bool STRIPE = W == 16;
-    static_assert(!(MULTI && (STRIPE || LISTS)), "a stripe is part of one segment");
-    constexpr int SLOT = 32 * W, PF = FLOW_PF;
-    constexpr int SC = StackWin<W>::ROWS, PITCH = StackWin<W>::PITCH, ZERO = 32 * W, IMP = ZERO + 4;
-    constexpr int NG = W / 4;  // 16-byte pieces a lane copies per row
+                                         const XChunk &ch, unsigned zeros, int32_t *ring, int32_t *gstk) {
+    constexpr int W = FLOW_W, PF = FLOW_PF, SC = FLOW_STACK_ROWS, ZERO = FLOW_ZERO, IMP = ZERO + 4;
+    constexpr unsigned SLOT_B = 4 * XTED_SW, RING_B = PF * SLOT_B, PITCH_B = 4 * FLOW_PITCH;
     const int lane = threadIdx.x & 31;
     const int2 *rows = P.rowinfo + pr.row_base, *nodes = P.rowinfo + pr.col_base;
     int32_t *dt = P.dt + pr.dt_off;
@@ -206,24 +215,25 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
     // delete + insert saves nothing: the maximum then takes another term)
     const int bm = P.c_del + P.c_ins, bn = max(bm - P.c_ren, 0);
     const int R = run.rows;
-    const unsigned ring_a = smem_addr(ring), stk_a = ring_a + 4 * FLOW_RING;  // stack rows are PITCH ints apart
-    constexpr unsigned SLOT_B = 4 * SLOT, RING_B = PF * SLOT_B, PITCH_B = 4 * PITCH;
-    // single segment: where column c of a row lies in its ring slot (piece p at
-    // p ^ ((p >> 3) & (NG - 1)): eight lanes reading their g-th pieces touch
+    const bool multi = ch.nseg > 1;
+    const unsigned ring_a = smem_addr(ring), stk_a = ring_a + 4 * FLOW_RING;  // (stack rows are PITCH_B apart)
+    const unsigned tl_a = stk_a + 4 * FLOW_STACK, lab_a = tl_a + 4 * XTED_SW, el_a = lab_a + 4 * XTED_SW;
+    // where column c of a row lies in its ring slot (piece p of four words at
+    // p ^ ((p >> 3) & 1): eight lanes reading their first or second pieces touch
     // eight different bank groups)
-    auto swz = [](int c) { return 4 * ((c >> 2) ^ ((c >> 5) & (NG - 1))) + (c & 3); };
+    auto swz = [](int c) { return 4 * ((c >> 2) ^ ((c >> 5) & 1)) + (c & 3); };
 
     // ---- columns ----
-    int key[W], node[W];
-    int lab[LISTS ? 1 : W];
-    int fb[W];                       // far column: byte offset in a stack row (not LISTS, another stripe's: export index)
-    unsigned tcol = 0;               // bit k: column k is on its segment's right path
-    unsigned xfar = 0, expm = 0;     // STRIPE: far column in another stripe; exported column
-    int ebase = 0;                   // STRIPE: export index of this lane's (LISTS: the stripe's) first exported column
-    int sbase = 0, cend = ch.width;  // single: node of local column 0; columns [.., cend) exist
-    int lead = 0, K = 1, X = 0, s = 0;
+    int key[W];           // its segment's key
+    int fb[W];            // its far column: byte offset in a stack row
+    unsigned tcol = 0;    // bit k: column k is on its segment's right path
+    unsigned xfar = 0;    // bit k: its far column is in another stripe
+    unsigned expm = 0;    // bit k: stripes further left read it
+    int ebase = 0x7fffffff;
+    int sbase = 0, cend = ch.width, lead = 0, K = 1, X = 0, s = 0;
     __syncwarp();
-    if (MULTI) {
+    // multi: the columns' nodes, through the ring (nothing is under way there)
+    if (multi) {
         // segment of the lane's first column by binary search, then a walk over the keyroots
         int q = ch.k_lo, j = 0, j0 = 0, je = 0;
         const int c0 = lane * W;
@@ -244,8 +254,8 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
         for (int k = 0; k < W; k++) {
             const int c = c0 + k;
             fb[k] = 4 * ZERO;
-            node[k] = key[k] = 0;
-            if (!LISTS) lab[k] = 0;
+            key[k] = 0;
+            int nd_j = -1;
             if (c < ch.width) {
                 if (j >= je) {
                     q++;
@@ -253,10 +263,8 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
                     je = (nodes[j0].y & XTED_ROW_ORL_MASK) + 1;
                     j = j0;
                 }
-                const int2 nd = nodes[j];
-                const int f = (nd.y & XTED_ROW_ORL_MASK) + 1;  // far column's node
-                node[k] = j;
-                if (!LISTS) lab[k] = nd.x;
+                const int f = (nodes[j].y & XTED_ROW_ORL_MASK) + 1;  // far column's node
+                nd_j = j;
                 key[k] = (ch.k_lo + ch.nseg - 1 - q) * XTED_KEY_BIG;
                 if (f == je) {
                     tcol |= 1u << k;
@@ -266,42 +274,39 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
                 }
                 j++;
             }
+            ring[c] = nd_j;
         }
     } else {
         const int j0 = P.krd[ch.k_lo], je = j0 + ch.width;
         lead = j0 & (XTED_PITCH - 1);
-        const int base = j0 - lead;
+        sbase = j0 - lead;
         const int32_t *map = nullptr;
-        if (STRIPE) {
+        if (lead + ch.width > XTED_SW) {
             const XChunkX cx = P.chunkx[it.chunk];
             K = cx.K;
             X = cx.X;
             s = it.stripe;
             map = P.smap + cx.map;
+            sbase += s * XTED_SW;
+            if (s > 0) lead = 0;
         }
-        sbase = base + s * XTED_SW;
-        cend = min(je - sbase, 32 * W);
-        if (STRIPE && s > 0) lead = 0;
+        cend = min(je - sbase, XTED_SW);
 #pragma unroll
         for (int k = 0; k < W; k++) {
             const int c = lane * W + k, j = sbase + c;
             fb[k] = 4 * ZERO;
-            key[k] = node[k] = 0;
-            if (!LISTS) lab[k] = 0;
+            key[k] = 0;
             if (c >= lead && c < cend) {
-                const int2 nd = nodes[j];
-                const int f = (nd.y & XTED_ROW_ORL_MASK) + 1;
-                if (!LISTS) lab[k] = nd.x;
+                const int f = (nodes[j].y & XTED_ROW_ORL_MASK) + 1, fc = f - sbase;
                 if (f == je) {
                     tcol |= 1u << k;
-                } else if (!STRIPE || f - sbase < 32 * W) {
-                    const int fc = f - sbase;
+                } else if (fc < XTED_SW) {
                     fb[k] = 4 * ((fc & (W - 1)) * 32 + fc / W);
                 } else {
                     xfar |= 1u << k;
-                    fb[k] = map[f - j0];
+                    fb[k] = map[f - j0];  // (its export index, until it has a place beside the stack row)
                 }
-                if (STRIPE && K > 1) {
+                if (K > 1) {
                     const int e = map[j - j0];  // exports are numbered in column order
                     if (e >= 0) {
                         if (expm == 0) ebase = e;
@@ -309,94 +314,102 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
                     }
                 }
             }
+            ring[c] = j;
         }
     }
-    // LISTS: the q-th such column of the stripe, q = lane and lane + 32
-    int tq[2] = {0, 0}, tlab[2] = {0, 0};  // right path: column | its word in a ring slot << 10 | the next column's << 20
-    bool tlast = false;                    // one of them is the stripe's last column
-    int xq[2] = {0, 0}, iv[2] = {0, 0};    // far column elsewhere: export index; its value for the next row
-    int eq[2] = {0, 0};                    // exported: its word in a stack row
-    int nt = 0, nx = 0, ne = 0;
-    if (LISTS) {
-        auto listed = [&](unsigned mask, int &first) {  // this lane's first place in the list; the list's length
-            int n = __popc(mask);
+    __syncwarp();
+    // ---- the lists: path columns, exported columns, far columns elsewhere ----
+    auto first_of = [&](unsigned mask, int &n) {  // the lane's first place in a list; the list's length
+        int v = __popc(mask);
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int o = __shfl_up_sync(FULLMASK, n, d);
-                if (lane >= d) n += o;
-            }
-            first = n - __popc(mask);
-            return __shfl_sync(FULLMASK, n, 31);
-        };
-        int tf, xf, ef;
-        nt = listed(tcol, tf);
-        if (STRIPE) {
-            nx = listed(xfar, xf);
-            ne = listed(expm, ef);
+        for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(FULLMASK, v, d);
+            if (lane >= d) v += o;
         }
-        if (nt > 64 || nx > 64 || ne > 64) return FLOW_LISTS;
-        int32_t *tl = ring, *xl = ring + 64, *el = ring + 128;
+        n = __shfl_sync(FULLMASK, v, 31);
+        return v - __popc(mask);
+    };
+    int nt, nx, ne;
+    int tf = first_of(tcol, nt), xf = first_of(xfar, nx), ef = first_of(expm, ne);
+    ebase = (int)__reduce_min_sync(FULLMASK, (unsigned)ebase);
+    unsigned short *el = (unsigned short *)(ring + FLOW_RING + FLOW_STACK + 2 * XTED_SW);
+    int32_t *tlist = ring + FLOW_RING + FLOW_STACK, *tlab = tlist + XTED_SW;
+    // far columns elsewhere, in column order, then the places of their values
+    int32_t *xl = ring + FLOW_RING, *xplace = xl + XTED_SW, *xd = xplace + XTED_SW;  // (in the stack window, empty as yet)
+    int x1 = xf;
 #pragma unroll
-        for (int k = 0; k < W; k++) {
-            const int c = lane * W + k;
-            if ((tcol >> k) & 1u) tl[tf++] = c;
-            if (STRIPE && ((xfar >> k) & 1u)) {
-                xl[xf] = fb[k];
-                fb[k] = 4 * (IMP + xf++);
-            }
-            if (STRIPE && ((expm >> k) & 1u)) el[ef++] = k * 32 + lane;
+    for (int k = 0; k < W; k++) {
+        const int c = lane * W + k;
+        if ((tcol >> k) & 1u) {
+            const int j = ring[c];
+            tlab[tf] = nodes[j].x;
+            tlist[tf++] = (int)((unsigned)c | ((unsigned)(key[k] / XTED_KEY_BIG) << 8) | ((unsigned)j << 16));
         }
+        if ((expm >> k) & 1u) el[ef++] = (unsigned short)(k * 32 + lane);
+        if ((xfar >> k) & 1u) xl[x1++] = fb[k];
+    }
+    __syncwarp();
+    unsigned xover = 0;  // OVER, bit k: a far column elsewhere with no place beside the stack row
+    int xq[2] = {0, 0};  // export index of the value in place q, q = lane, lane + 32
+    int iv[2] = {0, 0};  // ... and the value for the next row
+    if (nx > 0) {
+        // columns with one far column follow each other (subtrees across a
+        // boundary are nested): they share a place
+        int places = 0;
+#pragma unroll 1
+        for (int q0 = 0; q0 < nx; q0 += 32) {
+            const int q = q0 + lane;
+            const bool first = q < nx && (q == 0 || xl[q] != xl[q - 1]);
+            const unsigned m = __ballot_sync(FULLMASK, first);
+            const int place = places + __popc(m & (0xffffffffu >> (31 - lane))) - 1;
+            if (q < nx) xplace[q] = place;
+            if (first && place < FLOW_IMPORTS) xd[place] = xl[q];
+            places += __popc(m);
+        }
+        nx = places;
+        if (!OVER && nx > FLOW_IMPORTS) return FLOW_OVER;
         __syncwarp();
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int q = lane + 32 * h;
-            if (q < nt) {
-                const int c = tl[q];
-                tlab[h] = nodes[sbase + c].x;
-                tq[h] = c | (swz(c) << 10) | ((c + 1 < 32 * W ? swz(c + 1) : 0) << 20);
-                tlast |= c + 1 == 32 * W;
+        for (int k = 0; k < W; k++)
+            if ((xfar >> k) & 1u) {
+                const int place = xplace[xf++];
+                if (place >= FLOW_IMPORTS) xover |= 1u << k;
+                fb[k] = 4 * (place < FLOW_IMPORTS ? IMP + place : ZERO);
             }
-            if (STRIPE && q < nx) xq[h] = xl[q];
-            if (STRIPE && q < ne) eq[h] = el[q];
-        }
-        if (STRIPE) ebase = __reduce_min_sync(FULLMASK, (unsigned)(expm ? ebase : 0x7fffffff));
+        if (lane < nx) xq[0] = xd[lane];
+        if (lane + 32 < min(nx, FLOW_IMPORTS)) xq[1] = xd[lane + 32];
     }
-    const bool right = STRIPE && s + 1 < K, left = STRIPE && s > 0;
-    const int32_t *Hin = P.buf + it.buf + (int64_t)s * R;          // the right neighbour's first column, per row
-    int32_t *Hout = P.buf + it.buf + (int64_t)(s - 1) * R;         // this stripe's, for the left one
-    int32_t *E = P.buf + it.buf + (int64_t)(K - 1) * R;            // exported columns, per row
-    const bool xwarp = STRIPE && __any_sync(FULLMASK, xfar != 0);
-    const bool lead_any = __any_sync(FULLMASK, lead != 0);
-
-    // ---- shared memory ----
+    // the lane's copies of a row. multi: word lane + 32 k from column cpn[k] (-1: none); else pieces lane and lane + 32
+    int cpn[W];
+#pragma unroll
+    for (int k = 0; k < W; k++) cpn[k] = multi ? ring[lane + 32 * k] : 4 * (lane + 32 * k) < cend ? 0 : -1;
     __syncwarp();
     if (lane < SC) sts(stk_a + lane * PITCH_B + 4 * ZERO, 0);
-    int cpn[MULTI ? W : 1], csz[MULTI ? W : NG];  // the lane's copies of a row: multi, node of column lane + 32 k; bytes
-    if (MULTI) {
-        // the lane's copy plan through the ring (nothing is under way there)
+    // words past the chunk's copies stay zero; those that come with its first
+    // or last piece are zeroed row by row, by lanes 0-2 and 3-5
+    const int copied = multi ? ch.width : (cend + XTED_PITCH - 1) & ~(XTED_PITCH - 1);
 #pragma unroll
-        for (int k = 0; k < W; k++) ring[lane * W + k] = node[k];
-        __syncwarp();
-#pragma unroll
-        for (int k = 0; k < W; k++) {
-            const bool v = lane + 32 * k < ch.width;
-            cpn[MULTI ? k : 0] = v ? ring[lane + 32 * k] : 0;
-            csz[MULTI ? k : 0] = v ? 4 : 0;  // past the chunk: zeroed
-        }
-    } else {
-#pragma unroll
-        for (int g = 0; g < NG; g++) csz[MULTI ? 0 : g] = 4 * max(0, min(4, cend - 4 * (lane + 32 * g)));
-    }
-    unsigned coff[NG];  // where the lane's own columns lie in a slot
-#pragma unroll
-    for (int g = 0; g < NG; g++) coff[g] = MULTI ? 4 * (lane * W + 4 * g) : 4 * swz(lane * W + 4 * g);
+    for (int k = 0; k < W; k++)
+        if (lane * W + k >= copied)
+            for (int q = 0; q < PF; q++) ring[q * XTED_SW + swz(lane * W + k)] = 0;
+    const int ec = lane < 3 ? lane : cend + lane - 3;
+    const bool edge = !multi && (lane < 3 ? lane < lead : lane < 6 && ec < copied);
+    const unsigned edge_o = 4 * swz(edge ? ec : 0);
+    const unsigned coff0 = 4 * swz(lane * W), coff1 = 4 * swz(lane * W + 4);  // the lane's columns in a slot
+    const bool right = s + 1 < K, left = s > 0;
+    const unsigned ask = (multi ? ITEM_MULTI : 0u) | (right ? ITEM_RIGHT : 0u) | (left ? ITEM_LEFT : 0u) |
+                         (nx > 0 ? ITEM_IMPORTS : 0u) | (ne > 0 ? ITEM_EXPORTS : 0u) |
+                         (__any_sync(FULLMASK, edge) ? ITEM_EDGE : 0u);
+    const int32_t *Hin = P.buf + it.buf + (int64_t)s * R;   // the right neighbour's first column, per row
+    int32_t *Hout = P.buf + it.buf + (int64_t)(s - 1) * R;  // this stripe's, for the left one
+    int32_t *E = P.buf + it.buf + (int64_t)(K - 1) * R;     // exported columns, per row
     __syncwarp();
 
     // ---- row sequence: the run's tables one after another, each from its last row up ----
     // Lane l holds row tb + l of the sequence (its node, its record with the
     // table flags, its label) and, loaded 32 rows ahead, row tb + 32 + l.
     int bi = 0, by = 0, bl = 0, ni = 0, ny = 0, nl = 0;
-    auto load_rows = [&](int f, int &i, int &y, int &l) {
+    auto load_rows = [&](int f) {
         f = min(f, R - 1);
         int q = run.kr_lo;
         int off = f;
@@ -411,170 +424,162 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
             off = f - (P.cumw[q] - p0);
         }
         const int i0 = P.krd[q], e0 = rows[i0].y & XTED_ROW_ORL_MASK;
-        i = e0 - off;
-        const int2 r = rows[i];
-        l = r.x;
+        ni = e0 - off;
+        const int2 r = rows[ni];
+        nl = r.x;
         unsigned fl = off == 0 ? ROW_FIRST : 0u;
         if ((r.y & XTED_ROW_ORL_MASK) == e0) fl |= ROW_TREE;
-        if (i == i0) fl |= ROW_LAST;
-        else if ((rows[i - 1].y & XTED_ROW_ORL_MASK) == e0) fl |= ROW_NEXTTREE;
-        y = (int)((unsigned)r.y | fl);
+        if (ni == i0) fl |= ROW_LAST;
+        else if ((rows[ni - 1].y & XTED_ROW_ORL_MASK) == e0) fl |= ROW_NEXTTREE;
+        ny = (int)((unsigned)r.y | fl | ask);
     };
 #pragma unroll 1
     for (int h = 0; h < 2; h++) {
         bi = ni, by = ny, bl = nl;
-        load_rows(32 * h + lane, ni, ny, nl);
+        load_rows(32 * h + lane);
     }
-    // row PF - 1 places on, by lane as above
-    int ai = __shfl_sync(FULLMASK, bi, (lane + PF - 1) & 31);
-    {
-        const int o = __shfl_sync(FULLMASK, ni, (lane + PF - 1) & 31);
-        if (lane + PF - 1 >= 32) ai = o;
-    }
-    const int32_t *src0 = MULTI ? dt : dt + sbase + 4 * lane;
-    const unsigned dst0 = ring_a + (MULTI ? 4 * lane : 16 * (lane ^ ((lane >> 3) & (NG - 1))));
-    auto copy_row = [&](unsigned so, int r) {  // row r into the slot at byte so of the ring
+    int ci = bi;  // the rows being copied, PF - 1 ahead
+    const int32_t *src0 = multi ? dt : dt + sbase + 4 * lane;
+    const unsigned dst0 = ring_a + (multi ? 4 * lane : 16 * (lane ^ ((lane >> 3) & 1)));
+    const unsigned dst1 = ring_a + (4 * lane ^ 16);  // multi: odd words of the lane (swz(lane + 32 k))
+    auto copy_row = [&](unsigned so, int r, unsigned y) {  // row r into the slot at byte so of the ring
         const int32_t *src = src0 + (unsigned long long)(unsigned)r * (unsigned)pitch;
-        const unsigned d = dst0 + so;
-        if (MULTI) {
+        const unsigned d = dst0 + so, d1 = dst1 + so;
+        if (y & ITEM_MULTI) {
 #pragma unroll
-            for (int k = 0; k < W; k++) cp_async4(d + 128 * k, src + (unsigned)cpn[MULTI ? k : 0], csz[MULTI ? k : 0]);
+            for (int k = 0; k < W; k++)
+                if (cpn[k] >= 0) cp_async4((k & 1 ? d1 : d) + 128 * k, src + (unsigned)cpn[k]);
         } else {
-#pragma unroll
-            for (int g = 0; g < NG; g++) cp_async16(d + 512 * g, src + 128 * g, csz[MULTI ? 0 : g]);
+            if (cpn[0] >= 0) cp_async16(d, src);
+            if (cpn[1] >= 0) cp_async16(d + 512, src + 128);
         }
     };
 #pragma unroll 1
     for (int q = 0; q < PF - 1; q++) {
-        copy_row(q * SLOT_B, __shfl_sync(FULLMASK, bi, q));  // (past the run's end: its last row again)
+        copy_row(q * SLOT_B, __shfl_sync(FULLMASK, bi, q), ask);  // (past the run's end: its last row again)
         cp_async_commit();
     }
 
     int prev[W];
 #pragma unroll
     for (int k = 0; k < W; k++) prev[k] = key[k];
-    int sp = 0, lo = 0;      // stack depth; lowest position held in the shared window
+    int sp = 0, lo = 0;             // stack depth; lowest position held in the shared window
     int c0 = 0, c1 = 0, cprev = 0;  // stripes: the right neighbour's first column in this row, the next, the one above
     if (right) {
         c0 = ld_relaxed(Hin);
-        c1 = R > 1 ? ld_relaxed(Hin + 1) : 0;
-    }
-    int pfw[STRIPE && !LISTS ? W : 1];  // far values of other stripes for this row (-1: not there yet)
-    if (STRIPE && !LISTS) {
-#pragma unroll
-        for (int k = 0; k < W; k++) pfw[k] = 0;
+        c1 = ld_relaxed(Hin + min(1, R - 1));
     }
 
 #pragma unroll 1
     for (int t = 0; t < R; t++) {
         const unsigned so = (unsigned)(t & (PF - 1)) * SLOT_B, slot = ring_a + so;
-        if (!LISTS) {
-            // the masks' bits are tested where they are used: kept apart in
-            // registers over the whole loop they would spill it
-            asm volatile("" : "+r"(tcol), "+r"(xfar), "+r"(expm));
-        }
+        const unsigned above = ring_a + ((so + RING_B - SLOT_B) & (RING_B - 1));  // the slot of row t - 1
+        const int tl = t & 31;
         cp_async_wait<PF - 2>();  // row t has landed
         __syncwarp();             // ... every lane's copies; row t - 1's readers are done
-        const int tl = t & 31;
-        const int i = __shfl_sync(FULLMASK, bi, tl);
         const unsigned y = (unsigned)__shfl_sync(FULLMASK, by, tl);
         const bool trow = (y & ROW_TREE) != 0;
-        int rl = 0;
-        if (trow) rl = __shfl_sync(FULLMASK, bl, tl);
-        if (LISTS && trow) {  // tree rows: the path columns' words become what the diagonal gives
-            const unsigned above = ring_a + ((so + RING_B - SLOT_B) & (RING_B - 1));  // the row above, if the table's
-#pragma unroll
-            for (int h = 0; h < 2; h++)
-                if (lane + 32 * h < nt) {
-                    int x = lds(above + (((unsigned)tq[h] >> 18) & 0xffcu));
-                    if (y & ROW_FIRST) x = 0;
-                    if (tlast && (tq[h] & 1023) + 1 == 32 * W) x = cprev;
-                    sts(slot + (((unsigned)tq[h] >> 8) & 0xffcu), x + (rl == tlab[h] ? bm : bn));
-                }
+        if (trow) {  // the path columns' words become what the diagonal gives
+            const int rl = __shfl_sync(FULLMASK, bl, tl);
+#pragma unroll 1
+            for (int q0 = 0; q0 < nt; q0 += 32) {
+                const int q = q0 + lane;
+                if (q >= nt) continue;
+                const unsigned e = (unsigned)lds(tl_a + 4 * q);
+                const int c = e & 255, kc = (int)((e >> 8) & 255) * XTED_KEY_BIG;
+                int x = c + 1 < XTED_SW ? lds(above + 4 * swz(c + 1)) : cprev;
+                x = y & ROW_FIRST ? 0 : max(x - kc, 0);  // past a segment's end: its border
+                sts(slot + 4 * swz(c), x + (rl == lds(lab_a + 4 * q) ? bm : bn));
+            }
             __syncwarp();  // (and every lane has read the row above, whose slot is copied into next)
         }
-        copy_row((so + RING_B - SLOT_B) & (RING_B - 1), __shfl_sync(FULLMASK, ai, tl));  // into row t - 1's slot
+        if (tl == 32 - (PF - 1)) ci = ni;
+        copy_row(above - ring_a, __shfl_sync(FULLMASK, ci, (t + PF - 1) & 31), y);
         cp_async_commit();
-        int c2 = 0;
-        if (right && t + 2 < R) c2 = ld_relaxed(Hin + t + 2);
         int a[W];
         for (;;) {
-#pragma unroll
-            for (int g = 0; g < NG; g++) {
-                const int4 v = lds4(slot + coff[g]);
-                a[4 * g] = v.x, a[4 * g + 1] = v.y, a[4 * g + 2] = v.z, a[4 * g + 3] = v.w;
+            if (y & ITEM_EDGE) {
+                if (edge) sts(slot + edge_o, 0);
+                __syncwarp();
             }
-            if (!MULTI && lead_any) {  // words left of the segment
-#pragma unroll
-                for (int k = 0; k < 3; k++)
-                    if (lane == 0 && k < lead) a[k] = 0;
-            }
-            if (!LISTS && trow) {
-                int dn = __shfl_down_sync(FULLMASK, prev[0], 1);
-                if (lane == 31) dn = cprev;
-#pragma unroll
-                for (int k = 0; k < W; k++) {
-                    int x = k == W - 1 ? dn : prev[k + 1];
-                    if (MULTI) x = max(x, key[k]) - key[k];  // past a segment's end: its border
-                    x += rl == lab[k] ? bm : bn;
-                    if ((tcol >> k) & 1u) a[k] = x;
-                }
-            }
+            const int4 u = lds4(slot + coff0), v = lds4(slot + coff1);
+            a[0] = u.x, a[1] = u.y, a[2] = u.z, a[3] = u.w, a[4] = v.x, a[5] = v.y, a[6] = v.z, a[7] = v.w;
             // a word that is still -1: another item has yet to write it
-            int m = a[0];
-#pragma unroll
-            for (int k = 1; k < W; k++) m |= a[k];
-            const unsigned who = __ballot_sync(FULLMASK, m < 0);
+            const unsigned who = __ballot_sync(FULLMASK, (a[0] | a[1] | a[2] | a[3] | a[4] | a[5] | a[6] | a[7]) < 0);
             if (__builtin_expect(who == 0, 1)) break;
             // the leftmost missing word is the last to come: wait for it, then
             // fetch this row and those already under way again
-            int kk = 0, v = 0;
+            int kk = 0, w = 0;
 #pragma unroll
             for (int k = W - 1; k >= 0; k--)
-                if (a[k] < 0) kk = MULTI ? node[k] : sbase + lane * W + k;
-            kk = __shfl_sync(FULLMASK, kk, __ffs(who) - 1);
-            if (!warp_wait(P, dt + (int64_t)i * pitch + kk, true, v)) return FLOW_FAILED;
-            int td[2] = {0, 0};  // a tree row's path words do not change
-            if (LISTS && trow) {
-#pragma unroll
-                for (int h = 0; h < 2; h++)
-                    if (lane + 32 * h < nt) td[h] = lds(slot + (((unsigned)tq[h] >> 8) & 0xffcu));
+                if (a[k] < 0) kk = k;
+            kk = lane * W + kk;
+            int j = sbase + kk;
+            if (y & ITEM_MULTI) {  // its node: that of the keyroot's segment it lies in
+                const int pos = P.cumw[ch.k_lo] + min(kk, ch.width - 1);
+                int l2 = ch.k_lo, h2 = ch.k_lo + ch.nseg - 1;
+                while (l2 < h2) {
+                    const int mid = (l2 + h2 + 1) >> 1;
+                    if (P.cumw[mid] <= pos) l2 = mid;
+                    else h2 = mid - 1;
+                }
+                j = P.krd[l2] + pos - P.cumw[l2];
             }
+            const int i = __shfl_sync(FULLMASK, bi, tl);
+            if (!warp_wait(P, dt + (int64_t)i * pitch + __shfl_sync(FULLMASK, j, __ffs(who) - 1), true, w)) return FLOW_FAILED;
             cp_async_wait<0>();
             __syncwarp();
+            if (trow) {  // its path words stay: kept where the labels are while the row is copied again
+#pragma unroll 1
+                for (int q0 = 0; q0 < nt; q0 += 32) {
+                const int q = q0 + lane;
+                if (q >= nt) continue;
+                    const int c = lds(tl_a + 4 * q) & 255, o = 4 * swz(c);
+                    sts(lab_a + 4 * q, lds(slot + o));
+                }
+                __syncwarp();
+            }
 #pragma unroll 1
             for (int q = 0; q < PF; q++) {
                 const int r = __shfl_sync(FULLMASK, tl + q < 32 ? bi : ni, (tl + q) & 31);
                 const unsigned sq = (so + q * SLOT_B) & (RING_B - 1);
-                if (MULTI) {  // through L2, past whatever an L1 line holds
+                if (y & ITEM_MULTI) {  // through L2, past whatever an L1 line holds
                     const int32_t *src = dt + (int64_t)r * pitch;
 #pragma unroll
                     for (int k = 0; k < W; k++)
-                        if (csz[MULTI ? k : 0] > 0) sts(dst0 + sq + 128 * k, ld_relaxed(src + cpn[MULTI ? k : 0]));
+                        if (cpn[k] >= 0) sts((k & 1 ? dst1 : dst0) + sq + 128 * k, ld_relaxed(src + cpn[k]));
                 } else {
-                    copy_row(sq, r);
+                    copy_row(sq, r, y);
                 }
             }
             cp_async_commit();
             cp_async_wait<0>();
             __syncwarp();
-            if (LISTS && trow) {
-#pragma unroll
-                for (int h = 0; h < 2; h++)
-                    if (lane + 32 * h < nt) sts(slot + (((unsigned)tq[h] >> 8) & 0xffcu), td[h]);
+            if (trow) {
+#pragma unroll 1
+                for (int q0 = 0; q0 < nt; q0 += 32) {
+                const int q = q0 + lane;
+                if (q >= nt) continue;
+                    const unsigned e = (unsigned)lds(tl_a + 4 * q);
+                    const int c = e & 255;
+                    sts(slot + 4 * swz(c), lds(lab_a + 4 * q));
+                    sts(lab_a + 4 * q, nodes[e >> 16].x);
+                }
                 __syncwarp();
             }
         }
-        if (right) {
+        int c2 = 0;
+        if (y & ITEM_RIGHT) {
             // (lanes reading one word at the same time need not see the same value)
             if (__builtin_expect(__any_sync(FULLMASK, c0 < 0), 0)) {
                 if (!warp_wait(P, Hin + t, true, c0)) return FLOW_FAILED;
-                if (t + 1 < R) c1 = ld_relaxed(Hin + t + 1);
-                if (t + 2 < R) c2 = ld_relaxed(Hin + t + 2);
+                c1 = ld_relaxed(Hin + min(t + 1, R - 1));
             }
+            c2 = ld_relaxed(Hin + min(t + 2, R - 1));
         }
         // ---- the row's cells, before the suffix maximum ----
         unsigned top = zeros;  // a tree row's far row is the table's border
+        int far[W];
         if (!trow) {
             top = stk_a + ((sp - 1) & (SC - 1)) * PITCH_B;
             if (__builtin_expect(sp - 1 < lo, 0)) {  // the top of the stack left the window: bring it back
@@ -584,74 +589,65 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
                 for (int k = 0; k < W; k++) sts(top + 4 * lane + 128 * k, g[32 * k]);
                 __syncwarp();
             }
-            if (xwarp) {  // some far columns lie in stripes to the right: the far row's exports
-                const int32_t *erow = E + (int64_t)(t - ((int)(y & XTED_ROW_ORL_MASK) + 1 - i)) * X;
-                if (LISTS) {
-                    if (__builtin_expect(__any_sync(FULLMASK, (iv[0] | iv[1]) < 0), 0)) {
-                        if (!warp_wait(P, erow + xq[0], iv[0] < 0, iv[0]) || !warp_wait(P, erow + xq[1], iv[1] < 0, iv[1]))
-                            return FLOW_FAILED;
-                    }
-                    sts(top + 4 * (IMP + lane), iv[0]);
-                    if (nx > 32) sts(top + 4 * (IMP + 32 + lane), iv[1]);
-                    __syncwarp();
-                } else if (STRIPE) {
-#pragma unroll
-                    for (int k = 0; k < W; k++) {
-                        const bool lack = ((xfar >> k) & 1u) && pfw[k] < 0;
-                        if (__any_sync(FULLMASK, lack) && !warp_wait(P, erow + (lack ? fb[k] : 0), lack, pfw[k]))
-                            return FLOW_FAILED;
-                    }
+            if (y & ITEM_IMPORTS) {  // some far columns lie in stripes to the right: the far row's exports
+                if (__builtin_expect(__any_sync(FULLMASK, (iv[0] | iv[1]) < 0), 0)) {
+                    const int i = __shfl_sync(FULLMASK, bi, tl);
+                    const int32_t *erow = E + (unsigned)(t - ((int)(y & XTED_ROW_ORL_MASK) + 1 - i)) * (unsigned)X;  // (R X < 2^32)
+                    if (!warp_wait(P, erow + xq[0], iv[0] < 0, iv[0]) || !warp_wait(P, erow + xq[1], iv[1] < 0, iv[1]))
+                        return FLOW_FAILED;
                 }
+                sts(top + 4 * (IMP + lane), iv[0]);
+                sts(top + 4 * (IMP + 32 + lane), iv[1]);
+                __syncwarp();
             }
         }
 #pragma unroll
-        for (int k = 0; k < W; k++) {
-            int far;
-            if (STRIPE && !LISTS) {
-                const bool x = (xfar >> k) & 1u;
-                far = lds(top + (x ? 4 * ZERO : fb[k]));
-                if (x && !trow) far = pfw[k];
-            } else {
-                far = lds(top + fb[k]);
-            }
-            if (MULTI) far = max(far, key[k]);  // a path column's far value is its segment's border
-            a[k] = __viaddmax_s32(a[k], far, prev[k]);
-        }
-        // ---- suffix maximum: the lane's columns (two chains when there are 16), then the lanes ----
-        constexpr int H = W > 8 ? W / 2 : W;
+        for (int k = 0; k < W; k++) far[k] = lds(top + fb[k]);
+        if (OVER && !trow) {  // more than have a place: straight from their words
+            const int i = __shfl_sync(FULLMASK, bi, tl);
+            const int32_t *erow = E + (unsigned)(t - ((int)(y & XTED_ROW_ORL_MASK) + 1 - i)) * (unsigned)X;  // (R X < 2^32)
+            const int32_t *map = P.smap + P.chunkx[it.chunk].map - P.krd[ch.k_lo];
+#pragma unroll 1
+            for (int k = 0; k < W; k++) {  // through the first import place, free on this path once all are stored
+                const bool over = (xover >> k) & 1u;
+                int v = 0;
+                const int f = over ? (nodes[sbase + lane * W + k].y & XTED_ROW_ORL_MASK) + 1 : 0;
+                if (!warp_wait(P, over ? erow + map[f] : erow, over, v)) return FLOW_FAILED;
 #pragma unroll
-        for (int k = W - 2; k >= 0; k--)
-            if (k != H - 1) a[k] = max(a[k], a[k + 1]);
-        int mine = W > 8 ? max(a[0], a[H]) : a[0];
-        if (STRIPE && lane == 31) mine = max(mine, c0);
-        const int incl = warp_suffix_max(mine);
+                for (int h = 0; h < W; h++)
+                    if (over && h == k) far[h] = v;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < W; k++)  // a path column's far value is its segment's border
+            a[k] = __viaddmax_s32(a[k], max(far[k], key[k]), prev[k]);
+        // ---- suffix maximum: the lane's columns, then the lanes ----
+#pragma unroll
+        for (int k = W - 2; k >= 0; k--) a[k] = max(a[k], a[k + 1]);
+        const int incl = warp_suffix_max(lane == 31 ? max(a[0], c0) : a[0]);
         int carry = __shfl_down_sync(FULLMASK, incl, 1);
-        if (lane == 31) carry = STRIPE ? c0 : 0;
-        const int carry_lo = W > 8 ? max(carry, a[H]) : carry;
+        if (lane == 31) carry = c0;
 #pragma unroll
-        for (int k = 0; k < W; k++) prev[k] = max(a[k], k < H ? carry_lo : carry);
+        for (int k = 0; k < W; k++) prev[k] = max(a[k], carry);
         // ---- what others read ----
-        if (left && lane == 0) st_relaxed(Hout + t, prev[0]);
-        if (LISTS && (y & (ROW_TREE | ROW_NEXTTREE))) {
+        if ((y & ITEM_LEFT) && lane == 0) st_relaxed(Hout + t, prev[0]);
+        if (y & (ROW_TREE | ROW_NEXTTREE)) {
             // the row goes into its own ring slot (free until the next row's
             // copies): the next row's diagonal, and this row's path columns
-#pragma unroll
-            for (int g = 0; g < NG; g++)
-                sts4(slot + coff[g], make_int4(prev[4 * g], prev[4 * g + 1], prev[4 * g + 2], prev[4 * g + 3]));
+            sts4(slot + coff0, make_int4(prev[0], prev[1], prev[2], prev[3]));
+            sts4(slot + coff1, make_int4(prev[4], prev[5], prev[6], prev[7]));
             if (trow) {
                 __syncwarp();
-                int32_t *o = dt + (int64_t)i * pitch + sbase;
-#pragma unroll
-                for (int h = 0; h < 2; h++)
-                    if (h == 0 || nt > 32)
-                        if (lane + 32 * h < nt) st_relaxed(o + (tq[h] & 1023), lds(slot + (((unsigned)tq[h] >> 8) & 0xffcu)));
+                int32_t *o = dt + (int64_t)__shfl_sync(FULLMASK, bi, tl) * pitch;
+#pragma unroll 1
+                for (int q0 = 0; q0 < nt; q0 += 32) {
+                const int q = q0 + lane;
+                if (q >= nt) continue;
+                    const unsigned e = (unsigned)lds(tl_a + 4 * q);
+                    const int c = e & 255;
+                    st_relaxed(o + (e >> 16), lds(slot + 4 * swz(c)) - (int)((e >> 8) & 255) * XTED_KEY_BIG);
+                }
             }
-        }
-        if (!LISTS && trow) {
-            int32_t *o = dt + (int64_t)i * pitch + (MULTI ? 0 : sbase + lane * W);
-#pragma unroll
-            for (int k = 0; k < W; k++)
-                if ((tcol >> k) & 1u) st_relaxed(o + (MULTI ? node[k] : k), prev[k] - key[k]);
         }
         if (y & ROW_LAST) {  // the table is done
 #pragma unroll
@@ -680,45 +676,39 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
 #pragma unroll
                 for (int k = 0; k < W; k++) sts(d + 4 * lane + 128 * k, prev[k]);
                 sp++;
-                if (LISTS && ne > 0) {
+                if (y & ITEM_EXPORTS) {  // the pushed row's exported columns
                     __syncwarp();
-                    int32_t *e = E + (int64_t)t * X + ebase + lane;
-                    if (lane < ne) st_relaxed(e, lds(d + 4 * eq[0]));
-                    if (lane + 32 < ne) st_relaxed(e + 32, lds(d + 4 * eq[1]));
-                }
-                if (STRIPE && !LISTS && expm) {
-                    int32_t *e = E + (int64_t)t * X + ebase;
-#pragma unroll
-                    for (int k = 0; k < W; k++)
-                        if ((expm >> k) & 1u) st_relaxed(e + __popc(expm & ((1u << k) - 1u)), prev[k]);
+                    int32_t *e = E + (unsigned)t * (unsigned)X + ebase;
+#pragma unroll 1
+                    for (int q0 = 0; q0 < ne; q0 += 32)
+                        if (q0 + lane < ne) st_relaxed(e + q0 + lane, lds(d + 4 * el[q0 + lane]));
                 }
             }
-            if (xwarp && !(y & ROW_NEXTTREE)) {  // the next row's far values in other stripes
-                const int nro = __shfl_sync(FULLMASK, tl + 1 < 32 ? by : ny, (tl + 1) & 31) & XTED_ROW_ORL_MASK;
-                const int32_t *e = E + (int64_t)(t + 1 - (nro + 1 - (i - 1))) * X;
-                if (LISTS) {
-                    if (lane < nx) iv[0] = ld_relaxed(e + xq[0]);
-                    if (lane + 32 < nx) iv[1] = ld_relaxed(e + xq[1]);
-                } else if (STRIPE) {
-#pragma unroll
-                    for (int k = 0; k < W; k++)
-                        if ((xfar >> k) & 1u) pfw[k] = ld_relaxed(e + fb[k]);
-                }
+            if ((y & ITEM_IMPORTS) && !(y & ROW_NEXTTREE)) {  // the next row's far values in other stripes
+                const int r = __shfl_sync(FULLMASK, tl < 31 ? bi : ni, (tl + 1) & 31);
+                const int nro = __shfl_sync(FULLMASK, tl < 31 ? by : ny, (tl + 1) & 31) & XTED_ROW_ORL_MASK;
+                const int32_t *e = E + (unsigned)(t - nro + r) * (unsigned)X;
+                if (lane < nx) iv[0] = ld_relaxed(e + xq[0]);
+                if (lane + 32 < min(nx, FLOW_IMPORTS)) iv[1] = ld_relaxed(e + xq[1]);
             }
         }
         c0 = c1;
         c1 = c2;
         if (tl == 31) {
             bi = ni, by = ny, bl = nl;
-            load_rows(t + 33 + lane, ni, ny, nl);
-            ai = __shfl_sync(FULLMASK, bi, (lane + PF - 1) & 31);
-            const int o = __shfl_sync(FULLMASK, ni, (lane + PF - 1) & 31);
-            if (lane + PF - 1 >= 32) ai = o;
+            load_rows(t + 33 + lane);
         }
     }
     cp_async_wait<0>();
     __syncwarp();
     return 0;
+}
+
+// (Inline: a call anywhere in the kernel makes every shuffle of the loop check for divergence, 29.1 against 25.1 ms on
+// 1,500 pairs of 200-500 nodes.)
+__device__ __forceinline__ int run_item_over(const XKernelParams &P, const XItem &it, const XPair &pr, const XRun &run,
+                                          const XChunk &ch, unsigned zeros, int32_t *ring, int32_t *gstk) {
+    return run_item<true>(P, it, pr, run, ch, zeros, ring, gstk);
 }
 
 // Trace record of an item (XTED_TRACE): claim, start and end time, and
@@ -803,16 +793,14 @@ __device__ void finish_served(const XKernelParams &P, const XPair &pr, const XIt
     }
 }
 
-// Three blocks of four warps per SM: 73 KB of shared memory and up to 168
-// registers a thread each (16 columns a lane hold the row above, far indices
-// and, in a stripe, the far values of other stripes in registers).
-__global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, 3) xted_flow_kernel(const __grid_constant__ XKernelParams P) {
+// Four blocks of four warps per SM: 48 KB of shared memory a block, 128 registers a thread.
+__global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, 4) xted_flow_kernel(const __grid_constant__ XKernelParams P) {
     extern __shared__ __align__(16) int32_t s_dyn[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int32_t *ring = s_dyn + FLOW_ZERO + warp * FLOW_WARP_INTS;
+    int32_t *ring = s_dyn + FLOW_PITCH + warp * FLOW_WARP_INTS;
     int32_t *gstk = P.scratch + (int64_t)(blockIdx.x * XTED_FLOW_WARPS + warp) * P.scratch_per_warp;
     for (int x = lane; x < FLOW_WARP_INTS; x += 32) ring[x] = 0;
-    for (int x = threadIdx.x; x < FLOW_ZERO; x += blockDim.x) s_dyn[x] = 0;
+    for (int x = threadIdx.x; x < FLOW_PITCH; x += blockDim.x) s_dyn[x] = 0;
     __syncthreads();
     for (;;) {
         int g = -1, slot = 0;
@@ -832,19 +820,13 @@ __global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, 3) xted_flow_kernel(cons
         const XPair pr = P.pairs[it.pair];
         const XRun run = P.runs[it.run];
         const XChunk ch = P.chunks[it.chunk];
-        int rc = 0;
-        if (it.pair == P.hold_pair && run.depth + ch.depth == 0) {
-            // test hook: nothing that reads this table's values becomes ready
-        } else if (ch.nseg > 1) {
-            rc = run_item<8, true, false>(P, it, pr, run, ch, smem_addr(s_dyn), ring, gstk);
-        } else if ((P.krd[ch.k_lo] & (XTED_PITCH - 1)) + ch.width <= 256) {
-            rc = run_item<8, false, true>(P, it, pr, run, ch, smem_addr(s_dyn), ring, gstk);
-            if (rc == FLOW_LISTS) rc = run_item<8, false, false>(P, it, pr, run, ch, smem_addr(s_dyn), ring, gstk);
-        } else {
-            rc = run_item<16, false, true>(P, it, pr, run, ch, smem_addr(s_dyn), ring, gstk);
-            if (rc == FLOW_LISTS) rc = run_item<16, false, false>(P, it, pr, run, ch, smem_addr(s_dyn), ring, gstk);
+        // (test hook: of a held pair, nothing that reads its level 0 becomes ready)
+        const bool held = it.pair == P.hold_pair && run.depth + ch.depth == 0;
+        if (!held) {
+            int rc = run_item<false>(P, it, pr, run, ch, smem_addr(s_dyn), ring, gstk);
+            if (rc == FLOW_OVER) rc = run_item_over(P, it, pr, run, ch, smem_addr(s_dyn), ring, gstk);
+            if (rc) break;
         }
-        if (rc) break;
         if (lane == 0) {
             // run and chunk of the two roots: the pair's last table (its leftmost stripe ends last)
             if (P.serve) {

@@ -697,7 +697,7 @@ int load(xted_ctx *c, ServeState *s, const xted_tree *tr, int32_t ntrees) {
     rc |= dev_alloc(s, &s->d_ctl, XTED_CTL_INTS);
     rc |= dev_alloc(s, &s->d_slot, 4 * XTED_SERVE_SLOTS);
     rc |= dev_alloc(s, &s->d_err, 8);
-    rc |= dev_alloc(s, &s->d_dt, (size_t)dt_cap + XTED_SW);  // (slack: see ctx_prepare)
+    rc |= dev_alloc(s, &s->d_dt, (size_t)dt_cap);
     // per-warp scratch: the far-row stack's rows outside the shared window
     const int64_t per = (int64_t)H.stack_rows * XTED_SW;
     rc |= dev_alloc(s, &s->d_scratch, (size_t)per * (size_t)c->grid * XTED_FLOW_WARPS);

@@ -173,7 +173,7 @@ struct XEntry {
 // there yet waits for it: every word that one item writes for another starts
 // at -1 and is written once, with a value >= 0.
 #define XTED_PITCH 4          // rows of a table start on 16 bytes
-#define XTED_SW 512           // columns of a stripe: the widest slice one warp holds (16 per lane)
+#define XTED_SW 256           // columns of a stripe: the widest slice one warp holds (8 per lane)
 #define XTED_FLOW_WARPS 4     // warps per block, each with its own shared memory
 
 struct XItem {
