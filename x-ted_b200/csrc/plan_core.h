@@ -347,6 +347,11 @@ XT_HD inline void orient_tree(const PlanPools &P, int ot) {
     P.otrees[ot] = O;
 }
 
+// The decomposition of a pair of non-empty trees: 0 right path, 1 left path.
+XT_HD inline int pair_orientation(const DTree &A, const DTree &B, int orientation) {
+    return orientation == XTED_ORIENT_LEFT || (orientation == XTED_ORIENT_AUTO && A.S[1] * B.S[1] < A.S[0] * B.S[0]);
+}
+
 // Orientation, level count and table offset of pair p.
 XT_HD inline void pair_setup(const DTree *trees, const DOTree *ot, const int32_t *pair_trees, int orientation,
                              int p, DPair *pairs) {
@@ -363,9 +368,8 @@ XT_HD inline void pair_setup(const DTree *trees, const DOTree *ot, const int32_t
     if (A.n == 0 || B.n == 0) {  // X-TED_CPU/TED.cpp:181-186
         q.trivial = A.n == 0 ? B.n : A.n;
     } else {
-        const int64_t cr = A.S[0] * B.S[0], cl = A.S[1] * B.S[1];
-        q.o = orientation == XTED_ORIENT_LEFT || (orientation == XTED_ORIENT_AUTO && cl < cr);
-        q.cells = q.o ? cl : cr;
+        q.o = pair_orientation(A, B, orientation);
+        q.cells = A.S[q.o] * B.S[q.o];
         q.L = ot[2 * q.ta + q.o].D + ot[2 * q.tb + q.o].D + 1;
     }
     pairs[p] = q;

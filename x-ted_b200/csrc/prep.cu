@@ -4,10 +4,10 @@
 // for every depth level fetches, sizes, sorts and bins tables with host
 // round trips (X-TED_CPU/TED.cpp:163-166, X-TED_GPU/parallel_X_TED.cu:184-224,
 // 304-387). Here the raw trees go up once and everything else is built on the
-// device, one warp per tree / oriented tree, one thread per pair / (pair, level):
+// device, a warp or a block per tree / oriented tree, one thread per pair / (pair, level):
 //
-//   k_tree_basic_warp  sizes, depths, parents, keyroot-size sums (both decompositions)
-//   k_orient_warp  per orientation: node records, kdepth, keyroots by depth,
+//   k_tree_basic   sizes, depths, parents, keyroot-size sums (both decompositions)
+//   k_orient       per orientation: node records, kdepth, keyroots by depth,
 //                  column-list positions, row runs, column chunks (the records
 //                  plan_core.h's orient_tree builds for the host planners)
 //   k_pair_setup   decomposition choice, level count
@@ -33,92 +33,6 @@ namespace xted {
 
 namespace {
 
-// The outputs of tree_basic (plan_core.h: sizes, depths and parents of every
-// node, the keyroot-size sums of both decompositions) with a warp per tree
-// and the work spread over its lanes instead of one thread walking the tree:
-// parents straight from the child lists; each node's orl (rightmost leaf) by
-// pointer jumping along last children, its size orl - v + 1; depths as a
-// prefix sum of +1 at every node and -1 just past its subtree (u is an
-// ancestor of v exactly when u <= v <= orl(u)); the sums as lane sums. One
-// thread per tree waited on a dependent global load per node visited.
-__global__ void k_tree_basic_warp(PlanPools P, DTree *trees_out) {
-    const int lane = threadIdx.x & 31;
-    const int t = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (t >= P.ntrees) return;  // whole warps: t is the same in every lane
-    DTree T = P.trees[t];
-    const int n = T.n;
-    const int32_t *off = P.raw + T.raw + n, *idx = P.raw + T.raw + 2 * n + 1;
-    int32_t *size = P.size + T.nbase, *depth = P.depth + T.nbase, *par = P.parent + T.nbase;
-    int32_t *jump = P.opar + 2 * (int64_t)T.nbase;  // scratch: this tree's orientation pool, unused until k_orient_warp
-    T.S[0] = T.S[1] = 0;
-    if (n > 0) {
-        for (int v = lane; v < n; v += 32) {
-            const int32_t lo = off[v], hi = off[v + 1];
-            for (int32_t e = lo; e < hi; e++) par[idx[e]] = v;
-            size[v] = hi > lo ? idx[hi - 1] : v;  // last child, or the node itself for a leaf
-        }
-        if (lane == 0) par[0] = -1;
-        __syncwarp();
-        int32_t *cur = size, *nxt = jump;
-        for (int round = 0; round < 32; round++) {
-            bool changed = false;
-            for (int v = lane; v < n; v += 32) {
-                const int32_t a = cur[v], b = cur[a];
-                nxt[v] = b;
-                changed |= b != a;
-            }
-            __syncwarp();
-            int32_t *tmp = cur;
-            cur = nxt;
-            nxt = tmp;
-            if (!__any_sync(0xffffffffu, changed)) break;
-        }
-        // cur[v] = orl(v). Depth: +1 at every u, -1 at orl(u) + 1, then an inclusive prefix sum
-        for (int v = lane; v < n; v += 32) depth[v] = 0;
-        __syncwarp();
-        for (int u = lane; u < n; u += 32) {
-            atomicAdd(&depth[u], 1);
-            const int32_t o1 = cur[u] + 1;
-            if (o1 < n) atomicSub(&depth[o1], 1);
-        }
-        __syncwarp();
-        const int per = (n + 31) / 32, a0 = min(lane * per, n), a1 = min(a0 + per, n);
-        int32_t sum = 0;
-        for (int v = a0; v < a1; v++) sum += depth[v];
-        int32_t incl = sum;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int32_t o = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d) incl += o;
-        }
-        int32_t run = incl - sum;
-        for (int v = a0; v < a1; v++) {
-            run += depth[v];
-            depth[v] = run - 1;
-        }
-        __syncwarp();
-        for (int v = lane; v < n; v += 32) size[v] = cur[v] - v + 1;
-        __syncwarp();
-        int64_t sr = 0, sl = 0;
-        for (int v = lane; v < n; v += 32) {
-            const int32_t lo = off[v], hi = off[v + 1];
-            for (int32_t e = lo; e < hi; e++) {
-                const int64_t z = size[idx[e]];
-                if (e != hi - 1) sr += z;
-                if (e != lo) sl += z;
-            }
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            sr += __shfl_down_sync(0xffffffffu, sr, d);
-            sl += __shfl_down_sync(0xffffffffu, sl, d);
-        }
-        T.S[0] = sr + size[0];
-        T.S[1] = sl + size[0];
-    }
-    if (lane == 0) trees_out[t] = T;
-}
-
 __device__ __forceinline__ int warp_incl_sum(int v, int lane) {
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -128,26 +42,186 @@ __device__ __forceinline__ int warp_incl_sum(int v, int lane) {
     return v;
 }
 
-// One warp per oriented tree: the same records as orient_tree (plan_core.h,
-// which the host planners run), with its passes spread over the lanes (a
-// thread per oriented tree took 10 ms for the 8,192 trees of the 4,096-pair
-// batch, its passes waiting on one global load after another; this takes 1.8).
-//   * node records and the previous-node-is-leaf flags: one node per lane;
+// The threads that plan one tree together: a warp for trees of up to
+// PLAN_WARP_NODES nodes (four trees to a block), a block of 1,024 threads
+// beyond. A batch's thousands of small trees fill the GPU with warps; one
+// large tree leaves it idle: the two 20,000-node caterpillars took 2.2 ms in
+// k_tree_basic and 13.1 ms in k_orient with a warp each.
+#define PLAN_WARP_NODES 1024
+#define PLAN_BLOCK_TREES 296  // more trees than this (two blocks an SM) fill the GPU with a warp each
+template <int NT>
+struct Team {
+    static constexpr int WARPS = NT / 32;
+    int tid;
+    int *part;  // shared, [WARPS + 1] (blocks)
+    __device__ void sync() const {
+        if (NT == 32) __syncwarp();
+        else __syncthreads();
+    }
+    // inclusive sum over the team's threads, and its total
+    __device__ int incl_sum(int v, int *total) const {
+        const int lane = tid & 31, w = tid >> 5;
+        int x = warp_incl_sum(v, lane);
+        if (NT == 32) {
+            *total = __shfl_sync(0xffffffffu, x, 31);
+            return x;
+        }
+        if (lane == 31) part[w] = x;
+        __syncthreads();
+        if (w == 0) {
+            const int y = warp_incl_sum(lane < WARPS ? part[lane] : 0, lane);
+            if (lane < WARPS) part[lane] = y;
+        }
+        __syncthreads();
+        if (w > 0) x += part[w - 1];
+        *total = part[WARPS - 1];
+        __syncthreads();
+        return x;
+    }
+    __device__ bool any(bool p) const {
+        if (NT == 32) return __any_sync(0xffffffffu, p);
+        return __syncthreads_or(p) != 0;
+    }
+};
+
+// The outputs of tree_basic (plan_core.h: sizes, depths and parents of every
+// node, the keyroot-size sums of both decompositions), with the work spread
+// over the team: parents straight from the child lists; each node's orl
+// (rightmost leaf) by pointer jumping along last children, its size orl - v +
+// 1; depths as a prefix sum of +1 at every node and -1 just past its subtree (u
+// is an ancestor of v exactly when u <= v <= orl(u)); the sums as thread sums.
+template <int NT>
+__global__ void k_tree_basic(PlanPools P, DTree *trees_out) {
+    __shared__ int part[33];
+    const Team<NT> team{NT == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x, part};
+    const int t = NT == 32 ? (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) : (int)blockIdx.x;
+    if (t >= P.ntrees) return;  // whole teams
+    DTree T = P.trees[t];
+    const int n = T.n, tid = team.tid;
+    const int32_t *off = P.raw + T.raw + n, *idx = P.raw + T.raw + 2 * n + 1;
+    int32_t *size = P.size + T.nbase, *depth = P.depth + T.nbase, *par = P.parent + T.nbase;
+    int32_t *jump = P.opar + 2 * (int64_t)T.nbase;  // scratch: this tree's orientation pool, unused until k_orient
+    if (n > 0) {
+        for (int v = tid; v < n; v += NT) {
+            const int32_t lo = off[v], hi = off[v + 1];
+            for (int32_t e = lo; e < hi; e++) par[idx[e]] = v;
+            size[v] = hi > lo ? idx[hi - 1] : v;  // last child, or the node itself for a leaf
+            depth[v] = 0;
+        }
+        if (tid == 0) par[0] = -1;
+        team.sync();
+        int32_t *cur = size, *nxt = jump;
+        for (int round = 0; round < 32; round++) {
+            bool changed = false;
+            for (int v = tid; v < n; v += NT) {
+                const int32_t a = cur[v], b = cur[a];
+                nxt[v] = b;
+                changed |= b != a;
+            }
+            team.sync();
+            int32_t *tmp = cur;
+            cur = nxt;
+            nxt = tmp;
+            if (!team.any(changed)) break;
+        }
+        // cur[v] = orl(v). Depth: +1 at every u, -1 at orl(u) + 1, then an inclusive prefix sum
+        for (int u = tid; u < n; u += NT) {
+            atomicAdd(&depth[u], 1);
+            const int32_t o1 = cur[u] + 1;
+            if (o1 < n) atomicSub(&depth[o1], 1);
+        }
+        team.sync();
+        int carry = 0;
+        for (int base = 0; base < n; base += NT) {
+            const int v = base + tid;
+            int total;
+            const int x = team.incl_sum(v < n ? __ldcg(&depth[v]) : 0, &total);
+            if (v < n) depth[v] = carry + x - 1;
+            carry += total;
+        }
+        for (int v = tid; v < n; v += NT) size[v] = cur[v] - v + 1;
+        team.sync();
+        // keyroot-size sums, right path and left path: all subtree sizes less
+        // those of last (first) children
+        int64_t sr = 0, sl = 0;
+        for (int v = tid; v < n; v += NT) {
+            const int32_t lo = off[v], hi = off[v + 1];
+            const int64_t z = size[v];
+            sr += z;
+            sl += z;
+            if (hi > lo) {
+                sr -= size[idx[hi - 1]];
+                sl -= size[idx[lo]];
+            }
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            sr += __shfl_down_sync(0xffffffffu, sr, d);
+            sl += __shfl_down_sync(0xffffffffu, sl, d);
+        }
+        if (NT == 32) {
+            T.S[0] = sr;
+            T.S[1] = sl;
+        } else {
+            __shared__ int64_t acc[2][32];
+            if ((tid & 31) == 0) {
+                acc[0][tid >> 5] = sr;
+                acc[1][tid >> 5] = sl;
+            }
+            __syncthreads();
+            T.S[0] = T.S[1] = 0;
+            for (int w = 0; w < Team<NT>::WARPS; w++) {
+                T.S[0] += acc[0][w];
+                T.S[1] += acc[1][w];
+            }
+        }
+    } else {
+        T.S[0] = T.S[1] = 0;
+    }
+    if (tid == 0) trees_out[t] = T;
+}
+
+// The decomposition of every pair (as pair_setup chooses it), so that k_orient
+// builds each tree in the orientations that some pair needs only: the left
+// path of a caterpillar has a keyroot depth per spine node and took nearly all
+// of its planning, for nothing.
+__global__ void k_pair_orient(const DTree *trees, const int32_t *pair_trees, int orientation, int npairs,
+                              int32_t *need) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= npairs) return;
+    const int ta = pair_trees[2 * p], tb = pair_trees[2 * p + 1];
+    const DTree &A = trees[ta], &B = trees[tb];
+    if (A.n == 0 || B.n == 0) return;
+    const int o = pair_orientation(A, B, orientation);
+    need[2 * ta + o] = 1;
+    need[2 * tb + o] = 1;
+}
+
+// One team per oriented tree: the records of orient_tree (plan_core.h, which
+// the host planners run), with its passes spread over the threads:
+//   * node records and the previous-node-is-leaf flags: one node per thread;
 //   * A(x), the keyroots on x's root path (x included): a prefix sum over
 //     preorder of +1 at each keyroot and -1 just past its subtree;
 //   * keyroot depth kd(u) = (max of A over u's subtree) - A(u), the height of u
-//     among the keyroots nested in it: each lane scans the subtrees of its
-//     keyroots (the keyroot-size sum of the tree in all);
-//   * keyroots grouped by depth in preorder: a counting sort, 32 nodes at a time,
-//     lanes of one depth ranked by lane;
-//   * row runs and column chunks per depth: sizes and column positions loaded
-//     and summed 32 keyroots at a time, the greedy packing then decided by the
-//     whole warp from shuffled sizes (every lane holds the same packing state).
-__global__ void k_orient_warp(PlanPools P) {
+//     among the keyroots nested in it: each thread scans the subtrees of its
+//     keyroots, over the maxima of 32 nodes at a time where they fit;
+//   * keyroots grouped by depth in preorder: a counting sort by one warp, 32
+//     nodes at a time, lanes of one depth ranked by lane;
+//   * row runs and column chunks per depth, a depth per warp: sizes and column
+//     positions loaded and summed 32 keyroots at a time, the greedy packing
+//     then decided by the whole warp from shuffled sizes (every lane holds the
+//     same packing state). A depth's runs and chunks start at its first keyroot's
+//     place in the pools, so the depths do not wait for each other. The launch
+//     takes chunks of every width alike: all count as narrow.
+template <int NT>
+__global__ void k_orient(PlanPools P, const int32_t *need) {
     const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int ot = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (ot >= 2 * P.ntrees) return;  // whole warps
+    __shared__ int part[33];
+    __shared__ int s_maxa;
+    const Team<NT> team{NT == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x, part};
+    const int ot = NT == 32 ? (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) : (int)blockIdx.x;
+    if (ot >= 2 * P.ntrees) return;  // whole teams
+    const int tid = team.tid, lane = tid & 31, warp = tid >> 5;
     const int t = ot >> 1, o = ot & 1;
     const DTree T = P.trees[t];
     const int n = T.n;
@@ -159,8 +233,8 @@ __global__ void k_orient_warp(PlanPools P) {
     O.maxka = 0;
     O.maxw_wide = 0;
     O.S = T.S[o];
-    if (n == 0) {
-        if (lane == 0) P.otrees[ot] = O;
+    if (n == 0 || !need[ot]) {
+        if (tid == 0) P.otrees[ot] = O;
         return;
     }
     const int32_t *lab = P.raw + T.raw;
@@ -168,29 +242,26 @@ __global__ void k_orient_warp(PlanPools P) {
     const int32_t *idx = P.raw + T.raw + 2 * n + 1;
     const int32_t *size = P.size + T.nbase, *depth = P.depth + T.nbase, *par = P.parent + T.nbase;
     int2 *node = P.node + O.node_base;
-    int32_t *opar = P.opar + O.node_base, *okd = P.okd + O.node_base, *oka = P.oka + O.node_base;
+    int32_t *okd = P.okd + O.node_base, *oka = P.oka + O.node_base, *bmax = P.opar + O.node_base;
     // node records in this orientation
-    for (int v = lane; v < n; v += 32) {
+    for (int v = tid; v < n; v += NT) {
         const int32_t u = o ? mirror_id(v, n, size, depth) : v;
         bool kr = true;
         if (v > 0) {
             const int32_t p = par[v];
             kr = o ? idx[off[p]] != v : idx[off[p + 1] - 1] != v;
-            opar[u] = o ? mirror_id(p, n, size, depth) : p;
-        } else {
-            opar[u] = -1;
         }
         node[u].x = lab[v];
         node[u].y = (int32_t)((uint32_t)(u + size[v] - 1) | (kr ? XTED_ROW_ISKR : 0u));
         oka[u] = 0;
     }
-    __syncwarp();
-    for (int u = 1 + lane; u < n; u += 32) {
+    team.sync();
+    for (int u = 1 + tid; u < n; u += NT) {
         const int32_t prev_orl = node[u - 1].y & XTED_ROW_ORL_MASK;  // (its flag bits may change meanwhile)
         if (prev_orl == u - 1) node[u].y = (int32_t)((uint32_t)node[u].y | XTED_ROW_PREVLEAF);
     }
     // A(x): +1 at a keyroot, -1 just past its subtree, summed over preorder
-    for (int u = lane; u < n; u += 32) {
+    for (int u = tid; u < n; u += NT) {
         const int32_t y = node[u].y;
         if (y & XTED_ROW_ISKR) {
             atomicAdd(&oka[u], 1);
@@ -198,88 +269,101 @@ __global__ void k_orient_warp(PlanPools P) {
             if (e < n) atomicSub(&oka[e], 1);
         }
     }
-    __syncwarp();
+    if (tid == 0) s_maxa = 1;
+    team.sync();
     int carry = 0, maxa = 1;
-    for (int base = 0; base < n; base += 32) {
-        const int x = base + lane;
-        const int dv = x < n ? __ldcg(&oka[x]) : 0;
-        const int a = carry + warp_incl_sum(dv, lane);
+    for (int base = 0; base < n; base += NT) {
+        const int x = base + tid;
+        int total;
+        const int a = carry + team.incl_sum(x < n ? __ldcg(&oka[x]) : 0, &total);
         if (x < n) {
             oka[x] = a;
             maxa = max(maxa, a);
         }
-        carry = __shfl_sync(FULL, a, 31);
+        const int wm = __reduce_max_sync(FULL, x < n ? a : 0);
+        if (lane == 0 && x < n) bmax[x >> 5] = wm;  // the maximum of 32 nodes
+        carry += total;
     }
-    for (int d = 16; d > 0; d >>= 1) maxa = max(maxa, __shfl_xor_sync(FULL, maxa, d));
-    O.maxka = maxa;
-    __syncwarp();
+    maxa = __reduce_max_sync(FULL, maxa);
+    if (NT == 32) {
+        O.maxka = maxa;
+        __syncwarp();
+    } else {
+        if (lane == 0) atomicMax(&s_maxa, maxa);
+        __syncthreads();
+        O.maxka = s_maxa;
+    }
     // keyroot depths
-    for (int u = lane; u < n; u += 32) {
+    DDepth *dep = P.depths + O.depth_base;
+    for (int u = tid; u < n; u += NT) {
         const int32_t y = node[u].y;
         int kd = -1;
         if (y & XTED_ROW_ISKR) {
-            const int e = y & XTED_ROW_ORL_MASK, au = oka[u];
-            int m = au;
-            for (int x = u + 1; x <= e; x++) m = max(m, oka[x]);
+            const int e = (y & XTED_ROW_ORL_MASK) + 1, au = oka[u];
+            int m = au, x = u + 1;
+            for (; x < e && (x & 31); x++) m = max(m, oka[x]);
+            for (; x + 32 <= e; x += 32) m = max(m, bmax[x >> 5]);
+            for (; x < e; x++) m = max(m, oka[x]);
             kd = m - au;
         }
         okd[u] = kd;
     }
-    __syncwarp();
+    team.sync();
     const int D = okd[0];  // the root is a keyroot
     O.D = D;
     // keyroots grouped by depth (counting sort, preorder inside a depth)
-    DDepth *dep = P.depths + O.depth_base;
-    for (int d = lane; d <= D; d += 32) {
+    for (int d = tid; d <= D; d += NT) {
         dep[d].krd_lo = 0;
         dep[d].krd_hi = 0;
     }
-    __syncwarp();
-    for (int u = lane; u < n; u += 32)
+    team.sync();
+    for (int u = tid; u < n; u += NT)
         if (okd[u] >= 0) atomicAdd(&dep[okd[u]].krd_hi, 1);
-    __syncwarp();
+    team.sync();
     carry = O.node_base;
-    for (int base = 0; base <= D; base += 32) {
-        const int d = base + lane;
+    for (int base = 0; base <= D; base += NT) {
+        const int d = base + tid;
         const int c = d <= D ? __ldcg(&dep[d].krd_hi) : 0;
-        const int incl = warp_incl_sum(c, lane);
+        int total;
+        const int incl = team.incl_sum(c, &total);
         if (d <= D) {
             dep[d].krd_lo = carry + incl - c;
             dep[d].krd_hi = carry + incl - c;  // fill cursor
         }
-        carry += __shfl_sync(FULL, incl, 31);
+        carry += total;
     }
-    __syncwarp();
-    const unsigned below = (1u << lane) - 1u;
-    for (int base = 0; base < n; base += 32) {
-        const int u = base + lane;
-        const int kd = u < n ? okd[u] : -1;
-        const unsigned same = __match_any_sync(FULL, kd);  // lanes holding keyroots of this depth
-        if (kd >= 0) {
-            const int leader = __ffs(same) - 1;
-            int at = 0;
-            if (lane == leader) {
-                at = dep[kd].krd_hi;
-                dep[kd].krd_hi = at + __popc(same);
+    team.sync();
+    if (NT == 32 || warp == 0) {
+        const unsigned below = (1u << lane) - 1u;
+        for (int base = 0; base < n; base += 32) {
+            const int u = base + lane;
+            const int kd = u < n ? okd[u] : -1;
+            const unsigned same = __match_any_sync(FULL, kd);  // lanes holding keyroots of this depth
+            if (kd >= 0) {
+                const int leader = __ffs(same) - 1;
+                int at = 0;
+                if (lane == leader) {
+                    at = dep[kd].krd_hi;
+                    dep[kd].krd_hi = at + __popc(same);
+                }
+                at = __shfl_sync(same, at, leader);
+                P.krd[at + __popc(same & below)] = u;
             }
-            at = __shfl_sync(same, at, leader);
-            P.krd[at + __popc(same & below)] = u;
+            __syncwarp();
         }
-        __syncwarp();
     }
+    team.sync();
     // column-list positions, row runs and chunks per depth
     int run_rows, nw, hw;
     tree_granularity(P, n, &run_rows, &nw, &hw);
     const int group_w = nw > 0 ? nw : XTED_NARROW_MAX;
-    const int half_w = hw > nw ? (hw < XTED_HALF_MAX ? hw : XTED_HALF_MAX) : nw;
-    int32_t run_cur = O.node_base, chunk_cur = O.node_base;
-    for (int d = 0; d <= D; d++) {
+    for (int d = warp; d <= D; d += Team<NT>::WARPS) {
         DDepth dd = dep[d];  // krd_lo, krd_hi
         const int klo = dd.krd_lo, khi = dd.krd_hi;
-        // runs
-        dd.run_lo = run_cur;
-        dd.maxrows = 0;
-        int pos = 0, r_lo = -1, r_hi = -1, r_rows = 0;
+        int run_cur = klo, chunk_cur = klo;
+        dd.run_lo = dd.chunk_lo = klo;
+        dd.maxrows = dd.maxw_n = 0;
+        int pos = 0, r_lo = klo, r_rows = 0, c_lo = klo, c_w = 0;
         for (int kb = klo; kb < khi; kb += 32) {
             const int k = kb + lane;
             int sz = 0;
@@ -292,80 +376,39 @@ __global__ void k_orient_warp(PlanPools P) {
             pos += __shfl_sync(FULL, incl, 31);
             const int cnt = min(32, khi - kb);
             for (int j = 0; j < cnt; j++) {
-                const int szj = __shfl_sync(FULL, sz, j);
-                if (r_lo >= 0 && r_rows + szj > run_rows) {
-                    if (r_rows > dd.maxrows) dd.maxrows = r_rows;
-                    if (lane == 0) P.runs[run_cur] = XRun{r_lo, r_hi, r_rows, d};
+                const int szj = __shfl_sync(FULL, sz, j), kk = kb + j;
+                if (r_rows > 0 && r_rows + szj > run_rows) {
+                    dd.maxrows = max(dd.maxrows, r_rows);
+                    if (lane == 0) P.runs[run_cur] = XRun{r_lo, kk, r_rows, d};
                     run_cur++;
-                    r_lo = -1;
+                    r_lo = kk;
                     r_rows = 0;
                 }
-                if (r_lo < 0) r_lo = kb + j;
-                r_hi = kb + j + 1;
                 r_rows += szj;
+                if (c_w > 0 && c_w + szj > group_w) {
+                    dd.maxw_n = max(dd.maxw_n, c_w);
+                    if (lane == 0) P.chunks[chunk_cur] = XChunk{c_lo, c_w, d, kk - c_lo};
+                    chunk_cur++;
+                    c_lo = kk;
+                    c_w = 0;
+                }
+                c_w += szj;
             }
         }
-        if (r_lo >= 0) {
-            if (r_rows > dd.maxrows) dd.maxrows = r_rows;
-            if (lane == 0) P.runs[run_cur] = XRun{r_lo, r_hi, r_rows, d};
-            run_cur++;
+        dd.maxrows = max(dd.maxrows, r_rows);
+        dd.maxw_n = max(dd.maxw_n, c_w);
+        if (lane == 0) {
+            P.runs[run_cur] = XRun{r_lo, khi, r_rows, d};
+            P.chunks[chunk_cur] = XChunk{c_lo, c_w, d, khi - c_lo};
         }
-        dd.run_hi = run_cur;
-        // chunks: three passes, narrow chunks first, then half-block ones, then whole-block ones
-        dd.chunk_lo = chunk_cur;
-        dd.nnarrow = dd.nwide = dd.nhalf = 0;
-        dd.maxw_n = dd.maxw_w = dd.maxw_h = 0;
-        for (int pass = 0; pass < 3; pass++) {
-            int c_lo = -1, c_w = 0, c_n = 0;
-            bool done = false;
-            for (int kb = klo; kb <= khi && !done; kb += 32) {
-                const int k = kb + lane;
-                int w = 0;
-                if (k < khi) {
-                    const int32_t u = P.krd[k];
-                    w = (node[u].y & XTED_ROW_ORL_MASK) - u + 1;
-                }
-                const int cnt = min(32, khi + 1 - kb);
-                for (int j = 0; j < cnt; j++) {
-                    const int kk = kb + j;
-                    const int wj = __shfl_sync(FULL, w, j);
-                    const bool flush = c_n > 0 && (kk == khi || c_w + wj > group_w);
-                    if (flush) {
-                        const int kind = c_w <= nw ? 0 : (c_w <= half_w ? 1 : 2);
-                        if (kind == pass) {
-                            if (lane == 0) P.chunks[chunk_cur] = XChunk{c_lo, c_w, d, c_n};
-                            chunk_cur++;
-                            if (kind == 2) {
-                                dd.nwide++;
-                                if (c_w > dd.maxw_w) dd.maxw_w = c_w;
-                            } else if (kind == 1) {
-                                dd.nhalf++;
-                                if (c_w > dd.maxw_h) dd.maxw_h = c_w;
-                            } else {
-                                dd.nnarrow++;
-                                if (c_w > dd.maxw_n) dd.maxw_n = c_w;
-                            }
-                        }
-                        c_lo = -1;
-                        c_w = 0;
-                        c_n = 0;
-                    }
-                    if (kk == khi) {
-                        done = true;
-                        break;
-                    }
-                    if (c_n == 0) c_lo = kk;  // first segment (keyroot pool index)
-                    c_w += wj;
-                    c_n += 1;
-                }
-            }
-        }
-        if (dd.maxw_h > O.maxw_wide) O.maxw_wide = dd.maxw_h;
-        if (dd.maxw_w > O.maxw_wide) O.maxw_wide = dd.maxw_w;
+        dd.run_hi = run_cur + 1;
+        dd.nnarrow = chunk_cur + 1 - klo;
+        dd.nhalf = dd.nwide = 0;
+        dd.maxw_h = dd.maxw_w = 0;
         if (lane == 0) dep[d] = dd;
         __syncwarp();
     }
-    if (lane == 0) P.otrees[ot] = O;
+    if (tid == 0) P.otrees[ot] = O;
 }
 
 __global__ void k_pair_setup(const DTree *trees, const DOTree *ot, const int32_t *pair_trees, int orientation,
@@ -509,7 +552,7 @@ __global__ void k_depth_totals(PlanPools P, XChunkX *chunkx) {
     const int lane = threadIdx.x & 31;
     const int ot = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (ot >= 2 * P.ntrees) return;
-    const DOTree O = P.otrees[ot];
+    const DOTree O = P.otrees[ot];  // (D = -1: not built)
     for (int d = 0; d <= O.D; d++) {
         DDepth &dd = P.depths[O.depth_base + d];
         const int lo = dd.chunk_lo, hi = lo + dd.nnarrow + dd.nhalf + dd.nwide;
@@ -798,7 +841,7 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     need += 3 * sizeof(int32_t) * (size_t)std::max<int64_t>(N, 1);  // size, depth, parent
     need += N2 * (sizeof(int2) + 2 * sizeof(int32_t) + sizeof(XRun) + sizeof(XChunk) + sizeof(XChunkX) + 4 * sizeof(int32_t));
     need += sizeof(DDepth) * (N2 + 2 * (size_t)T) + sizeof(DOTree) * 2 * (size_t)T + sizeof(DTree) * (size_t)T +
-            2 * sizeof(int32_t) * (size_t)T;
+            4 * sizeof(int32_t) * (size_t)T;
     need += (size_t)npairs * (sizeof(DPair) + sizeof(XPair) + 4 + 4 * 8) + 24 * 256 + sizeof(Summary);
     rc = ctx_dev_reserve(c, c->meta, need);
     if (rc) return rc;
@@ -843,15 +886,19 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     int64_t *d_dts = cv.take<int64_t>((size_t)npairs + 1);
     XChunkX *d_chunkx = cv.take<XChunkX>(N2);
     int32_t *d_list = cv.take<int32_t>(N2);
-    int32_t *d_used = cv.take<int32_t>(2 * (size_t)T);
+    int32_t *d_used = cv.take<int32_t>(2 * (size_t)T), *d_need = cv.take<int32_t>(2 * (size_t)T);
     Summary *d_sum = cv.take<Summary>(1);
     if (cv.off > c->meta.cap) return XTED_ENOMEM;
     const bool stripes = maxn + XTED_PITCH > XTED_SW;  // some chunk may be wider than a warp holds
 
     const int BS = 128;
     cudaMemsetAsync(d_used, 0, (size_t)((char *)(d_sum + 1) - (char *)d_used), s);
-    k_tree_basic_warp<<<blocks_for(32 * (int64_t)T, BS), BS, 0, s>>>(P, d_trees);
-    k_orient_warp<<<blocks_for(64 * (int64_t)T, BS), BS, 0, s>>>(P);
+    const bool big = maxn > PLAN_WARP_NODES && T <= PLAN_BLOCK_TREES;
+    if (big) k_tree_basic<1024><<<(unsigned)T, 1024, 0, s>>>(P, d_trees);
+    else k_tree_basic<32><<<blocks_for(32 * (int64_t)T, BS), BS, 0, s>>>(P, d_trees);
+    k_pair_orient<<<blocks_for(std::max(npairs, 1), BS), BS, 0, s>>>(d_trees, d_pt, c->opts.orientation, npairs, d_need);
+    if (big) k_orient<1024><<<2 * (unsigned)T, 1024, 0, s>>>(P, d_need);
+    else k_orient<32><<<blocks_for(64 * (int64_t)T, BS), BS, 0, s>>>(P, d_need);
     k_pair_setup<<<blocks_for(std::max(npairs, 1), BS), BS, 0, s>>>(d_trees, P.otrees, d_pt, c->opts.orientation, npairs,
                                                                     d_pairs, d_L, d_cells, d_used);
     k_scan64<<<1, 1024, 0, s>>>(d_L, npairs, d_Ls);
