@@ -1,0 +1,75 @@
+"""One pair planned by one block (needs a B200): sizes around the block's
+1,024 threads and the limit of the one-block plan, against the batch's planner
+(which a prepared batch uses) and the oracle; plans that do not fit its lists;
+and the arena entry point's own checks of its trees."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle
+import xted
+from xted import _lib, gen, trees
+
+pytestmark = pytest.mark.gpu
+
+
+def _noalloc(a, b):
+    keep = []
+    ta, tb = _lib.ctree(a, keep), _lib.ctree(b, keep)
+    out = ctypes.c_int32(-1)
+    return _lib.lib().xted_distance_noalloc(ctypes.byref(ta), ctypes.byref(tb), 0, ctypes.byref(out)), out.value
+
+
+@pytest.mark.timeout(300)
+@pytest.mark.parametrize("m,n", [(1, 1), (1, 300), (32, 33), (257, 256), (1023, 260), (1024, 1025), (2048, 2048), (2049, 2048)])
+def test_sizes(m, n):
+    for k, (sa, sb) in enumerate((("random", "random"), ("wide", "deep"), ("caterpillar", "random"))):
+        a, b = gen.tree(sa, m, 3 * m + k, "uniform", 5), gen.tree(sb, n, 7 * n + k, "uniform", 5)
+        want = int(oracle.distance_batch([(a, b)], nthreads=8)[0])
+        with xted.Context() as ctx:
+            assert ctx.distance(a, b) == want
+            cells = ctx.stats()["cells"]
+            ctx.prepare_batch([(a, b)])
+            assert int(ctx.run_prepared()[0]) == want
+            assert ctx.stats()["cells"] == cells
+        rc, d = _noalloc(a, b)
+        assert (rc, d) == (xted.XTED_ETOOBIG, -1) if m > 1500 else (0, want)
+
+
+def _nested(n):
+    adj = [[c for c in (v + 1, v + 2) if c < n] if v % 2 == 0 and v + 1 < n else [] for v in range(n)]
+    return trees.from_adjacency([v % 3 for v in range(n)], adj)
+
+
+@pytest.mark.timeout(300)
+def test_plans_that_do_not_fit():
+    a = _nested(801)  # keyroot depth 400: more levels than the one-block plan lists
+    b = gen.tree("random", 90, 5, "uniform", 3)
+    for x, y in ((a, b), (b, a), (a, a)):
+        want = int(oracle.distance_batch([(x, y)], nthreads=8)[0])
+        with xted.Context(orientation=xted.ORIENT_RIGHT) as ctx:
+            assert ctx.distance(x, y) == want
+        assert _noalloc(x, y) == (0, want)
+    wide, small = gen.tree("wide", 60000, 9, "uniform", 3), gen.tree("random", 3, 1, "uniform", 3)
+    want = int(oracle.distance_batch([(wide, small)], nthreads=8)[0])
+    assert _noalloc(wide, small) == (0, want)  # its plan is larger than the arena
+    assert _noalloc(small, small)[0] == 0
+
+
+@pytest.mark.timeout(300)
+def test_arena_checks_trees_like_the_host():
+    rng = np.random.default_rng(3)
+    bad = 0
+    for k in range(120):
+        t = gen.tree(("random", "wide", "deep")[k % 3], int(rng.integers(2, 70)), k, "uniform", 4)
+        labels, off, idx = (np.array(x, dtype=np.int32) for x in (t.labels, t.off, t.idx))
+        for _ in range(int(rng.integers(1, 3))):
+            arr = off if rng.integers(2) else idx
+            arr[int(rng.integers(len(arr)))] += int(rng.integers(-2, 3)) if k % 4 else int(rng.choice([-2**30, 2**30]))
+        c = trees.Tree(labels, off, idx)
+        keep = []
+        want = _lib.lib().xted_validate(ctypes.byref(_lib.ctree(c, keep)))
+        assert _noalloc(c, t)[0] == want and _noalloc(t, c)[0] == want
+        bad += want != 0
+    assert 30 < bad < 120

@@ -91,15 +91,81 @@ int ctx_host_reserve(HostBuf &b, size_t bytes) {
     return XTED_OK;
 }
 
+// One pair is planned by one block up to this many nodes together, by the
+// batch's kernels beyond. A call on two trees of 40 nodes takes 165 us this way
+// and 239 the other, of 1,000 nodes each 1,531 and 1,730, of 2,048 each 2,701
+// and 2,720; of 2,500 each the batch's kernels are level.
+#define XTED_PAIR_NODES 4096
+// Its items, hand-off words and stacks: what does not fit is planned by the batch's kernels.
+#define XTED_PAIR_ROOM ((size_t)32 << 20)
+
+// Lays one pair out and enqueues its plan; nothing is read back (ctx_run finds
+// out whether the plan fitted).
+static int pair_prepare(xted_ctx *c, const xted_tree &a, const xted_tree &b) {
+    const xted_tree *t[2] = {&a, &b};
+    for (int k = 0; k < 2; k++) {
+        const int rc = validate_tree(TreeView{t[k]->n, t[k]->labels, t[k]->child_off, t[k]->child_idx});
+        if (rc) return rc;
+    }
+    PairLayout &L = c->pair;
+    pair_layout(nullptr, 0, a.n, b.n, &L);
+    const size_t fixed = (size_t)((char *)L.room - (char *)nullptr);
+    int rc = ctx_dev_reserve(c, c->meta, fixed + XTED_PAIR_ROOM);
+    if (!rc) rc = ctx_host_reserve(c->stage, (size_t)L.upload_ints * 4);
+    if (!rc) rc = ctx_host_reserve(c->result, (PAIR_HDR_INTS + 1) * sizeof(int32_t));
+    if (rc) return rc;
+    pair_layout(c->meta.p, fixed + XTED_PAIR_ROOM, a.n, b.n, &L);
+    L.P.run_rows = c->opts.run_rows;
+    L.P.narrow_width = c->opts.narrow_width;
+    L.P.half_width = c->opts.half_width == 0 ? XTED_HALF_DEFAULT : c->opts.half_width;
+    L.P.ntune = 0;
+    if (c->opts.tuned) {
+        int nt = 0;
+        const XTuneRow *tt = ctx_tune_table(c, &nt);
+        for (int k = 0; k < nt && k < XTED_TUNE_ROWS; k++) L.P.tune[L.P.ntune++] = tt[k];
+    }
+    int32_t *h = (int32_t *)c->stage.p;
+    std::memset(h + L.upload_ints - PAIR_HDR_INTS, 0, PAIR_HDR_INTS * sizeof(int32_t));
+    for (int k = 0; k < 2; k++) {
+        const size_t n = (size_t)t[k]->n;
+        std::memcpy(h, t[k]->labels, 4 * n);
+        std::memcpy(h + n, t[k]->child_off, 4 * (n + 1));
+        if (n > 1) std::memcpy(h + 2 * n + 1, t[k]->child_idx, 4 * (n - 1));
+        h += 3 * n + 1;
+    }
+    c->h2d_bytes = L.upload_ints * 4;
+    if (cudaMemcpyAsync(L.raw, c->stage.p, (size_t)c->h2d_bytes, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
+        launch_plan_pair(L, c->opts.orientation, false, c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        return XTED_ECUDA;
+    }
+    XKernelParams &K = c->kp;
+    std::memset(&K, 0, sizeof(K));
+    pair_params(L, K);
+    K.c_del = c->opts.cost_del;
+    K.c_ins = c->opts.cost_ins;
+    K.c_ren = c->opts.cost_ren;
+    K.timeout_ns = (uint64_t)(c->opts.wait_timeout_s * 1e9);
+    c->npairs = 1;
+    c->prepared = true;
+    return XTED_OK;
+}
+
 // Plans a batch on the device (prep.cu) and sizes every buffer the DP launch
 // needs; the kernel parameters stay in the context so the batch can be run
-// repeatedly from device-resident inputs.
-int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs) {
+// repeatedly from device-resident inputs. With one_block, one small pair is
+// planned by a block instead (not under a memory limit, whose lists are sized
+// by reading their lengths back, nor for a trace of the items).
+int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs, bool one_block) {
     c->prepared = false;
     ctx_drop_graph(c);  // the graph holds the previous plan's buffers and sizes
     for (int32_t p = 0; p < npairs; p++)
         if (!costs_fit(c->opts, a[p].n, b[p].n)) return XTED_EINVAL;
     XKernelParams &K = c->kp;
+    const char *tr = std::getenv("XTED_TRACE");
+    if (one_block && npairs == 1 && a->n > 0 && b->n > 0 && (int64_t)a->n + b->n <= XTED_PAIR_NODES &&
+        c->opts.mem_limit == 0 && !(tr && *tr))
+        return pair_prepare(c, *a, *b);
     int rc = dev_plan(c, a, b, npairs, K);
     if (rc) return rc;
     K.c_del = c->opts.cost_del;
@@ -127,7 +193,6 @@ int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npa
     K.timeout_ns = (uint64_t)(c->opts.wait_timeout_s * 1e9);
     // Optional per-item trace (XTED_TRACE=<file>): timestamps of every item,
     // written as raw uint64 quadruples after each run.
-    const char *tr = std::getenv("XTED_TRACE");
     K.trace = nullptr;
     if (tr && *tr && K.nitems > 0) {
         rc = ctx_dev_reserve(c, c->trace, (size_t)K.nitems * 4 * sizeof(unsigned long long));
@@ -151,6 +216,21 @@ static int enqueue_step(xted_ctx *c, bool events) {
     int32_t *hres = (int32_t *)c->result.p;
     const size_t res_bytes = (size_t)npairs * sizeof(int32_t);
     if (events && cudaEventRecord(c->ev0, c->stream) != cudaSuccess) return XTED_ECUDA;
+    if (K.plan) {
+        const PairLayout &L = c->pair;
+        const int grid = pair_grid(c->grid, L.m, L.n);
+        if ((c->runs_prepared > 1 &&  // (the first run finds the words zero, as uploaded)
+             cudaMemsetAsync(L.hdr, 0, PAIR_CTL_INTS * sizeof(int32_t), c->stream) != cudaSuccess) ||
+            launch_pair_clear(L, grid, c->stream) != cudaSuccess ||
+            (events && cudaEventRecord(c->evk0, c->stream) != cudaSuccess) ||
+            launch_dp(K, grid, c->stream) != cudaSuccess ||
+            (events && cudaEventRecord(c->evk1, c->stream) != cudaSuccess) ||
+            (events && cudaEventRecord(c->ev1, c->stream) != cudaSuccess) ||
+            cudaMemcpyAsync(hres, L.hdr, (PAIR_HDR_INTS + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream) !=
+                cudaSuccess)
+            return XTED_ECUDA;
+        return XTED_OK;
+    }
     // per-run reset: the error words and the claim counter; every table and hand-off word to -1 (not written)
     if (cudaMemsetAsync(cnt, 0, 8 * sizeof(int32_t), c->stream) != cudaSuccess ||
         (K.nitems > 0 &&
@@ -240,6 +320,22 @@ int ctx_run(xted_ctx *c, int32_t *out, bool allow_graph) {
     c->stats.device_ms = ms;
     c->stats.dp_ms = kms;
     c->stats.h2d_bytes = c->h2d_bytes;
+    if (K.plan) {
+        const XPlanOut plan = *(const XPlanOut *)(hres + PAIR_OUT);
+        c->stats.d2h_bytes = (PAIR_HDR_INTS + 1) * sizeof(int32_t);
+        c->stats.grid = pair_grid(c->grid, c->pair.m, c->pair.n);
+        if (plan.status != 0) return plan.status;
+        c->kp.nitems = plan.items;  // (for the statistics: the launch reads the plan's)
+        c->plan_cells = plan.cells;
+        c->plan_cells_right = plan.cells_right;
+        c->plan_levels_max = plan.levels;
+        std::memcpy(c->err_info, hres + PAIR_ERROR + 1, sizeof(c->err_info));
+        if (hres[PAIR_ERROR] != 0) return hres[PAIR_ERROR];
+        const int32_t v = hres[PAIR_HDR_INTS];  // the root table's saving
+        if (v < 0) return XTED_ETIMEOUT;
+        out[0] = c->pair.m * K.c_del + c->pair.n * K.c_ins - v;
+        return XTED_OK;
+    }
     c->stats.d2h_bytes = (int64_t)(res_bytes + 8 * sizeof(int32_t));
     c->stats.grid = c->grid;
     std::memcpy(c->err_info, hres + 2, sizeof(c->err_info));
@@ -384,8 +480,8 @@ int xted_distance_batch(xted_ctx *c, const xted_tree *a, const xted_tree *b, int
     if (!c || npairs < 0 || (npairs > 0 && (!a || !b || !out))) return XTED_EINVAL;
     const double t0 = now_ms();
     if (cudaSetDevice(c->opts.device) != cudaSuccess) return XTED_ECUDA;
-    int rc = ctx_prepare(c, a, b, npairs);
-    const double t1 = now_ms();
+    int rc = ctx_prepare(c, a, b, npairs, true);
+    double t1 = now_ms();
     std::memset(&c->stats, 0, sizeof(c->stats));
     if (rc) return rc;
     const bool hold = c->fault == XTED_FAULT_HOLD_PAIR && npairs > 0;
@@ -394,6 +490,13 @@ int xted_distance_batch(xted_ctx *c, const xted_tree *a, const xted_tree *b, int
         c->kp.hold_pair = 0;
     }
     rc = ctx_run(c, out, false);
+    if (rc == PLAN_OVERFLOW) {  // one pair, planned by one block: a list did not fit
+        rc = ctx_prepare(c, a, b, npairs, false);
+        t1 = now_ms();
+        if (rc) return rc;
+        if (hold) c->kp.hold_pair = 0;
+        rc = ctx_run(c, out, false);
+    }
     c->kp.hold_pair = -1;
     fill_stats(c, t1 - t0);
     c->stats.total_ms = now_ms() - t0;
@@ -404,7 +507,7 @@ int xted_prepare_batch(xted_ctx *c, const xted_tree *a, const xted_tree *b, int3
     if (!c || npairs < 0 || (npairs > 0 && (!a || !b))) return XTED_EINVAL;
     if (cudaSetDevice(c->opts.device) != cudaSuccess) return XTED_ECUDA;
     const double t0 = now_ms();
-    int rc = ctx_prepare(c, a, b, npairs);
+    int rc = ctx_prepare(c, a, b, npairs, false);
     std::memset(&c->stats, 0, sizeof(c->stats));
     if (rc) return rc;
     c->prep_ms = now_ms() - t0;

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/xted.h"
+#include "pair_plan.h"
 #include "plan.h"
 #include "plan_core.h"
 
@@ -56,6 +57,7 @@ struct xted_ctx {
     int32_t plan_stack_rows = 1, plan_levels_max = 0;
     // the prepared plan (xted_prepare_batch / every batch call)
     XKernelParams kp{};
+    xted::PairLayout pair;    // kp.plan set: one pair, planned by one block (pair_plan.h)
     int32_t npairs = 0;
     int64_t h2d_bytes = 0;
     double prep_ms = 0;
@@ -72,7 +74,7 @@ int ctx_dev_reserve(xted_ctx *c, DevBuf &b, size_t bytes);
 // A pair of m and n nodes fits the row scan's key range under the context's costs.
 bool costs_fit(const xted_opts &o, int64_t m, int64_t n);
 int ctx_host_reserve(HostBuf &b, size_t bytes);
-int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs);
+int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs, bool one_block);
 int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs, XKernelParams &K);
 int ctx_run(xted_ctx *c, int32_t *out, bool allow_graph);
 void ctx_drop_graph(xted_ctx *c);

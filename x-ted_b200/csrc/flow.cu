@@ -661,13 +661,13 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
                 if (__builtin_expect((unsigned)(sp - lo) >= (unsigned)SC, 0)) {
                     if (sp < lo) {
                         lo = sp - 1;
-                    } else if (lo < P.stack_rows) {  // the window is full: its lowest row moves out
+                    } else if (lo < (P.plan ? P.plan->stack_rows : P.stack_rows)) {  // the window is full: its lowest row moves out
                         int32_t *g = gstk + (int64_t)lo * ZERO + lane;
                         const unsigned d = stk_a + (lo & (SC - 1)) * PITCH_B + 4 * lane;
 #pragma unroll 1
                         for (int k = 0; k < W; k++) g[32 * k] = lds(d + 128 * k);
                     } else if (lane == 0) {
-                        set_error(P, XTED_ENOMEM, 2, lo, P.stack_rows);
+                        set_error(P, XTED_ENOMEM, 2, lo, 0);
                     }
                     lo++;
                 }
@@ -798,10 +798,14 @@ __global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, 4) xted_flow_kernel(cons
     extern __shared__ __align__(16) int32_t s_dyn[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int32_t *ring = s_dyn + FLOW_PITCH + warp * FLOW_WARP_INTS;
-    int32_t *gstk = P.scratch + (int64_t)(blockIdx.x * XTED_FLOW_WARPS + warp) * P.scratch_per_warp;
+    const int nitems = P.plan ? P.plan->items : P.nitems;
+    const int64_t per = P.plan ? (int64_t)P.plan->stack_rows * XTED_SW : P.scratch_per_warp;
+    const int64_t gwarp = (int64_t)blockIdx.x * XTED_FLOW_WARPS + warp;
+    int32_t *gstk = P.scratch + (P.plan ? -(gwarp + 1) * per : gwarp * per);
     for (int x = lane; x < FLOW_WARP_INTS; x += 32) ring[x] = 0;
     for (int x = threadIdx.x; x < FLOW_PITCH; x += blockDim.x) s_dyn[x] = 0;
     __syncthreads();
+    if (P.plan && (gwarp + 1) * per > P.plan->scratch) return;
     for (;;) {
         int g = -1, slot = 0;
         uint64_t t_claim = P.trace ? global_ns() : 0;
@@ -810,7 +814,7 @@ __global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, 4) xted_flow_kernel(cons
         } else {
             if (lane == 0 && ld_relaxed(P.error) == 0) {
                 g = atomicAdd(P.next, 1);
-                if (g >= P.nitems) g = -1;
+                if (g >= nitems) g = -1;
             }
             g = __shfl_sync(FULLMASK, g, 0);
         }
@@ -868,23 +872,11 @@ int dp_occupancy(int *blocks_per_sm) {
                                                               FLOW_SMEM);
 }
 
-// Cooperative launch (every warp resident at once: a waiting warp never keeps
-// the one it waits for off the GPU), expressed as a launch attribute so that
-// the same call also records into a CUDA graph.
+// A plain launch: a block that is not resident has claimed nothing, and what
+// the resident warps have claimed needs only items claimed before.
 cudaError_t launch_dp(const XKernelParams &P, int grid, cudaStream_t s) {
-    XKernelParams p = P;
-    void *args[] = {&p};
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(32 * XTED_FLOW_WARPS);
-    cfg.dynamicSmemBytes = FLOW_SMEM;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelExC(&cfg, (const void *)xted_flow_kernel, args);
+    xted_flow_kernel<<<grid, 32 * XTED_FLOW_WARPS, FLOW_SMEM, s>>>(P);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_gather(const XPair *pairs, const int32_t *trivial, const int32_t *dt, int npairs, int32_t *out,

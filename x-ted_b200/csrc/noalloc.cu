@@ -23,8 +23,14 @@
 // pool makes one warm-up call at start-up, before it does so. The caller's
 // current device is restored before every return.
 //
-// Algorithm: the same right-path keyroot decomposition as the batched path
-// (orl(v) = v + size(v) - 1 in preorder; keyroots = root and every child that
+// The pair is planned by one block (k_plan_pair, prep.cu) and run by the
+// batched path's DP kernel (flow.cu), whose warps each need room for a stack
+// in what the plan leaves of the arena; warps that find none leave. A pair of
+// 300 and 251 nodes took 37.4 ms in the kernel below and takes 0.62 ms so.
+//
+// The kernel below needs less memory and remains for pairs whose plan does not
+// fit (a tree of 60,000 nodes against one of a few, or very many tables): the
+// same right-path keyroot decomposition as the batched path (orl(v) = v + size(v) - 1 in preorder; keyroots = root and every child that
 // is not a last child), tables processed by keyroot level
 // kd(i0) + kd(j0) so that every tree-distance entry a table reads was written
 // at a lower level. One block; each warp fills whole tables row by row, the
@@ -36,6 +42,12 @@
 #include <mutex>
 
 #include "xted.h"
+#include "pair_plan.h"
+
+namespace xted {
+int dp_occupancy(int *blocks_per_sm);
+cudaError_t launch_dp(const XKernelParams &P, int grid, cudaStream_t s);
+}  // namespace xted
 
 namespace {
 
@@ -241,11 +253,13 @@ __global__ void __launch_bounds__(kThreads) xted_noalloc_kernel(int32_t *A, Layo
     }
 }
 
-// Per-device arena address, looked up once with that device current.
+// Per-device arena address and DP grid, looked up once with that device
+// current; the kernels are loaded then, too (nothing is left to a later call).
 std::mutex g_setup_mu;
 int32_t *g_arena_ptr[kMaxDevices];
+int g_grid[kMaxDevices];
 
-int arena_for(int device, int32_t **out) {
+int arena_for(int device, int32_t **out, int *grid) {
     std::lock_guard<std::mutex> lock(g_setup_mu);
     if (!g_arena_ptr[device]) {
         cudaDeviceProp prop;
@@ -259,18 +273,60 @@ int arena_for(int device, int32_t **out) {
             cudaGetLastError();
             return XTED_ECUDA;
         }
+        int occ = 0;
+        cudaFuncAttributes fa;
+        if (xted::dp_occupancy(&occ) != 0 || occ < 1 || xted::pair_kernels_load() != cudaSuccess ||
+            cudaFuncGetAttributes(&fa, xted_noalloc_kernel) != cudaSuccess) {
+            cudaGetLastError();
+            return XTED_ECUDA;
+        }
+        g_grid[device] = occ * prop.multiProcessorCount;
         g_arena_ptr[device] = (int32_t *)p;
     }
     *out = g_arena_ptr[device];
+    *grid = g_grid[device];
     return XTED_OK;
 }
 
-int copy_tree(int32_t *A, const TreeRegs &r, const xted_tree &t, cudaStream_t s) {
+bool copy_tree(int32_t *lab, int32_t *off, int32_t *idx, const xted_tree &t, cudaStream_t s) {
     const size_t n = (size_t)t.n;
-    bool ok = cudaMemcpyAsync(A + r.lab, t.labels, 4 * n, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-              cudaMemcpyAsync(A + r.off, t.child_off, 4 * (n + 1), cudaMemcpyHostToDevice, s) == cudaSuccess;
-    if (ok && n > 1) ok = cudaMemcpyAsync(A + r.idx, t.child_idx, 4 * (n - 1), cudaMemcpyHostToDevice, s) == cudaSuccess;
-    return ok ? XTED_OK : XTED_ECUDA;
+    return cudaMemcpyAsync(lab, t.labels, 4 * n, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+           cudaMemcpyAsync(off, t.child_off, 4 * (n + 1), cudaMemcpyHostToDevice, s) == cudaSuccess &&
+           (n < 2 || cudaMemcpyAsync(idx, t.child_idx, 4 * (n - 1), cudaMemcpyHostToDevice, s) == cudaSuccess);
+}
+
+// The pair on the batched path's kernels; PLAN_OVERFLOW: its plan does not fit the arena.
+int run_planned(int32_t *A, int grid, const xted_tree &a, const xted_tree &b, int32_t *out, cudaStream_t s) {
+    xted::PairLayout L;
+    if (!xted::pair_layout(A, XTED_NOALLOC_ARENA_BYTES, a.n, b.n, &L)) return PLAN_OVERFLOW;
+    L.P.run_rows = 64;
+    L.P.narrow_width = XTED_SW;
+    L.P.half_width = XTED_HALF_DEFAULT;
+    L.P.ntune = 0;
+    const int64_t second = 3 * (int64_t)a.n + 1;
+    int32_t *ra = L.raw, *rb = L.raw + second;
+    XKernelParams K{};
+    xted::pair_params(L, K);
+    K.c_del = K.c_ins = K.c_ren = 1;
+    K.timeout_ns = 20000000000ull;
+    grid = xted::pair_grid(grid, a.n, b.n);
+    int32_t res[PAIR_HDR_INTS + 1];
+    if (cudaMemsetAsync(L.hdr, 0, 4 * PAIR_CTL_INTS, s) != cudaSuccess || !copy_tree(ra, ra + a.n, ra + 2 * a.n + 1, a, s) ||
+        !copy_tree(rb, rb + b.n, rb + 2 * b.n + 1, b, s) ||
+        xted::launch_plan_pair(L, XTED_ORIENT_AUTO, true, s) != cudaSuccess ||
+        xted::launch_pair_clear(L, grid, s) != cudaSuccess || xted::launch_dp(K, grid, s) != cudaSuccess ||
+        cudaMemcpyAsync(res, L.hdr, sizeof(res), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess) {
+        cudaGetLastError();
+        return XTED_ECUDA;
+    }
+    const XPlanOut *plan = (const XPlanOut *)(res + PAIR_OUT);
+    if (plan->status != 0) return plan->status;
+    if (res[PAIR_ERROR] != 0) return res[PAIR_ERROR];
+    const int32_t v = res[PAIR_HDR_INTS];  // the root table's saving
+    if (v < 0) return XTED_ETIMEOUT;
+    *out = a.n + b.n - v;
+    return XTED_OK;
 }
 
 // Restores the calling thread's current device on scope exit (the entry
@@ -305,7 +361,8 @@ extern "C" int xted_distance_noalloc(const xted_tree *a, const xted_tree *b, int
     }
     const DeviceRestore restore;
     int32_t *A = nullptr;
-    int rc = arena_for(device, &A);
+    int grid = 0;
+    int rc = arena_for(device, &A, &grid);
     if (rc) return rc;
     // Empty trees follow standard_ted's rules (the distance is the other
     // tree's size); a non-empty partner is still validated, by running it
@@ -328,10 +385,16 @@ extern "C" int xted_distance_noalloc(const xted_tree *a, const xted_tree *b, int
     if (cudaSetDevice(device) != cudaSuccess) return XTED_ECUDA;
     cudaGetLastError();  // drop a non-sticky error left by an earlier, unrelated runtime call on this thread
     cudaStream_t s = cudaStreamPerThread;
+    rc = run_planned(A, grid, *a, *b, out, s);
+    if (rc != PLAN_OVERFLOW) return rc;
     if (cudaMemsetAsync(A, 0, 4 * kHeaderInts, s) != cudaSuccess) return XTED_ECUDA;
-    rc = copy_tree(A, L.t[0], *a, s);
-    if (!rc) rc = copy_tree(A, L.t[1], *b, s);
-    if (rc) return rc;
+    for (int k = 0; k < 2; k++) {
+        const TreeRegs &r = L.t[k];
+        if (!copy_tree(A + r.lab, A + r.off, A + r.idx, k ? *b : *a, s)) {
+            cudaGetLastError();
+            return XTED_ECUDA;
+        }
+    }
     void *args[] = {&A, &L};
     if (cudaLaunchKernel((const void *)xted_noalloc_kernel, dim3(1), dim3(kThreads), args, 0, s) != cudaSuccess) {
         cudaGetLastError();

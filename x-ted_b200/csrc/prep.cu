@@ -27,6 +27,7 @@
 
 #include "ctx.h"
 #include "flow_plan.h"
+#include "pair_plan.h"
 #include "plan_core.h"
 
 namespace xted {
@@ -91,11 +92,7 @@ struct Team {
 // 1; depths as a prefix sum of +1 at every node and -1 just past its subtree (u
 // is an ancestor of v exactly when u <= v <= orl(u)); the sums as thread sums.
 template <int NT>
-__global__ void k_tree_basic(PlanPools P, DTree *trees_out) {
-    __shared__ int part[33];
-    const Team<NT> team{NT == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x, part};
-    const int t = NT == 32 ? (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) : (int)blockIdx.x;
-    if (t >= P.ntrees) return;  // whole teams
+__device__ void tree_basic_team(const Team<NT> &team, const PlanPools &P, int t, DTree *trees_out, int64_t (*acc)[32]) {
     DTree T = P.trees[t];
     const int n = T.n, tid = team.tid;
     const int32_t *off = P.raw + T.raw + n, *idx = P.raw + T.raw + 2 * n + 1;
@@ -163,7 +160,6 @@ __global__ void k_tree_basic(PlanPools P, DTree *trees_out) {
             T.S[0] = sr;
             T.S[1] = sl;
         } else {
-            __shared__ int64_t acc[2][32];
             if ((tid & 31) == 0) {
                 acc[0][tid >> 5] = sr;
                 acc[1][tid >> 5] = sl;
@@ -179,6 +175,16 @@ __global__ void k_tree_basic(PlanPools P, DTree *trees_out) {
         T.S[0] = T.S[1] = 0;
     }
     if (tid == 0) trees_out[t] = T;
+    team.sync();
+}
+
+template <int NT>
+__global__ void k_tree_basic(PlanPools P, DTree *trees_out) {
+    __shared__ int part[33];
+    __shared__ int64_t acc[2][32];
+    const Team<NT> team{NT == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x, part};
+    const int t = NT == 32 ? (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) : (int)blockIdx.x;
+    if (t < P.ntrees) tree_basic_team<NT>(team, P, t, trees_out, acc);  // whole teams
 }
 
 // The decomposition of every pair (as pair_setup chooses it), so that k_orient
@@ -214,13 +220,8 @@ __global__ void k_pair_orient(const DTree *trees, const int32_t *pair_trees, int
 //     place in the pools, so the depths do not wait for each other. The launch
 //     takes chunks of every width alike: all count as narrow.
 template <int NT>
-__global__ void k_orient(PlanPools P, const int32_t *need) {
+__device__ void orient_team(const Team<NT> &team, const PlanPools &P, int ot, bool needed, int *s_max) {
     const unsigned FULL = 0xffffffffu;
-    __shared__ int part[33];
-    __shared__ int s_maxa;
-    const Team<NT> team{NT == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x, part};
-    const int ot = NT == 32 ? (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) : (int)blockIdx.x;
-    if (ot >= 2 * P.ntrees) return;  // whole teams
     const int tid = team.tid, lane = tid & 31, warp = tid >> 5;
     const int t = ot >> 1, o = ot & 1;
     const DTree T = P.trees[t];
@@ -233,7 +234,7 @@ __global__ void k_orient(PlanPools P, const int32_t *need) {
     O.maxka = 0;
     O.maxw_wide = 0;
     O.S = T.S[o];
-    if (n == 0 || !need[ot]) {
+    if (n == 0 || !needed) {
         if (tid == 0) P.otrees[ot] = O;
         return;
     }
@@ -269,7 +270,7 @@ __global__ void k_orient(PlanPools P, const int32_t *need) {
             if (e < n) atomicSub(&oka[e], 1);
         }
     }
-    if (tid == 0) s_maxa = 1;
+    if (tid == 0) *s_max = 1;
     team.sync();
     int carry = 0, maxa = 1;
     for (int base = 0; base < n; base += NT) {
@@ -289,9 +290,9 @@ __global__ void k_orient(PlanPools P, const int32_t *need) {
         O.maxka = maxa;
         __syncwarp();
     } else {
-        if (lane == 0) atomicMax(&s_maxa, maxa);
+        if (lane == 0) atomicMax(s_max, maxa);
         __syncthreads();
-        O.maxka = s_maxa;
+        O.maxka = *s_max;
     }
     // keyroot depths
     DDepth *dep = P.depths + O.depth_base;
@@ -409,6 +410,16 @@ __global__ void k_orient(PlanPools P, const int32_t *need) {
         __syncwarp();
     }
     if (tid == 0) P.otrees[ot] = O;
+    team.sync();
+}
+
+template <int NT>
+__global__ void k_orient(PlanPools P, const int32_t *need) {
+    __shared__ int part[33];
+    __shared__ int s_max;
+    const Team<NT> team{NT == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x, part};
+    const int ot = NT == 32 ? (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) : (int)blockIdx.x;
+    if (ot < 2 * P.ntrees) orient_team<NT>(team, P, ot, need[ot] != 0, &s_max);  // whole teams
 }
 
 __global__ void k_pair_setup(const DTree *trees, const DOTree *ot, const int32_t *pair_trees, int orientation,
@@ -445,6 +456,9 @@ __global__ void k_scan64(const int64_t *v, int n, int64_t *out) {
     }
     if (tid == nt - 1) out[n] = part[nt - 1];
 }
+
+#define PLAN_PAIR_THREADS 1024
+#define ITEM_INTS ((int64_t)(sizeof(XItem) / sizeof(int32_t)))
 
 struct Summary {
     int64_t entries, dt_elems;
@@ -496,16 +510,40 @@ __global__ void k_map_reserve(PlanPools P, const int32_t *used, XChunkX *chunkx,
     }
 }
 
-// One block per striped chunk: its export map, the far columns that a stripe
+// The export map of a striped chunk, by a block: the far columns that a stripe
 // reads from a stripe to its right, numbered in column order (-1 elsewhere).
-// The tree whose node records it needs is found from the chunk's
-// keyroot pool index, which lies in the tree's range of the node pool.
+// nodes are the column tree's records. Returns the number of exports.
+template <int NT>
+__device__ int chunk_map_team(const Team<NT> &team, const XChunk &ch, const int32_t *krd, const int2 *nodes, int32_t *map) {
+    const int w = ch.width, j0 = krd[ch.k_lo], lead = j0 & (XTED_PITCH - 1), tid = team.tid;
+    for (int c = tid; c < w; c += NT) map[c] = 0;
+    team.sync();
+    for (int c = tid; c < w; c += NT) {
+        const int foff = (nodes[j0 + c].y & XTED_ROW_ORL_MASK) + 1 - (j0 + c);
+        if (far_crosses(c, foff, w, lead)) map[c + foff] = 1;
+    }
+    team.sync();
+    int before = 0;
+    for (int base = 0; base < w; base += NT) {
+        const int c = base + tid, m = c < w ? map[c] : 0;
+        int total;
+        const int incl = team.incl_sum(m, &total);
+        if (c < w) map[c] = m ? before + incl - 1 : -1;
+        before += total;
+    }
+    return before;
+}
+
+// One block per striped chunk. The tree whose node records it needs is found
+// from the chunk's keyroot pool index, which lies in the tree's range of the
+// node pool.
 __global__ void k_chunk_maps(PlanPools P, const int32_t *list, XChunkX *chunkx, int32_t *smap) {
-    __shared__ int ends[XTED_WARPS];
+    __shared__ int part[33];
     __shared__ int s_base;
-    const int c0 = list[blockIdx.x], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Team<XTED_CTA_THREADS> team{(int)threadIdx.x, part};
+    const int c0 = list[blockIdx.x];
     const XChunk ch = P.chunks[c0];
-    if (tid == 0) {  // the oriented tree whose pool range holds the chunk
+    if (team.tid == 0) {  // the oriented tree whose pool range holds the chunk
         int lo = 0, hi = 2 * P.ntrees - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -515,72 +553,48 @@ __global__ void k_chunk_maps(PlanPools P, const int32_t *list, XChunkX *chunkx, 
         s_base = P.otrees[lo].node_base;
     }
     __syncthreads();
-    const int w = ch.width, j0 = P.krd[ch.k_lo], lead = j0 & (XTED_PITCH - 1);
-    const int2 *nodes = P.node + s_base;
-    int32_t *map = smap + chunkx[c0].map;
-    for (int c = tid; c < w; c += XTED_CTA_THREADS) map[c] = 0;
-    __syncthreads();
-    for (int c = tid; c < w; c += XTED_CTA_THREADS) {
-        const int foff = (nodes[j0 + c].y & XTED_ROW_ORL_MASK) + 1 - (j0 + c);
-        if (far_crosses(c, foff, w, lead)) map[c + foff] = 1;
-    }
-    __syncthreads();
-    const int per = (w + XTED_CTA_THREADS - 1) / XTED_CTA_THREADS;
-    const int a0 = min(tid * per, w), a1 = min(a0 + per, w);
-    int cnt = 0;
-    for (int c = a0; c < a1; c++) cnt += map[c];
-    const int incl = warp_incl_sum(cnt, lane);
-    if (lane == 31) ends[warp] = incl;
-    __syncthreads();
-    int before = incl - cnt, total = 0;
-    for (int q = 0; q < XTED_WARPS; q++) {
-        if (q < warp) before += ends[q];
-        total += ends[q];
-    }
-    for (int c = a0; c < a1; c++) {
-        const int m = map[c];
-        map[c] = m ? before : -1;
-        before += m;
-    }
-    if (tid == 0) chunkx[c0].X = total;
+    const int X = chunk_map_team(team, ch, P.krd, P.node + s_base, smap + chunkx[c0].map);
+    if (team.tid == 0) chunkx[c0].X = X;
 }
 
-// A warp per oriented tree: stripes and hand-off words of its chunks summed
-// per depth (flow_depth_totals, flow_plan.h, with the lanes over the chunks).
-__global__ void k_depth_totals(PlanPools P, XChunkX *chunkx) {
+// Stripes and hand-off words of one depth's chunks summed by a warp
+// (flow_depth_totals, flow_plan.h, with the lanes over the chunks).
+__device__ void depth_totals_warp(const PlanPools &P, XChunkX *chunkx, DDepth &dd, int lane) {
     const unsigned FULL = 0xffffffffu;
+    const int lo = dd.chunk_lo, hi = lo + dd.nnarrow + dd.nhalf + dd.nwide;
+    int k = 0, w = 0;
+    for (int cb = lo; cb < hi; cb += 32) {
+        const int c = cb + lane;
+        int K = 0, words = 0;
+        if (c < hi) {
+            K = chunk_stripes(P.chunks[c], P.krd);
+            if (K == 1) chunkx[c].X = 0;
+            words = chunk_words(K, chunkx[c].X);
+        }
+        const int ki = warp_incl_sum(K, lane), wi = warp_incl_sum(words, lane);
+        if (c < hi) {
+            chunkx[c].K = K;
+            chunkx[c].kpre = k + ki - K;
+            chunkx[c].wpre = w + wi - words;
+        }
+        k += __shfl_sync(FULL, ki, 31);
+        w += __shfl_sync(FULL, wi, 31);
+    }
+    if (lane == 0) {
+        dd.nitems = k;
+        dd.wsum = w;
+        const int last = dd.run_hi - 1;
+        dd.rows = P.cumw[P.runs[last].kr_lo] + P.runs[last].rows;  // every depth up to D has a keyroot
+    }
+}
+
+// A warp per oriented tree: the totals of its depths.
+__global__ void k_depth_totals(PlanPools P, XChunkX *chunkx) {
     const int lane = threadIdx.x & 31;
     const int ot = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (ot >= 2 * P.ntrees) return;
-    const DOTree O = P.otrees[ot];  // (D = -1: not built)
-    for (int d = 0; d <= O.D; d++) {
-        DDepth &dd = P.depths[O.depth_base + d];
-        const int lo = dd.chunk_lo, hi = lo + dd.nnarrow + dd.nhalf + dd.nwide;
-        int k = 0, w = 0;
-        for (int cb = lo; cb < hi; cb += 32) {
-            const int c = cb + lane;
-            int K = 0, words = 0;
-            if (c < hi) {
-                K = chunk_stripes(P.chunks[c], P.krd);
-                if (K == 1) chunkx[c].X = 0;
-                words = chunk_words(K, chunkx[c].X);
-            }
-            const int ki = warp_incl_sum(K, lane), wi = warp_incl_sum(words, lane);
-            if (c < hi) {
-                chunkx[c].K = K;
-                chunkx[c].kpre = k + ki - K;
-                chunkx[c].wpre = w + wi - words;
-            }
-            k += __shfl_sync(FULL, ki, 31);
-            w += __shfl_sync(FULL, wi, 31);
-        }
-        if (lane == 0) {
-            dd.nitems = k;
-            dd.wsum = w;
-            const int last = dd.run_hi - 1;
-            dd.rows = P.cumw[P.runs[last].kr_lo] + P.runs[last].rows;  // every depth up to D has a keyroot
-        }
-    }
+    const DOTree O = P.otrees[ot];
+    for (int d = 0; d <= O.D; d++) depth_totals_warp(P, chunkx, P.depths[O.depth_base + d], lane);
 }
 
 // One (pair, level) of the batch.
@@ -591,16 +605,25 @@ struct Level {
     int64_t item_off, buf_off;
 };
 
-// A pair's levels: their counts, and the time left of the pair from each on.
-__global__ void k_level_count(FlowCtx C, const DPair *pairs, int npairs, Level *lv, Summary *sum) {
-    const int lane = threadIdx.x & 31;
-    const int p = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (p >= npairs) return;
-    const DPair q = pairs[p];
-    if (q.L == 0) return;
-    const DOTree A = C.ot[2 * q.ta + q.o], B = C.ot[2 * q.tb + q.o];
+// Where k_plan_pair writes, and how much fits.
+struct PairPlan {
+    int32_t n[2];  // the trees' sizes (raw: the first's arrays, then the second's)
+    int32_t orientation, check;
+    XPair *pair;
+    XChunkX *chunkx;
+    int32_t *smap, *list;
+    Level *levels;
+    int32_t *room;  // items, then hand-off words; stacks from the end down
+    XPlanOut *out;
+    int32_t cap_map, cap_list, cap_levels;
+    int64_t room_ints;
+};
+
+// A pair's levels (a warp): their counts, and the time left of the pair from
+// each on. Returns the whole pair's time.
+__device__ int64_t level_count_warp(const FlowCtx &C, const DOTree &A, const DOTree &B, int p, int L, Level *lv, int lane) {
     int64_t rem = 0;
-    for (int hi = q.L; hi > 0; hi -= 32) {  // from the last level down, 32 at a time
+    for (int hi = L; hi > 0; hi -= 32) {  // from the last level down, 32 at a time
         const int d = hi - 1 - lane;
         int64_t items = 0, words = 0, est = 0;
         if (d >= 0) flow_level_count(C, A, B, d, &items, &words, &est);
@@ -611,7 +634,7 @@ __global__ void k_level_count(FlowCtx C, const DPair *pairs, int npairs, Level *
             if (lane >= o) incl += y;
         }
         if (d >= 0) {
-            Level &E = lv[q.lvl_base + d];
+            Level &E = lv[d];
             E.pair = p;
             E.level = d;
             E.items = items;
@@ -620,6 +643,16 @@ __global__ void k_level_count(FlowCtx C, const DPair *pairs, int npairs, Level *
         }
         rem += __shfl_sync(0xffffffffu, incl, 31);
     }
+    return rem;
+}
+
+__global__ void k_level_count(FlowCtx C, const DPair *pairs, int npairs, Level *lv, Summary *sum) {
+    const int lane = threadIdx.x & 31;
+    const int p = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (p >= npairs) return;
+    const DPair q = pairs[p];
+    if (q.L == 0) return;
+    const int64_t rem = level_count_warp(C, C.ot[2 * q.ta + q.o], C.ot[2 * q.tb + q.o], p, q.L, lv + q.lvl_base, lane);
     if (lane == 0) atomicMax((unsigned long long *)&sum->chain_max, (unsigned long long)rem);
 }
 
@@ -699,23 +732,210 @@ __global__ void __launch_bounds__(ORDER_THREADS) k_level_order(Level *lv, int n,
     }
 }
 
-// The items of the list, a block per level: by row depth from the deepest
-// down (the longest runs first), then by run, then by chunk.
+// The items of one level, by a block: by row depth from the deepest down (the
+// longest runs first), then by run, then by chunk.
+__device__ void level_fill_block(const FlowCtx &C, const DOTree &A, const DOTree &B, const Level &E, XItem *items) {
+    const int lo = max(E.level - B.D, 0), hi = min(A.D, E.level);
+    int64_t at = E.item_off, buf = E.buf_off;
+    for (int a = hi; a >= lo; a--) {
+        const DDepth ra = C.depths[A.depth_base + a], cb = C.depths[B.depth_base + E.level - a];
+        const int64_t n = (int64_t)(ra.run_hi - ra.run_lo) * cb.nitems;
+        for (int64_t k = threadIdx.x; k < n; k += blockDim.x) items[at + k] = flow_item(C, ra, cb, E.pair, k, buf);
+        at += n;
+        buf += (int64_t)ra.rows * cb.wsum;
+    }
+}
+
 __global__ void k_level_fill(FlowCtx C, const DPair *pairs, const Level *lv, int64_t nent, XItem *items) {
     for (int64_t e = blockIdx.x; e < nent; e += gridDim.x) {
         const Level E = lv[e];
         const DPair q = pairs[E.pair];
-        const DOTree A = C.ot[2 * q.ta + q.o], B = C.ot[2 * q.tb + q.o];
-        const int lo = max(E.level - B.D, 0), hi = min(A.D, E.level);
-        int64_t at = E.item_off, buf = E.buf_off;
-        for (int a = hi; a >= lo; a--) {
-            const DDepth ra = C.depths[A.depth_base + a], cb = C.depths[B.depth_base + E.level - a];
-            const int64_t n = (int64_t)(ra.run_hi - ra.run_lo) * cb.nitems;
-            for (int64_t k = threadIdx.x; k < n; k += blockDim.x) items[at + k] = flow_item(C, ra, cb, E.pair, k, buf);
-            at += n;
-            buf += (int64_t)ra.rows * cb.wsum;
+        level_fill_block(C, C.ot[2 * q.ta + q.o], C.ot[2 * q.tb + q.o], E, items);
+    }
+}
+
+// A preorder CSR tree is well formed (validate_tree, plan.cpp, by a block, every
+// index checked before it is used): offsets rise from 0 to n - 1, every node but
+// the root is one node's child, and the children of v start at v + 1 and follow
+// each other's last nodes (cur: 2 n ints of scratch).
+template <int NT>
+__device__ bool valid_team(const Team<NT> &team, int n, const int32_t *off, const int32_t *idx, int32_t *cur) {
+    const int tid = team.tid;
+    int32_t *nxt = cur + n;
+    bool bad = off[0] != 0 || off[n] != n - 1;
+    for (int v = tid; v < n; v += NT) {
+        bad |= off[v + 1] < off[v] || off[v] < 0 || off[v + 1] > n - 1;
+        nxt[v] = 0;
+    }
+    if (team.any(bad)) return false;
+    for (int v = tid; v < n; v += NT) {
+        const int32_t lo = off[v], hi = off[v + 1];
+        int32_t last = v;
+        for (int32_t e = lo; e < hi; e++) {
+            const int32_t c = idx[e];
+            if (c <= last || c >= n || (e == lo && c != v + 1)) {
+                bad = true;
+                break;
+            }
+            atomicAdd(&nxt[c], 1);
+            last = c;
+        }
+        cur[v] = last;
+    }
+    if (team.any(bad)) return false;
+    for (int v = 1 + tid; v < n; v += NT) bad |= __ldcg(&nxt[v]) != 1;
+    if (team.any(bad)) return false;
+    for (int round = 0; round < 32; round++) {  // each node's last descendant (links rise: they end)
+        bool changed = false;
+        for (int v = tid; v < n; v += NT) {
+            const int32_t x = cur[v], y = cur[x];
+            nxt[v] = y;
+            changed |= y != x;
+        }
+        team.sync();
+        int32_t *tmp = cur;
+        cur = nxt;
+        nxt = tmp;
+        if (!team.any(changed)) break;
+    }
+    bad = cur[0] != n - 1;
+    for (int v = tid; v < n; v += NT)
+        for (int32_t e = off[v] + 1; e < off[v + 1]; e++) bad |= idx[e] != cur[idx[e - 1]] + 1;
+    return !team.any(bad);
+}
+
+// The whole plan of one pair in one block, in memory of fixed size: nothing
+// is read back, so a call on two small trees makes one launch for its plan and
+// none of its waits (a pair of 100 nodes spent 118 us on eleven planning kernels
+// and two reads; the trees of one pair never fill more than a block or two
+// anyway). out->status: 0, XTED_EINVAL (check: the trees are validated here),
+// or PLAN_OVERFLOW when a list does not fit (the launch then runs nothing).
+__global__ void __launch_bounds__(PLAN_PAIR_THREADS) k_plan_pair(PlanPools P, DTree *trees, PairPlan B) {
+    constexpr int NT = PLAN_PAIR_THREADS;
+    __shared__ int part[33];
+    __shared__ int64_t acc[2][32];
+    __shared__ int s_max, s_maps, s_nmaps;
+    const Team<NT> team{(int)threadIdx.x, part};
+    const int tid = team.tid, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        s_maps = s_nmaps = 0;
+        B.out->status = PLAN_OVERFLOW;  // until all is in place
+        B.out->items = 0;
+        B.out->stack_rows = 1;
+        B.out->words = 0;
+        B.out->scratch = 0;
+        for (int t = 0; t < P.ntrees; t++) {
+            DTree T;
+            T.n = B.n[t];
+            T.raw = t == 0 ? 0 : 3 * B.n[0] + 1;
+            T.nbase = t == 0 ? 0 : B.n[0];
+            T.t = t;
+            T.S[0] = T.S[1] = 0;
+            trees[t] = T;
         }
     }
+    __syncthreads();
+    if (B.check)
+        for (int t = 0; t < P.ntrees; t++) {
+            const DTree T = trees[t];
+            const int32_t *off = P.raw + T.raw + T.n;
+            if (!valid_team(team, T.n, off, off + T.n + 1, P.opar + 2 * (int64_t)T.nbase)) {
+                if (tid == 0) B.out->status = XTED_EINVAL;
+                return;
+            }
+        }
+    for (int t = 0; t < P.ntrees; t++) tree_basic_team(team, P, t, trees, acc);
+    const int tb = P.ntrees - 1;  // (one tree: against itself)
+    const int o = pair_orientation(trees[0], trees[tb], B.orientation);
+    for (int t = 0; t < P.ntrees; t++) orient_team(team, P, 2 * t + o, true, &s_max);
+    const DOTree A = P.otrees[o], Bt = P.otrees[2 * tb + o];
+    // striped chunks of the column tree: export maps, then the depths' totals
+    for (int d = warp; d <= Bt.D; d += NT / 32) {
+        const DDepth &dd = P.depths[Bt.depth_base + d];
+        for (int c = dd.chunk_lo + lane; c < dd.chunk_lo + dd.nnarrow; c += 32)
+            if (chunk_stripes(P.chunks[c], P.krd) > 1) {
+                B.chunkx[c].map = atomicAdd(&s_maps, P.chunks[c].width);
+                const int i = atomicAdd(&s_nmaps, 1);
+                if (i < B.cap_list) B.list[i] = c;
+            }
+    }
+    __syncthreads();
+    if (s_maps > B.cap_map || s_nmaps > B.cap_list) return;
+    for (int i = 0; i < s_nmaps; i++) {
+        const int c = B.list[i];
+        const int X = chunk_map_team(team, P.chunks[c], P.krd, P.node + Bt.node_base, B.smap + B.chunkx[c].map);
+        if (tid == 0) B.chunkx[c].X = X;
+    }
+    __syncthreads();
+    for (int t = 0; t < P.ntrees; t++) {
+        const DOTree &O = t == 0 ? A : Bt;
+        for (int d = warp; d <= O.D; d += NT / 32) depth_totals_warp(P, B.chunkx, P.depths[O.depth_base + d], lane);
+    }
+    __syncthreads();
+    FlowCtx C;
+    C.ot = P.otrees;
+    C.depths = P.depths;
+    C.runs = P.runs;
+    C.chunks = P.chunks;
+    C.chunkx = B.chunkx;
+    C.cumw = P.cumw;
+    const int L = A.D + Bt.D + 1;
+    if (L > B.cap_levels) return;
+    if (warp == 0) {
+        level_count_warp(C, A, Bt, 0, L, B.levels, lane);
+        __syncwarp();
+        if (lane == 0) {  // one pair: its levels in order
+            int64_t items = 0, words = 0;
+            for (int d = 0; d < L; d++) items += B.levels[d].items;
+            const int64_t total = items;
+            items = 0;
+            for (int d = 0; d < L; d++) {
+                Level &E = B.levels[d];
+                E.item_off = items;
+                E.buf_off = ITEM_INTS * total + words;
+                items += E.items;
+                words += E.words;
+            }
+            acc[0][0] = items;
+            acc[0][1] = words;
+        }
+    }
+    __syncthreads();
+    const int64_t items = acc[0][0], words = acc[0][1];
+    const int64_t left = B.room_ints - ITEM_INTS * items - ((words + 3) & ~(int64_t)3);
+    if (left < (A.maxka + 1) * (int64_t)XTED_SW) return;  // at least one warp's stack
+    for (int d = 0; d < L; d++) level_fill_block(C, A, Bt, B.levels[d], (XItem *)B.room);
+    if (tid == 0) {
+        XPair x;
+        x.dt_off = 0;
+        x.m = trees[0].n;
+        x.n = trees[tb].n;
+        x.row_base = A.node_base;
+        x.col_base = Bt.node_base;
+        x.pitch = table_pitch(x.n);
+        x.pad = 0;
+        *B.pair = x;
+        XPlanOut out;
+        out.items = (int32_t)items;
+        out.stack_rows = A.maxka + 1;
+        out.levels = L;
+        out.status = 0;
+        out.cells = A.S * Bt.S;
+        out.cells_right = trees[0].S[0] * trees[tb].S[0];
+        out.words = words;
+        out.scratch = left;
+        *B.out = out;
+    }
+}
+
+// A planned pair's tables and hand-off words to -1, 16 bytes a store.
+__global__ void k_pair_clear(const XPlanOut *out, int4 *dt, int64_t dt4, int32_t *room) {
+    if (out->status != 0) return;
+    const int64_t w4 = (out->words + 3) / 4, step = (int64_t)gridDim.x * blockDim.x;
+    int4 *w = (int4 *)(room + ITEM_INTS * (int64_t)out->items);
+    const int4 none = make_int4(-1, -1, -1, -1);
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < dt4 + w4; k += step)
+        *(k < dt4 ? dt + k : w + (k - dt4)) = none;
 }
 
 __global__ void k_pair_finalize(const DPair *pairs, const DTree *trees, const DOTree *ot, int npairs, XPair *xp,
@@ -751,6 +971,103 @@ struct Carver {
         return p;
     }
 };
+
+size_t pair_layout(void *base, size_t bytes, int32_t m, int32_t n, PairLayout *L) {
+    const size_t N = (size_t)m + n, N2 = 2 * N;
+    Carver cv{(char *)base};
+    L->m = m;
+    L->n = n;
+    const size_t raw_ints = (3 * N + 2 + 63) & ~(size_t)63;
+    L->dt_ints = (int64_t)m * table_pitch(n);
+    L->upload_ints = (int64_t)raw_ints + PAIR_HDR_INTS;
+    L->raw = cv.take<int32_t>(raw_ints + PAIR_HDR_INTS + (size_t)L->dt_ints);
+    L->hdr = L->raw + raw_ints;
+    L->dt = L->hdr + PAIR_HDR_INTS;
+    PlanPools &P = L->P;
+    P.raw = L->raw;
+    L->trees = cv.take<DTree>(2);
+    P.trees = L->trees;
+    P.ntrees = 2;
+    P.size = cv.take<int32_t>(N);
+    P.depth = cv.take<int32_t>(N);
+    P.parent = cv.take<int32_t>(N);
+    P.node = cv.take<int2>(N2);
+    P.krd = cv.take<int32_t>(N2);
+    P.cumw = cv.take<int32_t>(N2);
+    P.runs = cv.take<XRun>(N2);
+    P.chunks = cv.take<XChunk>(N2);
+    P.opar = cv.take<int32_t>(N2);
+    P.okd = cv.take<int32_t>(N2);
+    P.oka = cv.take<int32_t>(N2);
+    P.depths = cv.take<DDepth>(N2 + 4);
+    P.otrees = cv.take<DOTree>(4);
+    L->chunkx = cv.take<XChunkX>(N2);
+    L->list = cv.take<int32_t>((size_t)n);
+    L->cap_list = n;
+    L->cap_map = 32 * n;  // (each column of 32 tables wider than a warp holds)
+    L->smap = cv.take<int32_t>((size_t)L->cap_map);
+    L->cap_levels = 64;  // keyroot depths grow with the logarithm of the nodes
+    L->levels = cv.take<Level>((size_t)L->cap_levels);
+    L->room = cv.take<int32_t>(0);
+    const size_t used = (size_t)((char *)L->room - (char *)base);
+    if (bytes <= used) return 0;
+    L->room_ints = (int64_t)(bytes - used) / 4;
+    return used;
+}
+
+cudaError_t launch_plan_pair(const PairLayout &L, int32_t orientation, bool check, cudaStream_t s) {
+    PairPlan B;
+    B.n[0] = L.m;
+    B.n[1] = L.n;
+    B.orientation = orientation;
+    B.check = check;
+    B.pair = (XPair *)(L.hdr + PAIR_PAIR);
+    B.chunkx = L.chunkx;
+    B.smap = L.smap;
+    B.list = L.list;
+    B.levels = (Level *)L.levels;
+    B.room = L.room;
+    B.out = (XPlanOut *)(L.hdr + PAIR_OUT);
+    B.cap_map = L.cap_map;
+    B.cap_list = L.cap_list;
+    B.cap_levels = L.cap_levels;
+    B.room_ints = L.room_ints;
+    k_plan_pair<<<1, PLAN_PAIR_THREADS, 0, s>>>(L.P, L.trees, B);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pair_clear(const PairLayout &L, int32_t blocks, cudaStream_t s) {
+    k_pair_clear<<<(unsigned)blocks, 256, 0, s>>>((const XPlanOut *)(L.hdr + PAIR_OUT), (int4 *)L.dt, L.dt_ints / 4, L.room);
+    return cudaGetLastError();
+}
+
+cudaError_t pair_kernels_load() {
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, k_plan_pair);
+    return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pair_clear);
+}
+
+void pair_params(const PairLayout &L, XKernelParams &K) {
+    K.rowinfo = L.P.node;
+    K.krd = L.P.krd;
+    K.cumw = L.P.cumw;
+    K.runs = L.P.runs;
+    K.chunks = L.P.chunks;
+    K.chunkx = L.chunkx;
+    K.pairs = (const XPair *)(L.hdr + PAIR_PAIR);
+    K.items = (const XItem *)L.room;
+    K.dt = L.dt;
+    K.buf = L.room;
+    K.smap = L.smap;
+    K.scratch = L.room + L.room_ints;
+    K.plan = (const XPlanOut *)(L.hdr + PAIR_OUT);
+    K.npairs = 1;
+    K.next = L.hdr + PAIR_NEXT;
+    K.progress = L.hdr + PAIR_PROGRESS;
+    K.error = L.hdr + PAIR_ERROR;
+    K.error_info = L.hdr + PAIR_ERROR + 1;
+    K.hold_pair = -1;
+}
 
 int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs, XKernelParams &K) {
     cudaStream_t s = c->stream;

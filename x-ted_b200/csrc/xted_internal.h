@@ -192,6 +192,15 @@ struct XChunkX {
     int64_t map;   // striped: its export map in XKernelParams::smap (width ints: export index or -1)
 };
 
+// A plan made without reading anything back (k_plan_pair): what the launch
+// needs of it, in device memory.
+struct XPlanOut {
+    int32_t items, stack_rows, levels;
+    int32_t status;  // nonzero: no plan, nothing to run
+    int64_t cells, cells_right;
+    int64_t words, scratch;  // hand-off words; ints left for the warps' stacks
+};
+
 struct XKernelParams {
     const int2 *rowinfo;  // node records of every oriented tree
     const int32_t *krd;   // keyroots grouped by depth (node ids within their tree)
@@ -208,6 +217,8 @@ struct XKernelParams {
     int64_t scratch_per_warp;  // int32 elements
     int32_t stack_rows;   // stack capacity in rows
     int32_t nitems, npairs;
+    const XPlanOut *plan;  // if set: in place of nitems and stack_rows; the stacks lie below scratch, and
+                           // warps whose stack does not fit leave at once
     int32_t *next;        // items claimed (batch launch)
     int32_t *progress;    // items finished
     int32_t *error;       // 0 = ok; else an XTED error code
