@@ -115,15 +115,7 @@ static int pair_prepare(xted_ctx *c, const xted_tree &a, const xted_tree &b) {
     if (!rc) rc = ctx_host_reserve(c->result, (PAIR_HDR_INTS + 1) * sizeof(int32_t));
     if (rc) return rc;
     pair_layout(c->meta.p, fixed + XTED_PAIR_ROOM, a.n, b.n, &L);
-    L.P.run_rows = c->opts.run_rows;
-    L.P.narrow_width = c->opts.narrow_width;
-    L.P.half_width = c->opts.half_width == 0 ? XTED_HALF_DEFAULT : c->opts.half_width;
-    L.P.ntune = 0;
-    if (c->opts.tuned) {
-        int nt = 0;
-        const XTuneRow *tt = ctx_tune_table(c, &nt);
-        for (int k = 0; k < nt && k < XTED_TUNE_ROWS; k++) L.P.tune[L.P.ntune++] = tt[k];
-    }
+    ctx_granularity(c, (int64_t)a.n * b.n, L.P);
     int32_t *h = (int32_t *)c->stage.p;
     std::memset(h + L.upload_ints - PAIR_HDR_INTS, 0, PAIR_HDR_INTS * sizeof(int32_t));
     for (int k = 0; k < 2; k++) {
@@ -369,6 +361,32 @@ const XTuneRow *ctx_tune_table(const xted_ctx *c, int *nrows) {
     }
     *nrows = kTuneRows;
     return kTuneTable;
+}
+
+// The granularity a launch is planned with. A run of rows ends the wait of the
+// tables that need it, so short runs shorten the chain of a launch that does
+// not fill the GPU; a full one pays for every run's start (its copies are not
+// yet in flight). The lines lie where the node products of the launch's pairs
+// together pass 2, 20 and 100 million. Device ms at runs of 16 / 32 / 128 / 256 rows:
+//   one pair of 60 0.095 / 0.113 / 0.125 / 0.126, of 1,000 1.22 / 1.25 / 1.57 / 2.00;
+//   64 pairs of 400 (10 M) 0.908 / 0.890 / 0.967 / 1.03, 16 of 1,000 (16 M) 1.93 / 1.91 / 2.00 / 2.25;
+//   256 of 400 (41 M) 2.09 / 1.97 / 1.89 / 1.94, 64 of 1,000 (64 M) 4.25 / 4.15 / 4.17 / 4.16;
+//   1,024 of 400 (164 M) 6.38 / 5.89 / 5.47 / 5.38, 256 of 1,000 11.8 / 11.1 / 10.5 / 10.4.
+// A table set by xted_set_tune_table, or the options of an untuned context, is taken as it is.
+void ctx_granularity(const xted_ctx *c, int64_t products, PlanPools &P) {
+    P.run_rows = c->opts.run_rows;
+    P.narrow_width = c->opts.narrow_width;
+    P.half_width = c->opts.half_width == 0 ? XTED_HALF_DEFAULT : c->opts.half_width;
+    P.ntune = 0;
+    if (!c->opts.tuned) return;
+    const int32_t cap = products < 2000000 ? 16 : products < 20000000 ? 32 : products < 100000000 ? 128 : INT32_MAX;
+    int nt = 0;
+    const XTuneRow *tt = ctx_tune_table(c, &nt);
+    for (int k = 0; k < nt && k < XTED_TUNE_ROWS; k++) {
+        P.tune[k] = tt[k];
+        if (c->ntune <= 0) P.tune[k].run_rows = std::min(tt[k].run_rows, cap);
+        P.ntune++;
+    }
 }
 
 void fill_stats(xted_ctx *c, double plan_ms) {

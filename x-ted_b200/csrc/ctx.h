@@ -82,6 +82,7 @@ void fill_stats(xted_ctx *c, double plan_ms);
 // The size-bucket granularity table the context plans with: the one set by
 // xted_set_tune_table, else the autotuned table compiled into the library.
 const XTuneRow *ctx_tune_table(const xted_ctx *c, int *nrows);
+void ctx_granularity(const xted_ctx *c, int64_t products, PlanPools &P);
 void serve_shutdown(xted_ctx *c);
 std::mutex &serve_mutex(xted_ctx *c);  // the serving state's lock (c->serve must be set)
 

@@ -299,7 +299,7 @@ bool copy_tree(int32_t *lab, int32_t *off, int32_t *idx, const xted_tree &t, cud
 int run_planned(int32_t *A, int grid, const xted_tree &a, const xted_tree &b, int32_t *out, cudaStream_t s) {
     xted::PairLayout L;
     if (!xted::pair_layout(A, XTED_NOALLOC_ARENA_BYTES, a.n, b.n, &L)) return PLAN_OVERFLOW;
-    L.P.run_rows = 64;
+    L.P.run_rows = (int64_t)a.n * b.n < 2000000 ? 16 : 32;  // (one pair never fills the GPU: short runs)
     L.P.narrow_width = XTED_SW;
     L.P.half_width = XTED_HALF_DEFAULT;
     L.P.ntune = 0;

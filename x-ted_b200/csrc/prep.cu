@@ -1076,9 +1076,10 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     c->uniq.clear();
     std::vector<int32_t> &pt = c->pair_trees;
     pt.resize(2 * (size_t)npairs);
-    int64_t N = 0, R = 0;
+    int64_t N = 0, R = 0, products = 0;
     int32_t maxn = 0;
     for (int p = 0; p < npairs; p++) {
+        products += (int64_t)std::max(a[p].n, 0) * std::max(b[p].n, 0);
         for (int side = 0; side < 2; side++) {
             const xted_tree &t = side ? b[p] : a[p];
             TreeKey key{t.labels, t.child_off, t.child_idx, t.n};
@@ -1185,15 +1186,7 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     P.oka = cv.take<int32_t>(N2);
     P.depths = cv.take<DDepth>(N2 + 2 * (size_t)T);
     P.otrees = cv.take<DOTree>(2 * (size_t)T);
-    P.run_rows = c->opts.run_rows;
-    P.narrow_width = c->opts.narrow_width;
-    P.half_width = c->opts.half_width == 0 ? XTED_HALF_DEFAULT : c->opts.half_width;
-    P.ntune = 0;
-    if (c->opts.tuned) {
-        int nt = 0;
-        const XTuneRow *tt = ctx_tune_table(c, &nt);
-        for (int k = 0; k < nt && k < XTED_TUNE_ROWS; k++) P.tune[P.ntune++] = tt[k];
-    }
+    ctx_granularity(c, products, P);
     DPair *d_pairs = cv.take<DPair>((size_t)npairs);
     XPair *d_xpairs = cv.take<XPair>((size_t)npairs);
     int32_t *d_trivial = cv.take<int32_t>((size_t)npairs);
