@@ -89,3 +89,18 @@ def test_more_far_values_than_places(n):
     a, b = _comb(9, 5, False), _comb(n, 6, False)
     with xted.Context(orientation=xted.ORIENT_RIGHT) as ctx:
         assert ctx.distance(a, b) == oracle.distance(a, b)
+
+
+@pytest.mark.timeout(300)
+@pytest.mark.parametrize("npairs", [1023, 1024])
+def test_launch_of_many_pairs(npairs):
+    """From 1,024 pairs on the launch takes five blocks an SM: every chunk kind,
+    first as a batch, then prepared and run again from a graph."""
+    small = [(gen.tree("random", 1 + k % 37, k, "uniform", 4), gen.tree("deep", 1 + k % 61, 2 * k, "uniform", 4)) for k in range(npairs - 6)]
+    pairs = small + [(_comb(130, 1, a), _comb(n, 2, a)) for a in (True, False) for n in (255, 600, 1100)]
+    want = oracle.distance_batch(pairs, nthreads=8)
+    with xted.Context() as ctx:
+        assert np.array_equal(ctx.distance_batch(pairs), want)
+        ctx.prepare_batch(pairs)
+        for _ in range(3):
+            assert np.array_equal(ctx.run_prepared(), want)

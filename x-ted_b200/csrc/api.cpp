@@ -26,8 +26,8 @@
 #include "tune_table.h"
 
 namespace xted {
-int dp_occupancy(int *blocks_per_sm);
-cudaError_t launch_dp(const XKernelParams &P, int grid, cudaStream_t s);
+int dp_occupancy(int *blocks_per_sm, bool full);
+cudaError_t launch_dp(const XKernelParams &P, int grid, bool full, cudaStream_t s);
 cudaError_t launch_gather(const XPair *pairs, const int32_t *trivial, const int32_t *dt, int npairs,
                           int32_t *out, int c_del, int c_ins, int32_t *error, cudaStream_t s);
 }  // namespace xted
@@ -90,6 +90,10 @@ int ctx_host_reserve(HostBuf &b, size_t bytes) {
     b.cap = want;
     return XTED_OK;
 }
+
+// From this many pairs on a launch takes five blocks an SM (flow.cu has the
+// times of both): the work then outlasts the longest pair's chain.
+#define XTED_FULL_PAIRS 1024
 
 // One pair is planned by one block up to this many nodes together, by the
 // batch's kernels beyond. A call on two trees of 40 nodes takes 165 us this way
@@ -168,7 +172,13 @@ int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npa
     // per-warp scratch: the far-row stack's rows outside the shared window
     const int64_t stack_rows = c->plan_stack_rows;
     const int64_t per = stack_rows * XTED_SW;
-    rc = ctx_dev_reserve(c, c->scratch, (size_t)per * (size_t)c->grid * XTED_FLOW_WARPS * sizeof(int32_t));
+    c->full = npairs >= XTED_FULL_PAIRS && c->grid_full > 0;
+    c->run_grid = c->full ? c->grid_full : c->grid;
+    for (;;) {  // (a launch of fewer blocks needs less: under a memory limit, as many as fit)
+        rc = ctx_dev_reserve(c, c->scratch, (size_t)per * (size_t)c->run_grid * XTED_FLOW_WARPS * sizeof(int32_t));
+        if (rc != XTED_ENOMEM || c->run_grid == 1) break;
+        c->run_grid = (c->run_grid + 1) / 2;
+    }
     if (rc) return rc;
     // counters: [1] error, [2..5] error info, then out[npairs]
     rc = ctx_dev_reserve(c, c->counters, (8 + 2 * (size_t)npairs) * sizeof(int32_t));
@@ -215,7 +225,7 @@ static int enqueue_step(xted_ctx *c, bool events) {
              cudaMemsetAsync(L.hdr, 0, PAIR_CTL_INTS * sizeof(int32_t), c->stream) != cudaSuccess) ||
             launch_pair_clear(L, grid, c->stream) != cudaSuccess ||
             (events && cudaEventRecord(c->evk0, c->stream) != cudaSuccess) ||
-            launch_dp(K, grid, c->stream) != cudaSuccess ||
+            launch_dp(K, grid, false, c->stream) != cudaSuccess ||
             (events && cudaEventRecord(c->evk1, c->stream) != cudaSuccess) ||
             (events && cudaEventRecord(c->ev1, c->stream) != cudaSuccess) ||
             cudaMemcpyAsync(hres, L.hdr, (PAIR_HDR_INTS + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream) !=
@@ -232,7 +242,7 @@ static int enqueue_step(xted_ctx *c, bool events) {
            cudaMemsetAsync(K.buf, 0xff, (size_t)c->plan_words * sizeof(int32_t), c->stream) != cudaSuccess))))
         return XTED_ECUDA;
     if (events && cudaEventRecord(c->evk0, c->stream) != cudaSuccess) return XTED_ECUDA;
-    if (K.nitems > 0 && launch_dp(K, c->grid, c->stream) != cudaSuccess) return XTED_ECUDA;
+    if (K.nitems > 0 && launch_dp(K, c->run_grid, c->full, c->stream) != cudaSuccess) return XTED_ECUDA;
     if (events && cudaEventRecord(c->evk1, c->stream) != cudaSuccess) return XTED_ECUDA;
     if (launch_gather(K.pairs, c->d_trivial, K.dt, npairs, d_out, K.c_del, K.c_ins, K.error, c->stream) != cudaSuccess)
         return XTED_ECUDA;
@@ -329,7 +339,7 @@ int ctx_run(xted_ctx *c, int32_t *out, bool allow_graph) {
         return XTED_OK;
     }
     c->stats.d2h_bytes = (int64_t)(res_bytes + 8 * sizeof(int32_t));
-    c->stats.grid = c->grid;
+    c->stats.grid = c->run_grid;
     std::memcpy(c->err_info, hres + 2, sizeof(c->err_info));
     if (K.trace) {
         std::vector<unsigned long long> tr((size_t)K.nitems * 4);
@@ -460,10 +470,13 @@ int xted_create(xted_ctx **out, const xted_opts *opts) {
     c->opts = o;
     c->sms = prop.multiProcessorCount;
     int occ = 0;
-    if (dp_occupancy(&occ) != 0 || occ < 1) {
+    int occ_full = 0;
+    if (dp_occupancy(&occ, false) != 0 || occ < 1 || dp_occupancy(&occ_full, true) != 0) {
         delete c;
         return XTED_ECUDA;
     }
+    // (under a limit on blocks or on memory, whose stacks would be a quarter more, only the smaller launch)
+    if (occ_full > occ && o.ctas_per_sm == 0 && o.mem_limit == 0) c->grid_full = occ_full * c->sms;
     if (o.ctas_per_sm > 0) occ = std::min(occ, o.ctas_per_sm);
     c->grid = occ * c->sms;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||

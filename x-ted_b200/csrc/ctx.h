@@ -34,7 +34,8 @@ struct DTree;       // plan_core.h
 struct xted_ctx {
     xted_opts opts;
     int sms = 0;
-    int grid = 0;
+    int grid = 0;          // blocks of a launch bound by its pairs' chains of tables
+    int grid_full = 0;     // ... of one with many pairs (0: never)
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evk0 = nullptr, evk1 = nullptr;
     xted::DevBuf meta, levels, work, dt, scratch, counters, trace, smap, sbuf;
@@ -59,6 +60,8 @@ struct xted_ctx {
     XKernelParams kp{};
     xted::PairLayout pair;    // kp.plan set: one pair, planned by one block (pair_plan.h)
     int32_t npairs = 0;
+    int32_t run_grid = 0;
+    bool full = false;        // the launch takes grid_full blocks
     int64_t h2d_bytes = 0;
     double prep_ms = 0;
     bool prepared = false;

@@ -124,17 +124,16 @@ __device__ __forceinline__ int warp_suffix_max(int v) {
 // leaves a window of 4 rows on 2.5% of the mixed batch's rows, one of 8 on 1.7%.
 #define FLOW_W 8                   // columns per lane
 #define FLOW_PF 4
-#define FLOW_IMPORTS 64            // far values of other stripes kept beside a stack row
+#define FLOW_IMPORTS 48            // far values of other stripes kept beside a stack row
 #define FLOW_STACK_ROWS 4
 #define FLOW_ZERO (32 * FLOW_W)    // place of the zero word in a stack row
 #define FLOW_PITCH (FLOW_ZERO + 4 + FLOW_IMPORTS)
 #define FLOW_RING (FLOW_PF * XTED_SW)
 #define FLOW_STACK (FLOW_STACK_ROWS * FLOW_PITCH)
-// path columns (column | segment << 8 | node << 16), their labels, exported columns (16 bits each)
-#define FLOW_LISTS (XTED_SW + XTED_SW + XTED_SW / 2)
+// path columns (column | segment << 8 | node << 16), their labels, exported columns (8 bits each)
+#define FLOW_LISTS (XTED_SW + XTED_SW + XTED_SW / 4)
 #define FLOW_WARP_INTS (FLOW_RING + FLOW_STACK + FLOW_LISTS)
-// a stack row of zeros, one per block: what tree rows read as far values
-#define FLOW_SMEM ((FLOW_PITCH + XTED_FLOW_WARPS * FLOW_WARP_INTS) * 4)
+#define FLOW_SMEM (XTED_FLOW_WARPS * FLOW_WARP_INTS * 4)
 static_assert(XTED_SW == 32 * FLOW_W && XTED_MAX_NODES < 65536 && FLOW_PITCH % 4 == 0, "list entries and row places");
 // A row's flags in a run's row sequence, beside orl (20 bits) and the flags of
 // its node record (bits 29, 30). The ITEM_ flags are the same for every row of
@@ -204,7 +203,7 @@ __device__ __forceinline__ bool warp_wait(const XKernelParams &P, const int32_t 
 #define FLOW_OVER 2
 template <bool OVER>
 __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it, const XPair &pr, const XRun &run,
-                                         const XChunk &ch, unsigned zeros, int32_t *ring, int32_t *gstk) {
+                                         const XChunk &ch, int32_t *ring, int32_t *gstk) {
     constexpr int W = FLOW_W, PF = FLOW_PF, SC = FLOW_STACK_ROWS, ZERO = FLOW_ZERO, IMP = ZERO + 4;
     constexpr unsigned SLOT_B = 4 * XTED_SW, RING_B = PF * SLOT_B, PITCH_B = 4 * FLOW_PITCH;
     const int lane = threadIdx.x & 31;
@@ -332,7 +331,7 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
     int nt, nx, ne;
     int tf = first_of(tcol, nt), xf = first_of(xfar, nx), ef = first_of(expm, ne);
     ebase = (int)__reduce_min_sync(FULLMASK, (unsigned)ebase);
-    unsigned short *el = (unsigned short *)(ring + FLOW_RING + FLOW_STACK + 2 * XTED_SW);
+    unsigned char *el = (unsigned char *)(ring + FLOW_RING + FLOW_STACK + 2 * XTED_SW);
     int32_t *tlist = ring + FLOW_RING + FLOW_STACK, *tlab = tlist + XTED_SW;
     // far columns elsewhere, in column order, then the places of their values
     int32_t *xl = ring + FLOW_RING, *xplace = xl + XTED_SW, *xd = xplace + XTED_SW;  // (in the stack window, empty as yet)
@@ -345,7 +344,7 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
             tlab[tf] = nodes[j].x;
             tlist[tf++] = (int)((unsigned)c | ((unsigned)(key[k] / XTED_KEY_BIG) << 8) | ((unsigned)j << 16));
         }
-        if ((expm >> k) & 1u) el[ef++] = (unsigned short)(k * 32 + lane);
+        if ((expm >> k) & 1u) el[ef++] = (unsigned char)(k * 32 + lane);
         if ((xfar >> k) & 1u) xl[x1++] = fb[k];
     }
     __syncwarp();
@@ -578,10 +577,11 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
             c2 = ld_relaxed(Hin + min(t + 2, R - 1));
         }
         // ---- the row's cells, before the suffix maximum ----
-        unsigned top = zeros;  // a tree row's far row is the table's border
-        int far[W];
+        int far[W];  // a tree row's far row is the table's border
+#pragma unroll
+        for (int k = 0; k < W; k++) far[k] = 0;
         if (!trow) {
-            top = stk_a + ((sp - 1) & (SC - 1)) * PITCH_B;
+            const unsigned top = stk_a + ((sp - 1) & (SC - 1)) * PITCH_B;
             if (__builtin_expect(sp - 1 < lo, 0)) {  // the top of the stack left the window: bring it back
                 lo = sp - 1;
                 const int32_t *g = gstk + (int64_t)lo * ZERO + lane;
@@ -597,12 +597,12 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
                         return FLOW_FAILED;
                 }
                 sts(top + 4 * (IMP + lane), iv[0]);
-                sts(top + 4 * (IMP + 32 + lane), iv[1]);
+                if (lane < FLOW_IMPORTS - 32) sts(top + 4 * (IMP + 32 + lane), iv[1]);
                 __syncwarp();
             }
-        }
 #pragma unroll
-        for (int k = 0; k < W; k++) far[k] = lds(top + fb[k]);
+            for (int k = 0; k < W; k++) far[k] = lds(top + fb[k]);
+        }
         if (OVER && !trow) {  // more than have a place: straight from their words
             const int i = __shfl_sync(FULLMASK, bi, tl);
             const int32_t *erow = E + (unsigned)(t - ((int)(y & XTED_ROW_ORL_MASK) + 1 - i)) * (unsigned)X;  // (R X < 2^32)
@@ -707,8 +707,8 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
 // (Inline: a call anywhere in the kernel makes every shuffle of the loop check for divergence, 29.1 against 25.1 ms on
 // 1,500 pairs of 200-500 nodes.)
 __device__ __forceinline__ int run_item_over(const XKernelParams &P, const XItem &it, const XPair &pr, const XRun &run,
-                                          const XChunk &ch, unsigned zeros, int32_t *ring, int32_t *gstk) {
-    return run_item<true>(P, it, pr, run, ch, zeros, ring, gstk);
+                                          const XChunk &ch, int32_t *ring, int32_t *gstk) {
+    return run_item<true>(P, it, pr, run, ch, ring, gstk);
 }
 
 // Trace record of an item (XTED_TRACE): claim, start and end time, and
@@ -793,18 +793,24 @@ __device__ void finish_served(const XKernelParams &P, const XPair &pr, const XIt
     }
 }
 
-// Four blocks of four warps per SM: 48 KB of shared memory a block, 128 registers a thread.
-__global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, 4) xted_flow_kernel(const __grid_constant__ XKernelParams P) {
+// Blocks of four warps, 45 KB of shared memory each: four per SM with 128
+// registers a thread, or five with 96 (25 of them spilled). A row waits on
+// fixed latencies for three of four cycles, so a launch that always has items
+// to claim runs faster with the fifth block: 4,096 pairs 142.1 -> 135.7 ms, 1,024
+// pairs 38.2 -> 37.2, 4,560 small ones 13.03 -> 12.72. A launch bound by its
+// pairs' longest chains runs slower, row by row: 20,000 random 47.6 -> 48.9 ms,
+// 1,000 wide x deep 1.25 -> 1.40, a pair of 100 0.10 -> 0.115. 500 pairs: 7.83 -> 7.96.
+template <int BLOCKS>
+__global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, BLOCKS) xted_flow_kernel(const __grid_constant__ XKernelParams P) {
     extern __shared__ __align__(16) int32_t s_dyn[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int32_t *ring = s_dyn + FLOW_PITCH + warp * FLOW_WARP_INTS;
+    int32_t *ring = s_dyn + warp * FLOW_WARP_INTS;
     const int nitems = P.plan ? P.plan->items : P.nitems;
     const int64_t per = P.plan ? (int64_t)P.plan->stack_rows * XTED_SW : P.scratch_per_warp;
     const int64_t gwarp = (int64_t)blockIdx.x * XTED_FLOW_WARPS + warp;
     int32_t *gstk = P.scratch + (P.plan ? -(gwarp + 1) * per : gwarp * per);
     for (int x = lane; x < FLOW_WARP_INTS; x += 32) ring[x] = 0;
-    for (int x = threadIdx.x; x < FLOW_PITCH; x += blockDim.x) s_dyn[x] = 0;
-    __syncthreads();
+    __syncwarp();
     if (P.plan && (gwarp + 1) * per > P.plan->scratch) return;
     for (;;) {
         int g = -1, slot = 0;
@@ -827,8 +833,8 @@ __global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, 4) xted_flow_kernel(cons
         // (test hook: of a held pair, nothing that reads its level 0 becomes ready)
         const bool held = it.pair == P.hold_pair && run.depth + ch.depth == 0;
         if (!held) {
-            int rc = run_item<false>(P, it, pr, run, ch, smem_addr(s_dyn), ring, gstk);
-            if (rc == FLOW_OVER) rc = run_item_over(P, it, pr, run, ch, smem_addr(s_dyn), ring, gstk);
+            int rc = run_item<false>(P, it, pr, run, ch, ring, gstk);
+            if (rc == FLOW_OVER) rc = run_item_over(P, it, pr, run, ch, ring, gstk);
             if (rc) break;
         }
         if (lane == 0) {
@@ -865,17 +871,22 @@ __global__ void xted_gather_kernel(const XPair *pairs, const int32_t *trivial, c
 }
 
 // ---- host-side launch helpers ----
-int dp_occupancy(int *blocks_per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(xted_flow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FLOW_SMEM);
+template <int BLOCKS>
+static int occupancy_of(int *blocks_per_sm) {
+    cudaError_t e = cudaFuncSetAttribute(xted_flow_kernel<BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, FLOW_SMEM);
     if (e != cudaSuccess) return (int)e;
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, xted_flow_kernel, 32 * XTED_FLOW_WARPS,
-                                                              FLOW_SMEM);
+    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, xted_flow_kernel<BLOCKS>,
+                                                              32 * XTED_FLOW_WARPS, FLOW_SMEM);
+}
+int dp_occupancy(int *blocks_per_sm, bool full) {
+    return full ? occupancy_of<5>(blocks_per_sm) : occupancy_of<4>(blocks_per_sm);
 }
 
 // A plain launch: a block that is not resident has claimed nothing, and what
 // the resident warps have claimed needs only items claimed before.
-cudaError_t launch_dp(const XKernelParams &P, int grid, cudaStream_t s) {
-    xted_flow_kernel<<<grid, 32 * XTED_FLOW_WARPS, FLOW_SMEM, s>>>(P);
+cudaError_t launch_dp(const XKernelParams &P, int grid, bool full, cudaStream_t s) {
+    if (full) xted_flow_kernel<5><<<grid, 32 * XTED_FLOW_WARPS, FLOW_SMEM, s>>>(P);
+    else xted_flow_kernel<4><<<grid, 32 * XTED_FLOW_WARPS, FLOW_SMEM, s>>>(P);
     return cudaGetLastError();
 }
 

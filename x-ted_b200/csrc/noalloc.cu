@@ -45,8 +45,8 @@
 #include "pair_plan.h"
 
 namespace xted {
-int dp_occupancy(int *blocks_per_sm);
-cudaError_t launch_dp(const XKernelParams &P, int grid, cudaStream_t s);
+int dp_occupancy(int *blocks_per_sm, bool full);
+cudaError_t launch_dp(const XKernelParams &P, int grid, bool full, cudaStream_t s);
 }  // namespace xted
 
 namespace {
@@ -275,7 +275,7 @@ int arena_for(int device, int32_t **out, int *grid) {
         }
         int occ = 0;
         cudaFuncAttributes fa;
-        if (xted::dp_occupancy(&occ) != 0 || occ < 1 || xted::pair_kernels_load() != cudaSuccess ||
+        if (xted::dp_occupancy(&occ, false) != 0 || occ < 1 || xted::pair_kernels_load() != cudaSuccess ||
             cudaFuncGetAttributes(&fa, xted_noalloc_kernel) != cudaSuccess) {
             cudaGetLastError();
             return XTED_ECUDA;
@@ -314,7 +314,7 @@ int run_planned(int32_t *A, int grid, const xted_tree &a, const xted_tree &b, in
     if (cudaMemsetAsync(L.hdr, 0, 4 * PAIR_CTL_INTS, s) != cudaSuccess || !copy_tree(ra, ra + a.n, ra + 2 * a.n + 1, a, s) ||
         !copy_tree(rb, rb + b.n, rb + 2 * b.n + 1, b, s) ||
         xted::launch_plan_pair(L, XTED_ORIENT_AUTO, true, s) != cudaSuccess ||
-        xted::launch_pair_clear(L, grid, s) != cudaSuccess || xted::launch_dp(K, grid, s) != cudaSuccess ||
+        xted::launch_pair_clear(L, grid, s) != cudaSuccess || xted::launch_dp(K, grid, false, s) != cudaSuccess ||
         cudaMemcpyAsync(res, L.hdr, sizeof(res), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess) {
         cudaGetLastError();

@@ -47,7 +47,7 @@
 #include "serve_plan.h"
 
 namespace xted {
-cudaError_t launch_dp(const XKernelParams &P, int grid, cudaStream_t s);
+cudaError_t launch_dp(const XKernelParams &P, int grid, bool full, cudaStream_t s);
 }
 
 static_assert(XTED_SERVE_SLOTS == XTED_SERVE_SLOTS_MAX, "slot count of the ABI and the kernels");
@@ -599,7 +599,7 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
     if (inflight && !s->running) {
         cudaStreamSynchronize(s->cs);
         bool ok = cudaMemsetAsync(s->d_ctl, 0, XTED_CTL_INTS * 4, s->ks) == cudaSuccess &&
-                  launch_dp(s->K, s->c->grid, s->ks) == cudaSuccess &&
+                  launch_dp(s->K, s->c->grid, false, s->ks) == cudaSuccess &&
                   cudaEventRecord(s->kev, s->ks) == cudaSuccess;
         if (!ok) {
             cudaGetLastError();
