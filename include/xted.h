@@ -63,30 +63,22 @@ typedef struct xted_tree {
 typedef struct xted_opts {
     int32_t device;         /* CUDA device ordinal                          */
     int32_t orientation;    /* XTED_ORIENT_*                                */
-    int32_t narrow_width;   /* widest column chunk run by one warp (1..256);
-                               0 runs every chunk on a whole thread block   */
+    int32_t narrow_width;   /* widest column chunk of several segments
+                               (0..256)                                     */
     int32_t run_rows;       /* target rows per row run (>= 1)               */
-    int32_t ctas_per_sm;    /* persistent blocks per SM (0 = occupancy max) */
-    int32_t wide_rows;      /* > 0: a narrow chunk's unit whose row run is
-                               longer than this runs on the whole block
-                               (shortens critical paths, costs throughput);
-                               <= 0: never (default)                        */
-    int32_t half_width;     /* chunks wider than narrow_width up to this
-                               width (at most 1024) run on half a block, two
-                               at a time; 0 = 512 (fastest on the mixed
-                               batch), < 0: none                            */
+    int32_t ctas_per_sm;    /* persistent blocks per SM, at most (0: as many
+                               as fit)                                      */
+    int32_t wide_rows;      /* accepted; without effect on the launch       */
+    int32_t half_width;     /* accepted (at most 1024); without effect on
+                               the launch                                   */
     int32_t tuned;          /* nonzero (default): run_rows, narrow_width and
                                half_width come per tree from the autotuned
                                size-bucket table; 0: the fields above apply
                                to every tree                                */
     double wait_timeout_s;  /* bound on every device-side wait              */
     int64_t mem_limit;      /* device bytes the context may hold (0 = none) */
-    int64_t stripe_min_cells; /* a table whose column segment is wider than
-                               2,048 and whose unit has at least this many
-                               cells runs in column stripes of 512 columns
-                               (wider past 128 stripes), each stripe a task
-                               that any block may run (0 = 2^20; < 0: the
-                               whole table on one block)                    */
+    int64_t stripe_min_cells; /* accepted; without effect: every segment wider
+                               than 256 columns runs in column stripes      */
     int32_t cost_del;       /* edit costs (integers >= 0): deleting a node of */
     int32_t cost_ins;       /* the first tree, inserting a node of the second */
     int32_t cost_ren;       /* tree, and mapping two nodes whose labels differ

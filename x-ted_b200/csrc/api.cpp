@@ -3,7 +3,7 @@
 // xted_distance / xted_distance_batch replace the reference's
 // standard_ted (X-TED_CPU/TED.cpp:177-190; X-TED_GPU/TED.cu:116-128): the
 // planner (prep.cu) lays out every keyroot table of every pair as a list of
-// items, one cooperative launch of the persistent DP kernel (flow.cu) runs
+// items, one launch of the persistent DP kernel (flow.cu) runs
 // them, and a gather kernel reads Dtree[0][0] of each pair
 // (X-TED_CPU/TED.cpp:188). Errors are returned, never printed or exited on
 // (the reference prints CUDA errors and continues, X-TED_GPU/utils/cuda_utils.h:35-41,

@@ -82,6 +82,8 @@ struct XUnit {
     int32_t chunk; // global chunk index (column tree)
 };
 
+// (From here to XEntry: the block-by-block tasks of plan_core.h's level
+// schedule, which the host emulation of the planner's records runs. The DP launch has only items.)
 #define XTED_TASK_WIDE 0x80000000u  // one unit run by the whole block
 #define XTED_TASK_STRIPED 0x20000000u  // (with WIDE) one column stripe of a striped unit
 // Striped units: a single column segment wider than the register paths
@@ -135,18 +137,9 @@ struct XTask {
     int32_t unit_lo;  // first unit
 };
 
-// Ready queue. Every (pair, level) is an entry whose tasks are contiguous.
-// An entry is published into the ready queue of its priority bucket when the
-// last task of the pair's previous level finishes (level 0 at launch), so a
-// block only ever claims tasks whose tables' inputs are complete; the
-// reference instead runs one host-synchronised level at a time
-// (X-TED_CPU/parallel_computing.cpp:155-182, X-TED_GPU/parallel_X_TED.cu:312-387).
+// Entries and buckets: the level-by-level schedule that the host emulation of
+// the planner's records runs (plan_core.h); the DP launch uses the items below.
 #define XTED_BUCKETS 16
-// Every bucket has two rings: one for the narrow tasks of its entries (run by
-// single warps, a block's warps independently) and one for their group tasks
-// (half- and whole-block units, striped units), so that a block busy with
-// narrow units can keep claiming narrow work instead of stopping all its
-// warps for a group task. Ring index = kind * XTED_BUCKETS + bucket.
 #define XTED_KIND_NARROW 0
 #define XTED_KIND_GROUP 1
 #define XTED_RINGS (2 * XTED_BUCKETS)
