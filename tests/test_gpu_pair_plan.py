@@ -73,3 +73,19 @@ def test_arena_checks_trees_like_the_host():
         assert _noalloc(c, t)[0] == want and _noalloc(t, c)[0] == want
         bad += want != 0
     assert 30 < bad < 120
+
+
+@pytest.mark.timeout(300)
+@pytest.mark.parametrize("m,n", [(1, 1), (40, 57), (300, 251)])
+def test_a_pair_runs_again(m, n):
+    """A call leaves its plan prepared: run again it starts from cleared
+    counters, also from the graph that the second run captures."""
+    a, b = gen.tree("random", m, 5, "uniform", 5), gen.tree("deep", n, 6, "uniform", 5)
+    out = ctypes.c_int32(-1)
+    with xted.Context() as ctx:
+        want = ctx.distance(a, b)
+        assert want == oracle.distance(a, b)
+        for _ in range(4):
+            out.value = -1
+            assert _lib.lib().xted_run_prepared(ctx.handle, ctypes.byref(out)) == 0
+            assert out.value == want

@@ -210,7 +210,8 @@ int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npa
 // gather, and the copy of results + error word to pinned memory. Synchronous.
 // One step of the prepared plan, enqueued on the context's stream: counter
 // resets, the persistent DP launch, the gather, and the copy of results + error word to pinned memory.
-static int enqueue_step(xted_ctx *c, bool events) {
+// first: nothing has run since the plan was uploaded.
+static int enqueue_step(xted_ctx *c, bool events, bool first) {
     const XKernelParams &K = c->kp;
     const int npairs = c->npairs;
     int32_t *cnt = (int32_t *)c->counters.p;
@@ -221,7 +222,7 @@ static int enqueue_step(xted_ctx *c, bool events) {
     if (K.plan) {
         const PairLayout &L = c->pair;
         const int grid = pair_grid(c->grid, L.m, L.n);
-        if ((c->runs_prepared > 1 &&  // (the first run finds the words zero, as uploaded)
+        if ((!first &&  // (the first run finds the words zero, as uploaded)
              cudaMemsetAsync(L.hdr, 0, PAIR_CTL_INTS * sizeof(int32_t), c->stream) != cudaSuccess) ||
             launch_pair_clear(L, grid, c->stream) != cudaSuccess ||
             (events && cudaEventRecord(c->evk0, c->stream) != cudaSuccess) ||
@@ -267,7 +268,7 @@ static bool capture_step(xted_ctx *c) {
         cudaGetLastError();
         return false;
     }
-    const int rc = enqueue_step(c, false);  // events recorded inside a graph cannot be timed
+    const int rc = enqueue_step(c, false, false);  // events recorded inside a graph cannot be timed
     const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     bool ok = rc == XTED_OK && e == cudaSuccess && g != nullptr &&
               cudaGraphInstantiate(&c->step_graph, g, 0) == cudaSuccess;
@@ -293,6 +294,7 @@ int ctx_run(xted_ctx *c, int32_t *out, bool allow_graph) {
         if (!c->step_graph && !capture_step(c)) c->graph_failed = true;
         replay = c->step_graph != nullptr;
     }
+    const bool first = c->runs_prepared == 0;
     c->runs_prepared++;
     if (replay) {
         // timed from outside: the DP time of a replay includes the step's
@@ -304,7 +306,7 @@ int ctx_run(xted_ctx *c, int32_t *out, bool allow_graph) {
             return XTED_ECUDA;
         }
     } else {
-        const int rc = enqueue_step(c, true);
+        const int rc = enqueue_step(c, true, first);
         if (rc) {
             cudaGetLastError();
             return rc;
