@@ -51,24 +51,28 @@ bool costs_fit(const xted_opts &o, int64_t m, int64_t n) {
     return (int64_t)o.cost_del * m + (int64_t)o.cost_ins * n < XTED_COST_BOUND;
 }
 
+static void dev_release(xted_ctx *c, DevBuf &b) {
+    if (b.p) cudaFree(b.p);
+    c->held -= (int64_t)b.cap;
+    b = DevBuf{};
+}
+
 int ctx_dev_reserve(xted_ctx *c, DevBuf &b, size_t bytes) {
     if (b.cap >= bytes) return XTED_OK;
     size_t want = align_up(std::max(bytes, b.cap + b.cap / 2), (size_t)2 << 20);
-    if (c->opts.mem_limit > 0) {
-        const int64_t limit = c->opts.mem_limit;
-        if (c->held - (int64_t)b.cap + (int64_t)want > limit) want = align_up(bytes, 256);
-        if (c->held - (int64_t)b.cap + (int64_t)want > limit) return XTED_ENOMEM;
-    }
-    if (b.p) {
-        cudaFree(b.p);
-        c->held -= (int64_t)b.cap;
-        b.p = nullptr;
-        b.cap = 0;
-    }
+    dev_release(c, b);
     void *p = nullptr;
-    if (cudaMalloc(&p, want) != cudaSuccess) {
-        cudaGetLastError();
-        return XTED_ENOMEM;
+    for (;;) {
+        const int64_t room = c->opts.mem_limit > 0 ? c->opts.mem_limit - c->held : INT64_MAX;
+        if ((int64_t)want > room) want = align_up(bytes, 256);
+        if ((int64_t)want <= room) {
+            if (cudaMalloc(&p, want) == cudaSuccess) break;
+            cudaGetLastError();
+        }
+        // the stacks and hand-off words of an earlier plan may have taken all there is: they come in any size
+        if (&b == &c->scratch || &b == &c->sbuf || (!c->scratch.p && !c->sbuf.p)) return XTED_ENOMEM;
+        dev_release(c, c->scratch);
+        dev_release(c, c->sbuf);
     }
     b.p = p;
     b.cap = want;
@@ -147,6 +151,52 @@ static int pair_prepare(xted_ctx *c, const xted_tree &a, const xted_tree &b) {
     return XTED_OK;
 }
 
+// A launch holds as many bytes of hand-off words as of tables, and this many at least; a list with more runs in
+// parts. The words of a pair that is costly in both decompositions grow with the fourth power of its nodes (zigzags of
+// 1,000 nodes 11.6 GB beside 4 MB of tables, of 2,000 nodes 212 GB), those of most others stay below their tables or
+// this floor (4,096 mixed pairs 4.0 GB beside 4.7). Every part but the last ends with the GPU running empty: the deep
+// pair of 20,000 nodes takes 407 ms whole, with 10 GB, and 471 in parts of 2 GB.
+#define XTED_WORDS_MIN ((int64_t)8 << 30)
+
+// Reserves the launch's stacks and hand-off words and divides the list into
+// parts. Both come in any size: the stacks down to one block's, the words down
+// to the largest unit's. Where not all fits, the stacks take at most half.
+static int reserve_launch(xted_ctx *c) {
+    XKernelParams &K = c->kp;
+    const int64_t block = (int64_t)c->plan_stack_rows * XTED_SW * XTED_FLOW_WARPS * (int64_t)sizeof(int32_t);
+    const int64_t bytes = c->plan_words * (int64_t)sizeof(int32_t);
+    int64_t cap = std::max(XTED_WORDS_MIN, c->plan_dt_elems * (int64_t)sizeof(int32_t));
+    if (c->opts.mem_limit > 0 && bytes > 0) {
+        const int64_t left = c->opts.mem_limit - c->held + (int64_t)c->scratch.cap + (int64_t)c->sbuf.cap;
+        if (block * c->run_grid + std::min(bytes, cap) > left) {
+            dev_release(c, c->scratch);
+            dev_release(c, c->sbuf);
+            c->run_grid = (int32_t)std::max<int64_t>(std::min<int64_t>(c->run_grid, left / 2 / block), 1);
+            cap = std::min(cap, left - block * c->run_grid);
+        }
+    }
+    for (bool old = c->sbuf.p != nullptr;; old = false) {
+        int rc = ctx_dev_reserve(c, c->scratch, (size_t)(block * c->run_grid));
+        for (int64_t most = cap, before = INT64_MAX; !rc && bytes > 0;) {
+            int64_t need = 0;
+            rc = dev_parts(c, std::max<int64_t>(most / (int64_t)sizeof(int32_t), 1), &need);
+            if (!rc) rc = ctx_dev_reserve(c, c->sbuf, (size_t)need * sizeof(int32_t));
+            if (rc != XTED_ENOMEM || need >= before) break;
+            rc = XTED_OK;
+            before = need;
+            most = need * (int64_t)sizeof(int32_t) / 2;
+        }
+        if (!rc) rc = ctx_dev_reserve(c, c->scratch, (size_t)(block * c->run_grid));  // (given up for the list of parts?)
+        if (rc != XTED_ENOMEM || (c->run_grid == 1 && !old)) {
+            K.scratch = (int32_t *)c->scratch.p;
+            return rc;
+        }
+        dev_release(c, c->scratch);
+        dev_release(c, c->sbuf);
+        if (!old) c->run_grid = (c->run_grid + 1) / 2;  // (first without what an earlier plan left)
+    }
+}
+
 // Plans a batch on the device (prep.cu) and sizes every buffer the DP launch
 // needs; the kernel parameters stay in the context so the batch can be run
 // repeatedly from device-resident inputs. With one_block, one small pair is
@@ -174,12 +224,6 @@ int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npa
     const int64_t per = stack_rows * XTED_SW;
     c->full = npairs >= XTED_FULL_PAIRS && c->grid_full > 0;
     c->run_grid = c->full ? c->grid_full : c->grid;
-    for (;;) {  // (a launch of fewer blocks needs less: under a memory limit, as many as fit)
-        rc = ctx_dev_reserve(c, c->scratch, (size_t)per * (size_t)c->run_grid * XTED_FLOW_WARPS * sizeof(int32_t));
-        if (rc != XTED_ENOMEM || c->run_grid == 1) break;
-        c->run_grid = (c->run_grid + 1) / 2;
-    }
-    if (rc) return rc;
     // counters: [1] error, [2..5] error info, then out[npairs]
     rc = ctx_dev_reserve(c, c->counters, (8 + 2 * (size_t)npairs) * sizeof(int32_t));
     if (rc) return rc;
@@ -187,7 +231,6 @@ int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npa
     if (rc) return rc;
     int32_t *cnt = (int32_t *)c->counters.p;
     K.dt = (int32_t *)c->dt.p;
-    K.scratch = (int32_t *)c->scratch.p;
     K.scratch_per_warp = per;
     K.stack_rows = (int32_t)stack_rows;
     K.error = cnt + 1;
@@ -201,6 +244,9 @@ int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npa
         if (rc) return rc;
         K.trace = (unsigned long long *)c->trace.p;
     }
+    c->parts.assign({XPart{0, 0, 0}, XPart{0, K.nitems, 0}});
+    rc = reserve_launch(c);
+    if (rc) return rc;
     c->npairs = npairs;
     c->prepared = true;
     return XTED_OK;
@@ -234,16 +280,27 @@ static int enqueue_step(xted_ctx *c, bool events, bool first) {
             return XTED_ECUDA;
         return XTED_OK;
     }
-    // per-run reset: the error words and the claim counter; every table and hand-off word to -1 (not written)
+    // per-run reset: the error words; every table to -1 (not written), and of each part the claim counter and the
+    // hand-off words
     if (cudaMemsetAsync(cnt, 0, 8 * sizeof(int32_t), c->stream) != cudaSuccess ||
         (K.nitems > 0 &&
-         (cudaMemsetAsync(K.next, 0, 2 * sizeof(int32_t), c->stream) != cudaSuccess ||
-          cudaMemsetAsync(K.dt, 0xff, (size_t)c->plan_dt_elems * sizeof(int32_t), c->stream) != cudaSuccess ||
-          (c->plan_words > 0 &&
-           cudaMemsetAsync(K.buf, 0xff, (size_t)c->plan_words * sizeof(int32_t), c->stream) != cudaSuccess))))
+         cudaMemsetAsync(K.dt, 0xff, (size_t)c->plan_dt_elems * sizeof(int32_t), c->stream) != cudaSuccess))
         return XTED_ECUDA;
-    if (events && cudaEventRecord(c->evk0, c->stream) != cudaSuccess) return XTED_ECUDA;
-    if (K.nitems > 0 && launch_dp(K, c->run_grid, c->full, c->stream) != cudaSuccess) return XTED_ECUDA;
+    for (size_t k = 0; k + 1 < c->parts.size() && K.nitems > 0; k++) {
+        const XPart &p = c->parts[k], &q = c->parts[k + 1];
+        XKernelParams part = K;
+        part.items = K.items + p.item;
+        part.nitems = q.item - p.item;
+        part.buf = (int32_t *)((uintptr_t)c->sbuf.p - (uintptr_t)p.word * sizeof(int32_t));
+        if (K.trace) part.trace = K.trace + 4 * (int64_t)p.item;
+        if (cudaMemsetAsync(K.next, 0, 2 * sizeof(int32_t), c->stream) != cudaSuccess ||
+            (q.word > p.word &&
+             cudaMemsetAsync(c->sbuf.p, 0xff, (size_t)(q.word - p.word) * sizeof(int32_t), c->stream) != cudaSuccess) ||
+            (events && k == 0 && cudaEventRecord(c->evk0, c->stream) != cudaSuccess) ||
+            launch_dp(part, c->run_grid, c->full, c->stream) != cudaSuccess)
+            return XTED_ECUDA;
+    }
+    if (events && K.nitems == 0 && cudaEventRecord(c->evk0, c->stream) != cudaSuccess) return XTED_ECUDA;
     if (events && cudaEventRecord(c->evk1, c->stream) != cudaSuccess) return XTED_ECUDA;
     if (launch_gather(K.pairs, c->d_trivial, K.dt, npairs, d_out, K.c_del, K.c_ins, K.error, c->stream) != cudaSuccess)
         return XTED_ECUDA;

@@ -26,6 +26,12 @@ struct HostBuf {
     size_t cap = 0;
 };
 
+// Where a part of the launch's list starts (flow_plan.h: flow_cut).
+struct XPart {
+    int64_t word;  // its first hand-off word
+    int32_t item, pad;
+};
+
 struct ServeState;  // serve.cpp
 struct DTree;       // plan_core.h
 
@@ -56,6 +62,7 @@ struct xted_ctx {
     std::vector<xted::DTree> htrees;
     int64_t plan_dt_elems = 0, plan_cells = 0, plan_cells_right = 0, plan_words = 0;
     int32_t plan_stack_rows = 1, plan_levels_max = 0;
+    std::vector<xted::XPart> parts;  // of the list, each a launch; its end last
     // the prepared plan (xted_prepare_batch / every batch call)
     XKernelParams kp{};
     xted::PairLayout pair;    // kp.plan set: one pair, planned by one block (pair_plan.h)
@@ -79,6 +86,8 @@ bool costs_fit(const xted_opts &o, int64_t m, int64_t n);
 int ctx_host_reserve(HostBuf &b, size_t bytes);
 int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs, bool one_block);
 int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs, XKernelParams &K);
+// Divides the planned list into parts of at most cap hand-off words (c->parts); need: the most words of a part.
+int dev_parts(xted_ctx *c, int64_t cap, int64_t *need);
 int ctx_run(xted_ctx *c, int32_t *out, bool allow_graph);
 void ctx_drop_graph(xted_ctx *c);
 void fill_stats(xted_ctx *c, double plan_ms);

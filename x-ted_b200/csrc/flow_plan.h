@@ -91,6 +91,30 @@ XT_HD inline XItem flow_item(const FlowCtx &C, const DDepth &ra, const DDepth &c
     return it;
 }
 
+// A list whose hand-off words exceed the buffer runs in parts, launches one
+// after another that each use the buffer from its start: an item needs items
+// before it, whose part has ended. `buf` never falls along the list, and a unit's
+// words end where the next unit's begin. Returns the end of the part that
+// starts at item g: whole units of at most cap words together, or one unit alone.
+XT_HD inline int32_t flow_cut(const XItem *items, int32_t n, int64_t words, int32_t g, int64_t cap) {
+    const int64_t top = items[g].buf + cap;
+    if (words <= top) return n;
+    int32_t lo = g, hi = n - 1;  // the last item whose words start at or below top ...
+    while (lo < hi) {
+        const int32_t mid = lo + (hi - lo + 1) / 2;
+        if (items[mid].buf <= top) lo = mid;
+        else hi = mid - 1;
+    }
+    const int32_t last = lo;
+    lo = g, hi = last;  // ... and the first of those with the same start: its unit may end above top
+    while (lo < hi) {
+        const int32_t mid = lo + (hi - lo) / 2;
+        if (items[mid].buf < items[last].buf) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo > g ? lo : last + 1;
+}
+
 // Hand-off words per row of a chunk: the first column of every stripe but the
 // leftmost, and the exported columns.
 XT_HD inline int32_t chunk_words(int32_t K, int32_t X) { return K > 1 ? K - 1 + X : 0; }

@@ -955,6 +955,14 @@ __global__ void k_pair_finalize(const DPair *pairs, const DTree *trees, const DO
     trivial[p] = q.trivial;
 }
 
+// The parts of a list (flow_cut): where each starts, at most max of them, and
+// their count (one thread: some fifty loads a part, on lists that need more than one).
+__global__ void k_parts(const XItem *items, int n, int64_t words, int64_t cap, XPart *parts, int max, int32_t *count) {
+    int k = 0;
+    for (int g = 0; g < n && k < max; g = flow_cut(items, n, words, g, cap)) parts[k++] = XPart{items[g].buf, g, 0};
+    *count = k;
+}
+
 inline unsigned blocks_for(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 }  // namespace
@@ -1067,6 +1075,36 @@ void pair_params(const PairLayout &L, XKernelParams &K) {
     K.error = L.hdr + PAIR_ERROR;
     K.error_info = L.hdr + PAIR_ERROR + 1;
     K.hold_pair = -1;
+}
+
+int dev_parts(xted_ctx *c, int64_t cap, int64_t *need) {
+    std::vector<XPart> &parts = c->parts;
+    const int64_t words = c->plan_words;
+    const int n = c->kp.nitems;
+    parts.assign(1, XPart{0, 0, 0});
+    if (words > cap) {
+        // two neighbouring parts have more than cap words together
+        const int64_t max = std::min<int64_t>(2 * (words / std::max<int64_t>(cap, 1)) + 2, n);
+        int rc = ctx_dev_reserve(c, c->levels, sizeof(XPart) * (size_t)max + 256);  // (the levels have been used)
+        if (rc) return rc;
+        int32_t *d_count = (int32_t *)c->levels.p, count = 0;
+        XPart *d_parts = (XPart *)((char *)c->levels.p + 256);
+        k_parts<<<1, 1, 0, c->stream>>>(c->kp.items, n, words, cap, d_parts, (int)max, d_count);
+        if (cudaMemcpyAsync(&count, d_count, 4, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
+            cudaStreamSynchronize(c->stream) != cudaSuccess) {
+            cudaGetLastError();
+            return XTED_ECUDA;
+        }
+        parts.resize((size_t)count);
+        if (cudaMemcpy(parts.data(), d_parts, sizeof(XPart) * (size_t)count, cudaMemcpyDeviceToHost) != cudaSuccess) {
+            cudaGetLastError();
+            return XTED_ECUDA;
+        }
+    }
+    parts.push_back(XPart{words, n, 0});
+    *need = 0;
+    for (size_t k = 0; k + 1 < parts.size(); k++) *need = std::max(*need, parts[k + 1].word - parts[k].word);
+    return XTED_OK;
 }
 
 int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs, XKernelParams &K) {
@@ -1259,16 +1297,12 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     }
     const int64_t nitems = hs->items;
     if (nitems > INT32_MAX / 2) return XTED_ENOMEM;
-    // ---- buffer C: the items and the launch's counters; the hand-off words ----
+    // ---- buffer C: the items and the launch's counters ----
     rc = ctx_dev_reserve(c, c->work, sizeof(XItem) * (size_t)(nitems + 1) + 2 * 256 + 64);
     if (rc) return rc;
     Carver cw{(char *)c->work.p};
     XItem *d_items = cw.take<XItem>((size_t)nitems);
     int32_t *d_ctl = cw.take<int32_t>(2);  // items claimed, items finished
-    if (hs->words > 0) {
-        rc = ctx_dev_reserve(c, c->sbuf, (size_t)hs->words * sizeof(int32_t));
-        if (rc) return rc;
-    }
     if (nent > 0)
         k_level_fill<<<(unsigned)std::min<int64_t>(nent, 1 << 16), 128, 0, s>>>(C, d_pairs, d_lv, nent, d_items);
     if (cudaGetLastError() != cudaSuccess) return XTED_ECUDA;
@@ -1287,7 +1321,6 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     K.next = d_ctl;
     K.progress = d_ctl + 1;
     K.smap = (const int32_t *)c->smap.p;
-    K.buf = (int32_t *)c->sbuf.p;
     K.hold_pair = -1;
     c->d_trivial = d_trivial;
     c->plan_dt_elems = hs->dt_elems;
