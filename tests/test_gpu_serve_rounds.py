@@ -1,0 +1,65 @@
+"""Serving rounds inside one launch (needs a B200)."""
+import time
+
+import numpy as np
+import pytest
+
+import oracle
+import xted
+from xted import gen
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = ("random", "wide", "deep", "caterpillar")
+
+
+def _trees(n, seed, lo, hi):
+    rng = np.random.default_rng(seed)
+    return [gen.tree(SHAPES[i % 4], int(rng.integers(lo, hi + 1)), seed * 1000 + i, "zipf", 12) for i in range(n)]
+
+
+def _check(ids, ds, q, corpus, k):
+    d = oracle.distance_batch([(q, t) for t in corpus], nthreads=8)
+    order = sorted(range(len(corpus)), key=lambda i: (d[i], i))[:k]
+    assert ids.tolist() == order and ds.tolist() == [int(d[i]) for i in order]
+
+
+@pytest.mark.timeout(300)
+def test_second_round_joins_the_running_launch():
+    """Queries one after another, each with a second round: the tables are
+    cleared by the launch itself, so a round need not wait for its end (it did,
+    and every query took two launches)."""
+    corpus, queries = _trees(300, 5, 20, 90), _trees(24, 6, 20, 90)
+    with xted.Context() as ctx:
+        ctx.corpus_load(corpus)
+        for q in queries[:4]:
+            ctx.query_wait(ctx.query_submit(q, 5), timeout_s=60)
+        before = ctx.serve_stats()
+        for q in queries[4:]:
+            t = ctx.query_submit(q, 5)
+            ids, ds, _, _ = ctx.query_wait(t, timeout_s=60)
+            _check(ids, ds, q, corpus, 5)
+            time.sleep(0.01)  # (the launch goes idle and ends)
+        after = ctx.serve_stats()
+        rounds = len(queries) - 4 + after["second_rounds"] - before["second_rounds"]
+        assert rounds >= 30
+        assert after["launches"] - before["launches"] <= 25  # 20 queries; a slow host may miss the launch now and then
+
+
+@pytest.mark.timeout(300)
+def test_queries_that_arrive_while_others_run():
+    """Tables of a new query are cleared while other queries' items run: sizes
+    around one piece of the clearing, without and with pruning."""
+    corpus, queries = _trees(40, 7, 1, 140), _trees(20, 8, 1, 140)
+    with xted.Context() as ctx:
+        ctx.corpus_load(corpus)
+        for prune in (0, 2):
+            ctx.serve_options(prune)
+            tickets = []
+            for q in queries:
+                tickets.append(ctx.query_submit(q, len(corpus)))
+                time.sleep(0.001)
+            for q, t in zip(queries, tickets):
+                ids, ds, _, _ = ctx.query_wait(t, timeout_s=60)
+                _check(ids, ds, q, corpus, len(corpus))
+        ctx.serve_drain()

@@ -134,6 +134,7 @@ __device__ __forceinline__ int warp_suffix_max(int v) {
 #define FLOW_LISTS (XTED_SW + XTED_SW + XTED_SW / 4)
 #define FLOW_WARP_INTS (FLOW_RING + FLOW_STACK + FLOW_LISTS)
 #define FLOW_SMEM (XTED_FLOW_WARPS * FLOW_WARP_INTS * 4)
+#define FLOW_SERVE_SMEM (FLOW_SMEM + XTED_FLOW_WARPS * 4)  // and each warp's generation
 static_assert(XTED_SW == 32 * FLOW_W && XTED_MAX_NODES < 65536 && FLOW_PITCH % 4 == 0, "list entries and row places");
 // A row's flags in a run's row sequence, beside orl (20 bits) and the flags of
 // its node record (bits 29, 30). The ITEM_ flags are the same for every row of
@@ -724,12 +725,62 @@ __device__ void trace_item(const XKernelParams &P, int g, uint64_t claim, uint64
                                   ((unsigned long long)(width & 0xffff) << 16) | ((unsigned long long)(unsigned)rows << 32);
 }
 
+// Before a warp's first item of a list (a whole warp): clears pieces of the
+// list's tables and hand-off words while there are any, then waits for the
+// pieces of others; false once the launch has failed. The launch clears them
+// itself because it leaves an SM no registers: a memset beside it waited for all
+// work in flight to end and for the idle exit (a lone query of 20-100 nodes with
+// a second round took 4.1 ms against 0.9 so). The fences also order what was
+// posted before the list, and drop whatever this SM's L1 holds of it: once a list
+// and warp, where the claim of every item had one. (The claims' loop is tested
+// at its top: left by a break behind the shuffle, it made the compiler guard
+// every shuffle of the launch and spill, 16% of a query's time.)
+__device__ __noinline__ bool open_list(const XKernelParams &P, int slot, int lane) {
+    __threadfence();
+    XServeClear *c = P.clears + slot;
+    const int pieces = ld_relaxed(&c->pieces);
+    const int64_t off = ((volatile XServeClear *)c)->off, n = ((volatile XServeClear *)c)->n;
+    int k = 0;
+    if (lane == 0) k = atomicAdd(&c->claimed, 1);
+    k = __shfl_sync(FULLMASK, k, 0);
+    while (__any_sync(FULLMASK, k < pieces)) {
+        const int64_t lo = (int64_t)k * XTED_CLEAR_INTS;
+        const int len = (int)min(n - lo, (int64_t)XTED_CLEAR_INTS);
+        int32_t *p = P.dt + off + lo;
+        for (int i = 4 * lane; i + 4 <= len; i += 128) *(int4 *)(p + i) = make_int4(-1, -1, -1, -1);
+        if (lane < (len & 3)) p[(len & ~3) + lane] = -1;
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) {
+            atomicAdd(&c->done, 1);
+            k = atomicAdd(&c->claimed, 1);
+        }
+        k = __shfl_sync(FULLMASK, k, 0);
+    }
+    uint64_t t0 = 0;
+    while (__any_sync(FULLMASK, ld_relaxed(&c->done) < pieces)) {
+        __nanosleep(100);
+        bool out = ld_relaxed(P.error) != 0;
+        const uint64_t now = global_ns();
+        if (t0 == 0) t0 = now;
+        if (now - t0 > P.timeout_ns) {
+            set_error(P, XTED_ETIMEOUT, 3, slot, 0);
+            out = true;
+        }
+        if (__any_sync(FULLMASK, out)) return false;
+    }
+    __threadfence();
+    return true;
+}
+
 // The next item of a serving session (a whole warp): the lists of the queries
 // in flight, the oldest query's first. -1: leave the launch. Warps leave once
 // every one of them has been idle for a while (then the launch is closed and
 // the host starts another when work arrives); an item claimed meanwhile
-// runs to its end, the rest of its list waits for the next launch.
-__device__ __noinline__ int claim_served(const XKernelParams &P, int lane, int *slot) {
+// runs to its end, the rest of its list waits for the next launch. opened: the
+// generation of the list whose item the warp had last (through L2: L1 may hold
+// an item of an earlier list).
+__device__ __noinline__ int claim_served(const XKernelParams &P, int lane, int *slot, int *opened) {
     const int total = (int)(gridDim.x * (blockDim.x >> 5));
     bool idle = false;
     uint64_t t0 = 0;
@@ -754,8 +805,13 @@ __device__ __noinline__ int claim_served(const XKernelParams &P, int lane, int *
             }
             g = __shfl_sync(FULLMASK, g, 0);
             if (g >= 0) {
-                __threadfence();  // acquire: the query's plan and its cleared tables are visible from here on
                 *slot = q;
+                const int gen = __ldcg(&P.items[g].gen);
+                if (__any_sync(FULLMASK, gen != *(volatile int *)opened)) {
+                    if (!open_list(P, q, lane)) return -1;
+                    if (lane == 0) *(volatile int *)opened = gen;
+                    __syncwarp();
+                }
                 return g;
             }
             continue;
@@ -800,23 +856,27 @@ __device__ void finish_served(const XKernelParams &P, const XPair &pr, const XIt
 // pairs 38.2 -> 37.2, 4,560 small ones 13.03 -> 12.72. A launch bound by its
 // pairs' longest chains runs slower, row by row: 20,000 random 47.6 -> 48.9 ms,
 // 1,000 wide x deep 1.25 -> 1.40, a pair of 100 0.10 -> 0.115. 500 pairs: 7.83 -> 7.96.
-template <int BLOCKS>
+// SERVE: a serving session's launch, which claims from the lists of its queries.
+template <int BLOCKS, bool SERVE>
 __global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, BLOCKS) xted_flow_kernel(const __grid_constant__ XKernelParams P) {
     extern __shared__ __align__(16) int32_t s_dyn[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int32_t *ring = s_dyn + warp * FLOW_WARP_INTS;
-    const int nitems = P.plan ? P.plan->items : P.nitems;
-    const int64_t per = P.plan ? (int64_t)P.plan->stack_rows * XTED_SW : P.scratch_per_warp;
+    const XPlanOut *plan = SERVE ? nullptr : P.plan;
+    const int nitems = plan ? plan->items : P.nitems;
+    const int64_t per = plan ? (int64_t)plan->stack_rows * XTED_SW : P.scratch_per_warp;
     const int64_t gwarp = (int64_t)blockIdx.x * XTED_FLOW_WARPS + warp;
-    int32_t *gstk = P.scratch + (P.plan ? -(gwarp + 1) * per : gwarp * per);
+    int32_t *gstk = P.scratch + (plan ? -(gwarp + 1) * per : gwarp * per);
     for (int x = lane; x < FLOW_WARP_INTS; x += 32) ring[x] = 0;
     __syncwarp();
-    if (P.plan && (gwarp + 1) * per > P.plan->scratch) return;
+    if (plan && (gwarp + 1) * per > plan->scratch) return;
+    int *opened = s_dyn + XTED_FLOW_WARPS * FLOW_WARP_INTS + warp;  // SERVE: the generation of the list that the warp is on
+    if (SERVE && lane == 0) *opened = 0;
     for (;;) {
         int g = -1, slot = 0;
-        uint64_t t_claim = P.trace ? global_ns() : 0;
-        if (P.serve) {
-            g = claim_served(P, lane, &slot);
+        const uint64_t t_claim = !SERVE && P.trace ? global_ns() : 0;
+        if (SERVE) {
+            g = claim_served(P, lane, &slot, opened);
         } else {
             if (lane == 0 && ld_relaxed(P.error) == 0) {
                 g = atomicAdd(P.next, 1);
@@ -825,7 +885,7 @@ __global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, BLOCKS) xted_flow_kernel
             g = __shfl_sync(FULLMASK, g, 0);
         }
         if (g < 0) break;
-        const uint64_t t_start = P.trace ? global_ns() : 0;
+        const uint64_t t_start = !SERVE && P.trace ? global_ns() : 0;
         const XItem it = P.items[g];
         const XPair pr = P.pairs[it.pair];
         const XRun run = P.runs[it.run];
@@ -839,13 +899,13 @@ __global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, BLOCKS) xted_flow_kernel
         }
         if (lane == 0) {
             // run and chunk of the two roots: the pair's last table (its leftmost stripe ends last)
-            if (P.serve) {
+            if (SERVE) {
                 const bool root = it.stripe == 0 && run.rows == pr.m && ch.width == pr.n && run.kr_hi - run.kr_lo == 1 &&
                                   ch.nseg == 1;
                 finish_served(P, pr, it, root, slot);
             }
             atomicAdd(P.progress, 1);
-            if (P.trace) trace_item(P, g, t_claim, t_start, it.stripe, ch.width, run.rows);
+            if (!SERVE && P.trace) trace_item(P, g, t_claim, t_start, it.stripe, ch.width, run.rows);
         }
         __syncwarp();
     }
@@ -871,22 +931,25 @@ __global__ void xted_gather_kernel(const XPair *pairs, const int32_t *trivial, c
 }
 
 // ---- host-side launch helpers ----
-template <int BLOCKS>
+template <int BLOCKS, bool SERVE>
 static int occupancy_of(int *blocks_per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(xted_flow_kernel<BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, FLOW_SMEM);
+    const int smem = SERVE ? FLOW_SERVE_SMEM : FLOW_SMEM;
+    cudaError_t e = cudaFuncSetAttribute(xted_flow_kernel<BLOCKS, SERVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, xted_flow_kernel<BLOCKS>,
-                                                              32 * XTED_FLOW_WARPS, FLOW_SMEM);
+    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, xted_flow_kernel<BLOCKS, SERVE>,
+                                                              32 * XTED_FLOW_WARPS, smem);
 }
 int dp_occupancy(int *blocks_per_sm, bool full) {
-    return full ? occupancy_of<5>(blocks_per_sm) : occupancy_of<4>(blocks_per_sm);
+    return full ? occupancy_of<5, false>(blocks_per_sm) : occupancy_of<4, false>(blocks_per_sm);
 }
+int serve_occupancy(int *blocks_per_sm) { return occupancy_of<4, true>(blocks_per_sm); }
 
 // A plain launch: a block that is not resident has claimed nothing, and what
 // the resident warps have claimed needs only items claimed before.
 cudaError_t launch_dp(const XKernelParams &P, int grid, bool full, cudaStream_t s) {
-    if (full) xted_flow_kernel<5><<<grid, 32 * XTED_FLOW_WARPS, FLOW_SMEM, s>>>(P);
-    else xted_flow_kernel<4><<<grid, 32 * XTED_FLOW_WARPS, FLOW_SMEM, s>>>(P);
+    if (P.serve) xted_flow_kernel<4, true><<<grid, 32 * XTED_FLOW_WARPS, FLOW_SERVE_SMEM, s>>>(P);
+    else if (full) xted_flow_kernel<5, false><<<grid, 32 * XTED_FLOW_WARPS, FLOW_SMEM, s>>>(P);
+    else xted_flow_kernel<4, false><<<grid, 32 * XTED_FLOW_WARPS, FLOW_SMEM, s>>>(P);
     return cudaGetLastError();
 }
 

@@ -70,7 +70,7 @@ XT_HD inline XItem flow_item(const FlowCtx &C, const DDepth &ra, const DDepth &c
     XItem it;
     it.run = r;
     it.pair = pair;
-    it.pad[0] = it.pad[1] = 0;
+    it.gen = it.pad = 0;
     int32_t c = cb.chunk_lo + k;
     it.stripe = 0;
     it.buf = buf;

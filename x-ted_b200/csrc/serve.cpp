@@ -15,8 +15,8 @@
 // items fit ("DP scratch bytes"), in arrival order.
 //
 // Continuous batching. An admitted query's plan is copied to the device on a
-// copy stream, its tables set to "not written", and its slot's list word
-// (first item, end) written last. The warps of the DP kernel, launched once
+// copy stream, its slot's list word written last; the launch sets its tables to
+// "not written" before it runs the list's items. The warps of the DP kernel, launched once
 // and kept running while there is work, claim items from the lists of all
 // slots, the oldest query's first, so earlier queries finish first while later
 // ones fill idle warps. The item that ends a pair writes its distance into
@@ -47,6 +47,7 @@
 #include "serve_plan.h"
 
 namespace xted {
+int serve_occupancy(int *blocks_per_sm);
 cudaError_t launch_dp(const XKernelParams &P, int grid, bool full, cudaStream_t s);
 }
 
@@ -132,6 +133,7 @@ struct ServeState {
     xted_ctx *c = nullptr;
     int T = 0, S = XTED_SERVE_SLOTS, Qmax = XTED_SERVE_MAX_QUERY;  // XTED_SERVE_SLOTS == XTED_SERVE_SLOTS_MAX
     int32_t max_tree = 0;  // largest corpus tree
+    int grid = 0;          // blocks of the launch
     int64_t Nc_nonempty = 0;
     ServePools pools;  // host planning pools: the corpus, then one region per slot
     // device
@@ -145,6 +147,7 @@ struct ServeState {
     XChunkX *d_chunkx = nullptr;
     XItem *d_items = nullptr;
     unsigned long long *d_lists = nullptr;
+    XServeClear *d_clears = nullptr;
     int32_t *h_results = nullptr, *h_flags = nullptr;  // mapped pinned host memory
     Extents dt_ext, i_ext;
     XKernelParams K{};
@@ -245,14 +248,13 @@ void release(ServeState *s, Slot &sl) {
     sl = Slot{};
 }
 
-// Fixes the plan up to its device offsets, clears its tables, and copies it,
-// its slot words and last its list word to the device, in that order, on the
-// copy stream.
+// Fixes the plan up to its device offsets and copies it, its slot words and
+// last its list word to the device, in that order, on the copy stream.
 int post(ServeState *s, int slot, Slot &sl) {
     QPlan &p = sl.plan;
     const int T = s->T;
     const int64_t pair_base = (int64_t)slot * T;
-    serve_fixup_items(s->pools, p, slot, sl.dt_off);
+    serve_fixup_items(s->pools, p, slot, sl.dt_off, sl.gen);
     const ServePools &H = s->pools;
     const DTree &Q = H.trees[(size_t)(T + slot)];
     const size_t nb = 2 * (size_t)Q.nbase, n2 = 2 * (size_t)Q.n;
@@ -264,12 +266,12 @@ int post(ServeState *s, int slot, Slot &sl) {
                       p.items.end());
         s->c->fault = 0;
     }
+    const int64_t clear = p.dt_elems + p.words;
+    const XServeClear cl{sl.dt_off, clear, (int32_t)((clear + XTED_CLEAR_INTS - 1) / XTED_CLEAR_INTS), 0, 0, 0};
     const unsigned long long list =
         ((unsigned long long)(sl.i_off + (int64_t)p.items.size()) << 32) | (unsigned long long)sl.i_off;
     const int32_t age = (int32_t)sl.seq;
     int rc = XTED_OK;
-    if (cudaMemsetAsync(s->d_dt + sl.dt_off, 0xff, (size_t)(p.dt_elems + p.words) * 4, st) != cudaSuccess)
-        rc = XTED_ECUDA;
     rc |= upload(s->d_dt + sl.dt_off + p.dt_elems + p.words, p.smap.data(), p.smap.size() * 4, st);
     rc |= upload(s->d_node + nb, H.node.data() + nb, n2 * sizeof(int2), st);
     rc |= upload(s->d_krd + nb, H.krd.data() + nb, n2 * 4, st);
@@ -282,6 +284,7 @@ int post(ServeState *s, int slot, Slot &sl) {
     rc |= upload(s->d_slot + XTED_SERVE_SLOTS + slot, &words[0], 4, st);      // slot_need
     rc |= upload(s->d_slot + 2 * XTED_SERVE_SLOTS + slot, &words[1], 4, st);  // slot_gen
     rc |= upload(s->d_slot + 3 * XTED_SERVE_SLOTS + slot, &age, 4, st);
+    rc |= upload(s->d_clears + slot, &cl, sizeof(cl), st);
     rc |= upload(s->d_lists + slot, &list, sizeof(list), st);
     return rc ? XTED_ECUDA : XTED_OK;
 }
@@ -599,7 +602,7 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
     if (inflight && !s->running) {
         cudaStreamSynchronize(s->cs);
         bool ok = cudaMemsetAsync(s->d_ctl, 0, XTED_CTL_INTS * 4, s->ks) == cudaSuccess &&
-                  launch_dp(s->K, s->c->grid, false, s->ks) == cudaSuccess &&
+                  launch_dp(s->K, s->grid, false, s->ks) == cudaSuccess &&
                   cudaEventRecord(s->kev, s->ks) == cudaSuccess;
         if (!ok) {
             cudaGetLastError();
@@ -680,6 +683,9 @@ int load(xted_ctx *c, ServeState *s, const xted_tree *tr, int32_t ntrees) {
                       c->opts.tuned ? tune : nullptr, c->opts.tuned ? ntune : 0);
     const ServePools &H = s->pools;
     const size_t n2 = H.node.size();
+    int occ = 0;  // (a launch ends once all its warps are idle: no more blocks than are resident)
+    if (serve_occupancy(&occ) != 0 || occ < 1) return XTED_ECUDA;
+    s->grid = std::min(c->grid, occ * c->sms);
     // device memory
     int64_t dt_cap = std::min<int64_t>(kDtCapMax, (int64_t)S * Qm * std::max<int64_t>(nonempty, 1));
     if (c->opts.mem_limit > 0) dt_cap = std::min<int64_t>(dt_cap, c->opts.mem_limit / 8);  // half of the limit
@@ -695,12 +701,13 @@ int load(xted_ctx *c, ServeState *s, const xted_tree *tr, int32_t ntrees) {
     rc |= dev_alloc(s, &s->d_items, (size_t)kItemCap);
     rc |= dev_alloc(s, &s->d_lists, XTED_SERVE_SLOTS);
     rc |= dev_alloc(s, &s->d_ctl, XTED_CTL_INTS);
+    rc |= dev_alloc(s, &s->d_clears, XTED_SERVE_SLOTS);
     rc |= dev_alloc(s, &s->d_slot, 4 * XTED_SERVE_SLOTS);
     rc |= dev_alloc(s, &s->d_err, 8);
     rc |= dev_alloc(s, &s->d_dt, (size_t)dt_cap);
     // per-warp scratch: the far-row stack's rows outside the shared window
     const int64_t per = (int64_t)H.stack_rows * XTED_SW;
-    rc |= dev_alloc(s, &s->d_scratch, (size_t)per * (size_t)c->grid * XTED_FLOW_WARPS);
+    rc |= dev_alloc(s, &s->d_scratch, (size_t)per * (size_t)s->grid * XTED_FLOW_WARPS);
     if (rc) return XTED_ENOMEM;
     if (cudaHostAlloc((void **)&s->h_results, sizeof(int32_t) * std::max<size_t>((size_t)S * T, 1),
                       cudaHostAllocMapped) != cudaSuccess ||
@@ -757,6 +764,7 @@ int load(xted_ctx *c, ServeState *s, const xted_tree *tr, int32_t ntrees) {
     K.serve_pairs = T;
     K.idle_exit_ns = 2000000;  // 2 ms
     K.lists = s->d_lists;
+    K.clears = s->d_clears;
     K.ages = s->d_slot + 3 * XTED_SERVE_SLOTS;
     K.ctl = s->d_ctl;
     K.slot_done = s->d_slot;

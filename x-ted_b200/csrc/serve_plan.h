@@ -283,15 +283,16 @@ inline void serve_plan_items(ServePools &s, int slot, const int32_t *lab, const 
     });
 }
 
-// Moves a plan's items to their slot: pairs of slot `slot` start at slot * T;
+// Moves a plan's items to their slot as list generation gen: pairs of slot `slot` start at slot * T;
 // the query's device range at `off` holds its tables, hand-off words and
 // export maps in that order.
-inline void serve_fixup_items(ServePools &s, QPlan &p, int slot, int64_t off) {
+inline void serve_fixup_items(ServePools &s, QPlan &p, int slot, int64_t off, int32_t gen) {
     const int32_t pair_base = (int32_t)((int64_t)slot * s.T);
     for (XPair &x : p.pairs) x.dt_off += off;
     for (XItem &i : p.items) {
         i.pair += pair_base;
         i.buf += off + p.dt_elems;
+        i.gen = gen;
     }
     for (int o = 0; o < 2; o++) {
         const DOTree &O = s.otrees[2 * (size_t)(s.T + slot) + o];

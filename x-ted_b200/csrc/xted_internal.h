@@ -173,7 +173,8 @@ struct XItem {
     int32_t run, chunk, pair;
     int32_t stripe;           // stripe of the unit's chunk (0 for a chunk one warp holds)
     int64_t buf;              // striped unit: its hand-off words in XKernelParams::buf
-    int32_t pad[2];
+    int32_t gen;              // serving: the generation of its list
+    int32_t pad;
 };
 
 // What a column chunk adds to the plan (same index as its XChunk).
@@ -192,6 +193,14 @@ struct XPlanOut {
     int32_t status;  // nonzero: no plan, nothing to run
     int64_t cells, cells_right;
     int64_t words, scratch;  // hand-off words; ints left for the warps' stacks
+};
+
+// What a serving list's warps set to -1 before they run its items: n words of
+// the table pool from off on (16-byte aligned), in pieces of XTED_CLEAR_INTS.
+#define XTED_CLEAR_INTS 16384
+struct XServeClear {
+    int64_t off, n;
+    int32_t pieces, claimed, done, pad;
 };
 
 struct XKernelParams {
@@ -223,6 +232,7 @@ struct XKernelParams {
     int32_t serve_pairs;    // pairs per query slot (the corpus size)
     uint64_t idle_exit_ns;  // the launch ends once every warp has had no work for this long
     unsigned long long *lists;  // [XTED_SERVE_SLOTS] (end << 32) | next item of the slot's list
+    XServeClear *clears;    // [XTED_SERVE_SLOTS]
     const int32_t *ages;    // [XTED_SERVE_SLOTS] arrival number of the slot's query
     int32_t *ctl;           // XTED_CTL_* words
     int32_t *slot_done;     // [XTED_SERVE_SLOTS] items finished in the slot's current round
