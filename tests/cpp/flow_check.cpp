@@ -9,6 +9,7 @@
 // hand-off words; every index lies in its pool; the distance is the oracle's.
 // The list is run whole and in parts (flow_cut) that share one buffer: parts
 // consist of whole units, hold at most their limit or one unit, and cover the list.
+// Then as serving divides and places it (serve_cut, serve_fixup_items).
 //   usage: flow_check <rounds> <max_nodes> <seed>
 #include <algorithm>
 #include <cstdio>
@@ -84,7 +85,8 @@ struct Plan {
 };
 
 // Runs items [from, to) of a plan; word w0 of the list is the buffer's first.
-static void run_items(const Plan &p, int from, int to, int64_t w0, std::vector<int32_t> &dt, std::vector<int32_t> &buf) {
+static void run_items(const Plan &p, int from, int to, int64_t w0, std::vector<int32_t> &dt, std::vector<int32_t> &buf,
+                      const std::vector<int32_t> &smap) {
     const ServePools &H = p.H;
     const XPair &pr = p.q.pairs[0];
     const int2 *rows = H.node.data() + pr.row_base, *nodes = H.node.data() + pr.col_base;
@@ -158,7 +160,7 @@ static void run_items(const Plan &p, int from, int to, int64_t w0, std::vector<i
                                 far = S[(size_t)(fi - i0)][(size_t)fc];
                             } else {
                                 if (K == 1) FAIL("a far column outside its chunk");
-                                const int32_t x = p.q.smap[(size_t)(cx.map + fj - j0)];
+                                const int32_t x = smap[(size_t)(cx.map + fj - j0)];
                                 if (x < 0 || x >= X) FAIL("export %d of %lld", x, (long long)X);
                                 far = word((K - 1) * R + at[(size_t)(fi - i0)] * X, x);
                                 if (far < 0) FAIL("an exported column is not there yet");
@@ -174,7 +176,7 @@ static void run_items(const Plan &p, int from, int to, int64_t w0, std::vector<i
                         o = row[(size_t)c];
                     }
                     if (K > 1) {
-                        const int32_t x = p.q.smap[(size_t)(cx.map + j - j0)];
+                        const int32_t x = smap[(size_t)(cx.map + j - j0)];
                         const bool pushed = i > i0 && far_of(rows, i - 1) == i;  // a row read as a far row
                         if (x >= 0 && pushed) {
                             int32_t &o = word((K - 1) * R + t * X, x);
@@ -226,13 +228,32 @@ int main(int argc, char **argv) {
                     for (int k = from; k < to; k++)
                         if (p.q.items[(size_t)k].buf != w0) FAIL("a part of several units has %lld words", (long long)(w1 - w0));
                 std::vector<int32_t> buf((size_t)(w1 - w0), -1);
-                run_items(p, from, to, w0, dt, buf);
+                run_items(p, from, to, w0, dt, buf, p.q.smap);
             }
             if (cap >= p.q.words && np != 1) FAIL("%d parts", np);
             parts += np;
             if (dt[(size_t)p.q.pairs[0].dt_off] != want) FAIL("distance: saving %d, want %d", dt[(size_t)p.q.pairs[0].dt_off], want);
         }
         striped += p.q.words > 0;
+        // as serving posts it: parts bounded in words and items, at an offset of
+        // a pool that holds tables, the part's words and export maps side by side
+        const int64_t item_cap = 1 + (int64_t)(g() % (uint64_t)(n + 1));
+        serve_cut(p.q, p.q.words / 4 + 1, item_cap);
+        const int64_t off = 4 * (int64_t)(g() % 100), at = off + p.q.dt_elems;
+        serve_fixup_items(p.H, p.q, 0, off);
+        std::vector<int32_t> pool((size_t)at, -1);
+        pool.resize((size_t)(at + p.q.max_words), 7);
+        pool.insert(pool.end(), p.q.smap.begin(), p.q.smap.end());
+        if (p.q.cuts.front() != 0 || p.q.cuts.back() != n) FAIL("parts do not cover the list");
+        for (size_t k = 0; k + 1 < p.q.cuts.size(); k++) {
+            const int from = p.q.cuts[k], to = p.q.cuts[k + 1];
+            if (to - from > p.q.max_items || p.q.part_words[k] > p.q.max_words) FAIL("a part beyond the largest");
+            std::fill(pool.begin() + (long)at, pool.begin() + (long)(at + p.q.part_words[k]), -1);
+            run_items(p, from, to, 0, pool, pool, pool);
+        }
+        if (pool[(size_t)p.q.pairs[0].dt_off] != want) FAIL("distance in parts of a pool");
+        for (size_t k = 0; k < p.q.smap.size(); k++)
+            if (pool[(size_t)(at + p.q.max_words) + k] != p.q.smap[k]) FAIL("an export map was overwritten");
     }
     if (striped == 0 && maxn > 600) FAIL("no striped units");
     std::printf("ok: %lld items, %lld words, %lld parts, %lld striped pairs\n", items, words, parts, striped);

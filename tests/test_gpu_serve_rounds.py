@@ -63,3 +63,22 @@ def test_queries_that_arrive_while_others_run():
                 ids, ds, _, _ = ctx.query_wait(t, timeout_s=60)
                 _check(ids, ds, q, corpus, len(corpus))
         ctx.serve_drain()
+
+
+@pytest.mark.timeout(300)
+def test_lists_larger_than_the_pool():
+    """A query whose hand-off words exceed the session's pool (spines with a leg
+    per node on a random side) runs in parts, beside small queries, with and
+    without a second round."""
+    from test_gpu_flow_memory import _zigzag
+    corpus = [_zigzag(400 + 3 * k, k) for k in range(6)] + _trees(40, 9, 5, 60)
+    queries = [_zigzag(410, 50), gen.tree("random", 33, 3, "zipf", 12), _zigzag(395, 51)]
+    with xted.Context(mem_limit=256 << 20) as ctx:
+        ctx.corpus_load(corpus)
+        for prune in (0, 2):
+            ctx.serve_options(prune)
+            tickets = [ctx.query_submit(q, 8) for q in queries]
+            for q, t in zip(queries, tickets):
+                ids, ds, _, _ = ctx.query_wait(t, timeout_s=100)
+                _check(ids, ds, q, corpus, 8)
+        ctx.serve_drain()

@@ -123,6 +123,7 @@ struct Slot {
     uint64_t ticket = 0;
     int64_t seq = 0;
     int32_t gen = 0;
+    int part = 0;                // of the plan's list
     int64_t dt_off = 0, dt_n = 0, i_off = 0, i_n = 0;  // table pool and item pool ranges
     QPlan plan;
 };
@@ -150,6 +151,7 @@ struct ServeState {
     XServeClear *d_clears = nullptr;
     int32_t *h_results = nullptr, *h_flags = nullptr;  // mapped pinned host memory
     Extents dt_ext, i_ext;
+    int64_t dt_cap = 0;  // distances of a query's tables, at most
     XKernelParams K{};
     cudaStream_t ks = nullptr, cs = nullptr;
     cudaEvent_t kev = nullptr;
@@ -180,7 +182,8 @@ struct ServeState {
 namespace {
 
 constexpr int kMaxPending = 1 << 16;
-constexpr int64_t kItemCap = 24 << 20;
+constexpr int64_t kItemCap = 12 << 20;
+constexpr int64_t kItemPart = kItemCap / 2;  // a longer list is posted in parts, beside which others fit
 constexpr int64_t kDtCapMax = (int64_t)4 << 30;  // int32 elements (16 GiB)
 
 template <class T>
@@ -213,18 +216,25 @@ void free_all(ServeState *s) {
     s->ks = s->cs = nullptr;
 }
 
-// Table-pool elements of a planned query: tables, hand-off words, export maps
-// (whole 16-byte pieces, so every query's tables start on one).
+// Table-pool elements of a planned query: tables, hand-off words of a part,
+// export maps (whole 16-byte pieces, so every query's tables start on one).
 int64_t pool_elems(const QPlan &p) {
-    const int64_t n = std::max<int64_t>(p.dt_elems + p.words + (int64_t)p.smap.size(), 1);
+    const int64_t n = std::max<int64_t>(p.dt_elems + p.max_words + (int64_t)p.smap.size(), 1);
     return (n + XTED_PITCH - 1) / XTED_PITCH * XTED_PITCH;
+}
+
+// Divides a planned query's list: hand-off words of at most a quarter of the
+// table pool, or what its tables leave of it, at a time.
+void divide(ServeState *s, QPlan &p) {
+    const int64_t left = s->dt_ext.cap() - p.dt_elems - (int64_t)p.smap.size() - XTED_PITCH;
+    serve_cut(p, std::max<int64_t>(std::min(left, s->dt_ext.cap() / 4), 1), kItemPart);
 }
 
 // Reserves device room for a planned query; false if it does not fit now.
 bool reserve(ServeState *s, Slot &sl) {
     const QPlan &p = sl.plan;
     sl.dt_n = pool_elems(p);
-    sl.i_n = std::max<int64_t>((int64_t)p.items.size(), 1);
+    sl.i_n = std::max<int64_t>(p.max_items, 1);
     if (!s->dt_ext.alloc(sl.dt_n, &sl.dt_off)) return false;
     if (!s->i_ext.alloc(sl.i_n, &sl.i_off)) {
         s->dt_ext.release(sl.dt_off, sl.dt_n);
@@ -234,7 +244,13 @@ bool reserve(ServeState *s, Slot &sl) {
 }
 
 bool never_fits(ServeState *s, const QPlan &p) {
-    return pool_elems(p) > s->dt_ext.cap() || (int64_t)p.items.size() > s->i_ext.cap();
+    return p.distances > s->dt_cap || pool_elems(p) > s->dt_ext.cap() || p.max_items > s->i_ext.cap();
+}
+
+int32_t next_gen(ServeState *s) {
+    const int32_t g = s->next_gen++;
+    if (s->next_gen <= 0) s->next_gen = 1;
+    return g;
 }
 
 void release_extents(ServeState *s, Slot &sl) {
@@ -248,31 +264,48 @@ void release(ServeState *s, Slot &sl) {
     sl = Slot{};
 }
 
-// Fixes the plan up to its device offsets and copies it, its slot words and
-// last its list word to the device, in that order, on the copy stream.
+// Copies part sl.part of the plan's list, its slot words and last its list
+// word to the device, in that order, on the copy stream.
+int post_part(ServeState *s, int slot, Slot &sl) {
+    QPlan &p = sl.plan;
+    cudaStream_t st = s->cs;
+    XItem *items = p.items.data() + p.cuts[(size_t)sl.part];
+    int64_t n = p.cuts[(size_t)sl.part + 1] - p.cuts[(size_t)sl.part];
+    const int32_t words[2] = {(int32_t)n, sl.gen};
+    for (int64_t k = 0; k < n; k++) items[k].gen = sl.gen;
+    if (s->c->fault == XTED_FAULT_HOLD_PAIR) {  // test hook: one computed pair is never computed
+        const int32_t held = items[0].pair;
+        n = std::remove_if(items, items + n, [&](const XItem &i) { return i.pair == held; }) - items;
+        s->c->fault = 0;
+    }
+    const int64_t done = sl.part > 0 ? p.dt_elems : 0;  // the tables stay between parts
+    const int64_t clear = p.dt_elems - done + p.part_words[(size_t)sl.part];
+    const XServeClear cl{sl.dt_off + done, clear, (int32_t)((clear + XTED_CLEAR_INTS - 1) / XTED_CLEAR_INTS), 0, 0, 0};
+    const unsigned long long list = ((unsigned long long)(sl.i_off + n) << 32) | (unsigned long long)sl.i_off;
+    const int32_t age = (int32_t)sl.seq;
+    int rc = XTED_OK;
+    rc |= upload(s->d_items + sl.i_off, items, (size_t)n * sizeof(XItem), st);
+    rc |= upload(s->d_slot + XTED_SERVE_SLOTS + slot, &words[0], 4, st);      // slot_need
+    rc |= upload(s->d_slot + 2 * XTED_SERVE_SLOTS + slot, &words[1], 4, st);  // slot_gen
+    rc |= upload(s->d_slot + 3 * XTED_SERVE_SLOTS + slot, &age, 4, st);
+    rc |= upload(s->d_clears + slot, &cl, sizeof(cl), st);
+    rc |= upload(s->d_lists + slot, &list, sizeof(list), st);
+    return rc ? XTED_ECUDA : XTED_OK;
+}
+
+// Fixes the plan up to its device offsets and copies it to the device, with the
+// first part of its list.
 int post(ServeState *s, int slot, Slot &sl) {
     QPlan &p = sl.plan;
     const int T = s->T;
     const int64_t pair_base = (int64_t)slot * T;
-    serve_fixup_items(s->pools, p, slot, sl.dt_off, sl.gen);
+    serve_fixup_items(s->pools, p, slot, sl.dt_off);
     const ServePools &H = s->pools;
     const DTree &Q = H.trees[(size_t)(T + slot)];
     const size_t nb = 2 * (size_t)Q.nbase, n2 = 2 * (size_t)Q.n;
     cudaStream_t st = s->cs;
-    const int32_t words[2] = {(int32_t)p.items.size(), sl.gen};
-    if (s->c->fault == XTED_FAULT_HOLD_PAIR) {  // test hook: one computed pair is never computed
-        const int32_t held = p.items[0].pair;
-        p.items.erase(std::remove_if(p.items.begin(), p.items.end(), [&](const XItem &i) { return i.pair == held; }),
-                      p.items.end());
-        s->c->fault = 0;
-    }
-    const int64_t clear = p.dt_elems + p.words;
-    const XServeClear cl{sl.dt_off, clear, (int32_t)((clear + XTED_CLEAR_INTS - 1) / XTED_CLEAR_INTS), 0, 0, 0};
-    const unsigned long long list =
-        ((unsigned long long)(sl.i_off + (int64_t)p.items.size()) << 32) | (unsigned long long)sl.i_off;
-    const int32_t age = (int32_t)sl.seq;
     int rc = XTED_OK;
-    rc |= upload(s->d_dt + sl.dt_off + p.dt_elems + p.words, p.smap.data(), p.smap.size() * 4, st);
+    rc |= upload(s->d_dt + sl.dt_off + p.dt_elems + p.max_words, p.smap.data(), p.smap.size() * 4, st);
     rc |= upload(s->d_node + nb, H.node.data() + nb, n2 * sizeof(int2), st);
     rc |= upload(s->d_krd + nb, H.krd.data() + nb, n2 * 4, st);
     rc |= upload(s->d_cumw + nb, H.cumw.data() + nb, n2 * 4, st);
@@ -280,13 +313,8 @@ int post(ServeState *s, int slot, Slot &sl) {
     rc |= upload(s->d_chunks + nb, H.chunks.data() + nb, n2 * sizeof(XChunk), st);
     rc |= upload(s->d_chunkx + nb, H.chunkx.data() + nb, n2 * sizeof(XChunkX), st);
     rc |= upload(s->d_pairs + pair_base, p.pairs.data(), p.pairs.size() * sizeof(XPair), st);
-    rc |= upload(s->d_items + sl.i_off, p.items.data(), p.items.size() * sizeof(XItem), st);
-    rc |= upload(s->d_slot + XTED_SERVE_SLOTS + slot, &words[0], 4, st);      // slot_need
-    rc |= upload(s->d_slot + 2 * XTED_SERVE_SLOTS + slot, &words[1], 4, st);  // slot_gen
-    rc |= upload(s->d_slot + 3 * XTED_SERVE_SLOTS + slot, &age, 4, st);
-    rc |= upload(s->d_clears + slot, &cl, sizeof(cl), st);
-    rc |= upload(s->d_lists + slot, &list, sizeof(list), st);
-    return rc ? XTED_ECUDA : XTED_OK;
+    sl.part = 0;
+    return rc ? XTED_ECUDA : post_part(s, slot, sl);
 }
 
 // Empties a slot's list, so that no launch claims the rest of it.
@@ -402,10 +430,19 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
         if (!sl.busy || sl.gen == 0) continue;
         if (((volatile int32_t *)s->h_flags)[i] != sl.gen) continue;
         std::atomic_thread_fence(std::memory_order_acquire);
-        s->pairs_served += sl.plan.need;
-        s->cells_served += sl.plan.cells;
         progress = true;
         auto it = s->queries.find(sl.ticket);
+        if ((size_t)sl.part + 2 < sl.plan.cuts.size() && it != s->queries.end()) {  // the next part of its list
+            sl.part++;
+            sl.gen = next_gen(s);
+            if (post_part(s, i, sl) != XTED_OK) {
+                it->second.state = XTED_ECUDA;
+                release(s, sl);
+            }
+            continue;
+        }
+        s->pairs_served += sl.plan.need;
+        s->cells_served += sl.plan.cells;
         if (it == s->queries.end()) {
             release(s, sl);
             continue;
@@ -426,6 +463,7 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
                 const double t1 = now_ms();
                 serve_plan_items(s->pools, i, qcopy.lab.data(), qcopy.off.data(), qcopy.idx.data(), qcopy.n,
                                  s->c->opts.orientation, sl.plan, sl.inc.data());
+                divide(s, sl.plan);
                 const double t2 = now_ms();
                 lk.lock();
                 s->plan_us += (int64_t)((t2 - t1) * 1e3);
@@ -448,8 +486,7 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
         Slot &sl = s->slots[i];
         if (!sl.busy || !sl.need_post || !reserve(s, sl)) continue;
         sl.need_post = false;
-        sl.gen = s->next_gen++;
-        if (s->next_gen <= 0) s->next_gen = 1;
+        sl.gen = next_gen(s);
         auto it = s->queries.find(sl.ticket);
         if (post(s, i, sl) != XTED_OK) {
             if (it != s->queries.end()) it->second.state = XTED_ECUDA;
@@ -541,6 +578,7 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
             const double t1 = now_ms();
             serve_plan_items(s->pools, slot, qcopy.lab.data(), qcopy.off.data(), qcopy.idx.data(), qcopy.n,
                              s->c->opts.orientation, sl.plan, inc.data());
+            divide(s, sl.plan);
             const double t2 = now_ms();
             lk.lock();
             s->bound_us += (int64_t)((t1 - t0) * 1e3);
@@ -569,8 +607,7 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
             continue;
         }
         if (!reserve(s, sl)) break;  // wait for memory to free up
-        sl.gen = s->next_gen++;
-        if (s->next_gen <= 0) s->next_gen = 1;
+        sl.gen = next_gen(s);
         const int rc = post(s, slot, sl);
         s->pending.pop_front();
         if (rc) {
@@ -690,6 +727,8 @@ int load(xted_ctx *c, ServeState *s, const xted_tree *tr, int32_t ntrees) {
     int64_t dt_cap = std::min<int64_t>(kDtCapMax, (int64_t)S * Qm * std::max<int64_t>(nonempty, 1));
     if (c->opts.mem_limit > 0) dt_cap = std::min<int64_t>(dt_cap, c->opts.mem_limit / 8);  // half of the limit
     dt_cap = std::max<int64_t>(dt_cap, 1);
+    s->dt_cap = dt_cap;
+    dt_cap += std::max<int64_t>(dt_cap / 32, 1 << 20);  // hand-off words and export maps beside the largest tables
     int rc = XTED_OK;
     rc |= dev_alloc(s, &s->d_node, n2);
     rc |= dev_alloc(s, &s->d_krd, n2);

@@ -51,7 +51,11 @@ struct QPlan {
     std::vector<XItem> items;     // the launch's items, in list order
     std::vector<int32_t> smap;    // export maps of the query's striped chunks
     int64_t words = 0;            // hand-off words of striped units
+    std::vector<int32_t> cuts;    // parts of the list, each posted once the one before has ended: their first items, the end
+    std::vector<int64_t> part_words;  // ... and the hand-off words of each
+    int64_t max_words = 0, max_items = 0;  // the most of a part
     int64_t dt_elems = 0, cells = 0;
+    int64_t distances = 0;        // of all tables (dt_elems: with their rows on 16 bytes)
     int32_t need = 0;             // pairs the device computes
 };
 
@@ -195,6 +199,7 @@ inline void serve_plan_pairs(ServePools &s, int slot, const int32_t *lab, const 
         x.col_base = s.otrees[2 * (size_t)tq + d.o].node_base;
         x.pitch = table_pitch(n);
         dt += (int64_t)x.m * x.pitch;
+        out.distances += (int64_t)x.m * x.n;
         d.lvl_base = (int32_t)lv.size();
         out.first[(size_t)t] = d.lvl_base;
         for (int l = 0; l < d.L; l++) {
@@ -283,23 +288,52 @@ inline void serve_plan_items(ServePools &s, int slot, const int32_t *lab, const 
     });
 }
 
-// Moves a plan's items to their slot as list generation gen: pairs of slot `slot` start at slot * T;
-// the query's device range at `off` holds its tables, hand-off words and
-// export maps in that order.
-inline void serve_fixup_items(ServePools &s, QPlan &p, int slot, int64_t off, int32_t gen) {
+// Divides a plan's list into parts of at most word_cap hand-off words and
+// item_cap items (or one unit alone, where that is more).
+inline void serve_cut(QPlan &p, int64_t word_cap, int64_t item_cap) {
+    const int32_t n = (int32_t)p.items.size();
+    p.cuts.assign(1, 0);
+    p.part_words.clear();
+    p.max_words = p.max_items = 0;
+    for (int32_t g = 0; g < n;) {
+        int32_t e = flow_cut(p.items.data(), n, p.words, g, word_cap);
+        if (e - g > item_cap) {
+            auto same = [&](int32_t k) {  // items k - 1 and k are stripes of one unit
+                const XItem &a = p.items[(size_t)k - 1], &b = p.items[(size_t)k];
+                return a.run == b.run && a.chunk == b.chunk && a.pair == b.pair;
+            };
+            int32_t k = g + (int32_t)item_cap;
+            while (k > g && same(k)) k--;
+            for (k = k > g ? k : g + (int32_t)item_cap; k < e && same(k);) k++;
+            e = k;
+        }
+        const int64_t w = (e < n ? p.items[(size_t)e].buf : p.words) - p.items[(size_t)g].buf;
+        p.part_words.push_back(w);
+        p.max_words = w > p.max_words ? w : p.max_words;
+        p.max_items = e - g > p.max_items ? e - g : p.max_items;
+        p.cuts.push_back(g = e);
+    }
+}
+
+// Moves a divided plan to its slot: pairs of slot `slot` start at slot * T; the
+// query's device range at `off` holds its tables, the hand-off words of the
+// part that runs, and its export maps in that order.
+inline void serve_fixup_items(ServePools &s, QPlan &p, int slot, int64_t off) {
     const int32_t pair_base = (int32_t)((int64_t)slot * s.T);
     for (XPair &x : p.pairs) x.dt_off += off;
-    for (XItem &i : p.items) {
-        i.pair += pair_base;
-        i.buf += off + p.dt_elems;
-        i.gen = gen;
+    for (size_t k = 0; k + 1 < p.cuts.size(); k++) {
+        const int64_t move = off + p.dt_elems - p.items[(size_t)p.cuts[k]].buf;
+        for (int32_t g = p.cuts[k]; g < p.cuts[k + 1]; g++) {
+            p.items[(size_t)g].pair += pair_base;
+            p.items[(size_t)g].buf += move;
+        }
     }
     for (int o = 0; o < 2; o++) {
         const DOTree &O = s.otrees[2 * (size_t)(s.T + slot) + o];
         if (O.D < 0) continue;
         const DDepth &last = s.depths[(size_t)(O.depth_base + O.D)];
         for (int32_t c = O.node_base; c < last.chunk_lo + last.nnarrow + last.nhalf + last.nwide; c++)
-            s.chunkx[(size_t)c].map += off + p.dt_elems + p.words;
+            s.chunkx[(size_t)c].map += off + p.dt_elems + p.max_words;
     }
 }
 
