@@ -82,3 +82,27 @@ def test_lists_larger_than_the_pool():
                 ids, ds, _, _ = ctx.query_wait(t, timeout_s=100)
                 _check(ids, ds, q, corpus, 8)
         ctx.serve_drain()
+
+
+@pytest.mark.timeout(300)
+def test_a_failed_query_leaves_its_slot_to_the_next():
+    """A query whose work is lost fails and its slot's list is emptied, in the
+    stream's order, before the next query's is posted there: more queries than
+    slots wait behind it, several times."""
+    corpus, queries = _trees(20, 10, 5, 60), _trees(20, 11, 5, 60)
+    with xted.Context() as ctx:
+        ctx.corpus_load(corpus)
+        ctx.serve_options(prune=0)
+        for _ in range(4):
+            ctx.test_fault(xted.XTED_FAULT_HOLD_PAIR)
+            tickets = [ctx.query_submit(q, 3) for q in queries]
+            failed = 0
+            for q, t in zip(queries, tickets):
+                try:
+                    ids, ds, _, _ = ctx.query_wait(t, timeout_s=60)
+                except xted.XtedError as e:
+                    assert e.code == xted.XTED_ETIMEOUT
+                    failed += 1
+                else:
+                    _check(ids, ds, q, corpus, 3)
+            assert failed == 1

@@ -317,10 +317,11 @@ int post(ServeState *s, int slot, Slot &sl) {
     return rc ? XTED_ECUDA : post_part(s, slot, sl);
 }
 
-// Empties a slot's list, so that no launch claims the rest of it.
+// Empties a slot's list, so that no launch claims the rest of it (on the copy
+// stream: what is posted to the slot next comes after it).
 void close_list(ServeState *s, int slot) {
-    if (cudaMemset(s->d_lists + slot, 0, sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMemset(s->d_slot + slot, 0, 4) != cudaSuccess)
+    const unsigned long long none = 0;
+    if (upload(s->d_lists + slot, &none, sizeof(none), s->cs) || upload(s->d_slot + slot, &none, 4, s->cs))
         cudaGetLastError();
 }
 
@@ -506,7 +507,7 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
         if (err != 0) {
             s->error = err;
             fail_inflight(s, err);
-            cudaMemset(s->d_err, 0, 8 * sizeof(int32_t));
+            cudaMemsetAsync(s->d_err, 0, 8 * sizeof(int32_t), s->cs);  // (a launch waits for this stream)
             for (int i = 0; i < s->S; i++) close_list(s, i);  // what is left of them is void
             s->cv_done.notify_all();
             progress = true;
