@@ -208,6 +208,14 @@ int main(int argc, char **argv) {
         static const int narrow[4] = {0, 256, 17, 100}, rr[4] = {16, 1, 256, 50};
         serve_pools_build(p.H, &ta, 1, 1, maxn, rr[g() % 4], narrow[g() % 4], XTED_HALF_DEFAULT);
         serve_plan_items(p.H, 0, b.lab.data(), b.off.data(), b.idx.data(), b.n, r % 3, p.q);
+        size_t maps = 0;  // of the column tree's decomposition that the pair uses, and no other
+        const DOTree &O = p.H.otrees[(size_t)(p.q.pairs[0].col_base == p.H.otrees[3].node_base ? 3 : 2)];
+        for (int d = 0; d <= O.D; d++) {
+            const DDepth &dd = p.H.depths[(size_t)(O.depth_base + d)];
+            for (int c = dd.chunk_lo; c < dd.chunk_lo + dd.nnarrow + dd.nhalf + dd.nwide; c++)
+                if (chunk_stripes(p.H.chunks[(size_t)c], p.H.krd.data()) > 1) maps += (size_t)p.H.chunks[(size_t)c].width;
+        }
+        if (p.q.smap.size() != maps) FAIL("%zu words of export maps, %zu of the columns in use", p.q.smap.size(), maps);
         const int n = (int)p.q.items.size();
         items += n;
         words += p.q.words;

@@ -223,9 +223,13 @@ inline void serve_plan_items(ServePools &s, int slot, const int32_t *lab, const 
     std::vector<DLevel> lv;
     serve_plan_pairs(s, slot, lab, off, idx, n, orientation, out, include, dp, lv);
     const int tq = s.T + slot;
+    bool used[2] = {false, false};
+    for (const DLevel &l : lv) used[dp[(size_t)l.pair].o] = true;
     for (int o = 0; o < 2; o++) {
         const DOTree &O = s.otrees[2 * (size_t)tq + o];
-        for (int d = 0; d <= O.D; d++) {
+        // a decomposition that no pair uses gets no export maps: the dearer one of a long comb has a map of
+        // a quarter of its nodes squared
+        for (int d = 0; used[o] && d <= O.D; d++) {
             DDepth &dd = s.depths[(size_t)(O.depth_base + d)];
             for (int32_t c = dd.chunk_lo; c < dd.chunk_lo + dd.nnarrow + dd.nhalf + dd.nwide; c++) {
                 const XChunk &ch = s.chunks[(size_t)c];
@@ -330,7 +334,9 @@ inline void serve_fixup_items(ServePools &s, QPlan &p, int slot, int64_t off) {
     }
     for (int o = 0; o < 2; o++) {
         const DOTree &O = s.otrees[2 * (size_t)(s.T + slot) + o];
-        if (O.D < 0) continue;
+        bool used = false;
+        for (const XPair &x : p.pairs) used |= x.m > 0 && x.col_base == O.node_base;
+        if (O.D < 0 || !used) continue;
         const DDepth &last = s.depths[(size_t)(O.depth_base + O.D)];
         for (int32_t c = O.node_base; c < last.chunk_lo + last.nnarrow + last.nhalf + last.nwide; c++)
             s.chunkx[(size_t)c].map += off + p.dt_elems + p.max_words;
