@@ -106,3 +106,28 @@ def test_a_failed_query_leaves_its_slot_to_the_next():
                 else:
                     _check(ids, ds, q, corpus, 3)
             assert failed == 1
+
+
+@pytest.mark.timeout(300)
+def test_calls_while_lists_are_posted():
+    """Polls and submissions from other threads while the worker plans and posts."""
+    import threading
+    corpus, queries = _trees(120, 12, 100, 400), _trees(30, 13, 100, 400)
+    with xted.Context() as ctx:
+        ctx.corpus_load(corpus)
+        ctx.serve_options(prune=0)
+        want = [ctx.query_wait(ctx.query_submit(q, 4), timeout_s=60)[:2] for q in queries]
+        got = [None] * len(queries)
+
+        def client(lo):
+            for i in range(lo, len(queries), 3):
+                got[i] = ctx.query_wait(ctx.query_submit(queries[i], 4), poll_s=0.0, timeout_s=60)[:2]
+
+        threads = [threading.Thread(target=client, args=(k,)) for k in range(3)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for (a, b), (c, d) in zip(want, got):
+            assert np.array_equal(a, c) and np.array_equal(b, d)
+        ctx.serve_drain()

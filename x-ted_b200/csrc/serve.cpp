@@ -247,6 +247,12 @@ bool never_fits(ServeState *s, const QPlan &p) {
     return p.distances > s->dt_cap || pool_elems(p) > s->dt_ext.cap() || p.max_items > s->i_ext.cap();
 }
 
+bool take_hold(ServeState *s) {
+    const bool hold = s->c->fault == XTED_FAULT_HOLD_PAIR;
+    if (hold) s->c->fault = 0;
+    return hold;
+}
+
 int32_t next_gen(ServeState *s) {
     const int32_t g = s->next_gen++;
     if (s->next_gen <= 0) s->next_gen = 1;
@@ -265,18 +271,19 @@ void release(ServeState *s, Slot &sl) {
 }
 
 // Copies part sl.part of the plan's list, its slot words and last its list
-// word to the device, in that order, on the copy stream.
-int post_part(ServeState *s, int slot, Slot &sl) {
+// word to the device, in that order, on the copy stream. Called without the
+// lock (a list may be 200 MB, and a poll would wait for its copy): the slot is
+// the worker's own. hold: the test hook, one computed pair is never computed.
+int post_part(ServeState *s, int slot, Slot &sl, bool hold) {
     QPlan &p = sl.plan;
     cudaStream_t st = s->cs;
     XItem *items = p.items.data() + p.cuts[(size_t)sl.part];
     int64_t n = p.cuts[(size_t)sl.part + 1] - p.cuts[(size_t)sl.part];
     const int32_t words[2] = {(int32_t)n, sl.gen};
     for (int64_t k = 0; k < n; k++) items[k].gen = sl.gen;
-    if (s->c->fault == XTED_FAULT_HOLD_PAIR) {  // test hook: one computed pair is never computed
+    if (hold) {
         const int32_t held = items[0].pair;
         n = std::remove_if(items, items + n, [&](const XItem &i) { return i.pair == held; }) - items;
-        s->c->fault = 0;
     }
     const int64_t done = sl.part > 0 ? p.dt_elems : 0;  // the tables stay between parts
     const int64_t clear = p.dt_elems - done + p.part_words[(size_t)sl.part];
@@ -295,7 +302,7 @@ int post_part(ServeState *s, int slot, Slot &sl) {
 
 // Fixes the plan up to its device offsets and copies it to the device, with the
 // first part of its list.
-int post(ServeState *s, int slot, Slot &sl) {
+int post(ServeState *s, int slot, Slot &sl, bool hold) {
     QPlan &p = sl.plan;
     const int T = s->T;
     const int64_t pair_base = (int64_t)slot * T;
@@ -314,7 +321,7 @@ int post(ServeState *s, int slot, Slot &sl) {
     rc |= upload(s->d_chunkx + nb, H.chunkx.data() + nb, n2 * sizeof(XChunkX), st);
     rc |= upload(s->d_pairs + pair_base, p.pairs.data(), p.pairs.size() * sizeof(XPair), st);
     sl.part = 0;
-    return rc ? XTED_ECUDA : post_part(s, slot, sl);
+    return rc ? XTED_ECUDA : post_part(s, slot, sl, hold);
 }
 
 // Empties a slot's list, so that no launch claims the rest of it (on the copy
@@ -434,10 +441,15 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
         progress = true;
         auto it = s->queries.find(sl.ticket);
         if ((size_t)sl.part + 2 < sl.plan.cuts.size() && it != s->queries.end()) {  // the next part of its list
+            Query &q = it->second;  // (stays where it is until it is done or has failed)
             sl.part++;
             sl.gen = next_gen(s);
-            if (post_part(s, i, sl) != XTED_OK) {
-                it->second.state = XTED_ECUDA;
+            const bool hold = take_hold(s);
+            lk.unlock();
+            const int rc = post_part(s, i, sl, hold);
+            lk.lock();
+            if (rc != XTED_OK) {
+                q.state = XTED_ECUDA;
                 release(s, sl);
             }
             continue;
@@ -488,8 +500,12 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
         if (!sl.busy || !sl.need_post || !reserve(s, sl)) continue;
         sl.need_post = false;
         sl.gen = next_gen(s);
+        const bool hold = take_hold(s);
+        lk.unlock();
+        const int rc = post(s, i, sl, hold);
+        lk.lock();
         auto it = s->queries.find(sl.ticket);
-        if (post(s, i, sl) != XTED_OK) {
+        if (rc != XTED_OK) {
             if (it != s->queries.end()) it->second.state = XTED_ECUDA;
             release(s, sl);
         }
@@ -609,15 +625,18 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
         }
         if (!reserve(s, sl)) break;  // wait for memory to free up
         sl.gen = next_gen(s);
-        const int rc = post(s, slot, sl);
         s->pending.pop_front();
+        q.state = 1;
+        const bool hold = take_hold(s);
+        lk.unlock();
+        const int rc = post(s, slot, sl, hold);
+        lk.lock();
         if (rc) {
             q.state = rc;
             release(s, sl);
             s->cv_done.notify_all();
             continue;
         }
-        q.state = 1;
         q.t_admit = now_ms();
         progress = true;
     }
