@@ -131,3 +131,16 @@ def test_calls_while_lists_are_posted():
         for (a, b), (c, d) in zip(want, got):
             assert np.array_equal(a, c) and np.array_equal(b, d)
         ctx.serve_drain()
+
+
+@pytest.mark.timeout(300)
+def test_closing_with_queries_in_every_state():
+    """A context closed while the worker plans, posts and runs."""
+    corpus, queries = _trees(120, 12, 100, 400), _trees(30, 13, 100, 400)
+    for pause in (0.0, 0.0005, 0.001, 0.002, 0.003, 0.005, 0.01, 0.05):
+        with xted.Context() as ctx:
+            ctx.corpus_load(corpus)
+            ctx.serve_options(2 if pause == 0.05 else 0)
+            for q in queries:
+                ctx.query_submit(q, 4)
+            time.sleep(pause)

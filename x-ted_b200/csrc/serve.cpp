@@ -470,15 +470,21 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
                 release_extents(s, sl);
                 sl.gen = 0;
                 sl.round = 2;
-                sl.inc = std::move(inc2);
                 Query qcopy = q;
                 lk.unlock();
                 const double t1 = now_ms();
+                QPlan plan;
                 serve_plan_items(s->pools, i, qcopy.lab.data(), qcopy.off.data(), qcopy.idx.data(), qcopy.n,
-                                 s->c->opts.orientation, sl.plan, sl.inc.data());
-                divide(s, sl.plan);
+                                 s->c->opts.orientation, plan, inc2.data());
+                divide(s, plan);
                 const double t2 = now_ms();
                 lk.lock();
+                if (s->stop) {  // shutting down: no further round
+                    sl = Slot{};
+                    continue;
+                }
+                sl.plan = std::move(plan);
+                sl.inc = std::move(inc2);
                 s->plan_us += (int64_t)((t2 - t1) * 1e3);
                 s->second_rounds++;
                 if (never_fits(s, sl.plan)) {  // round 2 covers more trees than round 1 did
@@ -593,9 +599,10 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
             std::vector<uint8_t> inc;
             first_round(s, qcopy, lb, dist, inc);
             const double t1 = now_ms();
+            QPlan plan;  // (a shutdown empties the slots meanwhile)
             serve_plan_items(s->pools, slot, qcopy.lab.data(), qcopy.off.data(), qcopy.idx.data(), qcopy.n,
-                             s->c->opts.orientation, sl.plan, inc.data());
-            divide(s, sl.plan);
+                             s->c->opts.orientation, plan, inc.data());
+            divide(s, plan);
             const double t2 = now_ms();
             lk.lock();
             s->bound_us += (int64_t)((t1 - t0) * 1e3);
@@ -603,6 +610,7 @@ bool step(ServeState *s, std::unique_lock<std::mutex> &lk) {
             if (s->stop || !sl.busy || sl.ticket != ticket) break;  // shut down meanwhile
             q.lb = std::move(lb);
             q.dist = std::move(dist);
+            sl.plan = std::move(plan);
             sl.inc = std::move(inc);
             sl.round = 1;
             progress = true;
