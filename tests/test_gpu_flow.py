@@ -104,3 +104,20 @@ def test_launch_of_many_pairs(npairs):
         ctx.prepare_batch(pairs)
         for _ in range(3):
             assert np.array_equal(ctx.run_prepared(), want)
+
+
+@pytest.mark.timeout(300)
+@pytest.mark.parametrize("n", [303, 304, 305, 340, 513])
+def test_far_values_of_other_stripes(n):
+    """The same combs with 47, 48 (the places beside the usual stack rows), 49,
+    84 and 255 far values of other stripes in a stripe, against rows that pop the
+    stack one by one and rows that leave and refill its window; in a batch wide
+    enough that stripes wait for each other."""
+    rows = [_comb(9, 5, False), _comb(61, 7, False), _comb(40, 8, True), gen.tree("deep", 90, 9, "uniform", 4),
+            gen.tree("random", 120, 10, "uniform", 4)]
+    pairs = [(a, _comb(n, s, False)) for a in rows for s in (6, 11)]
+    want = oracle.distance_batch(pairs, nthreads=8)
+    with xted.Context(orientation=xted.ORIENT_RIGHT) as ctx:
+        assert np.array_equal(ctx.distance_batch(pairs), want)
+        assert [ctx.distance(a, b) for a, b in pairs[:3]] == want[:3].tolist()
+        assert np.array_equal(ctx.distance_batch(pairs * 40), np.tile(want, 40))

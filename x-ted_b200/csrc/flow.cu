@@ -197,7 +197,11 @@ __device__ __forceinline__ bool warp_wait(const XKernelParams &P, const int32_t 
 // and their value goes out), those that stripes further left read, and those
 // whose far column lies in another stripe. What a row rarely needs (waiting,
 // the stack leaving its window) is marked unlikely. OVER: a stripe that takes
-// more far values from other stripes than have a place in shared memory.
+// more far values from other stripes than have a place beside the usual four
+// stack rows: two rows are kept, with a place for all, filled when a row first
+// needs them (200 pairs of zigzags of 500 nodes, whose stripes take up to 90
+// values: 1,207 ms with the values past 48 loaded column by column on every
+// row, 822 ms so).
 // Returns 0, FLOW_FAILED once the launch has failed, or FLOW_OVER (nothing
 // done) if OVER is needed.
 #define FLOW_FAILED 1
@@ -205,8 +209,11 @@ __device__ __forceinline__ bool warp_wait(const XKernelParams &P, const int32_t 
 template <bool OVER>
 __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it, const XPair &pr, const XRun &run,
                                          const XChunk &ch, int32_t *ring, int32_t *gstk) {
-    constexpr int W = FLOW_W, PF = FLOW_PF, SC = FLOW_STACK_ROWS, ZERO = FLOW_ZERO, IMP = ZERO + 4;
-    constexpr unsigned SLOT_B = 4 * XTED_SW, RING_B = PF * SLOT_B, PITCH_B = 4 * FLOW_PITCH;
+    constexpr int W = FLOW_W, PF = FLOW_PF, ZERO = FLOW_ZERO, IMP = ZERO + 4;
+    // OVER: a stack window of two rows, with a place for every column's far value, and the places' export indices
+    constexpr int SC = OVER ? 2 : FLOW_STACK_ROWS, PLACES = OVER ? XTED_SW : FLOW_IMPORTS;
+    constexpr unsigned SLOT_B = 4 * XTED_SW, RING_B = PF * SLOT_B, PITCH_B = 4 * (IMP + PLACES);
+    static_assert(SC * PITCH_B + (OVER ? 2 * PLACES : 0) <= 4 * FLOW_STACK, "the window's room");
     const int lane = threadIdx.x & 31;
     const int2 *rows = P.rowinfo + pr.row_base, *nodes = P.rowinfo + pr.col_base;
     int32_t *dt = P.dt + pr.dt_off;
@@ -349,9 +356,10 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
         if ((xfar >> k) & 1u) xl[x1++] = fb[k];
     }
     __syncwarp();
-    unsigned xover = 0;  // OVER, bit k: a far column elsewhere with no place beside the stack row
     int xq[2] = {0, 0};  // export index of the value in place q, q = lane, lane + 32
     int iv[2] = {0, 0};  // ... and the value for the next row
+    unsigned short *xs = (unsigned short *)((char *)(ring + FLOW_RING) + SC * PITCH_B);  // OVER: of all places
+    bool imported = false;  // OVER: the top row's places hold its values
     if (nx > 0) {
         // columns with one far column follow each other (subtrees across a
         // boundary are nested): they share a place
@@ -363,7 +371,7 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
             const unsigned m = __ballot_sync(FULLMASK, first);
             const int place = places + __popc(m & (0xffffffffu >> (31 - lane))) - 1;
             if (q < nx) xplace[q] = place;
-            if (first && place < FLOW_IMPORTS) xd[place] = xl[q];
+            if (first && place < PLACES) xd[place] = xl[q];
             places += __popc(m);
         }
         nx = places;
@@ -372,12 +380,15 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
 #pragma unroll
         for (int k = 0; k < W; k++)
             if ((xfar >> k) & 1u) {
-                const int place = xplace[xf++];
-                if (place >= FLOW_IMPORTS) xover |= 1u << k;
-                fb[k] = 4 * (place < FLOW_IMPORTS ? IMP + place : ZERO);
+                fb[k] = 4 * (IMP + xplace[xf++]);
             }
-        if (lane < nx) xq[0] = xd[lane];
-        if (lane + 32 < min(nx, FLOW_IMPORTS)) xq[1] = xd[lane + 32];
+        if (OVER) {
+#pragma unroll 1
+            for (int q = lane; q < nx; q += 32) xs[q] = (unsigned short)xd[q];
+        } else {
+            if (lane < nx) xq[0] = xd[lane];
+            if (lane + 32 < nx) xq[1] = xd[lane + 32];
+        }
     }
     // the lane's copies of a row. multi: word lane + 32 k from column cpn[k] (-1: none); else pieces lane and lane + 32
     int cpn[W];
@@ -590,7 +601,30 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
                 for (int k = 0; k < W; k++) sts(top + 4 * lane + 128 * k, g[32 * k]);
                 __syncwarp();
             }
-            if (y & ITEM_IMPORTS) {  // some far columns lie in stripes to the right: the far row's exports
+            if (OVER && !imported) {
+                // loaded here and not a row ahead: the values would take registers that the loop below spills
+                const int i = __shfl_sync(FULLMASK, bi, tl);
+                const int32_t *erow = E + (unsigned)(t - ((int)(y & XTED_ROW_ORL_MASK) + 1 - i)) * (unsigned)X;  // (R X < 2^32)
+                int v[W];
+#pragma unroll
+                for (int k = 0; k < W; k++) v[k] = lane + 32 * k < nx ? ld_relaxed(erow + xs[lane + 32 * k]) : 0;
+                for (;;) {
+                    int x = -1, w = 0;
+#pragma unroll
+                    for (int k = 0; k < W; k++)
+                        if (v[k] < 0) x = lane + 32 * k;
+                    if (!__any_sync(FULLMASK, x >= 0)) break;
+                    if (!warp_wait(P, erow + xs[max(x, 0)], x >= 0, w)) return FLOW_FAILED;
+#pragma unroll
+                    for (int k = 0; k < W; k++)
+                        if (v[k] < 0) v[k] = ld_relaxed(erow + xs[lane + 32 * k]);
+                }
+#pragma unroll
+                for (int k = 0; k < W; k++) sts(top + 4 * (IMP + lane + 32 * k), v[k]);
+                __syncwarp();
+                imported = true;
+            }
+            if (!OVER && (y & ITEM_IMPORTS)) {  // some far columns lie in stripes to the right: the far row's exports
                 if (__builtin_expect(__any_sync(FULLMASK, (iv[0] | iv[1]) < 0), 0)) {
                     const int i = __shfl_sync(FULLMASK, bi, tl);
                     const int32_t *erow = E + (unsigned)(t - ((int)(y & XTED_ROW_ORL_MASK) + 1 - i)) * (unsigned)X;  // (R X < 2^32)
@@ -603,21 +637,6 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
             }
 #pragma unroll
             for (int k = 0; k < W; k++) far[k] = lds(top + fb[k]);
-        }
-        if (OVER && !trow) {  // more than have a place: straight from their words
-            const int i = __shfl_sync(FULLMASK, bi, tl);
-            const int32_t *erow = E + (unsigned)(t - ((int)(y & XTED_ROW_ORL_MASK) + 1 - i)) * (unsigned)X;  // (R X < 2^32)
-            const int32_t *map = P.smap + P.chunkx[it.chunk].map - P.krd[ch.k_lo];
-#pragma unroll 1
-            for (int k = 0; k < W; k++) {  // through the first import place, free on this path once all are stored
-                const bool over = (xover >> k) & 1u;
-                int v = 0;
-                const int f = over ? (nodes[sbase + lane * W + k].y & XTED_ROW_ORL_MASK) + 1 : 0;
-                if (!warp_wait(P, over ? erow + map[f] : erow, over, v)) return FLOW_FAILED;
-#pragma unroll
-                for (int h = 0; h < W; h++)
-                    if (over && h == k) far[h] = v;
-            }
         }
 #pragma unroll
         for (int k = 0; k < W; k++)  // a path column's far value is its segment's border
@@ -654,9 +673,11 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
 #pragma unroll
             for (int k = 0; k < W; k++) prev[k] = key[k];
             sp = lo = 0;
+            if (OVER) imported = false;
             cprev = 0;
         } else {
             cprev = c0;
+            if (OVER && (y & (XTED_ROW_ISKR | XTED_ROW_PREVLEAF))) imported = false;
             if (y & XTED_ROW_ISKR) sp--;
             if (y & XTED_ROW_PREVLEAF) {
                 if (__builtin_expect((unsigned)(sp - lo) >= (unsigned)SC, 0)) {
@@ -685,12 +706,12 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
                         if (q0 + lane < ne) st_relaxed(e + q0 + lane, lds(d + 4 * el[q0 + lane]));
                 }
             }
-            if ((y & ITEM_IMPORTS) && !(y & ROW_NEXTTREE)) {  // the next row's far values in other stripes
+            if (!OVER && (y & ITEM_IMPORTS) && !(y & ROW_NEXTTREE)) {  // the next row's far values in other stripes
                 const int r = __shfl_sync(FULLMASK, tl < 31 ? bi : ni, (tl + 1) & 31);
                 const int nro = __shfl_sync(FULLMASK, tl < 31 ? by : ny, (tl + 1) & 31) & XTED_ROW_ORL_MASK;
                 const int32_t *e = E + (unsigned)(t - nro + r) * (unsigned)X;
                 if (lane < nx) iv[0] = ld_relaxed(e + xq[0]);
-                if (lane + 32 < min(nx, FLOW_IMPORTS)) iv[1] = ld_relaxed(e + xq[1]);
+                if (lane + 32 < nx) iv[1] = ld_relaxed(e + xq[1]);
             }
         }
         c0 = c1;
