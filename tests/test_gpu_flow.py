@@ -121,3 +121,34 @@ def test_far_values_of_other_stripes(n):
         assert np.array_equal(ctx.distance_batch(pairs), want)
         assert [ctx.distance(a, b) for a, b in pairs[:3]] == want[:3].tolist()
         assert np.array_equal(ctx.distance_batch(pairs * 40), np.tile(want, 40))
+
+
+def _path(n, seed):
+    labels = np.random.default_rng(seed).integers(0, 3, n)
+    return trees.from_adjacency([int(x) for x in labels], [[v + 1] if v + 1 < n else [] for v in range(n)])
+
+
+def _star(n, seed):
+    labels = np.random.default_rng(seed).integers(0, 3, n)
+    return trees.from_adjacency([int(x) for x in labels], [list(range(1, n))] + [[] for _ in range(n - 1)])
+
+
+@pytest.mark.timeout(300)
+@pytest.mark.parametrize("m", [31, 63, 64, 65, 97, 300])
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 66, 129, 255, 257, 513])
+def test_many_path_columns(m, n):
+    """Items whose rows and columns lie on their paths, all of them (paths;
+    runs and chunks of single nodes) or most (combs, whose chunks also hold
+    longer segments), around 64 columns, 64 rows and the stripes' edges; words of
+    later items are waited for (a batch), costs other than one."""
+    rows = [_path(m, 1), _star(m, 2), _comb(m, 3, False), _comb(m, 4, True)]
+    cols = [_path(n, 5), _star(n, 6), _comb(n, 7, False), gen.tree("caterpillar", n, 8, "uniform", 3)]
+    pairs = [(a, b) for a in rows for b in cols]
+    want = oracle.distance_batch(pairs, nthreads=8)
+    for orient in (xted.ORIENT_RIGHT, xted.ORIENT_LEFT):
+        with xted.Context(orientation=orient) as ctx:
+            assert np.array_equal(ctx.distance_batch(pairs), want)
+    with xted.Context(run_rows=256) as ctx:  # (runs of many small tables)
+        assert np.array_equal(ctx.distance_batch(pairs * 3), np.tile(want, 3))
+    with xted.Context(costs=(2, 3, 4)) as ctx:
+        assert ctx.distance_batch(pairs).tolist() == [oracle.distance(a, b, costs=(2, 3, 4)) for a, b in pairs]

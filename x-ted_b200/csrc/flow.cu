@@ -64,6 +64,9 @@ __device__ __forceinline__ int ld_relaxed(const int32_t *p) {
 __device__ __forceinline__ void st_relaxed(int32_t *p, int v) {
     asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+__device__ __forceinline__ void st_relaxed4(int32_t *p, int4 v) {  // (16-byte aligned; each word a store of its own)
+    asm volatile("st.relaxed.gpu.global.v4.s32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 __device__ __forceinline__ void set_error(const XKernelParams &P, int code, int a, int b, int c) {
     if (atomicCAS(P.error, 0, code) == 0) {
         P.error_info[0] = a;
@@ -196,24 +199,38 @@ __device__ __forceinline__ bool warp_wait(const XKernelParams &P, const int32_t 
 // those on their segment's right path (on tree rows they take the diagonal
 // and their value goes out), those that stripes further left read, and those
 // whose far column lies in another stripe. What a row rarely needs (waiting,
-// the stack leaving its window) is marked unlikely. OVER: a stripe that takes
-// more far values from other stripes than have a place beside the usual four
-// stack rows: two rows are kept, with a place for all, filled when a row first
-// needs them (200 pairs of zigzags of 500 nodes, whose stripes take up to 90
-// values: 1,207 ms with the values past 48 loaded column by column on every
-// row, 822 ms so).
-// Returns 0, FLOW_FAILED once the launch has failed, or FLOW_OVER (nothing
-// done) if OVER is needed.
+// the stack leaving its window) is marked unlikely.
+//
+// RARE is a second copy of the loop, for items that the lists do not serve:
+// - A stripe that takes more far values from other stripes than have a place
+//   beside the usual four stack rows keeps two rows, with a place for all, filled
+//   when a row first needs them. 200 pairs of zigzags of 500 nodes, whose stripes
+//   take up to 90 values: 1,207 ms with those past 48 loaded column by column on
+//   every row, 822 ms so.
+// - Many path columns and many tree rows (paths, combs, runs and chunks of single
+//   nodes): path columns take the diagonal from the row above in registers, eight
+//   a lane, where the lists take two passes of up to eight steps through shared
+//   memory; where every column is on its path a tree row reads nothing at all. Two
+//   paths of 8,000 nodes: 17.3 -> 5.9 ms, 1,024 mixed pairs 13.1 -> 12.6.
+// Returns 0, FLOW_FAILED once the launch has failed, or FLOW_RARE (nothing
+// done) if RARE is needed.
 #define FLOW_FAILED 1
-#define FLOW_OVER 2
-template <bool OVER>
+#define FLOW_RARE 2
+// Path columns from which lists lose, on items of 64 rows and more of which half or more of the first 64 are tree rows.
+// At 16 / 32 / 64 / 128 columns: 4,500 pairs of 20-250 nodes 12.13 / 11.95 / 11.86 / 11.84 ms, 1,024 mixed ones 12.69 /
+// 12.60 / 12.59 / 12.63, 200 random ones of 500 2.14 / 2.10 / 2.06 / 2.05, a star of 600 0.70 / 0.71 / 0.70 / 0.72. From
+// 32 / 64 / 128 / 256 rows: 4,500 pairs 11.97 / 11.86 / 11.84 / 11.85, 300 mixed 4.98 / 4.97 / 5.07 / 5.25, a pair of
+// paths of 100 nodes 0.123 / 0.123 / 0.174 / 0.173. (The setup before the choice is made is done twice.)
+#define FLOW_DENSE_COLS 64
+#define FLOW_DENSE_ROWS 64
+template <bool RARE>
 __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it, const XPair &pr, const XRun &run,
                                          const XChunk &ch, int32_t *ring, int32_t *gstk) {
     constexpr int W = FLOW_W, PF = FLOW_PF, ZERO = FLOW_ZERO, IMP = ZERO + 4;
-    // OVER: a stack window of two rows, with a place for every column's far value, and the places' export indices
-    constexpr int SC = OVER ? 2 : FLOW_STACK_ROWS, PLACES = OVER ? XTED_SW : FLOW_IMPORTS;
+    // RARE: a stack window of two rows, with a place for every column's far value, and the places' export indices
+    constexpr int SC = RARE ? 2 : FLOW_STACK_ROWS, PLACES = RARE ? XTED_SW : FLOW_IMPORTS;
     constexpr unsigned SLOT_B = 4 * XTED_SW, RING_B = PF * SLOT_B, PITCH_B = 4 * (IMP + PLACES);
-    static_assert(SC * PITCH_B + (OVER ? 2 * PLACES : 0) <= 4 * FLOW_STACK, "the window's room");
+    static_assert(SC * PITCH_B + (RARE ? 2 * PLACES : 0) <= 4 * FLOW_STACK, "the window's room");
     const int lane = threadIdx.x & 31;
     const int2 *rows = P.rowinfo + pr.row_base, *nodes = P.rowinfo + pr.col_base;
     int32_t *dt = P.dt + pr.dt_off;
@@ -347,7 +364,11 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
 #pragma unroll
     for (int k = 0; k < W; k++) {
         const int c = lane * W + k;
-        if ((tcol >> k) & 1u) {
+        if (RARE && ((tcol >> k) & 1u)) {  // by column, each read by its own lane only
+            const int j = ring[c];
+            tlab[swz(c)] = nodes[j].x;
+            tlist[swz(c)] = j;
+        } else if ((tcol >> k) & 1u) {
             const int j = ring[c];
             tlab[tf] = nodes[j].x;
             tlist[tf++] = (int)((unsigned)c | ((unsigned)(key[k] / XTED_KEY_BIG) << 8) | ((unsigned)j << 16));
@@ -358,8 +379,8 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
     __syncwarp();
     int xq[2] = {0, 0};  // export index of the value in place q, q = lane, lane + 32
     int iv[2] = {0, 0};  // ... and the value for the next row
-    unsigned short *xs = (unsigned short *)((char *)(ring + FLOW_RING) + SC * PITCH_B);  // OVER: of all places
-    bool imported = false;  // OVER: the top row's places hold its values
+    unsigned short *xs = (unsigned short *)((char *)(ring + FLOW_RING) + SC * PITCH_B);  // RARE: of all places
+    bool imported = false;  // RARE: the top row's places hold its values
     if (nx > 0) {
         // columns with one far column follow each other (subtrees across a
         // boundary are nested): they share a place
@@ -375,14 +396,14 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
             places += __popc(m);
         }
         nx = places;
-        if (!OVER && nx > FLOW_IMPORTS) return FLOW_OVER;
+        if (!RARE && nx > FLOW_IMPORTS) return FLOW_RARE;
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < W; k++)
             if ((xfar >> k) & 1u) {
                 fb[k] = 4 * (IMP + xplace[xf++]);
             }
-        if (OVER) {
+        if (RARE) {
 #pragma unroll 1
             for (int q = lane; q < nx; q += 32) xs[q] = (unsigned short)xd[q];
         } else {
@@ -449,6 +470,11 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
         bi = ni, by = ny, bl = nl;
         load_rows(32 * h + lane);
     }
+    const bool allp = nt == (multi ? ch.width : cend - lead);  // every column is on its segment's path
+    if (!RARE && R >= FLOW_DENSE_ROWS && (allp || nt > FLOW_DENSE_COLS)) {
+        const int trees = __popc(__ballot_sync(FULLMASK, by & ROW_TREE)) + __popc(__ballot_sync(FULLMASK, ny & ROW_TREE));
+        if (trees >= 32) return FLOW_RARE;
+    }
     int ci = bi;  // the rows being copied, PF - 1 ahead
     const int32_t *src0 = multi ? dt : dt + sbase + 4 * lane;
     const unsigned dst0 = ring_a + (multi ? 4 * lane : 16 * (lane ^ ((lane >> 3) & 1)));
@@ -467,7 +493,8 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
     };
 #pragma unroll 1
     for (int q = 0; q < PF - 1; q++) {
-        copy_row(q * SLOT_B, __shfl_sync(FULLMASK, bi, q), ask);  // (past the run's end: its last row again)
+        const bool skip = RARE && allp && (__shfl_sync(FULLMASK, by, q) & ROW_TREE);
+        if (!skip) copy_row(q * SLOT_B, __shfl_sync(FULLMASK, bi, q), ask);  // (past the run's end: its last row again)
         cp_async_commit();
     }
 
@@ -490,8 +517,10 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
         __syncwarp();             // ... every lane's copies; row t - 1's readers are done
         const unsigned y = (unsigned)__shfl_sync(FULLMASK, by, tl);
         const bool trow = (y & ROW_TREE) != 0;
-        if (trow) {  // the path columns' words become what the diagonal gives
-            const int rl = __shfl_sync(FULLMASK, bl, tl);
+        int rl = 0;
+        if (RARE && trow) rl = __shfl_sync(FULLMASK, bl, tl);
+        if (!RARE && trow) {  // the path columns' words become what the diagonal gives
+            rl = __shfl_sync(FULLMASK, bl, tl);
 #pragma unroll 1
             for (int q0 = 0; q0 < nt; q0 += 32) {
                 const int q = q0 + lane;
@@ -505,16 +534,33 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
             __syncwarp();  // (and every lane has read the row above, whose slot is copied into next)
         }
         if (tl == 32 - (PF - 1)) ci = ni;
-        copy_row(above - ring_a, __shfl_sync(FULLMASK, ci, (t + PF - 1) & 31), y);
+        const bool skip = RARE && allp && (__shfl_sync(FULLMASK, tl < 32 - (PF - 1) ? by : ny, (t + PF - 1) & 31) & ROW_TREE);
+        if (!skip) copy_row(above - ring_a, __shfl_sync(FULLMASK, ci, (t + PF - 1) & 31), y);
         cp_async_commit();
         int a[W];
-        for (;;) {
+        auto path_values = [&]() {  // RARE: the path columns take what the diagonal gives, from the row above in registers
+            const int4 l0 = lds4(lab_a + coff0), l1 = lds4(lab_a + coff1);
+            const int lab[W] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+            int next = __shfl_down_sync(FULLMASK, prev[0], 1);
+            if (lane == 31) next = cprev;
+#pragma unroll
+            for (int k = 0; k < W; k++) {
+                const int x = y & ROW_FIRST ? 0 : max((k + 1 < W ? prev[k + 1] : next) - key[k], 0);
+                if ((tcol >> k) & 1u) a[k] = x + (rl == lab[k] ? bm : bn);
+            }
+        };
+        if (RARE && trow && allp) {  // nothing of the row comes from elsewhere
+#pragma unroll
+            for (int k = 0; k < W; k++) a[k] = 0;
+            path_values();
+        } else for (;;) {
             if (y & ITEM_EDGE) {
                 if (edge) sts(slot + edge_o, 0);
                 __syncwarp();
             }
             const int4 u = lds4(slot + coff0), v = lds4(slot + coff1);
             a[0] = u.x, a[1] = u.y, a[2] = u.z, a[3] = u.w, a[4] = v.x, a[5] = v.y, a[6] = v.z, a[7] = v.w;
+            if (RARE && trow) path_values();
             // a word that is still -1: another item has yet to write it
             const unsigned who = __ballot_sync(FULLMASK, (a[0] | a[1] | a[2] | a[3] | a[4] | a[5] | a[6] | a[7]) < 0);
             if (__builtin_expect(who == 0, 1)) break;
@@ -540,7 +586,7 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
             if (!warp_wait(P, dt + (int64_t)i * pitch + __shfl_sync(FULLMASK, j, __ffs(who) - 1), true, w)) return FLOW_FAILED;
             cp_async_wait<0>();
             __syncwarp();
-            if (trow) {  // its path words stay: kept where the labels are while the row is copied again
+            if (!RARE && trow) {  // its path words stay: kept where the labels are while the row is copied again
 #pragma unroll 1
                 for (int q0 = 0; q0 < nt; q0 += 32) {
                 const int q = q0 + lane;
@@ -566,7 +612,7 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
             cp_async_commit();
             cp_async_wait<0>();
             __syncwarp();
-            if (trow) {
+            if (!RARE && trow) {
 #pragma unroll 1
                 for (int q0 = 0; q0 < nt; q0 += 32) {
                 const int q = q0 + lane;
@@ -601,8 +647,8 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
                 for (int k = 0; k < W; k++) sts(top + 4 * lane + 128 * k, g[32 * k]);
                 __syncwarp();
             }
-            if (OVER && !imported) {
-                // loaded here and not a row ahead: the values would take registers that the loop below spills
+            if (RARE && (y & ITEM_IMPORTS) && !imported) {
+                // (loaded a row ahead, into registers as the usual two, they gained 1%)
                 const int i = __shfl_sync(FULLMASK, bi, tl);
                 const int32_t *erow = E + (unsigned)(t - ((int)(y & XTED_ROW_ORL_MASK) + 1 - i)) * (unsigned)X;  // (R X < 2^32)
                 int v[W];
@@ -624,7 +670,7 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
                 __syncwarp();
                 imported = true;
             }
-            if (!OVER && (y & ITEM_IMPORTS)) {  // some far columns lie in stripes to the right: the far row's exports
+            if (!RARE && (y & ITEM_IMPORTS)) {  // some far columns lie in stripes to the right: the far row's exports
                 if (__builtin_expect(__any_sync(FULLMASK, (iv[0] | iv[1]) < 0), 0)) {
                     const int i = __shfl_sync(FULLMASK, bi, tl);
                     const int32_t *erow = E + (unsigned)(t - ((int)(y & XTED_ROW_ORL_MASK) + 1 - i)) * (unsigned)X;  // (R X < 2^32)
@@ -651,7 +697,21 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
         for (int k = 0; k < W; k++) prev[k] = max(a[k], carry);
         // ---- what others read ----
         if ((y & ITEM_LEFT) && lane == 0) st_relaxed(Hout + t, prev[0]);
-        if (y & (ROW_TREE | ROW_NEXTTREE)) {
+        if (RARE && trow) {
+            int32_t *o = dt + (int64_t)__shfl_sync(FULLMASK, bi, tl) * pitch;
+            if (!(y & ITEM_MULTI) && tcol == (1u << W) - 1) {
+                o += sbase + lane * W;
+                st_relaxed4(o, make_int4(prev[0], prev[1], prev[2], prev[3]));
+                st_relaxed4(o + 4, make_int4(prev[4], prev[5], prev[6], prev[7]));
+            } else if (tcol) {
+                const int4 n0 = lds4(tl_a + coff0), n1 = lds4(tl_a + coff1);
+                const int nd[W] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
+#pragma unroll
+                for (int k = 0; k < W; k++)
+                    if ((tcol >> k) & 1u) st_relaxed(o + nd[k], prev[k] - key[k]);
+            }
+        }
+        if (!RARE && (y & (ROW_TREE | ROW_NEXTTREE))) {
             // the row goes into its own ring slot (free until the next row's
             // copies): the next row's diagonal, and this row's path columns
             sts4(slot + coff0, make_int4(prev[0], prev[1], prev[2], prev[3]));
@@ -673,11 +733,11 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
 #pragma unroll
             for (int k = 0; k < W; k++) prev[k] = key[k];
             sp = lo = 0;
-            if (OVER) imported = false;
+            if (RARE) imported = false;
             cprev = 0;
         } else {
             cprev = c0;
-            if (OVER && (y & (XTED_ROW_ISKR | XTED_ROW_PREVLEAF))) imported = false;
+            if (RARE && (y & (XTED_ROW_ISKR | XTED_ROW_PREVLEAF))) imported = false;
             if (y & XTED_ROW_ISKR) sp--;
             if (y & XTED_ROW_PREVLEAF) {
                 if (__builtin_expect((unsigned)(sp - lo) >= (unsigned)SC, 0)) {
@@ -706,7 +766,7 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
                         if (q0 + lane < ne) st_relaxed(e + q0 + lane, lds(d + 4 * el[q0 + lane]));
                 }
             }
-            if (!OVER && (y & ITEM_IMPORTS) && !(y & ROW_NEXTTREE)) {  // the next row's far values in other stripes
+            if (!RARE && (y & ITEM_IMPORTS) && !(y & ROW_NEXTTREE)) {  // the next row's far values in other stripes
                 const int r = __shfl_sync(FULLMASK, tl < 31 ? bi : ni, (tl + 1) & 31);
                 const int nro = __shfl_sync(FULLMASK, tl < 31 ? by : ny, (tl + 1) & 31) & XTED_ROW_ORL_MASK;
                 const int32_t *e = E + (unsigned)(t - nro + r) * (unsigned)X;
@@ -724,13 +784,6 @@ __device__ __forceinline__ int run_item(const XKernelParams &P, const XItem &it,
     cp_async_wait<0>();
     __syncwarp();
     return 0;
-}
-
-// (Inline: a call anywhere in the kernel makes every shuffle of the loop check for divergence, 29.1 against 25.1 ms on
-// 1,500 pairs of 200-500 nodes.)
-__device__ __forceinline__ int run_item_over(const XKernelParams &P, const XItem &it, const XPair &pr, const XRun &run,
-                                          const XChunk &ch, int32_t *ring, int32_t *gstk) {
-    return run_item<true>(P, it, pr, run, ch, ring, gstk);
 }
 
 // Trace record of an item (XTED_TRACE): claim, start and end time, and
@@ -914,8 +967,11 @@ __global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, BLOCKS) xted_flow_kernel
         // (test hook: of a held pair, nothing that reads its level 0 becomes ready)
         const bool held = it.pair == P.hold_pair && run.depth + ch.depth == 0;
         if (!held) {
-            int rc = run_item<false>(P, it, pr, run, ch, ring, gstk);
-            if (rc == FLOW_OVER) rc = run_item_over(P, it, pr, run, ch, ring, gstk);
+            // (tables of single nodes against segments of single nodes: every row and column is on its path)
+            int rc = FLOW_RARE;
+            if (run.kr_hi - run.kr_lo < run.rows || ch.nseg < ch.width || ch.width <= FLOW_DENSE_COLS)
+                rc = run_item<false>(P, it, pr, run, ch, ring, gstk);
+            if (rc == FLOW_RARE) rc = run_item<true>(P, it, pr, run, ch, ring, gstk);
             if (rc) break;
         }
         if (lane == 0) {
