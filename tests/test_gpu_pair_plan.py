@@ -89,3 +89,19 @@ def test_a_pair_runs_again(m, n):
             out.value = -1
             assert _lib.lib().xted_run_prepared(ctx.handle, ctypes.byref(out)) == 0
             assert out.value == want
+
+
+@pytest.mark.timeout(300)
+@pytest.mark.parametrize("n", [1, 2, 13, 14, 15, 16, 63, 64, 65, 66])
+def test_arena_smallest_pairs(n):
+    """Around the sizes up to which the arena's own kernel runs a pair (14 nodes
+    a side, paths of 64), valid and malformed."""
+    path = trees.from_adjacency([v % 3 for v in range(n)], [[v + 1] if v + 1 < n else [] for v in range(n)])
+    for other in (gen.tree("random", n, 3, "uniform", 3), gen.tree("wide", max(n - 1, 1), 4, "uniform", 3), path,
+                  trees.from_adjacency([v % 2 for v in range(64)], [[v + 1] if v < 63 else [] for v in range(64)])):
+        for a, b in ((path, other), (other, path), (other, other)):
+            assert _noalloc(a, b) == (0, oracle.distance(a, b))
+    if n > 2:
+        bad = trees.Tree(np.array(path.labels, np.int32), np.array(path.off, np.int32), np.array(path.idx, np.int32))
+        bad.idx[n // 2] += 1
+        assert _noalloc(bad, path)[0] == _noalloc(path, bad)[0] == xted.XTED_EINVAL

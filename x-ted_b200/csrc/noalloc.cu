@@ -28,8 +28,9 @@
 // in what the plan leaves of the arena; warps that find none leave. A pair of
 // 300 and 251 nodes took 37.4 ms in the kernel below and takes 0.62 ms so.
 //
-// The kernel below needs less memory and remains for pairs whose plan does not
-// fit (a tree of 60,000 nodes against one of a few, or very many tables): the
+// The kernel below needs less memory and one launch. It remains for pairs whose
+// plan does not fit (a tree of 60,000 nodes against one of a few, or very many
+// tables) and for the smallest pairs (smallest_pair): the
 // same right-path keyroot decomposition as the batched path (orl(v) = v + size(v) - 1 in preorder; keyroots = root and every child that
 // is not a last child), tables processed by keyroot level
 // kd(i0) + kd(j0) so that every tree-distance entry a table reads was written
@@ -329,6 +330,19 @@ int run_planned(int32_t *A, int grid, const xted_tree &a, const xted_tree &b, in
     return XTED_OK;
 }
 
+// Pairs that one block finishes sooner than three launches: trees of a few nodes, and paths of up to 64, which are one
+// table. A call in this kernel / planned, us: random trees of 5 nodes 64 / 95, of 12 90 / 103, of 16 102 / 107, of 20
+// 135 / 118; combs of 12 101 / 104, of 16 148 / 104; paths of 20 62 / 103, of 60 111 / 142, of 300 982 / 629.
+bool smallest_pair(const xted_tree &a, const xted_tree &b) {
+    const int32_t most = std::max(a.n, b.n);
+    auto path = [](const xted_tree &t) {  // (every node but the last has a child; a malformed tree fails in either kernel)
+        for (int32_t v = 0; v + 1 < t.n; v++)
+            if (t.child_off[v + 1] == t.child_off[v]) return false;
+        return true;
+    };
+    return most <= 14 || (most <= 64 && path(a) && path(b));
+}
+
 // Restores the calling thread's current device on scope exit (the entry
 // point makes `device` current for its work, and must not leave it so).
 struct DeviceRestore {
@@ -385,7 +399,7 @@ extern "C" int xted_distance_noalloc(const xted_tree *a, const xted_tree *b, int
     if (cudaSetDevice(device) != cudaSuccess) return XTED_ECUDA;
     cudaGetLastError();  // drop a non-sticky error left by an earlier, unrelated runtime call on this thread
     cudaStream_t s = cudaStreamPerThread;
-    rc = run_planned(A, grid, *a, *b, out, s);
+    rc = smallest_pair(*a, *b) ? PLAN_OVERFLOW : run_planned(A, grid, *a, *b, out, s);
     if (rc != PLAN_OVERFLOW) return rc;
     if (cudaMemsetAsync(A, 0, 4 * kHeaderInts, s) != cudaSuccess) return XTED_ECUDA;
     for (int k = 0; k < 2; k++) {
