@@ -105,3 +105,31 @@ def test_arena_smallest_pairs(n):
         bad = trees.Tree(np.array(path.labels, np.int32), np.array(path.off, np.int32), np.array(path.idx, np.int32))
         bad.idx[n // 2] += 1
         assert _noalloc(bad, path)[0] == _noalloc(path, bad)[0] == xted.XTED_EINVAL
+
+
+@pytest.mark.timeout(300)
+def test_no_room_for_the_one_block_plan():
+    """With a few MB of device memory left a pair is planned by the batch's
+    kernels, whose buffers the context holds already."""
+    import torch
+    a, b = gen.tree("random", 300, 1, "uniform", 4), gen.tree("deep", 280, 2, "uniform", 4)
+    want = oracle.distance(a, b)
+    with xted.Context() as ctx:
+        ctx.prepare_batch([(a, b)])
+        assert ctx.run_prepared()[0] == want
+        torch.zeros(1, device="cuda")
+        hold = []
+        while (free := torch.cuda.mem_get_info()[0]) > 24 << 20:
+            size = max(free - (16 << 20), 1 << 20) if free < 64 << 30 else 32 << 30
+            try:
+                hold.append(torch.cuda.caching_allocator_alloc(size))
+            except torch.cuda.OutOfMemoryError:
+                break
+        try:
+            assert torch.cuda.mem_get_info()[0] < 32 << 20
+            assert ctx.distance(a, b) == want
+        finally:
+            for p in hold:
+                torch.cuda.caching_allocator_delete(p)
+            torch.cuda.empty_cache()
+        assert ctx.distance(a, b) == want

@@ -210,8 +210,10 @@ int ctx_prepare(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npa
     XKernelParams &K = c->kp;
     const char *tr = std::getenv("XTED_TRACE");
     if (one_block && npairs == 1 && a->n > 0 && b->n > 0 && (int64_t)a->n + b->n <= XTED_PAIR_NODES &&
-        c->opts.mem_limit == 0 && !(tr && *tr))
-        return pair_prepare(c, *a, *b);
+        c->opts.mem_limit == 0 && !(tr && *tr)) {
+        const int rc = pair_prepare(c, *a, *b);
+        if (rc != XTED_ENOMEM) return rc;  // (the batch's kernels size their lists and need less room)
+    }
     int rc = dev_plan(c, a, b, npairs, K);
     if (rc) return rc;
     K.c_del = c->opts.cost_del;
