@@ -65,3 +65,11 @@ def test_under_a_limit(limit_mb):
     with xted.Context(mem_limit=limit_mb << 20) as ctx:
         for pairs in (wide, many, wide):
             assert np.array_equal(ctx.distance_batch(pairs), oracle.distance_batch(pairs, nthreads=8))
+
+
+@pytest.mark.timeout(300)
+def test_room_of_many_trees():
+    """Planning 4,000 trees of 800,000 nodes together: 238 MB suffice."""
+    pairs = [(gen.tree("random", 400, k, "uniform", 4), gen.tree("random", 1, k, "uniform", 4)) for k in range(2000)]
+    with xted.Context(mem_limit=238 << 20) as ctx:
+        assert np.array_equal(ctx.distance_batch(pairs), oracle.distance_batch(pairs, nthreads=8))

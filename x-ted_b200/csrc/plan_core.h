@@ -39,11 +39,13 @@ struct DDepth {
     int32_t krd_lo, krd_hi;       // keyroots of this depth (pool indices, preorder)
     int32_t run_lo, run_hi;       // row runs
     int32_t chunk_lo, nnarrow, nwide;  // chunks: narrow, then half-block, then whole-block ones
-    int32_t maxrows, maxw_n, maxw_w;   // largest run and chunk widths (cost estimates)
-    int32_t nhalf, maxw_h;
-    int32_t nitems, wsum;  // as columns: items per row run, hand-off words per row (flow_plan.h)
-    int32_t rows;          // as rows: all rows of the depth's tables
-    int32_t pad;
+    int32_t maxrows, nhalf;            // largest run
+    // Largest chunk widths (for the level schedule's estimates), or the totals of the launch's list (flow_plan.h):
+    // as columns items per row run and hand-off words per row, as rows all rows of the depth's tables. No plan
+    // needs both, and a batch has two of these records for every node.
+    union { int32_t maxw_n, nitems; };
+    union { int32_t maxw_w, wsum; };
+    union { int32_t maxw_h, rows; };
 };
 
 // One tree in one orientation (index 2 * tree + o; o = 1 mirrored).

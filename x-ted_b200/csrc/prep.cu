@@ -363,7 +363,7 @@ __device__ void orient_team(const Team<NT> &team, const PlanPools &P, int ot, bo
         const int klo = dd.krd_lo, khi = dd.krd_hi;
         int run_cur = klo, chunk_cur = klo;
         dd.run_lo = dd.chunk_lo = klo;
-        dd.maxrows = dd.maxw_n = 0;
+        dd.maxrows = 0;
         int pos = 0, r_lo = klo, r_rows = 0, c_lo = klo, c_w = 0;
         for (int kb = klo; kb < khi; kb += 32) {
             const int k = kb + lane;
@@ -387,7 +387,6 @@ __device__ void orient_team(const Team<NT> &team, const PlanPools &P, int ot, bo
                 }
                 r_rows += szj;
                 if (c_w > 0 && c_w + szj > group_w) {
-                    dd.maxw_n = max(dd.maxw_n, c_w);
                     if (lane == 0) P.chunks[chunk_cur] = XChunk{c_lo, c_w, d, kk - c_lo};
                     chunk_cur++;
                     c_lo = kk;
@@ -397,7 +396,6 @@ __device__ void orient_team(const Team<NT> &team, const PlanPools &P, int ot, bo
             }
         }
         dd.maxrows = max(dd.maxrows, r_rows);
-        dd.maxw_n = max(dd.maxw_n, c_w);
         if (lane == 0) {
             P.runs[run_cur] = XRun{r_lo, khi, r_rows, d};
             P.chunks[chunk_cur] = XChunk{c_lo, c_w, d, khi - c_lo};
@@ -405,7 +403,6 @@ __device__ void orient_team(const Team<NT> &team, const PlanPools &P, int ot, bo
         dd.run_hi = run_cur + 1;
         dd.nnarrow = chunk_cur + 1 - klo;
         dd.nhalf = dd.nwide = 0;
-        dd.maxw_h = dd.maxw_w = 0;
         if (lane == 0) dep[d] = dd;
         __syncwarp();
     }
@@ -1195,7 +1192,7 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     const size_t N2 = 2 * (size_t)std::max<int64_t>(N, 1);
     size_t need = upload + 4096;
     need += 3 * sizeof(int32_t) * (size_t)std::max<int64_t>(N, 1);  // size, depth, parent
-    need += N2 * (sizeof(int2) + 2 * sizeof(int32_t) + sizeof(XRun) + sizeof(XChunk) + sizeof(XChunkX) + 4 * sizeof(int32_t));
+    need += N2 * (sizeof(int2) + 2 * sizeof(int32_t) + sizeof(XRun) + sizeof(XChunk) + sizeof(XChunkX) + sizeof(int32_t));
     need += sizeof(DDepth) * (N2 + 2 * (size_t)T) + sizeof(DOTree) * 2 * (size_t)T + sizeof(DTree) * (size_t)T +
             4 * sizeof(int32_t) * (size_t)T;
     need += (size_t)npairs * (sizeof(DPair) + sizeof(XPair) + 4 + 4 * 8) + 24 * 256 + sizeof(Summary);
@@ -1219,9 +1216,14 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     P.cumw = cv.take<int32_t>(N2);
     P.runs = cv.take<XRun>(N2);
     P.chunks = cv.take<XChunk>(N2);
-    P.opar = cv.take<int32_t>(N2);
-    P.okd = cv.take<int32_t>(N2);
-    P.oka = cv.take<int32_t>(N2);
+    // k_orient's scratch, and where it was, from k_map_reserve on, what the chunks add to the plan
+    char *chunk_room = cv.take<char>(N2 * (sizeof(XChunkX) + sizeof(int32_t)));
+    P.opar = (int32_t *)chunk_room;
+    P.okd = P.opar + N2;
+    P.oka = P.okd + N2;
+    static_assert(sizeof(XChunkX) + sizeof(int32_t) >= 3 * sizeof(int32_t), "room for both");
+    XChunkX *d_chunkx = (XChunkX *)chunk_room;
+    int32_t *d_list = (int32_t *)(d_chunkx + N2);
     P.depths = cv.take<DDepth>(N2 + 2 * (size_t)T);
     P.otrees = cv.take<DOTree>(2 * (size_t)T);
     ctx_granularity(c, products, P);
@@ -1232,8 +1234,6 @@ int dev_plan(xted_ctx *c, const xted_tree *a, const xted_tree *b, int32_t npairs
     int64_t *d_cells = cv.take<int64_t>((size_t)npairs + 1);
     int64_t *d_Ls = cv.take<int64_t>((size_t)npairs + 1);
     int64_t *d_dts = cv.take<int64_t>((size_t)npairs + 1);
-    XChunkX *d_chunkx = cv.take<XChunkX>(N2);
-    int32_t *d_list = cv.take<int32_t>(N2);
     int32_t *d_used = cv.take<int32_t>(2 * (size_t)T), *d_need = cv.take<int32_t>(2 * (size_t)T);
     Summary *d_sum = cv.take<Summary>(1);
     if (cv.off > c->meta.cap) return XTED_ENOMEM;
