@@ -636,7 +636,8 @@ def main():
         # the reference's distances of the sampled pairs against this run's
         dd = info["distances"]
         live = {"checked": len(dd), "mismatches": sum(int(ref_out[p]) != d for p, d in dd.items()),
-                "against": f"reference X-TED_CPU computed in this run ({info['kind']})"}
+                "against": ("reference X-TED_CPU" if info["kind"] == "reference" else "the oracle's restatement of X-TED_CPU")
+                + " computed in this run"}
         parity = dict(parity or {}, live_reference=live)
 
     # ---- single pairs (configs 1-3), 1 GPU ----

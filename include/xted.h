@@ -103,12 +103,12 @@ typedef struct xted_stats {
     int64_t pairs;
     int64_t cells;          /* interior forest-table cells executed          */
     int64_t cells_right;    /* cells X-TED's right-path decomposition needs  */
-    int64_t tasks;          /* block-level tasks in the device queue         */
-    int64_t units;          /* warp/block work units                         */
+    int64_t tasks;          /* items of the launch, each run by one warp     */
+    int64_t units;          /* the same                                      */
     int64_t h2d_bytes, d2h_bytes;
     double host_plan_ms;    /* host planning time                            */
     double device_ms;       /* device time of one run: counter reset, DP launch
-                               and gather (CUDA events on the launch stream) */
+                               (in parts: launches) and gather (CUDA events) */
     double total_ms;        /* wall time of the call                         */
     int32_t levels_max;     /* deepest keyroot-level count of any pair        */
     int32_t grid;           /* persistent blocks launched                    */

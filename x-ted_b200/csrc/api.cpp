@@ -95,8 +95,12 @@ int ctx_host_reserve(HostBuf &b, size_t bytes) {
     return XTED_OK;
 }
 
-// From this many pairs on a launch takes five blocks an SM (flow.cu has the
-// times of both): the work then outlasts the longest pair's chain.
+// From this many pairs on a launch takes five blocks an SM. It is a line on
+// mixed pairs of 50-2,000 nodes (ms with four / five): 128 pairs 5.35 / 5.50, 512
+// 20.5 / 20.2, 768 26.4 / 26.1, 1,023 36.7 / 35.5, 1,500 57.1 / 54.8. A count does
+// not see the shapes: pairs of deep trees gain from 20 pairs on (20 of 2,000 nodes
+// 59.4 / 56.5), random trees lose at any number (1,600 of 300 5.18 / 5.47, 16,000
+// of 100 8.84 / 9.23), and so do many small pairs beside a large one.
 #define XTED_FULL_PAIRS 1024
 
 // One pair is planned by one block up to this many nodes together, by the

@@ -924,12 +924,13 @@ __device__ void finish_served(const XKernelParams &P, const XPair &pr, const XIt
 }
 
 // Blocks of four warps, 45 KB of shared memory each: four per SM with 128
-// registers a thread, or five with 96 (25 of them spilled). A row waits on
-// fixed latencies for three of four cycles, so a launch that always has items
-// to claim runs faster with the fifth block: 4,096 pairs 142.1 -> 135.7 ms, 1,024
-// pairs 38.2 -> 37.2, 4,560 small ones 13.03 -> 12.72. A launch bound by its
-// pairs' longest chains runs slower, row by row: 20,000 random 47.6 -> 48.9 ms,
-// 1,000 wide x deep 1.25 -> 1.40, a pair of 100 0.10 -> 0.115. 500 pairs: 7.83 -> 7.96.
+// registers a thread, or five with 96 (seven of them spilled). A row waits on
+// fixed latencies for three of four cycles, so a launch of long rows that always
+// has items to claim runs faster with the fifth block, one bound by its pairs'
+// longest chains, or by the items' setup, runs slower: 1,023 mixed pairs 36.7 /
+// 35.5 ms with four / five, 1,000 of 50-300 nodes 3.17 / 3.24, 20,000 random 46.5 /
+// 49.0. The rule and more of its two sides are at XTED_FULL_PAIRS.
+//
 // SERVE: a serving session's launch, which claims from the lists of its queries.
 template <int BLOCKS, bool SERVE>
 __global__ void __launch_bounds__(32 * XTED_FLOW_WARPS, BLOCKS) xted_flow_kernel(const __grid_constant__ XKernelParams P) {

@@ -1011,7 +1011,9 @@ size_t pair_layout(void *base, size_t bytes, int32_t m, int32_t n, PairLayout *L
     L->cap_list = n;
     L->cap_map = 32 * n;  // (each column of 32 tables wider than a warp holds)
     L->smap = cv.take<int32_t>((size_t)L->cap_map);
-    L->cap_levels = 64;  // keyroot depths grow with the logarithm of the nodes
+    // keyroot depths of most trees grow with the logarithm of their nodes (a spine with a leg per node on the wrong side
+    // has half of them: its plan overflows and goes to the batch's kernels)
+    L->cap_levels = 64;
     L->levels = cv.take<Level>((size_t)L->cap_levels);
     L->room = cv.take<int32_t>(0);
     const size_t used = (size_t)((char *)L->room - (char *)base);

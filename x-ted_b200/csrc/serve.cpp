@@ -828,7 +828,6 @@ int load(xted_ctx *c, ServeState *s, const xted_tree *tr, int32_t ntrees) {
     K.timeout_ns = (uint64_t)(c->opts.wait_timeout_s * 1e9);
     K.trace = nullptr;
     K.serve = 1;
-    K.serve_pairs = T;
     K.idle_exit_ns = 2000000;  // 2 ms
     K.lists = s->d_lists;
     K.clears = s->d_clears;

@@ -16,11 +16,9 @@
 // column list. A *chunk* is a run of whole segments of one depth. A *row run*
 // is a run of whole keyroots of A of one depth. A *unit* = (row run, chunk):
 // every table (i0, j0) with i0 in the run and j0 in the chunk, computed row by
-// row (rows descending, a min-plus suffix scan across the chunk's columns).
-// A *task* is what one thread block claims from the device queue: one wide
-// unit (chunk wider than a warp can hold) or up to XTED_TASK_UNITS narrow
-// units that the block's warps claim one at a time, all of one pair and one
-// level.
+// row (rows descending, a suffix maximum across the chunk's columns). An *item*
+// is what one warp claims: a unit, or one column stripe of a unit whose chunk
+// is a segment wider than a warp holds.
 #pragma once
 
 #include <stdint.h>
@@ -28,8 +26,7 @@
 
 #define XTED_CTA_THREADS 256
 #define XTED_WARPS (XTED_CTA_THREADS / 32)
-#define XTED_NARROW_MAX 256       // widest chunk one warp holds in registers (8 per lane)
-#define XTED_WIDE_REG_MAX 2048    // widest chunk one block holds in registers (8 per thread)
+#define XTED_NARROW_MAX 256       // widest chunk of several segments (8 columns per lane)
 #define XTED_KEY_BIG (1 << 17)    // key step between segments of one chunk
 #define XTED_INF 0x3fffffff
 
@@ -38,17 +35,10 @@
 #define XTED_ROW_ISKR (1u << 29)     // node is a keyroot
 #define XTED_ROW_PREVLEAF (1u << 30) // node i-1 is a leaf
 
-// Per-column state derived in the kernels (the wide generic path keeps it in
-// scratch as int4: x = node j, y = label(j), z = foff | flags, w = dend):
-// foff = orl(j) + 1 - j (low 20 bits), dend = je - j with je = orl(j0) + 1 for
-// the segment's keyroot j0.
-#define XTED_COL_FOFF_MASK 0x000fffff
-#define XTED_COL_FARCOL (1u << 30)   // column j-1 is a leaf inside the segment: a far column
-
 // Node record (both trees use the same pool): x = label, y = orl | flags.
 
 // Granularity of one tree-size bucket: trees with fewer than max_n nodes use
-// this row-run length and these narrow / half-block chunk limits.
+// this row-run length and this widest chunk of several segments (half_width: no effect on the launch).
 #define XTED_TUNE_ROWS 8
 struct XTuneRow {
     int32_t max_n, run_rows, narrow_width, half_width;
@@ -77,75 +67,50 @@ struct XPair {
     int32_t pad;
 };
 
+// From here to XEntry: the level schedule of plan_core.h, blocks that run units
+// level by level. The launch has only items; the schedule is what
+// tests/cpp/plan_emu.cpp and serve_emu.cpp run over the same trees, runs and chunks.
 struct XUnit {
     int32_t run;   // global run index (row tree)
     int32_t chunk; // global chunk index (column tree)
 };
 
-// (From here to XEntry: the block-by-block tasks of plan_core.h's level
-// schedule, which the host emulation of the planner's records runs. The DP launch has only items.)
-#define XTED_TASK_WIDE 0x80000000u  // one unit run by the whole block
-#define XTED_TASK_STRIPED 0x20000000u  // (with WIDE) one column stripe of a striped unit
-// Striped units: a single column segment wider than the register paths
-// (XTED_WIDE_REG_MAX columns) is split into column stripes of 256 * sww
-// columns, and every stripe is a task of its own: kind_n = WIDE | STRIPED |
-// (stripe << XTED_STRIPE_SHIFT) | 1, unit_lo = the striped unit's index in
-// XKernelParams::stripes. The K stripes of a unit are consecutive tasks of
-// its level, rightmost first, and blocks claim a level's tasks in index order:
-// the stripe a block waits for (its right neighbour, which passes it the row
-// carries) has always been claimed before, by a block that is running it or
-// has finished it. Any block runs any stripe, one block runs them all in turn.
+#define XTED_WIDE_REG_MAX 2048      // widest chunk of a whole-block unit, wider ones in column stripes
+#define XTED_HALF_MAX 1024          // ... of a half-block unit
+#define XTED_HALF_DEFAULT 512
+#define XTED_TASK_WIDE 0x80000000u  // one unit run by a whole block
+#define XTED_TASK_HALF 0x40000000u  // units run by a block's two halves
+#define XTED_TASK_STRIPED 0x20000000u  // (with WIDE) one column stripe of a striped unit, rightmost first:
+                                    // kind_n = WIDE | STRIPED | (stripe << XTED_STRIPE_SHIFT) | 1
 #define XTED_STRIPE_SHIFT 16
 #define XTED_STRIPE_MASK 0xfffu
 #define XTED_STRIPE 2048        // widest stripe (8 columns per thread)
 #define XTED_STRIPE_MIN_W 2     // narrowest stripe: 2 columns per thread (512 columns)
 #define XTED_STRIPES_MAX 128    // stripes of one unit: a wider segment takes wider stripes
-#define XTED_STRIPE_PIPE_ROWS 32  // 512-column stripes of a unit with R >= this * K rows pipeline the hand-off
-#define XTED_STRIPE_MIN_CELLS_DEFAULT ((int64_t)1 << 20)
 
 struct XStripe {       // a striped unit
     int32_t unit;      // its unit
     int32_t K;         // stripes
     int32_t sww;       // columns per thread: a stripe is 256 * sww columns
-    int32_t X;         // far columns read across a stripe boundary (exported on every pushed row)
+    int32_t X;         // far columns read across a stripe boundary
     int32_t w, R;      // width (one segment) and rows
     int32_t pair, pad;
     int64_t map_off;   // its export map (w ints): column -> export index, or -1
-    int64_t buf_off;   // carries [K][R], first columns [K][R], exports [R][X]: 64-bit tagged words
+    int64_t buf_off;   // its hand-off words
 };
-#define XTED_TASK_HALF 0x40000000u  // units run by the block's two halves (4 warps each)
-#define XTED_HALF_MAX 1024          // widest chunk one half block holds in registers (8 per thread)
-#define XTED_HALF_DEFAULT 512       // default limit: wider chunks run faster on the whole block
-// Per-block scratch ints of a wide unit on the generic path (one segment of
-// w > XTED_WIDE_REG_MAX columns, far-row stack of sr rows): rows padded to
-// whole columns per thread, prev | loc | column records (int4) | stack.
-static inline int64_t xted_wide_big_scratch(int64_t w, int64_t sr) {
-    const int64_t wp = (w + XTED_CTA_THREADS - 1) / XTED_CTA_THREADS * XTED_CTA_THREADS;
-    return ((2 * wp + 4) & ~(int64_t)3) + 4 * wp + sr * wp;
-}
 
 #ifndef XTED_TASK_UNITS
-#define XTED_TASK_UNITS 32   // narrow units per task (claimed by the block's warps dynamically)
+#define XTED_TASK_UNITS 32   // narrow units per task
 #endif
-#define XTED_PREFETCH 2      // rows of tree distances in flight per unit (cp.async ring depth; 2 measured
-                             // faster than 4 or 8 on the mixed batch: the smaller ring leaves more L1)
 
 struct XTask {
     int32_t pair;
     int32_t entry;    // its (pair, level) entry
-    uint32_t kind_n;  // XTED_TASK_WIDE | number of units
+    uint32_t kind_n;  // XTED_TASK_* | number of units
     int32_t unit_lo;  // first unit
 };
 
-// Entries and buckets: the level-by-level schedule that the host emulation of
-// the planner's records runs (plan_core.h); the DP launch uses the items below.
 #define XTED_BUCKETS 16
-#define XTED_KIND_NARROW 0
-#define XTED_KIND_GROUP 1
-#define XTED_RINGS (2 * XTED_BUCKETS)
-// entry_state words per entry: narrow tasks claimed, group tasks claimed, tasks done
-#define XTED_ESTATE 3
-
 struct XEntry {
     int32_t task_off;  // first task
     int32_t ntasks;
@@ -229,7 +194,6 @@ struct XKernelParams {
     unsigned long long *trace; // optional, 4 words per item: claim ns, start ns, end ns, info
     // ---- serving session (serve = 1); a batch launch leaves these zero ----
     int32_t serve;
-    int32_t serve_pairs;    // pairs per query slot (the corpus size)
     uint64_t idle_exit_ns;  // the launch ends once every warp has had no work for this long
     unsigned long long *lists;  // [XTED_SERVE_SLOTS] (end << 32) | next item of the slot's list
     XServeClear *clears;    // [XTED_SERVE_SLOTS]
