@@ -2,8 +2,8 @@
 
 For each size bucket it builds a seeded batch of pairs whose trees all fall in
 the bucket (the four shapes of the mixed workload, Zipf(1.1) labels), runs the
-persistent DP with every candidate granularity (row-run length, widest narrow
-chunk, widest half-block chunk) and keeps the fastest. The result is written as
+persistent DP with every candidate granularity (row-run length, widest chunk of
+several segments) and keeps the fastest. The result is written as
 ``x-ted_b200/csrc/tune_table.h``, which the library compiles in: a context plans
 each tree with the row of its size bucket unless the caller sets the
 granularity explicitly.
@@ -43,9 +43,9 @@ BUCKETS = [  # (max_n, tree sizes drawn log-uniformly from [lo, hi), pairs in th
     (1 << 30, 2048, 4096, 96),
 ]
 MIXED_SIZES = (1024, 2048, 4096)  # pairs of gen.mixed_batch(n, seed=4) the guard times
-RUN_ROWS = [16, 32, 64, 128]
+RUN_ROWS = [16, 32, 64, 128, 256, 512]
 NARROW = [128, 256]
-HALF = [-1, 384, 512, 768, 1024]
+HALF = [-1]  # (the table's half-block column has no effect on the launch)
 
 HEADER = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc", "tune_table.h")
 
@@ -137,7 +137,7 @@ def write_header(rows, notes, path=HEADER):
         "//",
         "// Row k applies to trees with fewer than max_n nodes (the last row to all",
         "// larger ones): the row-run length of the tree as a row tree, and the widest",
-        "// narrow (one warp) and half-block chunks of the tree as a column tree.",
+        "// chunks of several segments of the tree as a column tree (the last column has no effect).",
     ]
     lines += ["// " + n for n in notes]
     lines += ["#pragma once", "", '#include "xted_internal.h"', "", "static const XTuneRow kTuneTable[] = {"]
@@ -159,7 +159,7 @@ def main(argv=None):
     args = ap.parse_args(argv)
     cands = list(itertools.product(RUN_ROWS, NARROW, HALF))
     if args.quick:
-        cands = [(32, 256, 512), (64, 256, 512), (64, 256, -1), (128, 256, 512)]
+        cands = [(64, 256, -1), (128, 256, -1), (256, 256, -1)]
     rows, notes = [], []
     t_all = time.time()
     for k, (max_n, lo, hi, npairs) in enumerate(BUCKETS):
@@ -172,10 +172,10 @@ def main(argv=None):
                               "dp_ms": round(ms, 3)}), flush=True)
         res.sort()
         best = res[0]
-        default = next((r for r in res if r[1:] == (64, 256, 512)), None)
+        default = next((r for r in res if r[1:] == (64, 256, -1)), None)
         rows.append((max_n, best[1], best[2], best[3]))
         notes.append(f"sizes [{lo}, {hi}), {npairs} pairs: best {best[0]:.2f} ms (run_rows {best[1]}, narrow "
-                     f"{best[2]}, half {best[3]})" + (f", untuned default {default[0]:.2f} ms" if default else ""))
+                     f"{best[2]})" + (f", untuned default {default[0]:.2f} ms" if default else ""))
     if not args.no_guard:
         current = read_header(args.out if os.path.exists(args.out) else HEADER)
         timer, seen = mixed_timer(device=args.device), []
